@@ -1,0 +1,609 @@
+"""What is timed when a change is meant to make the engine faster: requests through the step function.
+
+One pass serves a group of requests from their first token to their last: it opens them, feeds their prompts in
+portions under a token budget (decoding requests go first, as the scheduler does it), decodes the given number of
+tokens for each, and closes them.  The tokens fed are given by the case's seed, not drawn from the logits, so that a
+rounding does not change the work of the steps after it.  A pass returns the logits of every step, one row below the
+other: those of a prompt's last token and those of every decoded one.
+
+The engine (weights, cache, captured graphs) is what a serving program keeps; it is loaded once for a model and
+options, with the engine's own random weights.  Each state holds new prompts.
+
+Designs: Qwen2-MoE, the engine's main one, at the layer sizes that the benchmark names, and the three others that
+between them hold the further kinds of mixer: latent attention and a state-space recurrence (Vekasun), windowed
+attention whose values are its keys and linear attention with fixed decays (Difavik), softmax attention beside a
+state-space recurrence and capped attention beside a gated delta rule (Nolesun), at the layer sizes at which the
+benchmark compares them with Qwen2-MoE.
+
+Two choices keep the outputs comparable in bfloat16, where random weights make a model touchy: only some of the layers
+are run, 12 of the 24 of Qwen1.5-MoE-A2.7B, 6 over long prompts (over all of them roundings alone, and the close choices
+of experts that they decide, move a long context's logits by 3 to 4 %), and the other designs have their dense
+feed-forwards, or none (their norms and weights give a single routed expert so much of a layer that a close choice
+decided the other way moves the logits by 20 %).
+"""
+
+from __future__ import annotations
+
+import hashlib
+import math
+import random
+
+import torch
+
+from ninfer_amd_mi50_b200.config import EngineOptions
+from ninfer_amd_mi50_b200.engine import StepEntry, load_runner
+
+WEIGHT_SEED = 2
+MAX_REQUESTS, MAX_CONTEXT, CACHE_TOKENS = 64, 8448, 65536
+
+# width, heads, key heads, experts, experts a token, expert width, shared expert's width, vocabulary
+SIZES = {
+    "a2.7b": dict(width=2048, heads=16, kv_heads=16, experts=60, top=4, ff=1408, shared=5632, vocab=151936),
+    "57b": dict(width=3584, heads=28, kv_heads=4, experts=64, top=8, ff=2560, shared=20480, vocab=151936),
+    "tiny": dict(width=256, heads=4, kv_heads=2, experts=8, top=2, ff=128, shared=256, vocab=1024),
+    "w1024": dict(width=1024, heads=8, kv_heads=8, experts=32, top=4, ff=704, vocab=32000, q_rank=768, kv_rank=256,
+                  ssm_heads=32, state=64),
+    "w2048": dict(width=2048, heads=16, kv_heads=16, experts=60, top=4, ff=1408, vocab=32000, q_rank=1536, kv_rank=512,
+                  ssm_heads=64, state=128),
+}
+HEAD_DIM, ROT_DIM, SSM_HEAD_DIM, RET_DIM, GROUPS, TAPS = 128, 64, 64, 64, 8, 4
+WINDOW, KEEP_FIRST = 1024, 4
+EPS = 1e-6
+
+
+# ---- the cases ------------------------------------------------------------------------------------------------
+
+def _case(name, design, size, layers, requests, prompt, ragged, new, budget, dtype="bfloat16"):
+    """`requests` prompts of `prompt` tokens (with `ragged`: of 1/8 of that up to that), `new` decoded tokens for each,
+    at most `budget` tokens a step."""
+    return {"name": name, "design": design, "size": size, "layers": layers, "requests": requests, "prompt": prompt,
+            "ragged": ragged, "new": new, "budget": budget, "dtype": dtype}
+
+
+def listed():
+    return [
+        # the smallest model and calls, in 32-bit: three short prompts and eight decode steps, bound by launches
+        _case("tiny_fp32", "qwen2_moe", "tiny", 2, 3, 33, True, 8, 2048, "float32"),
+        # a chat turn of a single user: a short prompt, then decoding one row at a time
+        _case("chat_turn", "qwen2_moe", "a2.7b", 12, 1, 37, False, 16, 2048),
+        # a small service: eight chats of unequal prompts, decoded together
+        _case("eight_chats", "qwen2_moe", "a2.7b", 12, 8, 515, True, 32, 2048),
+        # a full batch: 64 short requests
+        _case("batch_64", "qwen2_moe", "a2.7b", 12, 64, 130, True, 12, 2048),
+        # time to the first token of a prompt of 2,048 tokens
+        _case("prompt_2048", "qwen2_moe", "a2.7b", 6, 1, 2048, False, 0, 2048),
+        # a long document read in portions, then a short answer over its long context
+        _case("document_8191", "qwen2_moe", "a2.7b", 6, 1, 8191, False, 8, 2048),
+        # steps that mix decoded tokens with portions of other requests' prompts, under a small token budget
+        _case("mixed_steps", "qwen2_moe", "a2.7b", 12, 12, 701, True, 16, 512),
+        # wide layers with few key heads (grouped queries) and wide experts
+        _case("wide_grouped", "qwen2_moe", "57b", 2, 6, 1024, True, 12, 2048),
+        # the all-32-bit path at full layer sizes
+        _case("full_fp32", "qwen2_moe", "a2.7b", 2, 2, 257, True, 4, 256, "float32"),
+        # the other designs: prompts and decoding, one long request, unequal ones, many short ones
+        _case("vekasun_prompts", "vekasun", "w2048", 4, 4, 2048, True, 12, 2048),
+        _case("difavik_prompt", "difavik", "w2048", 4, 1, 2048, False, 16, 2048),
+        _case("nolesun_chats", "nolesun", "w2048", 4, 8, 900, True, 16, 2048),
+    ]
+
+
+def _log_uniform(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def draw(rng):
+    design, size, layers = rng.choice([
+        ("qwen2_moe", "a2.7b", 12), ("qwen2_moe", "a2.7b", 12), ("qwen2_moe", "57b", 2), ("vekasun", "w2048", 4),
+        ("difavik", "w2048", 4), ("nolesun", "w2048", 4), (rng.choice(["vekasun", "difavik", "nolesun"]), "w1024", 4)])
+    dtype = "bfloat16"
+    if design == "qwen2_moe" and rng.random() < 0.15:
+        dtype, layers = "float32", 2
+    requests, budget = _log_uniform(rng, 1, 64), rng.choice([256, 511, 1024, 2048, 2048])
+    most = min(1024 if dtype == "float32" else 8192, 6 * budget) // requests     # what a whole pass costs is bounded
+    prompt = _log_uniform(rng, 2, max(2, most))
+    if layers == 12 and prompt > 600:
+        layers = 6
+    case = _case("", design, size, layers, requests, prompt, rng.random() < 0.5,
+                 rng.choice([0, 0, 4, 8, 15, 16]), budget, dtype)
+    del case["name"]
+    return case
+
+
+# ---- models ---------------------------------------------------------------------------------------------------
+
+def _decays(heads):
+    return [1.0 - 2.0 ** (-5.0 - 3.0 * h / max(1, heads - 1)) for h in range(heads)]
+
+
+def _config(case):
+    s, n = SIZES[case["size"]], case["layers"]
+    H, G = s["heads"], s["kv_heads"]
+    if case["design"] == "qwen2_moe":
+        return {"architectures": ["Qwen2MoeForCausalLM"], "model_type": "qwen2_moe", "num_hidden_layers": n,
+                "hidden_size": s["width"], "num_attention_heads": H, "num_key_value_heads": G, "head_dim": _head_dim(case),
+                "intermediate_size": 4 * s["ff"], "num_experts": s["experts"], "num_experts_per_tok": s["top"],
+                "moe_intermediate_size": s["ff"], "shared_expert_intermediate_size": s["shared"], "norm_topk_prob": False,
+                "decoder_sparse_step": 1, "mlp_only_layers": [], "vocab_size": s["vocab"], "rope_theta": 1e6,
+                "rms_norm_eps": EPS, "tie_word_embeddings": False, "use_sliding_window": False, "qkv_bias": True}
+    dense = {"kind": "dense", "ff": s["top"] * s["ff"]}          # as wide as a token's experts in the comparison
+    if case["design"] == "difavik":
+        left = {"heads": H, "kv_heads": G, "dim": HEAD_DIM, "vdim": HEAD_DIM, "scale": HEAD_DIM ** -0.5,
+                "mask": {"size": WINDOW, "keep_first": KEEP_FIRST}}
+        right = {"heads": H, "dim": RET_DIM, "vdim": HEAD_DIM, "decay": _decays(H), "rot": {"base": 10000.0, "dims": RET_DIM}}
+        light = {"heads": H, "dim": HEAD_DIM, "vdim": HEAD_DIM, "decay": _decays(H)}
+        return {"architecture": "Difavik", "vocab": s["vocab"], "width": s["width"], "norm": {"eps": EPS},
+                "embedding": {"bigram": {"buckets": 65521, "mul_prev": 1000003, "mul_cur": 31}},
+                "layers": [{"type": k, "mixer": light if k == "lightning" else {"left": left, "right": right},
+                            "mlp": dict(dense, limit=7.0)} for k in ("lightning", "parallel", "parallel", "lightning")]}
+    ssm = {"heads": s["ssm_heads"], "vdim": SSM_HEAD_DIM, "state": s["state"], "groups": GROUPS, "conv": TAPS,
+           "norm_groups": GROUPS}
+    if case["design"] == "vekasun":
+        att = {"heads": H, "dim": HEAD_DIM, "rot_dim": ROT_DIM, "vdim": HEAD_DIM, "kv_rank": s["kv_rank"],
+               "q_rank": s["q_rank"], "scale": (HEAD_DIM + ROT_DIM) ** -0.5, "rot": {"base": 10000.0, "dims": ROT_DIM}}
+        return {"architecture": "Vekasun", "vocab": s["vocab"], "width": s["width"], "norm": {"eps": EPS}, "logit_scale": 1.0,
+                "layers": [{"type": k, "mixer": att if k == "latent_attention" else ssm}
+                           for k in ("latent_attention", "mamba2", "mamba2", "latent_attention")]}
+    att = {"heads": H, "kv_heads": G, "dim": HEAD_DIM, "vdim": HEAD_DIM, "scale": HEAD_DIM ** -0.5,
+           "rot": {"base": 10000.0, "dims": ROT_DIM}}
+    rule = {"heads": H, "kv_heads": H // 2, "dim": HEAD_DIM, "vdim": HEAD_DIM, "conv": TAPS}
+    one = {"type": "parallel", "mixer": {"left": att, "right": ssm, "left_scale": 0.8, "right_scale": 1.2}}
+    two = {"type": "parallel_2", "mixer": {"left": dict(att, softcap=30.0), "right": rule, "left_scale": 0.9, "right_scale": 0.7}}
+    return {"architecture": "Nolesun", "vocab": s["vocab"], "width": s["width"], "norm": {"eps": EPS},
+            "embedding": {"scale": 8.0}, "loop": {"start": 1, "stop": 3, "times": 1},
+            "layers": [dict(m, mlp=dense) for m in (one, two, one, two)]}
+
+
+def _head_dim(case):
+    return 64 if case["size"] == "tiny" else HEAD_DIM
+
+
+_loaded = {}
+
+
+def _runner(case):
+    """The engine for the case's model; the one before it is given back when another model is asked for."""
+    key = (case["design"], case["size"], case["layers"], case["dtype"])
+    if key not in _loaded:
+        _loaded.clear()
+        torch.cuda.empty_cache()
+        _loaded[key] = load_runner(config=_config(case), random_seed=WEIGHT_SEED, options=EngineOptions(
+            dtype=case["dtype"], max_context=MAX_CONTEXT, prefill_chunk=2048, num_sequences=MAX_REQUESTS,
+            cache_tokens=CACHE_TOKENS))
+    return _loaded[key]
+
+
+# ---- one pass -------------------------------------------------------------------------------------------------
+
+def _requests(case, seed):
+    """Per request: (prompt's length, token ids of prompt and decoded part); the lengths are the case's own."""
+    rng, sizes = random.Random(seed), random.Random(case["requests"] * 100003 + case["prompt"])
+    vocab, got = SIZES[case["size"]]["vocab"], []
+    for i in range(case["requests"]):
+        n = case["prompt"] if not case["ragged"] or i == 0 else sizes.randint(max(1, case["prompt"] // 8), case["prompt"])
+        got.append((n, [rng.randrange(vocab) for _ in range(n + case["new"])]))
+    return got
+
+
+def _steps(case, requests):
+    """[[(request, first place, one past the last, whether its last token's logits are wanted)]] step by step."""
+    at, steps = [0] * len(requests), []
+    while any(a < len(t) for a, (_, t) in zip(at, requests)):
+        step, left = [], max(case["budget"], len(requests))
+        for r, (n, tokens) in enumerate(requests):
+            if n <= at[r] < len(tokens):
+                step.append((r, at[r], at[r] + 1, True))
+                left -= 1
+        for r, (n, tokens) in enumerate(requests):
+            if at[r] < n and left > 0:
+                end = min(n, at[r] + left)
+                step.append((r, at[r], end, end == n))
+                left -= end - at[r]
+        for r, _, end, _ in step:
+            at[r] = end
+        steps.append(step)
+    return steps
+
+
+_states = 0
+
+
+def prepare(case, seed):
+    global _states
+    _states += 1
+    requests = _requests(case, seed)
+    ids = [(_states, r) for r in range(len(requests))]
+    steps = [[StepEntry(ids[r], requests[r][1][a:b], [b - a - 1] if want else []) for r, a, b, want in step]
+             for step in _steps(case, requests)]
+    return {"runner": _runner(case), "ids": ids, "steps": steps}
+
+
+def run(state):
+    runner = state["runner"]
+    for r in state["ids"]:
+        runner.open(r)
+    logits = []
+    for step in state["steps"]:
+        out = runner.step(step)
+        if out.shape[0]:
+            logits.append(out.clone())             # a replayed step's logits lie in a buffer of the graph
+    for r in state["ids"]:
+        runner.close(r)
+    return torch.cat(logits)
+
+
+# ---- what a pass cannot do without ----------------------------------------------------------------------------
+
+def work(case):
+    """Weights that a step's rows use (a routed expert if a token is expected to choose it), once a step, since a step
+    needs the one before it; the cache entries its rows look at, once; new entries and logits written; states of the
+    recurrences read and written once a request and step."""
+    s, el = SIZES[case["size"]], 4 if case["dtype"] == "float32" else 2
+    W, H, G, D, E, k, ff = s["width"], s["heads"], s["kv_heads"], _head_dim(case), s["experts"], s["top"], s["ff"]
+    routed = case["layers"] if case["design"] == "qwen2_moe" else 0
+    proj = {"qwen2_moe": 0, "vekasun": 0, "difavik": 4 * 3, "nolesun": 4 * 2}[case["design"]] * W * k * ff      # weights that every row meets
+    kv_row, pair_flops, window = 0, 0, None            # cache entries a token, flops a (row, key) pair, over all layers
+    state, state_flops = 0, 0                          # bytes a request, flops a row, over all layers
+    n = case["layers"]
+    if case["design"] == "qwen2_moe":
+        proj += n * (W * (H + 2 * G) * D + H * D * W + 3 * W * s["shared"] + W * E)
+        kv_row, pair_flops = n * 2 * G * D, n * 4 * H * D
+    ssm_inner = s.get("ssm_heads", 0) * SSM_HEAD_DIM
+    ssm_proj = W * (2 * ssm_inner + 2 * GROUPS * s.get("state", 0) + s.get("ssm_heads", 0)) + ssm_inner * W
+    ssm_state = ssm_inner * s.get("state", 0)
+    if case["design"] == "vekasun":
+        q, r = s["q_rank"], s["kv_rank"]
+        proj += 2 * (W * (q + r + ROT_DIM) + q * H * (D + ROT_DIM) + r * H * 2 * D + W * H * D + H * D * W)
+        proj += 2 * ssm_proj
+        kv_row, pair_flops = 2 * (r + ROT_DIM), 2 * 2 * H * (2 * D + ROT_DIM)
+        state, state_flops = 2 * ssm_state * 4, 2 * 4 * ssm_state
+    if case["design"] == "difavik":
+        proj += 2 * (W * (H + G) * D + W * H + H * D * W + W * H * (2 * RET_DIM + 2 * D) + H * D * W)
+        proj += 2 * 5 * W * H * D
+        kv_row, pair_flops, window = 2 * 2 * G * D, 2 * 4 * H * D, WINDOW
+        state, state_flops = 2 * H * D * (D + RET_DIM) * 4, 2 * 4 * H * D * (D + RET_DIM)
+    if case["design"] == "nolesun":
+        proj += 4 * (W * (H + 2 * G) * D + H * D * W) + 2 * W * H * D + 2 * W * W
+        proj += 2 * ssm_proj + 2 * (W * H * D + 2 * W * H * D + 2 * W * H + H * D * W)
+        kv_row, pair_flops = 4 * 2 * G * D, 4 * 4 * H * D
+        state, state_flops = 2 * (ssm_state + H * D * D) * 4, 2 * (4 * ssm_state + 6 * H * D * D)
+    bytes_, flops = 0.0, 0.0
+    for step in _steps(case, _requests(case, 0)):
+        rows, wanted = sum(b - a for _, a, b, _ in step), sum(w for *_, w in step)
+        used = E * (1.0 - (1.0 - k / E) ** rows)
+        bytes_ += el * (proj + routed * used * 3 * W * ff + s["vocab"] * W * (wanted > 0) + rows * W)
+        bytes_ += 4 * wanted * s["vocab"] + el * rows * kv_row + 2 * state * len(step)
+        flops += 2.0 * rows * (proj + routed * k * 3 * W * ff) + 2.0 * wanted * W * s["vocab"] + rows * state_flops
+        for _, a, b, _ in step:
+            seen = b if window is None else min(b, b - a + window)
+            bytes_ += el * kv_row * (seen - (b - a))
+            pairs = (b * (b + 1) - a * (a + 1)) / 2 if window is None else sum(min(j + 1, window + KEEP_FIRST) for j in range(a, b))
+            flops += pair_flops * pairs
+    return {"bytes": bytes_, "flops": flops}
+
+
+def tolerance(case):
+    if case["dtype"] == "float32":
+        return {"rel": 1.2e-5}           # measured against 64 bits: 0.5e-6 to 3e-6
+    return {"rel": 0.03}                 # measured: 0.6 to 2 %
+
+
+# ---- the same in 64 bits --------------------------------------------------------------------------------------
+
+def _drawn(seed, name, shape, init, device):
+    """The engine's random weights, a function of (seed, tensor name, element) alone, as 64-bit numbers: two rounds of
+    a 32-bit mixing function over the element's number and the name's hash, four words of three 10-bit fields each,
+    their sum scaled to unit variance and rounded to bfloat16."""
+    digest = hashlib.sha256(f"{seed}:{name}".encode()).digest()
+    signed = lambda v: v - (1 << 32) if v >= 1 << 31 else v
+    k1, k2 = (signed(int.from_bytes(digest[i:i + 4], "little")) for i in (0, 4))
+
+    def mix(x):                                       # int32 products wrap; a shift's sign bits are masked off
+        x = x ^ ((x >> 16) & 0xFFFF)
+        x = x * 0x7FEB352D
+        x = x ^ ((x >> 15) & 0x1FFFF)
+        x = x * signed(0x846CA68B)
+        return x ^ ((x >> 16) & 0xFFFF)
+
+    count = math.prod(shape)
+    assert count < 1 << 31
+    out = torch.empty(count, dtype=torch.float64, device=device)
+    for a in range(0, count, 1 << 26):
+        i = torch.arange(a, min(count, a + (1 << 26)), dtype=torch.int32, device=device)
+        s = mix(mix(i ^ k1) ^ k2)
+        n = torch.full_like(s, -6138)
+        for c in (0x9E3779B9, 0x85EBCA6B, 0xC2B2AE35, 0x27D4EB2F):
+            w = mix(s ^ signed(c))
+            n += (w & 1023) + ((w >> 10) & 1023) + ((w >> 20) & 1023)
+        f32 = lambda v: torch.tensor(v, dtype=torch.float32, device=device)
+        z = n.to(torch.float32) * f32(9.765629656612873e-4)
+        v = f32(1.0) + f32(0.05) * z if init == "norm" else f32(0.02) * z
+        out[a:a + len(i)] = v.to(torch.bfloat16)
+    return out.view(shape)
+
+
+def _silu(x):
+    return x * torch.sigmoid(x)
+
+
+def _rms(x):
+    return x / torch.sqrt((x * x).mean(-1, keepdim=True) + EPS)
+
+
+def _turn(x, base, dims, neighbours=False):
+    """x [T, heads, D] turned by its positions 0 .. T - 1; pairs (i, i + dims / 2), or (2 i, 2 i + 1)."""
+    half = dims // 2
+    f = torch.tensor([base ** (-2.0 * i / dims) for i in range(half)], dtype=x.dtype, device=x.device)
+    angle = (torch.arange(len(x), dtype=x.dtype, device=x.device)[:, None] * f)[:, None]
+    c, s, out = torch.cos(angle), torch.sin(angle), x.clone()
+    p, q = (slice(0, dims, 2), slice(1, dims, 2)) if neighbours else (slice(0, half), slice(half, dims))
+    out[..., p], out[..., q] = x[..., p] * c - x[..., q] * s, x[..., q] * c + x[..., p] * s
+    return out
+
+
+def _attend(q, k, v, scale, cap=None, sink=None, window=None, slopes=None):
+    """q [T, H, D], k and v [T, G, .] of one request -> [T, H, Dv]; rows in blocks, so that scores stay small."""
+    T, H, _ = q.shape
+    rep, out, step = H // k.shape[1], [], max(1, 2048 * 2048 // T)
+    k, v = k.repeat_interleave(rep, 1).transpose(0, 1), v.repeat_interleave(rep, 1).transpose(0, 1)
+    j = torch.arange(T, device=q.device)
+    for a in range(0, T, step):
+        i = torch.arange(a, min(T, a + step), device=q.device)[:, None]
+        s = torch.matmul(q[a:a + step].transpose(0, 1), k.transpose(1, 2)) * scale
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        if slopes is not None:
+            s = s - slopes[:, None, None] * (i - j)
+        seen = j <= i
+        if window:
+            seen &= (i - j < window) | (j < KEEP_FIRST)
+        s = s.masked_fill(~seen, -math.inf)
+        if sink is not None:
+            s = torch.cat([s, sink[:, None, None].expand(H, s.shape[1], 1)], -1)
+        p = torch.softmax(s, -1)[..., :T]
+        out.append(torch.matmul(p, v).transpose(0, 1))
+    return torch.cat(out)
+
+
+def _conv_silu(u, taps, bias=None):
+    pad = torch.cat([u.new_zeros(TAPS - 1, u.shape[1]), u])
+    out = sum(pad[j:j + len(u)] * taps[:, j] for j in range(TAPS))
+    return _silu(out if bias is None else out + bias)
+
+
+class _Exact:
+    """A whole group of requests at once, layer by layer: rows of all requests one below the other."""
+
+    def __init__(self, case, seed):
+        self.case, self.s, self.dev = case, SIZES[case["size"]], torch.device("cuda" if torch.cuda.is_available() else "cpu")
+        self.requests = _requests(case, seed)
+        self.lengths = [len(t) for _, t in self.requests]
+        self.tokens = torch.tensor([t for _, ts in self.requests for t in ts], device=self.dev)
+
+    def w(self, name, *shape, init="linear"):
+        return _drawn(WEIGHT_SEED, name, shape, init, self.dev)
+
+    def each(self, fn, *rows):
+        """fn over every request's rows by itself."""
+        return torch.cat([fn(*r) for r in zip(*(torch.split(x, self.lengths) for x in rows))])
+
+    def experts(self, x, idx, weight, name, act):
+        s, W, ff, out = self.s, self.s["width"], self.s["ff"], torch.zeros_like(x)
+        gate, up, down = name
+        for e in range(s["experts"]):
+            rows, place = torch.nonzero(idx == e, as_tuple=True)
+            if len(rows):
+                u = x[rows]
+                y = act(u @ self.w(gate % e, ff, W).T, u @ self.w(up % e, ff, W).T) @ self.w(down % e, W, ff).T
+                out.index_add_(0, rows, y * weight[rows, place][:, None])
+        return out
+
+    def logits(self):
+        x = getattr(self, self.case["design"])()
+        at, wanted = torch.tensor([0] + self.lengths).cumsum(0).tolist(), []
+        for step in _steps(self.case, self.requests):
+            wanted += [at[r] + b - 1 for r, _, b, want in step if want]
+        head = {"qwen2_moe": "lm_head.weight", "difavik": "embed"}.get(self.case["design"], "head")
+        return self.final(x[wanted]) @ self.w(head, self.s["vocab"], self.s["width"]).T
+
+    # -- Qwen2-MoE
+    def qwen2_moe(self):
+        s, W, H, G, D = self.s, self.s["width"], self.s["heads"], self.s["kv_heads"], _head_dim(self.case)
+        glu = lambda g, u: _silu(g) * u
+        x = self.w("model.embed_tokens.weight", s["vocab"], W)[self.tokens]
+        self.final = lambda y: _rms(y) * self.w("model.norm.weight", W, init="norm")
+        for l in range(self.case["layers"]):
+            p = f"model.layers.{l}."
+            h = _rms(x) * self.w(p + "input_layernorm.weight", W, init="norm")
+            q, k, v = (h @ self.w(f"{p}self_attn.{n}_proj.weight", m * D, W).T + self.w(f"{p}self_attn.{n}_proj.bias", m * D)
+                       for n, m in (("q", H), ("k", G), ("v", G)))
+            turned = lambda y, m: _turn(y.view(-1, m, D), 1e6, D)
+            a = self.each(lambda q, k, v: _attend(turned(q, H), turned(k, G), v.view(-1, G, D), D ** -0.5), q, k, v)
+            x = x + a.flatten(1) @ self.w(p + "self_attn.o_proj.weight", W, H * D).T
+            h = _rms(x) * self.w(p + "post_attention_layernorm.weight", W, init="norm")
+            prob = torch.softmax(h @ self.w(p + "mlp.gate.weight", s["experts"], W).T, -1)
+            weight, idx = torch.topk(prob, s["top"], -1)
+            e = p + "mlp.experts.%d."
+            y = self.experts(h, idx, weight, (e + "gate_proj.weight", e + "up_proj.weight", e + "down_proj.weight"), glu)
+            e, S = p + "mlp.shared_expert.", s["shared"]
+            shared = glu(h @ self.w(e + "gate_proj.weight", S, W).T, h @ self.w(e + "up_proj.weight", S, W).T)
+            gate = torch.sigmoid(h @ self.w(p + "mlp.shared_expert_gate.weight", 1, W).T)
+            x = x + y + gate * (shared @ self.w(e + "down_proj.weight", W, S).T)
+        return x
+
+    # -- shared by the other designs
+    def state_space(self, h, p):
+        s, W, Hh, P, N = self.s, self.s["width"], self.s["ssm_heads"], SSM_HEAD_DIM, self.s["state"]
+        inner, C = Hh * P, Hh * P + 2 * GROUPS * N
+        proj = h @ self.w(p + "in", inner + C + Hh, W).T
+        taps, bias = self.w(p + "conv", C, TAPS), self.w(p + "conv.b", C)
+        dt_bias, rate, D = self.w(p + "dt_bias", Hh), torch.exp(self.w(p + "A_log", Hh)), self.w(p + "D", Hh)
+
+        def one(proj):
+            T = len(proj)
+            z, u, dt = torch.split(proj, [inner, C, Hh], 1)
+            x, B, Cm = torch.split(_conv_silu(u, taps, bias), [inner, GROUPS * N, GROUPS * N], 1)
+            x = x.reshape(T, Hh, P)
+            B, Cm = (y.reshape(T, GROUPS, N).repeat_interleave(Hh // GROUPS, 1) for y in (B, Cm))
+            dt = torch.nn.functional.softplus(dt + dt_bias, threshold=1e9)
+            decay, xd = torch.exp(-rate * dt), x * dt[..., None]
+            S, y = x.new_zeros(Hh, N, P), []
+            for t in range(T):
+                S = torch.baddbmm(S * decay[t][:, None, None], B[t][:, :, None], xd[t][:, None, :])
+                y.append(torch.bmm(Cm[t][:, None], S)[:, 0])
+            y = torch.stack(y) + D[:, None] * x
+            return (y.reshape(T, inner) * _silu(z)).view(T, GROUPS, inner // GROUPS)
+
+        y = _rms(self.each(one, proj)).flatten(1) * self.w(p + "norm", inner, init="norm")
+        return y @ self.w(p + "o", W, inner).T
+
+    # -- Vekasun
+    def vekasun(self):
+        s, W = self.s, self.s["width"]
+
+        def norm(y, name):
+            d = y - y.mean(-1, keepdim=True)
+            return d / torch.sqrt((d * d).mean(-1, keepdim=True) + EPS) * self.w(name, W, init="norm")
+
+        self.final = lambda y: norm(y, "final.norm")
+        x = self.w("embed", s["vocab"], W)[self.tokens]
+        for i, L in enumerate(_config(self.case)["layers"]):
+            p = f"l{i}."
+            h = norm(x, p + "norm1")
+            x = x + (self.state_space if L["type"] == "mamba2" else self.latent)(h, p + "mix.")
+        return x
+
+    def latent(self, h, p):
+        s, W, H, D, R = self.s, self.s["width"], self.s["heads"], HEAD_DIM, ROT_DIM
+        q = (_rms(h @ self.w(p + "dq", s["q_rank"], W).T) * self.w(p + "dq.norm", s["q_rank"], init="norm")) \
+            @ self.w(p + "uq", H * (D + R), s["q_rank"]).T
+        kv = h @ self.w(p + "dkv", s["kv_rank"] + R, W).T
+        c = _rms(kv[:, :s["kv_rank"]]) * self.w(p + "dkv.norm", s["kv_rank"], init="norm")
+        k, v = c @ self.w(p + "uk", H * D, s["kv_rank"]).T, c @ self.w(p + "uv", H * D, s["kv_rank"]).T
+        sink = self.w(p + "sink", H)
+
+        def one(q, k, rot, v):
+            q, k, rot = q.view(-1, H, D + R), k.view(-1, H, D), _turn(rot.reshape(-1, 1, R), 10000.0, R)
+            q = torch.cat([q[..., :D], _turn(q[..., D:], 10000.0, R)], -1)
+            return _attend(q, torch.cat([k, rot.expand(-1, H, R)], -1), v.view(-1, H, D), (D + R) ** -0.5, sink=sink)
+
+        o = self.each(one, q, k, kv[:, s["kv_rank"]:], v).flatten(1) * torch.sigmoid(h @ self.w(p + "g", H * D, W).T)
+        return o @ self.w(p + "o", W, H * D).T
+
+    # -- Difavik
+    def difavik(self):
+        s, W = self.s, self.s["width"]
+        scaled = lambda y, p, n: _rms(y) * (1.0 + self.w(f"{p}norm{n}", W)) * self.w(f"{p}ls{n}", W, init="norm")
+
+        def capped_glu(g, u):
+            g, u = torch.clamp(g, max=7.0), torch.clamp(u, min=-7.0, max=7.0)
+            return g * torch.sigmoid(1.702 * g) * (u + 1.0)
+
+        def pairs(tokens):
+            return torch.cat([tokens.new_tensor([65521]), (tokens[:-1] * 1000003 + tokens[1:] * 31) % 65521])
+
+        self.final = lambda y: _rms(y) * (1.0 + self.w("final.norm", W))
+        x = self.w("embed", s["vocab"], W)[self.tokens] + self.w("bigram", 65522, W)[self.each(pairs, self.tokens)]
+        for i, L in enumerate(_config(self.case)["layers"]):
+            p = f"l{i}."
+            m = p + "mix."
+            if L["type"] == "lightning":
+                y = self.decayed(x, m, HEAD_DIM, _silu, lambda o: _rms(o.flatten(1)) * self.w(m + "norm", s["heads"] * HEAD_DIM, init="norm"),
+                                 torch.sigmoid, rot=False)
+            else:
+                a = self.tied(x, m + "left.")
+                b = self.decayed(x, m + "right.", RET_DIM, lambda y: y, lambda o: _rms(o).flatten(1), _silu, rot=True)
+                y = 0.5 * (_rms(a) * self.w(m + "left.out", W, init="norm") + _rms(b) * self.w(m + "right.out", W, init="norm"))
+            x = x + scaled(y, p, 1)
+            q, ff = p + "mlp.", s["top"] * s["ff"]
+            y = capped_glu(*(x @ self.w(q + n, ff, W).T + self.w(f"{q}{n}.b", ff) for n in ("gate", "up")))
+            x = x + scaled(y @ self.w(q + "down", W, ff).T + self.w(q + "down.b", W), p, 2)
+        return x
+
+    def tied(self, h, p):
+        s, W, H, G, D = self.s, self.s["width"], self.s["heads"], self.s["kv_heads"], HEAD_DIM
+        q, k = (h @ self.w(p + n, m * D, W).T + self.w(f"{p}{n}.b", m * D) for n, m in (("q", H), ("k", G)))
+        qn, kn = (_rms(y) * self.w(f"{p}{n}.norm", m * D, init="norm") for y, n, m in ((q, "q", H), (k, "k", G)))
+        slopes = torch.tensor([2.0 ** (-8.0 * (i + 1) / H) for i in range(H)], dtype=h.dtype, device=h.device)
+        o = self.each(lambda q, k, v: _attend(q.view(-1, H, D), k.view(-1, G, D), v.view(-1, G, D), D ** -0.5,
+                                              window=WINDOW, slopes=slopes), qn, kn, k)
+        return (o * torch.sigmoid(h @ self.w(p + "g", H, W).T)[:, :, None]).flatten(1) @ self.w(p + "o", W, H * D).T
+
+    def decayed(self, h, p, D, act, norm, gate, rot):
+        W, H, V = self.s["width"], self.s["heads"], HEAD_DIM
+        q, k, v = (act(h @ self.w(p + n, H * d, W).T) for n, d in (("q", D), ("k", D), ("v", V)))
+        g = torch.tensor(_decays(H), dtype=h.dtype, device=h.device)[:, None, None]
+
+        def one(q, k, v):
+            q, k, v = q.view(-1, H, D), k.view(-1, H, D), v.view(-1, H, V)
+            if rot:
+                q, k = _turn(q, 10000.0, D), _turn(k, 10000.0, D) * D ** -0.5
+            S, o = q.new_zeros(H, D, V), []
+            for t in range(len(q)):
+                S = torch.baddbmm(S * g, k[t][:, :, None], v[t][:, None, :])
+                o.append(torch.bmm(q[t][:, None], S)[:, 0])
+            return torch.stack(o)
+
+        o = norm(self.each(one, q, k, v)) * gate(h @ self.w(p + "g", H * V, W).T)
+        return o @ self.w(p + "o", W, H * V).T
+
+    # -- Nolesun
+    def nolesun(self):
+        s, W = self.s, self.s["width"]
+        norm = lambda y, name: _rms(y) * (1.0 + self.w(name, W))
+        self.final = lambda y: norm(y, "final.norm")
+        x = x0 = self.w("embed", s["vocab"], W)[self.tokens] * 8.0
+        for i, L in enumerate(_config(self.case)["layers"]):
+            p, m = f"l{i}.", L["mixer"]
+            if i == 1:
+                x = torch.cat([x, x0], 1) @ self.w("loop.in", W, 2 * W).T + self.w("loop.step", 1, W)
+            h = norm(x, p + "norm1")
+            if L["type"] == "parallel":
+                y = self.plain_attention(h, p + "mix.left.", None), self.state_space(h, p + "mix.right.")
+            else:
+                y = self.plain_attention(h, p + "mix.left.", 30.0), self.delta_rule(h, p + "mix.right.")
+            y = m["left_scale"] * y[0] + m["right_scale"] * y[1]
+            x = x + norm(y, p + "norm1b") * self.w(p + "ls1", W, init="norm")
+            h, q, ff = norm(x, p + "norm2"), p + "mlp.", s["top"] * s["ff"]
+            y = torch.relu(h @ self.w(q + "up", ff, W).T) ** 2 @ self.w(q + "down", W, ff).T
+            x = x + norm(y, p + "norm2b") * self.w(p + "ls2", W, init="norm")
+        return x
+
+    def plain_attention(self, h, p, cap):
+        """With a cap on the scores also: rotation of neighbours, biases and an elementwise gate."""
+        s, W, H, G, D = self.s, self.s["width"], self.s["heads"], self.s["kv_heads"], HEAD_DIM
+        bias = lambda n, size: self.w(f"{p}{n}.b", size) if cap else 0.0
+        q, k, v = (h @ self.w(p + n, m * D, W).T + bias(n, m * D) for n, m in (("q", H), ("k", G), ("v", G)))
+        turned = lambda y, m: _turn(y.view(-1, m, D), 10000.0, ROT_DIM, neighbours=cap is not None)
+        o = self.each(lambda q, k, v: _attend(turned(q, H), turned(k, G), v.view(-1, G, D), D ** -0.5, cap=cap), q, k, v).flatten(1)
+        if cap:
+            o = o * torch.sigmoid(h @ self.w(p + "g", H * D, W).T)
+        return o @ self.w(p + "o", W, H * D).T + bias("o", W)
+
+    def delta_rule(self, h, p):
+        s, W, H, D = self.s, self.s["width"], self.s["heads"], HEAD_DIM
+        G = H // 2
+        taps = [self.w(f"{p}{n}.conv", m * D, TAPS) for n, m in (("q", G), ("k", G), ("v", H))]
+        q, k, v = (h @ self.w(p + n, m * D, W).T for n, m in (("q", G), ("k", G), ("v", H)))
+        beta = torch.sigmoid(h @ self.w(p + "b", H, W).T)
+        dt = torch.nn.functional.softplus(h @ self.w(p + "a", H, W).T + self.w(p + "dt_bias", H), threshold=1e9)
+        g = torch.exp(-torch.exp(self.w(p + "A_log", H)) * dt)
+
+        def one(q, k, v, beta, g):
+            q, k, v = (_conv_silu(y, t).view(len(y), -1, D) for y, t in zip((q, k, v), taps))
+            unit = lambda y: (y / torch.sqrt((y * y).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // G, 1)
+            q, k = unit(q) * D ** -0.5, unit(k)
+            S, o = q.new_zeros(H, D, D), []
+            for t in range(len(q)):
+                S = S * g[t][:, None, None]
+                new = beta[t][:, None, None] * (v[t][:, None] - torch.bmm(k[t][:, None], S))
+                S = torch.baddbmm(S, k[t][:, :, None], new)
+                o.append(torch.bmm(q[t][:, None], S)[:, 0])
+            return torch.stack(o)
+
+        o = (_rms(self.each(one, q, k, v, beta, g)) * self.w(p + "norm", D, init="norm")).flatten(1)
+        return (o * _silu(h @ self.w(p + "g", H * D, W).T)) @ self.w(p + "o", W, H * D).T
+
+
+def exact(case, seed):
+    with torch.no_grad():
+        return _Exact(case, seed).logits()
