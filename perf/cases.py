@@ -284,7 +284,7 @@ def work(case):
 def tolerance(case):
     if case["dtype"] == "float32":
         return {"rel": 1.2e-5}           # measured against 64 bits: 0.5e-6 to 3e-6
-    return {"rel": 0.03}                 # measured: 0.6 to 2 %
+    return {"rel": 0.03}                 # measured: 0.6 to 2 %, over long contexts 2.6 to 3.3 %
 
 
 # ---- the same in 64 bits --------------------------------------------------------------------------------------
