@@ -1,0 +1,570 @@
+// The recurrences  S_t = a_t S_{t-1} + w_t k_t v_t^T,  o_t = S_t^T q_t  of prompt portions on tensor cores (bfloat16
+// engines): the selective scan of ssm.cu (k = B, q = C, v = x, w = dt) and the linear attention of
+// linear_attention.cu (w = 1, a constant decay a head).  S is V x D per head, float32.
+//
+// Walking the rows one by one is bound by the chain from row to row (a prompt of 2,048 tokens, 64 heads of
+// 128 x 64: 771 us, about 1 % of the arithmetic's own time).  Over a chunk of Q rows the recurrence is three products:
+//
+//   o_t  = A_t S_0^T q_t + sum_{s <= t} (D(s, t) w_s q_t.k_s) v_s      A_t = a_1 ... a_t, D(s, t) = a_{s+1} ... a_t
+//   S_Q  = A_Q S_0 + sum_s D(s, Q) w_s k_s v_s^T
+//
+// so a step runs as (1) every chunk's own contribution to the state, all chunks and heads at once, (2) the chain over
+// the chunks' states, elementwise, which leaves in a chunk's place the state it starts from, (3) the outputs of all
+// chunks and heads at once.  Chunks are counted from a segment's first row of the step.  Decays are products, never
+// quotients or differences of logarithms, so a decay near zero does no harm.
+//
+// Everything beyond the activations stays float32 in what it carries: a float32 operand goes to the bfloat16 tensor
+// cores as three bfloat16 parts (8 + 8 + 8 bits: the number itself), a bfloat16 one as it is, and the partial
+// products whose weight is at least 2^-16 of the leading one are all taken (three where one operand is bfloat16, six
+// where both are float32) with float32 sums.
+//
+// One prompt of 2,048 tokens, before (row by row) and after: scan of 64 heads of 128 x 64 755 -> 172 us (the outputs take
+// 100 of it, the chunks' states 45, the chain over 16 chunks, which moves 67 MB, the rest), 32 heads of 64 x 64 394 -> 75;
+// linear attention of 16 heads of 128 x 128 with float32 q, k and v 499 -> 205 (six products each: bound by the tensor
+// pipe), 64 x 128 with bfloat16 values 347 -> 93.  Chunks of 128 rows halve the states' traffic where the operands are
+// bfloat16; with three parts of each operand in shared memory 64 rows fit.
+#define NF_CHAIN_CLASS 2
+#include "common.cuh"
+
+namespace nf {
+namespace {
+
+constexpr int kCrThreads = 256;
+constexpr int kCrPad = 8;               // elements of padding a shared-memory row: ldmatrix then meets no bank conflict
+
+enum CrMode : int { kCrScan = 0, kCrDecay = 1 };
+
+struct CrArgs {
+  const __nv_bfloat16 *q, *k, *v;       // rows of `ld` elements, columns from q0, k0, v0 on (q and k: a head group's D)
+  int ld, q0, k0, v0;
+  const float* prepared;                // float32 q and k [T, 2, H, D] instead
+  int v_silu;
+  int H, heads_per_group;
+  const __nv_bfloat16* dt;              // scan: raw step sizes
+  int ld_dt, dt0;
+  const float *dt_bias, *A_log, *skip;
+  const float* decay;                   // a decay a head
+  const int* chunks;                    // [n][3]: segment, first row, rows
+  const int* runs;                      // [m][3]: segment, first chunk, chunks
+  const int* seg_slot;
+  float* state;
+  long slot_stride;
+  float* chunk_state;                   // [n][H][V][D]
+  float* chunk_decay;                   // [n][H]
+  float* out;                           // [T][H * V]
+};
+
+__device__ __forceinline__ unsigned cr_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cr_ldm4(unsigned addr, unsigned (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void cr_ldm4t(unsigned addr, unsigned (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void cr_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two neighbouring numbers as PARTS packed pairs of bfloat16 that add up to them.  What has no remainder (an infinity,
+// a NaN) stands in the first part alone.
+template <int PARTS>
+__device__ __forceinline__ void cr_split(float x, float y, unsigned (&p)[PARTS]) {
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    p[i] = *reinterpret_cast<const unsigned*>(&h);
+    if (i + 1 < PARTS) {
+      const float hx = __low2float(h), hy = __high2float(h);
+      x = isinf(hx) || isnan(hx) ? 0.f : x - hx;
+      y = isinf(hy) || isnan(hy) ? 0.f : y - hy;
+    }
+  }
+}
+// Four consecutive numbers to the same place of PARTS planes.
+template <int PARTS>
+__device__ __forceinline__ void cr_store_parts(__nv_bfloat16* dst, size_t plane, const float (&x)[4]) {
+  unsigned lo[PARTS], hi[PARTS];
+  cr_split<PARTS>(x[0], x[1], lo);
+  cr_split<PARTS>(x[2], x[3], hi);
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) *reinterpret_cast<uint2*>(dst + i * plane) = make_uint2(lo[i], hi[i]);
+}
+
+// The chunk's decays and weights, one thread a row: 1 and 0 beyond its rows, so that those count nothing.
+template <int MODE>
+__device__ __forceinline__ void cr_row_gates(const CrArgs& a, int head, int row, bool live, float& decay, float& weight) {
+  decay = 1.f;
+  weight = 0.f;
+  if (!live) return;
+  if (MODE == kCrScan) {
+    const float v = to_float(a.dt[(size_t)row * a.ld_dt + a.dt0 + head]) + a.dt_bias[head];
+    weight = v > 20.f ? v : log1pf(expf(v));
+    decay = expf(-expf(a.A_log[head]) * weight);
+  } else {
+    decay = a.decay[head];
+    weight = 1.f;
+  }
+}
+
+// `rows` rows of the keys (or queries) into planes [PARTS][.][D + pad]; zeros from `live` rows on.
+template <int D, int PARTS>
+__device__ __forceinline__ void cr_load_qk(const CrArgs& a, bool keys, int head, int row0, int rows, int live,
+                                           __nv_bfloat16* dst, size_t plane) {
+  if (PARTS == 1) {
+    const __nv_bfloat16* src = (keys ? a.k + a.k0 : a.q + a.q0) + (size_t)(head / a.heads_per_group) * D;
+    for (int i = threadIdx.x; i < rows * (D / 8); i += kCrThreads) {
+      const int r = i / (D / 8), c = (i - r * (D / 8)) * 8;
+      uint4 x = make_uint4(0, 0, 0, 0);
+      if (r < live) x = *reinterpret_cast<const uint4*>(src + (size_t)(row0 + r) * a.ld + c);
+      *reinterpret_cast<uint4*>(dst + r * (D + kCrPad) + c) = x;
+    }
+  } else {
+    const float* src = a.prepared + (size_t)(keys ? a.H + head : head) * D;
+    for (int i = threadIdx.x; i < rows * (D / 4); i += kCrThreads) {
+      const int r = i / (D / 4), c = (i - r * (D / 4)) * 4;
+      float x[4] = {0.f, 0.f, 0.f, 0.f};
+      if (r < live) load4(src + (size_t)(row0 + r) * 2 * a.H * D + c, x);
+      cr_store_parts<PARTS>(dst + r * (D + kCrPad) + c, plane, x);
+    }
+  }
+}
+__device__ __forceinline__ float cr_value(float x, int silu) { return silu ? x / (1.f + expf(-x)) : x; }
+
+// ---- (1) a chunk's contribution to the state: [V, D] = sum_s (w_s D(s, end) v_s) k_s^T -------------------------------
+// 8 warps: a warp owns 32 value rows and D V / 256 state columns.
+template <int D, int V, int Q, int QKP, int MODE>
+__global__ void __launch_bounds__(kCrThreads)
+chunk_state_kernel(const CrArgs args) {
+  constexpr int WM = V / 32, WN = 8 / WM, NT = D / WN / 8;     // warps along V and D, column tiles a warp
+  constexpr int KS = D + kCrPad, VS = V + kCrPad;
+  static_assert(V % 32 == 0 && 8 % WM == 0 && D % (WN * 16) == 0 && Q % 32 == 0 && Q <= kCrThreads, "chunk shape");
+  extern __shared__ __align__(16) unsigned char cr_raw[];
+  __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(cr_raw);              // [QKP][Q][KS]
+  __nv_bfloat16* Vs = Ks + (size_t)QKP * Q * KS;                             // [3][Q][VS]
+  __shared__ float s_decay[Q], s_scale[Q];
+  const int chunk = blockIdx.x, head = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  CrArgs a = args;
+  chain_wait(a.q, a.k, a.v, a.dt, a.prepared);
+  const int row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
+  float weight = 0.f;
+  if (threadIdx.x < Q) {
+    float decay;
+    cr_row_gates<MODE>(a, head, row0 + threadIdx.x, (int)threadIdx.x < live, decay, weight);
+    s_decay[threadIdx.x] = decay;
+  }
+  cr_load_qk<D, QKP>(a, true, head, row0, Q, live, Ks, (size_t)Q * KS);
+  __syncthreads();
+  if (threadIdx.x < Q) {                 // w_s D(s, end): the rows after s in its 16, then whole sixteens
+    float run = 1.f;
+    const int end = (threadIdx.x & ~15) + 16;
+    for (int s = threadIdx.x + 1; s < end; ++s) run *= s_decay[s];
+    s_scale[threadIdx.x] = run;          // decays after s to the end of its sixteen
+  }
+  __syncthreads();
+  if (threadIdx.x < Q) {
+    float run = s_scale[threadIdx.x];
+    for (int b = (threadIdx.x >> 4) + 1; b < Q / 16; ++b) run *= s_scale[16 * b] * s_decay[16 * b];
+    if (threadIdx.x == 0) a.chunk_decay[(size_t)chunk * a.H + head] = run * s_decay[0];
+    weight *= run;
+  }
+  __syncthreads();
+  if (threadIdx.x < Q) s_scale[threadIdx.x] = weight;
+  __syncthreads();
+  {
+    const __nv_bfloat16* src = a.v + a.v0 + (size_t)head * V;
+    for (int i = threadIdx.x; i < Q * (V / 4); i += kCrThreads) {
+      const int r = i / (V / 4), c = (i - r * (V / 4)) * 4;
+      float x[4] = {0.f, 0.f, 0.f, 0.f};
+      if (r < live) {
+        load4(src + (size_t)(row0 + r) * a.ld + c, x);
+        const float f = s_scale[r];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = cr_value(x[e], a.v_silu) * f;
+      }
+      cr_store_parts<3>(Vs + r * VS + c, (size_t)Q * VS, x);
+    }
+  }
+  __syncthreads();
+  const int m0 = (warp % WM) * 32, n0 = (warp / WM) * (D / WN);
+  float acc[2][NT][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+  const int mat = lane >> 3, r8 = lane & 7;
+  const unsigned va = cr_smem(Vs + ((mat >> 1) * 8 + r8) * VS + m0 + (mat & 1) * 8);
+  const unsigned ka = cr_smem(Ks + ((mat & 1) * 8 + r8) * KS + n0 + (mat >> 1) * 8);
+#pragma unroll 1
+  for (int s0 = 0; s0 < Q; s0 += 16) {
+    if (s0 >= live) break;
+    unsigned A[3][2][4];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) cr_ldm4t(va + ((i * Q + s0) * VS + m * 16) * 2, A[i][m]);
+#pragma unroll
+    for (int n = 0; n < NT; n += 2)
+#pragma unroll
+      for (int j = QKP - 1; j >= 0; --j) {
+        unsigned B[4];
+        cr_ldm4t(ka + ((j * Q + s0) * KS + n * 8) * 2, B);
+#pragma unroll
+        for (int i = 2 - j; i >= 0; --i)
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            cr_mma(acc[m][n], A[i][m], B[0], B[1]);
+            cr_mma(acc[m][n + 1], A[i][m], B[2], B[3]);
+          }
+      }
+  }
+  float* dst = a.chunk_state + ((size_t)chunk * a.H + head) * V * D;
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      float* p = dst + (size_t)(m0 + m * 16 + (lane >> 2)) * D + n0 + n * 8 + (lane & 3) * 2;
+      *reinterpret_cast<float2*>(p) = make_float2(acc[m][n][0], acc[m][n][1]);
+      *reinterpret_cast<float2*>(p + 8 * D) = make_float2(acc[m][n][2], acc[m][n][3]);
+    }
+}
+
+// ---- (2) the chain over a segment's chunks --------------------------------------------------------------------------
+// A thread carries four of a head's V D state entries through the segment's chunks; loads run four chunks ahead.
+__global__ void __launch_bounds__(kCrThreads)
+chunk_chain_kernel(const CrArgs args, int entries) {
+  constexpr int AHEAD = 4;
+  const int run = blockIdx.x, head = blockIdx.y, e = (blockIdx.z * kCrThreads + threadIdx.x) * 4;
+  CrArgs a = args;
+  chain_wait(a.chunk_state, a.chunk_decay, a.state);
+  if (e >= entries) return;
+  const int seg = a.runs[3 * run], first = a.runs[3 * run + 1], n = a.runs[3 * run + 2];
+  float* slot = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + (size_t)head * entries + e;
+  float* mine = a.chunk_state + ((size_t)first * a.H + head) * entries + e;
+  const float* decay = a.chunk_decay + (size_t)first * a.H + head;
+  const size_t step = (size_t)a.H * entries;
+  float4 s = *reinterpret_cast<const float4*>(slot);
+  float4 next[AHEAD];
+  float d[AHEAD];
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i)
+    if (i < n) {
+      next[i] = *reinterpret_cast<const float4*>(mine + i * step);
+      d[i] = decay[(size_t)i * a.H];
+    }
+  for (int c0 = 0; c0 < n; c0 += AHEAD)
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      const int c = c0 + i;
+      if (c < n) {
+        const float4 x = next[i];
+        const float f = d[i];
+        *reinterpret_cast<float4*>(mine + c * step) = s;
+        if (c + AHEAD < n) {
+          next[i] = *reinterpret_cast<const float4*>(mine + (c + AHEAD) * step);
+          d[i] = decay[(size_t)(c + AHEAD) * a.H];
+        }
+        s.x = fmaf(f, s.x, x.x);
+        s.y = fmaf(f, s.y, x.y);
+        s.z = fmaf(f, s.z, x.z);
+        s.w = fmaf(f, s.w, x.w);
+      }
+    }
+  *reinterpret_cast<float4*>(slot) = s;
+}
+
+// ---- (3) a chunk's outputs --------------------------------------------------------------------------------------------
+// A warp owns 16 rows and V / (8 / (Q / 16)) columns.  Shared memory holds the queries throughout; beside them first the
+// state at the chunk's start, then the keys and values, SUB rows at a time.
+template <int D, int V, int Q, int SUB, int QKP, int VP, int MODE>
+__global__ void __launch_bounds__(kCrThreads, 2)
+chunk_output_kernel(const CrArgs args) {
+  constexpr int WQ = Q / 16, WV = 8 / WQ, NT = V / WV / 8;
+  constexpr int KS = D + kCrPad, VS = V + kCrPad;
+  static_assert(WQ * WV == 8 && NT % 2 == 0 && Q % SUB == 0 && SUB % 16 == 0, "chunk shape");
+  extern __shared__ __align__(16) unsigned char cr_raw[];
+  __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(cr_raw);              // [QKP][Q][KS]
+  __nv_bfloat16* Ss = Qs + (size_t)QKP * Q * KS;                             // [3][V][KS]
+  __nv_bfloat16* Ks = Ss;                                                    // [QKP][SUB][KS]
+  __nv_bfloat16* Vs = Ks + (size_t)QKP * SUB * KS;                           // [VP][SUB][VS]
+  __shared__ float s_decay[Q], s_weight[Q], s_upto[Q], s_after[Q];
+  __shared__ float s_diag[WQ][16][17];                                       // [.][s][t]: D(s, t) inside a sixteen
+  const int chunk = blockIdx.x, head = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  CrArgs a = args;
+  chain_wait(a.q, a.k, a.v, a.dt, a.prepared, a.chunk_state);
+  const int row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
+  if (threadIdx.x < Q)
+    cr_row_gates<MODE>(a, head, row0 + threadIdx.x, (int)threadIdx.x < live, s_decay[threadIdx.x], s_weight[threadIdx.x]);
+  cr_load_qk<D, QKP>(a, false, head, row0, Q, live, Qs, (size_t)Q * KS);
+  {
+    const float* src = a.chunk_state + ((size_t)chunk * a.H + head) * V * D;
+    for (int i = threadIdx.x; i < V * (D / 4); i += kCrThreads) {
+      const int r = i / (D / 4), c = (i - r * (D / 4)) * 4;
+      float x[4];
+      load4(src + (size_t)i * 4, x);
+      cr_store_parts<3>(Ss + r * KS + c, (size_t)V * KS, x);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < Q) {                 // a row's decays inside its sixteen: up to it, after it, from it to later rows
+    const int t = threadIdx.x, b = t & ~15;
+    float run = 1.f;
+    for (int s = b; s <= t; ++s) run *= s_decay[s];
+    s_upto[t] = run;
+    run = 1.f;
+    for (int u = 0; u < 16; ++u) {
+      if (b + u > t) run *= s_decay[b + u];
+      s_diag[t >> 4][t & 15][u] = b + u < t ? 0.f : run;
+    }
+    s_after[t] = run;
+  }
+  __syncthreads();
+  const int rb = warp % WQ, n0 = (warp / WQ) * (V / WV);       // this warp's sixteen and first column
+  const int g = lane >> 2, t4 = lane & 3, mat = lane >> 3, r8 = lane & 7;
+  const bool work = rb * 16 < live;
+  float acc[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
+  // rows as A (and, with eight rows more first, as B of two column tiles)
+  const unsigned qa = cr_smem(Qs + (rb * 16 + (mat & 1) * 8 + r8) * KS + (mat >> 1) * 8);
+  if (work) {
+    const unsigned sa = cr_smem(Ss + (n0 + (mat >> 1) * 8 + r8) * KS + (mat & 1) * 8);
+#pragma unroll 2
+    for (int k0 = 0; k0 < D; k0 += 16) {
+      unsigned A[QKP][4];
+#pragma unroll
+      for (int i = 0; i < QKP; ++i) cr_ldm4(qa + (i * Q * KS + k0) * 2, A[i]);
+#pragma unroll
+      for (int n = 0; n < NT; n += 2)
+#pragma unroll
+        for (int j = 2; j >= 0; --j) {
+          unsigned B[4];
+          cr_ldm4(sa + ((j * V + n * 8) * KS + k0) * 2, B);
+#pragma unroll
+          for (int i = (2 - j < QKP - 1 ? 2 - j : QKP - 1); i >= 0; --i) {
+            cr_mma(acc[n], A[i], B[0], B[1]);
+            cr_mma(acc[n + 1], A[i], B[2], B[3]);
+          }
+        }
+    }
+    float before = 1.f;                  // decays from the chunk's start to the sixteen's
+    for (int b = 0; b < rb; ++b) before *= s_upto[16 * b + 15];
+    const float f0 = before * s_upto[rb * 16 + g], f1 = before * s_upto[rb * 16 + g + 8];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      acc[n][0] *= f0; acc[n][1] *= f0;
+      acc[n][2] *= f1; acc[n][3] *= f1;
+    }
+  }
+  const float u0 = s_upto[rb * 16 + g], u1 = s_upto[rb * 16 + g + 8];
+  const unsigned kb = cr_smem(Ks + ((mat >> 1) * 8 + r8) * KS + (mat & 1) * 8);
+  const unsigned vb = cr_smem(Vs + ((mat & 1) * 8 + r8) * VS + n0 + (mat >> 1) * 8);
+#pragma unroll 1
+  for (int sub = 0; sub < Q; sub += SUB) {
+    if (sub >= live) break;
+    __syncthreads();                     // everyone is done with the state, or with the rows before
+    cr_load_qk<D, QKP>(a, true, head, row0 + sub, SUB, live - sub, Ks, (size_t)SUB * KS);
+    {
+      const __nv_bfloat16* src = a.v + a.v0 + (size_t)head * V;
+      if (VP == 1) {
+        for (int i = threadIdx.x; i < SUB * (V / 8); i += kCrThreads) {
+          const int r = i / (V / 8), c = (i - r * (V / 8)) * 8;
+          uint4 x = make_uint4(0, 0, 0, 0);
+          if (sub + r < live) x = *reinterpret_cast<const uint4*>(src + (size_t)(row0 + sub + r) * a.ld + c);
+          *reinterpret_cast<uint4*>(Vs + r * VS + c) = x;
+        }
+      } else {
+        for (int i = threadIdx.x; i < SUB * (V / 4); i += kCrThreads) {
+          const int r = i / (V / 4), c = (i - r * (V / 4)) * 4;
+          float x[4] = {0.f, 0.f, 0.f, 0.f};
+          if (sub + r < live) {
+            load4(src + (size_t)(row0 + sub + r) * a.ld + c, x);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] = cr_value(x[e], a.v_silu);
+          }
+          cr_store_parts<VP>(Vs + r * VS + c, (size_t)SUB * VS, x);
+        }
+      }
+    }
+    __syncthreads();
+    if (!work) continue;
+#pragma unroll 1
+    for (int sb = 0; sb < SUB; sb += 16) {
+      const int b = (sub + sb) >> 4;     // the sixteen of keys
+      if (b > rb) break;
+      float p[2][4];
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p[n][e] = 0.f;
+#pragma unroll 2
+      for (int k0 = 0; k0 < D; k0 += 16) {
+        unsigned A[QKP][4];
+#pragma unroll
+        for (int i = 0; i < QKP; ++i) cr_ldm4(qa + (i * Q * KS + k0) * 2, A[i]);
+#pragma unroll
+        for (int j = QKP - 1; j >= 0; --j) {
+          unsigned B[4];
+          cr_ldm4(kb + ((j * SUB + sb) * KS + k0) * 2, B);
+#pragma unroll
+          for (int i = (2 - j < QKP - 1 ? 2 - j : QKP - 1); i >= 0; --i) {
+            cr_mma(p[0], A[i], B[0], B[1]);
+            cr_mma(p[1], A[i], B[2], B[3]);
+          }
+        }
+      }
+      // times D(s, t) w_s
+      if (b == rb) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int s = n * 8 + t4 * 2 + (e & 1);
+            p[n][e] *= s_diag[rb][s][g + (e >> 1) * 8] * s_weight[b * 16 + s];
+          }
+      } else {
+        float between = 1.f;
+        for (int x = b + 1; x < rb; ++x) between *= s_upto[16 * x + 15];
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int s = b * 16 + n * 8 + t4 * 2 + e;
+            const float f = s_after[s] * between;
+            const float w = s_weight[s];
+            p[n][e] *= f * u0 * w;
+            p[n][e + 2] *= f * u1 * w;
+          }
+      }
+      unsigned P[3][4];
+      {
+        unsigned x[3];
+        cr_split<3>(p[0][0], p[0][1], x);
+        P[0][0] = x[0]; P[1][0] = x[1]; P[2][0] = x[2];
+        cr_split<3>(p[0][2], p[0][3], x);
+        P[0][1] = x[0]; P[1][1] = x[1]; P[2][1] = x[2];
+        cr_split<3>(p[1][0], p[1][1], x);
+        P[0][2] = x[0]; P[1][2] = x[1]; P[2][2] = x[2];
+        cr_split<3>(p[1][2], p[1][3], x);
+        P[0][3] = x[0]; P[1][3] = x[1]; P[2][3] = x[2];
+      }
+#pragma unroll
+      for (int n = 0; n < NT; n += 2)
+#pragma unroll
+        for (int j = VP - 1; j >= 0; --j) {
+          unsigned B[4];
+          cr_ldm4t(vb + ((j * SUB + sb) * VS + n * 8) * 2, B);
+#pragma unroll
+          for (int i = 2 - j; i >= 0; --i) {
+            cr_mma(acc[n], P[i], B[0], B[1]);
+            cr_mma(acc[n + 1], P[i], B[2], B[3]);
+          }
+        }
+    }
+  }
+  if (!work) return;
+#pragma unroll
+  for (int hi = 0; hi < 2; ++hi) {
+    const int r = rb * 16 + g + 8 * hi;
+    if (r >= live) continue;
+    const size_t row = (size_t)(row0 + r);
+    const float skip = MODE == kCrScan ? a.skip[head] : 0.f;
+    float* dst = a.out + row * a.H * V + (size_t)head * V + n0 + t4 * 2;
+    const __nv_bfloat16* x = a.v + row * a.ld + a.v0 + (size_t)head * V + n0 + t4 * 2;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      float y0 = acc[n][2 * hi], y1 = acc[n][2 * hi + 1];
+      if (MODE == kCrScan) {
+        const __nv_bfloat162 xx = *reinterpret_cast<const __nv_bfloat162*>(x + n * 8);
+        y0 = fmaf(skip, __low2float(xx), y0);
+        y1 = fmaf(skip, __high2float(xx), y1);
+      }
+      *reinterpret_cast<float2*>(dst + n * 8) = make_float2(y0, y1);
+    }
+  }
+}
+
+template <int D, int V, int Q, int SUB, int QKP, int VP, int MODE>
+static int launch_chunks(const CrArgs& a, int n_chunks, int n_runs, cudaStream_t stream) {
+  constexpr size_t smem1 = ((size_t)QKP * Q * (D + kCrPad) + 3 * (size_t)Q * (V + kCrPad)) * 2;
+  constexpr size_t part_s = 3 * (size_t)V * (D + kCrPad), part_kv = (size_t)QKP * SUB * (D + kCrPad) + (size_t)VP * SUB * (V + kCrPad);
+  constexpr size_t smem3 = ((size_t)QKP * Q * (D + kCrPad) + (part_s > part_kv ? part_s : part_kv)) * 2;
+  static_assert(smem1 <= 220 * 1024 && smem3 <= 220 * 1024, "shared memory of a chunk");
+  static bool set = false;                // (the attribute is the function's: set twice by two threads, it is the same)
+  if (!set) {
+    cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<D, V, Q, QKP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(chunk_output_kernel<D, V, Q, SUB, QKP, VP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
+    NF_REQUIRE(e == cudaSuccess, "chunk recurrence: cannot have %zu and %zu bytes of shared memory: %s", smem1, smem3, cudaGetErrorString(e));
+    set = true;
+  }
+  launch_chained(chunk_state_kernel<D, V, Q, QKP, MODE>, dim3(n_chunks, a.H), dim3(kCrThreads), smem1, stream, a);
+  launch_chained(chunk_chain_kernel, dim3(n_runs, a.H, (V * D / 4 + kCrThreads - 1) / kCrThreads), dim3(kCrThreads), 0, stream, a, V * D);
+  launch_chained(chunk_output_kernel<D, V, Q, SUB, QKP, VP, MODE>, dim3(n_chunks, a.H), dim3(kCrThreads), smem3, stream, a);
+  return check_launch("chunk_recurrence");
+}
+
+}  // namespace
+}  // namespace nf
+
+using namespace nf;
+
+// Rows a chunk; 0: these sizes are not served here.  scan: the selective scan, else linear attention.
+extern "C" int nf_chunk_recurrence_rows(int D, int V, int scan) {
+  if (scan) return (D == 64 || D == 128) && V == 64 ? 128 : 0;
+  return (D == 64 || D == 128) && V == 128 ? 64 : 0;
+}
+
+// The selective scan of the listed chunks; arguments as nf_ssd_scan's (bfloat16).  chunks int32 [n_chunks, 3] of
+// (segment, first row, rows), in order within a segment; runs int32 [n_runs, 3] of (segment, first chunk, chunks).
+// chunk_state float32 [n_chunks, heads, P, N], chunk_decay float32 [n_chunks, heads]: scratch.
+extern "C" int nf_chunk_scan(const void* xbc, int ldx, int x0, int b0, int c0, const void* dt, int ld_dt, int dt0,
+                             const float* dt_bias, const float* A_log, const float* skip, float* state, long long slot_stride,
+                             const int* seg_slot, const int* chunks, int n_chunks, const int* runs, int n_runs,
+                             float* chunk_state, float* chunk_decay, float* out, int heads, int P, int N, int groups,
+                             cudaStream_t stream) {
+  if (n_chunks == 0) return 0;
+  NF_REQUIRE(nf_chunk_recurrence_rows(N, P, 1) > 0 && groups > 0 && heads % groups == 0 && heads <= 65535, "chunk scan: sizes N=%d P=%d heads=%d", N, P, heads);
+  NF_REQUIRE(ldx % 8 == 0 && x0 % 8 == 0 && b0 % 8 == 0 && c0 % 8 == 0 && (uintptr_t)xbc % 16 == 0 && slot_stride % 4 == 0 &&
+             (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0, "chunk scan: rows and states must be 16-byte aligned");
+  CrArgs a = {};
+  a.q = a.k = a.v = (const __nv_bfloat16*)xbc;
+  a.ld = ldx; a.q0 = c0; a.k0 = b0; a.v0 = x0;
+  a.H = heads; a.heads_per_group = heads / groups;
+  a.dt = (const __nv_bfloat16*)dt; a.ld_dt = ld_dt; a.dt0 = dt0;
+  a.dt_bias = dt_bias; a.A_log = A_log; a.skip = skip;
+  a.chunks = chunks; a.runs = runs; a.seg_slot = seg_slot;
+  a.state = state; a.slot_stride = (long)slot_stride;
+  a.chunk_state = chunk_state; a.chunk_decay = chunk_decay; a.out = out;
+  if (N == 128) return launch_chunks<128, 64, 128, 64, 1, 1, kCrScan>(a, n_chunks, n_runs, stream);
+  return launch_chunks<64, 64, 128, 64, 1, 1, kCrScan>(a, n_chunks, n_runs, stream);
+}
+
+// Linear attention of the listed chunks: prepared float32 [T, 2, H, D] (q and k), v bfloat16 [T, ld] from v0 on
+// (through SiLU with v_silu), decay float32 [H]; the rest as above.
+extern "C" int nf_chunk_linear_attention(const float* prepared, const void* v, int ld, int v0, int v_silu, const float* decay,
+                                         float* state, long long slot_stride, const int* seg_slot,
+                                         const int* chunks, int n_chunks, const int* runs, int n_runs, float* chunk_state,
+                                         float* chunk_decay, float* out, int H, int D, int V, cudaStream_t stream) {
+  if (n_chunks == 0) return 0;
+  NF_REQUIRE(nf_chunk_recurrence_rows(D, V, 0) > 0 && H > 0 && H <= 65535 && decay, "chunk linear attention: sizes D=%d V=%d H=%d", D, V, H);
+  NF_REQUIRE(ld % 8 == 0 && v0 % 8 == 0 && (uintptr_t)v % 16 == 0 && (uintptr_t)prepared % 16 == 0 && slot_stride % 4 == 0 &&
+             (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0, "chunk linear attention: rows and states must be 16-byte aligned");
+  CrArgs a = {};
+  a.v = (const __nv_bfloat16*)v;
+  a.ld = ld; a.v0 = v0; a.v_silu = v_silu; a.prepared = prepared;
+  a.H = H; a.heads_per_group = 1;
+  a.decay = decay;
+  a.chunks = chunks; a.runs = runs; a.seg_slot = seg_slot;
+  a.state = state; a.slot_stride = (long)slot_stride;
+  a.chunk_state = chunk_state; a.chunk_decay = chunk_decay; a.out = out;
+  if (D == 128) return v_silu ? launch_chunks<128, 128, 64, 32, 3, 3, kCrDecay>(a, n_chunks, n_runs, stream)
+                              : launch_chunks<128, 128, 64, 32, 3, 1, kCrDecay>(a, n_chunks, n_runs, stream);
+  return v_silu ? launch_chunks<64, 128, 64, 32, 3, 3, kCrDecay>(a, n_chunks, n_runs, stream)
+                : launch_chunks<64, 128, 64, 32, 3, 1, kCrDecay>(a, n_chunks, n_runs, stream);
+}

@@ -88,7 +88,7 @@ decay_linear_attention_kernel(const T* __restrict__ src, int ld, int q_col0, int
                               float k_scale, float q_scale, int use_silu, float* __restrict__ state, long slot_stride,
                               const int* __restrict__ seg_row0, const int* __restrict__ seg_slot,
                               const int* __restrict__ seg_pos0, float* __restrict__ out, int H, int D, int V,
-                              const float* __restrict__ prepared, const float* __restrict__ gates) {
+                              const float* __restrict__ prepared, const float* __restrict__ gates, int skip_rows) {
   constexpr int COLS = kLaThreads / LANES;                 // value columns a CTA
   constexpr bool VEC = EPL % 4 == 0;
   constexpr int PAD = VEC ? 4 : 0;
@@ -106,6 +106,7 @@ decay_linear_attention_kernel(const T* __restrict__ src, int ld, int q_col0, int
   chain_release_if_small();
   chain_wait(src, state, prepared, gates);
   const int row0 = seg_row0[seg], rows = seg_row0[seg + 1] - row0;
+  if (rows >= skip_rows) return;                           // a segment that chunk_recurrence.cu serves
   const int pos0 = seg_pos0[seg];
   const float g = GATED ? 0.f : decay[head];
   float* sp = state + (size_t)seg_slot[seg] * slot_stride + ((size_t)head * V + (live ? col : 0)) * D + lane * EPL;
@@ -387,27 +388,27 @@ template <typename T, int EPL, int LANES, int CH, bool PREP>
 static void launch_la(const void* src, int ld, int q0, int k0, int v0, const float* decay, const float* inv_freq,
                       int rot, float k_scale, float q_scale, int use_silu, float* state, long long slot_stride,
                       const int* seg_row0, const int* seg_slot, const int* seg_pos0, float* out, int S, int H, int D,
-                      int V, const float* prepared, const float* gates, cudaStream_t stream) {
+                      int V, const float* prepared, const float* gates, int skip_rows, cudaStream_t stream) {
   constexpr int COLS = kLaThreads / LANES;
   dim3 grid(S, H, (V + COLS - 1) / COLS);
   if (gates)
     launch_chained(decay_linear_attention_kernel<T, EPL, LANES, CH, PREP, true>, grid, dim3(kLaThreads), 0, stream, (const T*)src, ld,
                    q0, k0, v0, decay, inv_freq, rot, k_scale, q_scale, use_silu, state, (long)slot_stride, seg_row0, seg_slot,
-                   seg_pos0, out, H, D, V, prepared, gates);
+                   seg_pos0, out, H, D, V, prepared, gates, skip_rows);
   else
     launch_chained(decay_linear_attention_kernel<T, EPL, LANES, CH, PREP, false>, grid, dim3(kLaThreads), 0, stream, (const T*)src, ld,
                    q0, k0, v0, decay, inv_freq, rot, k_scale, q_scale, use_silu, state, (long)slot_stride, seg_row0, seg_slot,
-                   seg_pos0, out, H, D, V, prepared, gates);
+                   seg_pos0, out, H, D, V, prepared, gates, skip_rows);
 }
 
 template <typename T>
 static int dispatch_la(const void* src, int ld, int q0, int k0, int v0, const float* decay, const float* inv_freq,
                        int rot, float k_scale, float q_scale, int use_silu, float* state, long long slot_stride,
                        const int* seg_row0, const int* seg_slot, const int* seg_pos0, float* out, int S, int H, int D,
-                       int V, const float* prepared, const float* gates, int single, cudaStream_t stream) {
+                       int V, const float* prepared, const float* gates, int single, int skip_rows, cudaStream_t stream) {
 #define NF_LA(E, L, C, P)                                                                                          \
   launch_la<T, E, L, C, P>(src, ld, q0, k0, v0, decay, inv_freq, rot, k_scale, q_scale, use_silu, state, slot_stride, \
-                           seg_row0, seg_slot, seg_pos0, out, S, H, D, V, prepared, gates, stream)
+                           seg_row0, seg_slot, seg_pos0, out, S, H, D, V, prepared, gates, skip_rows, stream)
   // single: every segment brings one row (a decode step): one token staged at a time, few registers
   if (prepared) {
     if (D <= 32) NF_LA(4, 8, 16, true);
@@ -446,13 +447,15 @@ extern "C" int nf_decay_linear_attention_max_dim() { return 256; }
 // every segment brings one row.
 // gates: null, or float32 [T, H, 3] of (decay, factor on k v^T, factor on the output) a (row, head), which
 // then stand in for `decay` (which may be null).  q_scale multiplies q after the turn, as k_scale does k.
+// skip_rows > 0: segments of that many rows or more are left alone.
 extern "C" int nf_decay_linear_attention(const void* src, int ld, int q_col0, int k_col0, int v_col0,
                                          const float* decay, const float* inv_freq, int rot, float k_scale,
                                          int use_silu, float* state, long long slot_stride, const int* seg_row0,
                                          const int* seg_slot, const int* seg_pos0, float* out, int S, int H, int D,
                                          int V, int dtype, const float* prepared, int single, float q_scale,
-                                         const float* gates, cudaStream_t stream) {
+                                         const float* gates, int skip_rows, cudaStream_t stream) {
   if (S == 0) return 0;
+  if (skip_rows <= 0) skip_rows = 0x7fffffff;
   NF_REQUIRE(decay || gates, "linear attention: neither a decay a head nor gates a row");
   NF_REQUIRE(S > 0 && H > 0 && D > 0 && V > 0 && D <= 256, "linear attention: bad sizes S=%d H=%d D=%d V=%d", S, H, D, V);
   NF_REQUIRE(rot >= 0 && rot % 2 == 0 && rot <= D && (rot == 0 || inv_freq), "linear attention: rot=%d with D=%d", rot, D);
@@ -460,9 +463,9 @@ extern "C" int nf_decay_linear_attention(const void* src, int ld, int q_col0, in
   NF_REQUIRE(!prepared || (D % 4 == 0 && D > 16 && (uintptr_t)prepared % 16 == 0), "linear attention: prepared q and k need D a multiple of 4 above 16");
   if (dtype == kF32)
     return dispatch_la<float>(src, ld, q_col0, k_col0, v_col0, decay, inv_freq, rot, k_scale, q_scale, use_silu, state,
-                              slot_stride, seg_row0, seg_slot, seg_pos0, out, S, H, D, V, prepared, gates, single, stream);
+                              slot_stride, seg_row0, seg_slot, seg_pos0, out, S, H, D, V, prepared, gates, single, skip_rows, stream);
   return dispatch_la<__nv_bfloat16>(src, ld, q_col0, k_col0, v_col0, decay, inv_freq, rot, k_scale, q_scale, use_silu, state,
-                                    slot_stride, seg_row0, seg_slot, seg_pos0, out, S, H, D, V, prepared, gates, single, stream);
+                                    slot_stride, seg_row0, seg_slot, seg_pos0, out, S, H, D, V, prepared, gates, single, skip_rows, stream);
 }
 
 // out float32 [T, 2 H D]: q then k of every row, activated, turned by positions[t] and (k) scaled.

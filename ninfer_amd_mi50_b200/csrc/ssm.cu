@@ -181,7 +181,7 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ldx, int x_col0, int b_col0, int 
                 const T* __restrict__ dt_src, int ld_dt, int dt_col0, const float* __restrict__ dt_bias,
                 const float* __restrict__ A_log, const float* __restrict__ Dskip, float* __restrict__ state,
                 long slot_stride, const int* __restrict__ seg_row0, const int* __restrict__ seg_slot,
-                float* __restrict__ y, int heads, int P, int N, int heads_per_group) {
+                float* __restrict__ y, int heads, int P, int N, int heads_per_group, int skip_rows) {
   constexpr int kCols = kScanGroups * CP;
   extern __shared__ float sm[];
   float* Bs = sm;                                  // [chunk][N]
@@ -198,6 +198,7 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ldx, int x_col0, int b_col0, int 
   const float rate = expf(A_log[h]), bias = dt_bias[h], skip = Dskip[h];
   chain_wait(xbc, dt_src);
   const int r0 = seg_row0[seg], n_rows = seg_row0[seg + 1] - r0;
+  if (n_rows >= skip_rows) return;                 // a segment that chunk_recurrence.cu serves
   float* S = state + (size_t)seg_slot[seg] * slot_stride + (size_t)h * P * N;
   float s[CP][NPER];
 #pragma unroll
@@ -361,7 +362,7 @@ template <typename T, int CP>
 static void launch_scan_cp(const void* xbc, int ldx, int x_col0, int b_col0, int c_col0, const void* dt_src, int ld_dt,
                            int dt_col0, const float* dt_bias, const float* A_log, const float* Dskip, float* state,
                            long slot_stride, const int* seg_row0, const int* seg_slot, float* y, int S, int heads, int P,
-                           int N, int groups, cudaStream_t stream) {
+                           int N, int groups, int skip_rows, cudaStream_t stream) {
   constexpr int kCols = kScanGroups * CP;
   const int nper = (N + kScanLanes - 1) / kScanLanes;
   const dim3 grid(S, heads * ((P + kCols - 1) / kCols)), block(kScanThreads);
@@ -369,7 +370,7 @@ static void launch_scan_cp(const void* xbc, int ldx, int x_col0, int b_col0, int
 #define NF_SCAN(NP)                                                                                                  \
   launch_chained(ssd_scan_kernel<T, NP, CP>, grid, block, smem, stream, (const T*)xbc, ldx, x_col0, b_col0, c_col0,   \
                  (const T*)dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, slot_stride, seg_row0, seg_slot, y, \
-                 heads, P, N, heads / groups)
+                 heads, P, N, heads / groups, skip_rows)
   if (nper <= 1) NF_SCAN(1);
   else if (nper <= 2) NF_SCAN(2);
   else if (nper <= 4) NF_SCAN(4);
@@ -384,15 +385,15 @@ template <typename T>
 static int launch_scan(const void* xbc, int ldx, int x_col0, int b_col0, int c_col0, const void* dt_src, int ld_dt,
                        int dt_col0, const float* dt_bias, const float* A_log, const float* Dskip, float* state,
                        long slot_stride, const int* seg_row0, const int* seg_slot, float* y, int S, int heads, int P,
-                       int N, int groups, cudaStream_t stream) {
+                       int N, int groups, int skip_rows, cudaStream_t stream) {
   const long ctas4 = (long)S * heads * ((P + 31) / 32), ctas2 = (long)S * heads * ((P + 15) / 16);
   const int forced = g_scan_columns;
   if (forced == 4 ? P % 32 == 0 : (forced == 0 && P % 32 == 0 && ctas4 >= 148))
-    launch_scan_cp<T, 4>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, stream);
+    launch_scan_cp<T, 4>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, skip_rows, stream);
   else if (forced == 2 ? P % 16 == 0 : (forced == 0 && P % 16 == 0 && ctas2 >= 148))
-    launch_scan_cp<T, 2>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, stream);
+    launch_scan_cp<T, 2>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, skip_rows, stream);
   else
-    launch_scan_cp<T, 1>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, stream);
+    launch_scan_cp<T, 1>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, skip_rows, stream);
   return 0;
 }
 
@@ -438,17 +439,19 @@ extern "C" int nf_causal_conv_silu(const void* src, int lds, int col0, int C, co
   return check_launch("causal_conv_silu");
 }
 
+// skip_rows > 0: segments of that many rows or more are left alone.
 extern "C" int nf_ssd_scan(const void* xbc, int ldx, int x_col0, int b_col0, int c_col0, const void* dt_src,
                            int ld_dt, int dt_col0, const float* dt_bias, const float* A_log, const float* Dskip,
                            float* state, long long slot_stride, const int* seg_row0, const int* seg_slot, float* y,
-                           int S, int heads, int P, int N, int groups, int dtype, cudaStream_t stream) {
+                           int S, int heads, int P, int N, int groups, int dtype, int skip_rows, cudaStream_t stream) {
   if (S == 0) return 0;
+  if (skip_rows <= 0) skip_rows = 0x7fffffff;
   NF_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0, "ssd_scan: %d heads do not split into %d groups", heads, groups);
   NF_REQUIRE(N > 0 && N <= kScanLanes * kScanMaxPer, "ssd_scan: state size %d (1..%d)", N, kScanLanes * kScanMaxPer);
   NF_REQUIRE(P > 0, "ssd_scan: bad head width");
   if (dtype == kF32)
-    launch_scan<float>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, (long)slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, stream);
+    launch_scan<float>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, (long)slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, skip_rows, stream);
   else
-    launch_scan<__nv_bfloat16>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, (long)slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, stream);
+    launch_scan<__nv_bfloat16>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, (long)slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, skip_rows, stream);
   return check_launch("ssd_scan");
 }

@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import ctypes
 from dataclasses import dataclass
-from typing import Optional, Tuple
+from typing import Optional, Sequence, Tuple
 
 import torch
 
@@ -43,6 +43,13 @@ TUNING = {
     # `latent_expand_max_mb`; a huge number keeps every row on the latent kernel
     "latent_expand_min_rows": 128,
     "latent_expand_max_mb": 1024,
+    # recurrences over prompt portions: segments of at least this many rows run as chunks on tensor cores (three launches
+    # that fill the device with a few hundred rows, where walking the rows costs the same each: the selective scan of 64
+    # heads takes 44 us against 55 at 128 rows, 32 against 32 at 64; linear attention of 16 heads of 128 x 128 takes 62
+    # against 134 at 512 rows, 57 against 44 at 128); a huge number leaves every row to the kernels that walk them
+    "chunk_scan_min_rows": 96,
+    "chunk_linear_min_rows": 192,
+    "chunk_recurrence_max_mb": 512,      # scratch for the chunks' states; a longer step's chunks run group after group
     "qkv_rope_fused": True,       # few bfloat16 rows: rotation and cache append in the projection's epilogue
     "router_tensor_min_rows": 128,   # router logits of more rows than this use tensor cores
     # up to this many rows, routing is a single launch (whole decode steps at 24 and 32 tokens:
@@ -1515,6 +1522,29 @@ def pair_hash_embed(table: torch.Tensor, ctx, last: torch.Tensor, h: torch.Tenso
 LINEAR_ATTENTION_MAX_DIM = 256
 
 
+def _recurrence_chunks(ctx, src: torch.Tensor, columns: Sequence[int], state: torch.Tensor, state_off: int, heads: int, D: int,
+                       V: int, scan: bool):
+    """What `ctx.recurrence_chunks` says for a step whose long segments the chunked recurrences (chunk_recurrence.cu) are to
+    serve, else None: bfloat16 rows and states that can be read 16 bytes at a time, sizes that those kernels have, and a
+    segment of at least as many rows as `TUNING` says."""
+    min_rows = TUNING["chunk_scan_min_rows" if scan else "chunk_linear_min_rows"]
+    if (src.dtype != torch.bfloat16 or getattr(ctx, "seg_len_host", None) is None or getattr(ctx, "graph_mode", False)
+            or ctx.max_rows_per_seg < min_rows or not hasattr(ctx, "recurrence_chunks")):
+        return None
+    rows = int(_lib.load().nf_chunk_recurrence_rows(c_int(D), c_int(V), c_int(1 if scan else 0)))
+    if (not rows or any(c % 8 for c in columns) or src.shape[1] % 8 or src.data_ptr() % 16 or state.stride(0) % 4
+            or (state.data_ptr() + 4 * state_off) % 16):
+        return None
+    return ctx.recurrence_chunks(rows, min_rows, max(1, (TUNING["chunk_recurrence_max_mb"] << 20) // (heads * D * V * 4)))
+
+
+def _chunk_scratch(lists, heads: int, D: int, V: int, device) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Float32 scratch for the largest group of chunks: their states, their decays."""
+    n = max(g[1] for g in lists)
+    return (torch.empty((n, heads, V, D), dtype=torch.float32, device=device),
+            torch.empty((n, heads), dtype=torch.float32, device=device))
+
+
 def decay_linear_attention(src: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, decay: torch.Tensor,
                            inv_freq: Optional[torch.Tensor], rot: int, k_scale: float, silu: bool,
                            state: torch.Tensor, ctx, heads: int, D: int, V: int, q_scale: float = 1.0,
@@ -1543,11 +1573,24 @@ def decay_linear_attention(src: torch.Tensor, q_col0: int, k_col0: int, v_col0: 
         _lib.call("nf_linear_attention_prepare", _p(src), c_int(src.shape[1]), c_int(q_col0), c_int(k_col0),
                   _p(inv_freq) if rot else None, c_int(rot), c_float(k_scale), c_int(1 if silu else 0), _p(ctx.positions),
                   _p(prepared), c_int(T), c_int(heads), c_int(D), c_int(_dt(src)), c_float(q_scale), _stream())
+    chunked = (_recurrence_chunks(ctx, src, (v_col0,), state, 0, heads, D, V, scan=False)
+               if prepared is not None and gates is None else None)
+    skip_rows = 0
+    if chunked is not None:
+        lists, others = chunked
+        states, decays = _chunk_scratch(lists, heads, D, V, src.device)
+        for chunks, n, runs, m in lists:
+            _lib.call("nf_chunk_linear_attention", _p(prepared), _p(src), c_int(src.shape[1]), c_int(v_col0), c_int(1 if silu else 0),
+                      _p(decay), _p(state), c_longlong(state.stride(0)), _p(ctx.seg_slot), _p(chunks), c_int(n),
+                      _p(runs), c_int(m), _p(states), _p(decays), _p(out), c_int(heads), c_int(D), c_int(V), _stream())
+        if not others:
+            return out
+        skip_rows = TUNING["chunk_linear_min_rows"]
     _lib.call("nf_decay_linear_attention", _p(src), c_int(src.shape[1]), c_int(q_col0), c_int(k_col0), c_int(v_col0),
               _p(decay), _p(inv_freq) if rot else None, c_int(rot), c_float(k_scale), c_int(1 if silu else 0),
               _p(state), c_longlong(state.stride(0)), _p(ctx.seg_row0), _p(ctx.seg_slot), _p(ctx.seg_pos0), _p(out),
               c_int(ctx.S), c_int(heads), c_int(D), c_int(V), c_int(_dt(src)), _p(prepared), c_int(1 if single else 0),
-              c_float(q_scale), _p(gates), _stream())
+              c_float(q_scale), _p(gates), c_int(skip_rows), _stream())
     return out
 
 
@@ -1644,11 +1687,24 @@ def ssd_scan(xbc: torch.Tensor, x_col0: int, b_col0: int, c_col0: int, dt_src: t
         _chk(t, n, torch.float32)
     T = xbc.shape[0]
     y = torch.empty((T, heads * P), dtype=torch.float32, device=xbc.device)
+    state_p = c_void_p(state.data_ptr() + 4 * state_off)
+    chunked = _recurrence_chunks(ctx, xbc, (x_col0, b_col0, c_col0), state, state_off, heads, N, P, scan=True)
+    skip_rows = 0
+    if chunked is not None:
+        lists, others = chunked
+        states, decays = _chunk_scratch(lists, heads, N, P, xbc.device)
+        for chunks, n, runs, m in lists:
+            _lib.call("nf_chunk_scan", _p(xbc), c_int(xbc.shape[1]), c_int(x_col0), c_int(b_col0), c_int(c_col0), _p(dt_src),
+                      c_int(dt_src.shape[1]), c_int(dt_col0), _p(dt_bias), _p(A_log), _p(D), state_p, c_longlong(state.stride(0)),
+                      _p(ctx.seg_slot), _p(chunks), c_int(n), _p(runs), c_int(m), _p(states), _p(decays), _p(y), c_int(heads),
+                      c_int(P), c_int(N), c_int(groups), _stream())
+        if not others:
+            return y
+        skip_rows = TUNING["chunk_scan_min_rows"]
     _lib.call("nf_ssd_scan", _p(xbc), c_int(xbc.shape[1]), c_int(x_col0), c_int(b_col0), c_int(c_col0), _p(dt_src),
               c_int(dt_src.shape[1]), c_int(dt_col0), _p(dt_bias), _p(A_log), _p(D),
-              c_void_p(state.data_ptr() + 4 * state_off), c_longlong(state.stride(0)), _p(ctx.seg_row0),
-              _p(ctx.seg_slot), _p(y), c_int(ctx.S), c_int(heads), c_int(P), c_int(N), c_int(groups),
-              c_int(_dt(xbc)), _stream())
+              state_p, c_longlong(state.stride(0)), _p(ctx.seg_row0), _p(ctx.seg_slot), _p(y), c_int(ctx.S), c_int(heads),
+              c_int(P), c_int(N), c_int(groups), c_int(_dt(xbc)), c_int(skip_rows), _stream())
     return y
 
 

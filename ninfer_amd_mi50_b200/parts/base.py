@@ -274,6 +274,35 @@ class StepContext:
             self._tiles["single_ctx"] = sub
         return self._tiles["single_ctx"]
 
+    def recurrence_chunks(self, rows_per_chunk: int, min_rows: int, max_chunks: int
+                          ) -> Tuple[List[Tuple[torch.Tensor, int, torch.Tensor, int]], bool]:
+        """Chunks of `rows_per_chunk` rows, counted from the first row, of the segments that bring at least `min_rows`
+        rows: a list of groups of at most `max_chunks` of them, to be run one after the other, each as (int32 [n, 3] of
+        (segment, first row, rows), n, int32 [m, 3] of the segments' runs in it as (segment, first chunk, chunks), m);
+        and whether other segments are left.  Built on the host; not available in graph mode."""
+        key = ("recurrence_chunks", rows_per_chunk, min_rows, max_chunks)
+        if key not in self._tiles:
+            groups, row, others = [], 0, False
+            for s, n in enumerate(self.seg_len_host):
+                others = others or n < min_rows
+                for r in range(0, n if n >= min_rows else 0, rows_per_chunk):
+                    if not groups or len(groups[-1][0]) == max_chunks:
+                        groups.append(([], []))
+                    chunks, runs = groups[-1]
+                    if not runs or runs[-1][0] != s:
+                        runs.append([s, len(chunks), 0])
+                    runs[-1][2] += 1
+                    chunks.append([s, row + r, min(rows_per_chunk, n - r)])
+                row += n
+            flat = self._ints([v for chunks, runs in groups for part in (chunks, runs) for c in part for v in c])
+            lists, at = [], 0
+            for chunks, runs in groups:
+                mid, end = at + 3 * len(chunks), at + 3 * (len(chunks) + len(runs))
+                lists.append((flat[at:mid], len(chunks), flat[mid:end], len(runs)))
+                at = end
+            self._tiles[key] = (lists, others)
+        return self._tiles[key]
+
     def context_rows(self, min_rows: int) -> Tuple[torch.Tensor, int]:
         """Where each segment's whole context (what it held and what it brings) starts in a matrix that holds the
         contexts of all segments of at least `min_rows` rows one after the other: (int32 [S], -1 for the others;

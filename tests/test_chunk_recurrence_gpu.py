@@ -1,0 +1,110 @@
+"""The chunked recurrences (csrc/chunk_recurrence.cu) against the recurrence walked row by row in float64."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# segments at the edges of a chunk (64 and 128 rows) and of its sixteens, beside short ones that the row-by-row kernel
+# keeps; the last entry is several groups of chunks when the scratch is small
+LENGTHS = [[64], [65, 1, 63], [127, 128, 129], [80, 3, 257], [700]]
+
+
+def context(lens):
+    from ninfer_amd_mi50_b200.parts.base import StepContext
+    dev = torch.device("cuda")
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    S, T = len(lens), sum(lens)
+    row0 = [sum(lens[:i]) for i in range(S + 1)]
+    pos0 = [7 * s for s in range(S)]
+    return StepContext(dtype=torch.bfloat16, device=dev, T=T, S=S, token_ids=ints([0] * T),
+                       positions=ints([p + i for p, n in zip(pos0, lens) for i in range(n)]),
+                       row_seg=ints([s for s, n in enumerate(lens) for _ in range(n)]), seg_row0=ints(row0), seg_pos0=ints(pos0),
+                       seg_slot=ints([S - s for s in range(S)]), logit_rows=ints([0]), seg_len_host=list(lens),
+                       seg_pos0_host=pos0, max_rows_per_seg=max(lens), max_context=max(p + n for p, n in zip(pos0, lens)))
+
+
+def walk(q, k, v, a, w, S):
+    """q, k [T, H, D], v [T, H, V], a, w [T, H], S [H, V, D], all float64."""
+    out = []
+    for t in range(len(q)):
+        S = a[t][:, None, None] * S + (w[t][:, None] * v[t])[:, :, None] * k[t][:, None, :]
+        out.append(torch.einsum("hvd,hd->hv", S, q[t]))
+    return torch.stack(out), S
+
+
+def close(got, want, what):
+    # float32 throughout: every number carries 24 bits and sums run over at most a few hundred terms (their error grows
+    # with the root of that); a dropped part of an operand (8 of its 24 bits) would show as 1e-5
+    err = ((got.double() - want).norm() / want.norm()).item()
+    assert err <= 2e-6, f"{what}: {err:.2e}"
+
+
+@pytest.mark.parametrize("lens", LENGTHS)
+@pytest.mark.parametrize("N", [64, 128])
+@pytest.mark.parametrize("slow", [False, True])
+def test_scan_in_chunks(lens, N, slow, monkeypatch):
+    from ninfer_amd_mi50_b200 import kernels
+    monkeypatch.setitem(kernels.TUNING, "chunk_scan_min_rows", 63)
+    H, P, G = 6, 64, 2
+    if lens == [700]:
+        monkeypatch.setitem(kernels.TUNING, "chunk_recurrence_max_mb", 1)
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + N)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ctx, T, C = context(lens), sum(lens), H * P + 2 * G * N
+    xbc, proj = rand(T, C).bfloat16(), rand(T, 8 + H + 2).bfloat16()
+    dt_bias, A_log, D = rand(H), rand(H) - (4.0 if slow else 0.0), rand(H)
+    A_log[0] = 6.0                                    # decays that underflow
+    off = 16
+    state = rand(len(lens) + 2, off + H * P * N)
+    before = state.double().clone()
+    y = kernels.ssd_scan(xbc, 0, H * P, H * P + G * N, proj, 8, dt_bias, A_log, D, state, off, ctx, H, P, N, G)
+    x = xbc.double()
+    dt = torch.nn.functional.softplus(proj[:, 8:8 + H].double() + dt_bias.double(), threshold=1e9)
+    heads = lambda c: x[:, c:c + G * N].view(T, G, N).repeat_interleave(H // G, 1)
+    v, row = x[:, :H * P].view(T, H, P), 0
+    for s, n in enumerate(lens):
+        r, slot = slice(row, row + n), len(lens) - s
+        want, S = walk(heads(H * P + G * N)[r], heads(H * P)[r], v[r], torch.exp(-torch.exp(A_log.double()) * dt[r]), dt[r],
+                       before[slot, off:].view(H, P, N))
+        close(y[r].view(n, H, P), want + D.double()[:, None] * v[r], f"outputs of segment {s}")
+        close(state[slot, off:].view(H, P, N), S, f"state of segment {s}")
+        row += n
+    for slot in (0, len(lens) + 1):
+        assert torch.equal(state[slot].double(), before[slot])
+    assert torch.equal(state[:, :off].double(), before[:, :off])
+
+
+@pytest.mark.parametrize("lens", LENGTHS)
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("silu", [False, True])
+def test_linear_attention_in_chunks(lens, D, silu, monkeypatch):
+    from ninfer_amd_mi50_b200 import kernels
+    monkeypatch.setitem(kernels.TUNING, "chunk_linear_min_rows", 63)
+    H, V = 5, 128
+    if lens == [700]:
+        monkeypatch.setitem(kernels.TUNING, "chunk_recurrence_max_mb", 1)
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + D)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ctx, T, width = context(lens), sum(lens), 2 * H * D + H * V
+    src = rand(T, width + 8).bfloat16()
+    decay = torch.tensor([1.0 - 2.0 ** -8, 0.9, 0.5, 1.0, 1e-30], device="cuda")
+    freq = torch.tensor([1000.0 ** (-2.0 * i / D) for i in range(D // 2)], device="cuda")
+    state = rand(len(lens) + 2, H * V * D)
+    before = state.double().clone()
+    out = kernels.decay_linear_attention(src, 0, H * D, 2 * H * D, decay, freq, D, 0.25, silu, state, ctx, H, D, V)
+    act = torch.nn.functional.silu if silu else (lambda x: x)
+    q, k, v = (act(src[:, c:c + H * d].double()).view(T, H, d) for c, d in ((0, D), (H * D, D), (2 * H * D, V)))
+    angle = ctx.positions.float()[:, None] * freq            # the kernel's angle, a float32 product
+    c, s = torch.cos(angle.double())[:, None], torch.sin(angle.double())[:, None]
+    turn = lambda x: torch.cat([x[..., :D // 2] * c - x[..., D // 2:] * s, x[..., D // 2:] * c + x[..., :D // 2] * s], -1)
+    q, k, row = turn(q), turn(k) * 0.25, 0
+    ones = torch.ones(T, H, dtype=torch.float64, device="cuda")
+    for i, n in enumerate(lens):
+        r, slot = slice(row, row + n), len(lens) - i
+        want, S = walk(q[r], k[r], v[r], ones[r] * decay.double(), ones[r], before[slot].view(H, V, D))
+        close(out[r].view(n, H, V), want, f"outputs of segment {i}")
+        close(state[slot].view(H, V, D), S, f"state of segment {i}")
+        row += n
+    for slot in (0, len(lens) + 1):
+        assert torch.equal(state[slot].double(), before[slot])
