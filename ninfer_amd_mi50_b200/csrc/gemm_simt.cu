@@ -1,5 +1,5 @@
-// C = A * B^T on CUDA cores with float32 accumulation: the matrix product of the
-// all-32-bit path, and the always-correct form of every product of the bfloat16 path.
+// C = A * B^T on CUDA cores with float32 accumulation: the always-correct form of every product
+// (float32 rows that can be read 16 bytes at a time go to gemm_f32.cu, with the same results).
 //
 // One kernel covers the dense linear layers (reference: rocBLAS ``gemm_ex`` with f32
 // compute, src/ops/linear.hip:9-59, and the GEMV kernels of src/ops/gemv.hip) and the
@@ -12,6 +12,10 @@
 #include "common.cuh"
 
 namespace nf {
+
+bool gemm_f32_takes(const void* A, int lda, const void* B, size_t bgs, int K);
+int gemm_f32(const void* A, int lda, const void* B, size_t bgs, void* C, int ldc, int M, int N, int K, int groups, int max_rows,
+             const int* offsets, const int* a_rows, int a_div, bool gated, GatedActParams act, cudaStream_t stream);
 
 constexpr int BM = 64, BN = 64, BK = 16;
 
@@ -135,6 +139,8 @@ extern "C" int nf_gemm_simt(const void* A, int lda, const void* B, long long b_g
   NF_REQUIRE((swiglu >= 0 && swiglu <= 2) || swiglu == kActGeluTanh || swiglu == kActRelu2, "gemm: epilogue %d (0 none, 1 silu-gated, 2 capped, 4 tanh-GELU-gated, 5 the square of relu)", swiglu);
   const bool gated = swiglu != 0 && swiglu != kActRelu2;
   const GatedActParams act{swiglu, act_limit, act_alpha};
+  if (in_dtype == kF32 && out_dtype == kF32 && gemm_f32_takes(A, lda, B, (size_t)b_group_stride, K))
+    return gemm_f32(A, lda, B, (size_t)b_group_stride, C, ldc, M, N, K, groups, max_rows_per_group, offsets, a_rows, a_div, gated, act, stream);
   if (in_dtype == kF32 && out_dtype == kF32)
     return launch<float, float>(A, lda, B, (size_t)b_group_stride, C, ldc, M, N, K, groups, max_rows_per_group, offsets, a_rows, a_div, gated, act, stream);
   if (in_dtype == kBF16 && out_dtype == kBF16)
