@@ -36,6 +36,15 @@
 // (what a latent cache's rows are expanded into for a prompt portion): a segment's rows lie together from kv_base[segment]
 // on, and a block is one copy an atom column.  `gate` multiplies head h's output by sigmoid(gate[row, h]).
 //
+// With ROT > 0 (dense only) queries and keys have ROT more dimensions behind their D: the keys' further ones are the same
+// for all heads and come from a second matrix (`map_rot`, columns from rot_x on; what a latent cache keeps beside its
+// latent), and the softmax's denominator also holds exp(sink[h]).  Shared memory then has room for one stage of keys and
+// values (a stage's copy still lies under the softmax), and P goes to the tensor cores as two bfloat16 numbers, its
+// rounding and the remainder, as in attention_latent_mma.cu, whose rows this form takes over: with one, a row that rests
+// on a single far key would lose half of its weight's bits.
+// Prompts of 256 to 2,048 tokens, four of them in steps of 2,048 rows, 16 heads over latents of 512: 39 us a layer and
+// step, in the folded form 455 (two such layers and two scans: 7.2 -> 5.5 ms).
+//
 // Everything between the roles goes through mbarriers; every wait is bounded: after a fixed
 // number of polls the kernel records a code in `g_fa_error`, tells its other warps to stop,
 // waits (bounded) for its own copies in flight, frees its tensor memory and returns.
@@ -110,9 +119,10 @@ __device__ __forceinline__ TileInfo tile_info(const int* tiles, int which, const
   return t;
 }
 
-template <int D, int FORM, bool DENSE>
+template <int D, int ROT, int FORM, bool DENSE>
 __global__ void __launch_bounds__(kFaThreads, 1)
 prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
+                            const __grid_constant__ CUtensorMap map_rot, int rot_x, const float* __restrict__ sink,
                             const int* __restrict__ block_table, int bt_width, const int* __restrict__ positions,
                             const int* __restrict__ seg_row0, const int* __restrict__ tiles,
                             __nv_bfloat16* __restrict__ out, int Hq, int Hkv, int page_size, int num_pages,
@@ -121,13 +131,16 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             float softcap) {
   constexpr bool SIGMOID = FORM == kFormSigmoid, CAPPED = FORM == kFormCapped;
   constexpr int ATOMS = D / 64;                   // 64-column swizzle atoms across the head
-  constexpr int QB = ATOMS * kAtom;               // bytes of the Q tile, of a K block, of a V block
+  constexpr int KATOMS = (D + ROT) / 64;          // ... across a query or key
+  constexpr int QB = KATOMS * kAtom, VB = ATOMS * kAtom;   // bytes of the Q tile and of a K block; of a V block
+  constexpr int STAGES = ROT ? 1 : 2, PARTS = ROT ? 2 : 1; // K and V stages; bfloat16 numbers a weight is given as
+  static_assert(!ROT || (DENSE && FORM == kFormSoftmax), "the further dimensions go with the dense softmax form");
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* Qs = smem;
-  unsigned char* KV = Qs + QB;                    // [2 stages][K block, V block]
-  unsigned char* Ps = KV + 4 * QB;                // [2 atoms][128 rows][128 bytes]
-  FaBarriers* bars = reinterpret_cast<FaBarriers*>(Ps + 2 * kAtom);
+  unsigned char* KV = Qs + QB;                    // [stages][K block, V block]
+  unsigned char* Ps = KV + STAGES * (QB + VB);    // [parts][2 atoms][128 rows][128 bytes]
+  FaBarriers* bars = reinterpret_cast<FaBarriers*>(Ps + PARTS * 2 * kAtom);
   float* s_rowsum = reinterpret_cast<float*>(bars + 1);      // [2 halves][128 rows]: the two threads of a row add up
   float* s_rowmax = s_rowsum + 2 * kQ;                       // [2 block parities][2 halves][128 rows]
   volatile int* stop = &bars->stop;
@@ -137,7 +150,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
   // zeros in both stages: a block's second page may not exist, and what the tensor core then
   // reads in its place (times a zero probability) must be finite
-  for (int i = threadIdx.x; i < 4 * QB / 16; i += blockDim.x) reinterpret_cast<uint4*>(KV)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < STAGES * (QB + VB) / 16; i += blockDim.x) reinterpret_cast<uint4*>(KV)[i] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
     mbar_init(&bars->q_empty, 1);
@@ -169,7 +182,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   // Launched chained: the zero-fill, the barriers and the tensor-memory allocation above touch
   // nothing outside the SM and ran while the kernel before this one drained; queries, keys and
   // values (and the first write of `out`) come after the wait.
-  chain_wait(block_table, positions, seg_row0, tiles, gate, kv_base);
+  chain_wait(block_table, positions, seg_row0, tiles, gate, kv_base, sink);
 
   if (warp == 0 || warp == 10) {
     // ---- producers: warp 0 brings Q and the keys, warp 10 the values --------------------------------
@@ -207,23 +220,25 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (kv == 0) {
           if (!mbar_wait(&bars->q_empty, (gq & 1) ^ 1, stop, 1, &g_fa_error)) { ok = false; break; }
           mbar_expect_tx(&bars->q_full, QB);
-          for (int a = 0; a < ATOMS; ++a) tma_load_2d(Qs + a * kAtom, &map_q, h * D + 64 * a, t.row0, &bars->q_full);
+          for (int a = 0; a < KATOMS; ++a) tma_load_2d(Qs + a * kAtom, &map_q, h * (D + ROT) + 64 * a, t.row0, &bars->q_full);
           q_pending = true;
         }
         for (int blk = 0; blk < t.n_blocks; ++blk, ++gb) {
-          const int s = gb & 1;
+          const int s = gb % STAGES;
           int n_ok = 0;
           for (int pi = 0; pi < per; ++pi) { page_now[pi] = page_next[pi]; n_ok += page_now[pi] >= 0; }
           lookup(blk + 1, page_next);
-          unsigned char* st = KV + (size_t)s * 2 * QB + kv * QB;
+          unsigned char* st = KV + (size_t)s * (QB + VB) + kv * QB;
           void* full = kv ? &bars->v_full[s] : &bars->k_full[s];
           void* empty = kv ? &bars->v_empty[s] : &bars->k_empty[s];
-          if (!mbar_wait(empty, ((gb >> 1) & 1) ^ 1, stop, 2, &g_fa_error)) { ok = false; break; }
+          if (!mbar_wait(empty, ((gb / STAGES) & 1) ^ 1, stop, 2, &g_fa_error)) { ok = false; break; }
           if constexpr (DENSE) {
             // (rows beyond the matrix read as zeros; rows of the next segment are finite and masked)
-            mbar_expect_tx(full, (unsigned)kKeys * D * 2);
+            mbar_expect_tx(full, (unsigned)kKeys * (kv ? D : D + ROT) * 2);
             for (int a = 0; a < ATOMS; ++a)
               tma_load_2d(st + a * kAtom, &map_kv, (kv * Hkv + kvh) * D + 64 * a, dense_row0 + blk * kKeys, full);
+            for (int a = ATOMS; a < KATOMS && kv == 0; ++a)
+              tma_load_2d(st + a * kAtom, &map_rot, rot_x + 64 * (a - ATOMS), dense_row0 + blk * kKeys, full);
             issued_stage[s] = gb;
             continue;
           }
@@ -242,11 +257,11 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (q_pending)
           for (unsigned i = 0; i < (1u << 20); ++i)
             if (mbar_try(&bars->q_full, (gq - 1) & 1)) break;
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
           if (issued_stage[s] < 0) continue;
           void* full = kv ? &bars->v_full[s] : &bars->k_full[s];
           for (unsigned i = 0; i < (1u << 20); ++i)
-            if (mbar_try(full, (issued_stage[s] >> 1) & 1)) break;
+            if (mbar_try(full, (issued_stage[s] / STAGES) & 1)) break;
         }
       }
     }
@@ -256,20 +271,24 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       const unsigned idesc_qk = fa_idesc(kKeys, false), idesc_pv = fa_idesc(D, true);
       int gb = 0, gp = 0, gq = 0;
       bool ok = true;
-      // O += P V of the block whose keys sit in stage (gp & 1); `first`: the first block of a tile
+      // O += P V of the block whose values sit in stage gp % STAGES; `first`: the first block of a tile
       auto issue_pv = [&](bool first) -> bool {
-        if (!mbar_wait(&bars->v_full[gp & 1], (gp >> 1) & 1, stop, 4, &g_fa_error)) return false;
+        const int vs = gp % STAGES;
+        if (!mbar_wait(&bars->v_full[vs], (gp / STAGES) & 1, stop, 4, &g_fa_error)) return false;
         if (!mbar_wait(&bars->p_full, gp & 1, stop, 5, &g_fa_error)) return false;
         if (first && gq > 0 && !mbar_wait(&bars->o_read, (gq - 1) & 1, stop, 6, &g_fa_error)) return false;
         tc_fence_after();
-        const unsigned char* vst = KV + (size_t)(gp & 1) * 2 * QB + QB;
+        const unsigned char* vst = KV + (size_t)vs * (QB + VB) + QB;
 #pragma unroll
         for (int kk = 0; kk < kKeys / 16; ++kk) {
-          const unsigned long long a = smem_desc(Ps + (kk >> 2) * kAtom) + 2 * (kk & 3);
           const unsigned long long b = smem_desc_mn(vst + kk * 16 * 128, kAtom);
-          tc_mma(tmem_o, a, b, idesc_pv, (!first || kk > 0) ? 1u : 0u);
+#pragma unroll
+          for (int part = 0; part < PARTS; ++part) {
+            const unsigned long long a = smem_desc(Ps + (2 * part + (kk >> 2)) * kAtom) + 2 * (kk & 3);
+            tc_mma(tmem_o, a, b, idesc_pv, (!first || kk > 0 || part > 0) ? 1u : 0u);
+          }
         }
-        tc_commit(&bars->v_empty[gp & 1]);       // the values of this block are free ...
+        tc_commit(&bars->v_empty[vs]);           // the values of this block are free ...
         tc_commit(&bars->p_free);                // ... and so are P and O, once these have run
         ++gp;
         return true;
@@ -279,19 +298,19 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (t.seg < 0) break;
         if (!mbar_wait(&bars->q_full, gq & 1, stop, 3, &g_fa_error)) { ok = false; break; }
         for (int blk = 0; blk < t.n_blocks && ok; ++blk, ++gb) {
-          const int s = gb & 1;
-          if (!mbar_wait(&bars->k_full[s], (gb >> 1) & 1, stop, 4, &g_fa_error)) { ok = false; break; }
+          const int s = gb & 1, ks = gb % STAGES;
+          if (!mbar_wait(&bars->k_full[ks], (gb / STAGES) & 1, stop, 4, &g_fa_error)) { ok = false; break; }
           if (!mbar_wait(&bars->s_empty[s], ((gb >> 1) & 1) ^ 1, stop, 7, &g_fa_error)) { ok = false; break; }
           tc_fence_after();
-          const unsigned char* kst = KV + (size_t)s * 2 * QB;
+          const unsigned char* kst = KV + (size_t)ks * (QB + VB);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) {
+          for (int kk = 0; kk < (D + ROT) / 16; ++kk) {
             const unsigned long long a = smem_desc(Qs + (kk >> 2) * kAtom) + 2 * (kk & 3);
             const unsigned long long b = smem_desc(kst + (kk >> 2) * kAtom) + 2 * (kk & 3);
             tc_mma(tmem + s * kKeys, a, b, idesc_qk, kk > 0 ? 1u : 0u);
           }
           tc_commit(&bars->s_full[s]);
-          tc_commit(&bars->k_empty[s]);                           // the keys are free once the scores are done
+          tc_commit(&bars->k_empty[ks]);                          // the keys are free once the scores are done
           if (blk == t.n_blocks - 1) tc_commit(&bars->q_empty);   // the tile's last use of Q
           if (blk > 0 && !issue_pv(blk == 1)) { ok = false; break; }
         }
@@ -434,6 +453,14 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           w.z = *reinterpret_cast<unsigned*>(&b2);
           w.w = *reinterpret_cast<unsigned*>(&b3);
           *reinterpret_cast<uint4*>(prow + ((q ^ (r & 7)) << 4)) = w;   // piece q: keys 8 q .. 8 q + 7 of the atom
+          if constexpr (PARTS == 2) {
+            auto rest = [](float x, float y, __nv_bfloat162 b) {
+              const __nv_bfloat162 d = __floats2bfloat162_rn(x - __low2float(b), y - __high2float(b));
+              return *reinterpret_cast<const unsigned*>(&d);
+            };
+            *reinterpret_cast<uint4*>(prow + 2 * kAtom + ((q ^ (r & 7)) << 4)) =
+                make_uint4(rest(p[0], p[1], b0), rest(p[2], p[3], b1), rest(p[4], p[5], b2), rest(p[6], p[7], b3));
+          }
           sum += ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
         }
         l_run += sum;
@@ -454,6 +481,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (!mbar_wait(&bars->o_final, gq & 1, stop, 10, &g_fa_error)) { ok = false; break; }
       tc_fence_after();
       float inv = l_row > 0.f ? 1.f / l_row : 0.f;
+      if constexpr (ROT > 0) {
+        if (sink) {                                              // one more term of the denominator, without a value
+          const float s2 = sink[h] * kLog2e, top = fmaxf(m_ref, s2), mine = ex2(m_ref - top);
+          inv = l_row > 0.f ? mine / fmaf(l_row, mine, ex2(s2 - top)) : 0.f;
+        }
+      }
       if (gate && row_ok) inv *= 1.f / (1.f + expf(-__bfloat162float(gate[(size_t)(t.row0 + r) * gate_ld + h])));
       __nv_bfloat16* dst = out + (size_t)(t.row0 + r) * Hq * D + (size_t)h * D + half * HD;
 #pragma unroll 1
@@ -491,21 +524,22 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   }
 }
 
-template <int D, int FORM, bool DENSE>
-int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mkv, const int* block_table, int bt_width,
+template <int D, int ROT, int FORM, bool DENSE>
+int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mrot, int rot_x, const float* sink,
+                      const int* block_table, int bt_width,
                       const int* positions, const int* seg_row0, const int* tiles, int n_tiles, void* out, int Hq,
                       int Hkv, int page_size, int num_pages, int window, float scale, const float* sig_bias,
                       const int* kv_base, const void* gate, int gate_ld, float softcap, cudaStream_t stream) {
-  constexpr int QB = (D / 64) * kAtom;
-  const size_t smem = 1024 + (size_t)5 * QB + 2 * kAtom + sizeof(FaBarriers) + 6 * kQ * sizeof(float);
+  constexpr int QB = (D + ROT) / 64 * kAtom, VB = D / 64 * kAtom;
+  const size_t smem = 1024 + QB + (ROT ? 1 : 2) * (size_t)(QB + VB) + (ROT ? 4 : 2) * kAtom + sizeof(FaBarriers) + 6 * kQ * sizeof(float);
   static bool set = false;
   if (!set) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<D, FORM, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<D, ROT, FORM, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     NF_REQUIRE(e == cudaSuccess, "prefill attention: cannot have %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     set = true;
   }
   dim3 grid(Hq, n_tiles);
-  launch_chained(prefill_attention_tc_kernel<D, FORM, DENSE>, grid, dim3(kFaThreads), smem, stream, mq, mkv, block_table, bt_width,
+  launch_chained(prefill_attention_tc_kernel<D, ROT, FORM, DENSE>, grid, dim3(kFaThreads), smem, stream, mq, mkv, mrot, rot_x, sink, block_table, bt_width,
                  positions, seg_row0, tiles, (__nv_bfloat16*)out, Hq, Hkv, page_size, num_pages, window, scale, sig_bias, kv_base,
                  (const __nv_bfloat16*)gate, gate_ld, softcap);
   return check_launch("prefill_attention_tc");
@@ -540,7 +574,7 @@ static int attention_tc(const void* qkv, long long T, int q_row_stride, const vo
   CUtensorMap mq, mkv;
   if (int rc = make_map(&mq, qkv, T, (long long)Hq * D, kQ, q_row_stride)) return rc;
   if (int rc = make_map(&mkv, pages, (long long)num_pages * 2 * Hkv * page_size, D, page_size)) return rc;
-#define NF_TC(DD, SG) launch_prefill_tc<DD, SG, false>(mq, mkv, block_table, bt_width, positions, seg_row0, tiles, n_tiles, out, Hq, Hkv, page_size, num_pages, window, scale, sig_bias, nullptr, nullptr, 0, softcap, stream)
+#define NF_TC(DD, SG) launch_prefill_tc<DD, 0, SG, false>(mq, mkv, mkv, 0, nullptr, block_table, bt_width, positions, seg_row0, tiles, n_tiles, out, Hq, Hkv, page_size, num_pages, window, scale, sig_bias, nullptr, nullptr, 0, softcap, stream)
 #define NF_TC_D(DD) (sig_bias ? NF_TC(DD, kFormSigmoid) : (softcap > 0.f ? NF_TC(DD, kFormCapped) : NF_TC(DD, kFormSoftmax)))
   return D == 64 ? NF_TC_D(64) : NF_TC_D(128);
 #undef NF_TC_D
@@ -592,9 +626,29 @@ extern "C" int nf_dense_attention_tc(const void* q, long long T, int q_row_strid
   CUtensorMap mq, mkv;
   if (int rc = make_map(&mq, q, T, (long long)Hq * D, kQ, q_row_stride)) return rc;
   if (int rc = make_map(&mkv, kv, kv_rows, 2ll * Hkv * D, kKeys)) return rc;
-#define NF_TC(DD) launch_prefill_tc<DD, kFormSoftmax, true>(mq, mkv, nullptr, 0, positions, seg_row0, tiles, n_tiles, out, Hq, Hkv, kKeys, 0, 0, scale, nullptr, kv_base, gate, gate_ld, 0.f, stream)
+#define NF_TC(DD) launch_prefill_tc<DD, 0, kFormSoftmax, true>(mq, mkv, mkv, 0, nullptr, nullptr, 0, positions, seg_row0, tiles, n_tiles, out, Hq, Hkv, kKeys, 0, 0, scale, nullptr, kv_base, gate, gate_ld, 0.f, stream)
   return D == 64 ? NF_TC(64) : NF_TC(128);
 #undef NF_TC
+}
+
+// The dense form with 64 further dimensions: q [T, q_row_stride] holds Hq heads of D + 64; the keys' further dimensions are
+// columns rot_x .. rot_x + 63 of rot [kv_rows, rot_ld], rows as kv's; sink float32 [Hq] or null.
+extern "C" int nf_dense_rot_attention_tc(const void* q, long long T, int q_row_stride, const void* kv, long long kv_rows,
+                                         const void* rot, int rot_ld, int rot_x, const int* kv_base, const int* positions,
+                                         const int* seg_row0, const int* tiles, int n_tiles, void* out, int Hq, int Hkv, int D,
+                                         float scale, const float* sink, cudaStream_t stream) {
+  if (n_tiles == 0) return 0;
+  NF_REQUIRE(n_tiles > 0 && n_tiles <= 65535 && T > 0 && kv_rows > 0 && kv_rows < (1ll << 31), "dense attention: bad sizes tiles=%d T=%lld rows=%lld", n_tiles, T, kv_rows);
+  NF_REQUIRE(D == 128 && Hkv > 0 && Hq % Hkv == 0, "dense attention: sizes the tensor-core kernel does not take (Hq=%d Hkv=%d D=%d)", Hq, Hkv, D);
+  NF_REQUIRE(q_row_stride % 8 == 0 && q_row_stride >= Hq * (D + 64) && (uintptr_t)q % 16 == 0 && (uintptr_t)kv % 16 == 0 &&
+             rot_ld % 8 == 0 && rot_x % 8 == 0 && rot_x + 64 <= rot_ld && (uintptr_t)rot % 16 == 0, "dense attention: rows must be 16-byte aligned");
+  NF_REQUIRE(kv_base, "dense attention: bad arguments");
+  CUtensorMap mq, mkv, mrot;
+  if (int rc = make_map(&mq, q, T, (long long)Hq * (D + 64), kQ, q_row_stride)) return rc;
+  if (int rc = make_map(&mkv, kv, kv_rows, 2ll * Hkv * D, kKeys)) return rc;
+  if (int rc = make_map(&mrot, rot, kv_rows, rot_ld, kKeys)) return rc;
+  return launch_prefill_tc<128, 64, kFormSoftmax, true>(mq, mkv, mrot, rot_x, sink, nullptr, 0, positions, seg_row0, tiles, n_tiles,
+                                                        out, Hq, Hkv, kKeys, 0, 0, scale, nullptr, kv_base, nullptr, 0, 0.f, stream);
 }
 
 // 0 if no tensor-core attention kernel has given up on a wait since the last call; else the code

@@ -38,9 +38,9 @@ TUNING = {
     # prompt portions: steps with at least this many rows use the tcgen05 attention kernel (head
     # size 64 or 128), fewer the mma.sync one; a huge number turns the tensor-core kernel off
     "prefill_attention_tc_min_rows": 128,
-    # latent attention (without a rotated part) in prompt portions of at least this many rows: the cached latents are
-    # expanded into keys and values and the tcgen05 kernel runs over them, as long as those take at most
-    # `latent_expand_max_mb`; a huge number keeps every row on the latent kernel
+    # latent attention in prompt portions of at least this many rows (a rotated part: of 64 dimensions, beside heads of
+    # 128): the cached latents are expanded into keys and values and the tcgen05 kernel runs over them, as long as those
+    # take at most `latent_expand_max_mb`; a huge number keeps every row on the latent kernel
     "latent_expand_min_rows": 128,
     "latent_expand_max_mb": 1024,
     # recurrences over prompt portions: segments of at least this many rows run as chunks on tensor cores (three launches
@@ -1784,10 +1784,11 @@ def latent_attention(q_abs: torch.Tensor, q: torch.Tensor, head_stride: int, rot
     return out
 
 
-def can_expand_latent(q: torch.Tensor, heads: int, D: int, Dv: int, R: int, ctx) -> bool:
-    """Whether `expanded_latent_attention` serves the step's segments of several rows."""
-    if not (q.is_cuda and q.dtype == torch.bfloat16 and TUNING["bf16_attention"] != "generic" and D == Dv and D in (64, 128)
-            and R % 8 == 0 and q.shape[1] % 8 == 0 and q.is_contiguous()
+def can_expand_latent(q: torch.Tensor, heads: int, D: int, Dv: int, R: int, ctx, Dr: int = 0) -> bool:
+    """Whether `expanded_latent_attention` serves the step's segments of several rows; `Dr`: rotated dimensions behind
+    every query's D and every cached row's R."""
+    if not (q.is_cuda and q.dtype == torch.bfloat16 and TUNING["bf16_attention"] != "generic" and D == Dv
+            and (D in (64, 128) if Dr == 0 else (D, Dr) == (128, 64)) and R % 8 == 0 and q.shape[1] % 8 == 0 and q.is_contiguous()
             and ctx.seg_len_host is not None and ctx.seg_pos0_host is not None):
         return False
     rows = sum(n for n in ctx.seg_len_host if n > 1)
@@ -1797,21 +1798,32 @@ def can_expand_latent(q: torch.Tensor, heads: int, D: int, Dv: int, R: int, ctx)
 
 def expanded_latent_attention(q: torch.Tensor, w_kv: torch.Tensor, heads: int, D: int, pages: torch.Tensor,
                               block_table: torch.Tensor, page_size: int, ctx, scale: float, out: torch.Tensor,
-                              gate: Optional[torch.Tensor] = None, gate_col0: int = 0) -> None:
+                              gate: Optional[torch.Tensor] = None, gate_col0: int = 0, Dr: int = 0,
+                              sink: Optional[torch.Tensor] = None) -> None:
     """Causal softmax attention of the step's segments of several rows over a latent cache, by expanding it: the
     segments' cached rows c (pages [n, page_size, R]) are gathered, one product with w_kv [2 * heads * D, R] (keys of
     all heads, then values) gives every token's keys and values, and the tcgen05 kernel runs over those.  q [T, ld]
     holds the queries in its first heads * D columns; head h's output times sigmoid(gate[t, gate_col0 + h]) (bfloat16)
-    goes to out [T, heads * D], whose rows of single-row segments are left as they are."""
+    goes to out [T, heads * D], whose rows of single-row segments are left as they are.
+
+    With `Dr` the cached rows are [c | Dr rotated dimensions that all heads share], the queries heads * (D + Dr), and
+    exp(sink[h]) joins the softmax's denominator (no gate then: it is the caller's)."""
     _chk(q, "q", torch.bfloat16); _chk(w_kv, "w_kv", q.dtype); _chk(pages, "pages", q.dtype); _chk(out, "out", q.dtype)
     R = w_kv.shape[1]
     base, total = ctx.context_rows(2)
-    c = torch.empty((total, R), dtype=q.dtype, device=q.device)
+    c = torch.empty((total, R + Dr), dtype=q.dtype, device=q.device)
     _lib.call("nf_gather_cached_rows", _p(pages), _p(block_table), c_int(block_table.shape[1]), _p(ctx.seg_pos0),
-              _p(ctx.seg_row0), _p(base), _p(c), c_int(ctx.S), c_int(R * 2), c_int(page_size), c_int(pages.shape[0]),
+              _p(ctx.seg_row0), _p(base), _p(c), c_int(ctx.S), c_int((R + Dr) * 2), c_int(page_size), c_int(pages.shape[0]),
               c_int(int(ctx.max_context)), c_int(total), _stream())
-    kv = linear(c, w_kv)
+    kv = linear(c, w_kv) if Dr == 0 else torch.mm(c[:, :R], w_kv.t())        # (a product over the rows' first part)
     tiles, n_tiles = ctx.paired_query_tiles(128, 0, 128, pair=False, min_rows=2)
+    if Dr:
+        if sink is not None:
+            _chk(sink, "sink", torch.float32)
+        _lib.call("nf_dense_rot_attention_tc", _p(q), c_longlong(q.shape[0]), c_int(q.shape[1]), _p(kv), c_longlong(total), _p(c),
+                  c_int(R + Dr), c_int(R), _p(base), _p(ctx.positions), _p(ctx.seg_row0), _p(tiles), c_int(n_tiles), _p(out),
+                  c_int(heads), c_int(heads), c_int(D), c_float(scale), _p(sink), _stream())
+        return
     gate_p = c_void_p(gate.data_ptr() + 2 * gate_col0) if gate is not None else None
     _lib.call("nf_dense_attention_tc", _p(q), c_longlong(q.shape[0]), c_int(q.shape[1]), _p(kv), c_longlong(total), _p(base),
               _p(ctx.positions), _p(ctx.seg_row0), _p(tiles), c_int(n_tiles), _p(out), c_int(heads), c_int(heads), c_int(D),

@@ -16,9 +16,10 @@ never materialise k_h or v_h: the key projection is folded into the query
 (``q_abs_h = W_uk[h]^T q_plain_h``, so ``q_plain_h . k_h = q_abs_h . c``) and the value projection
 is applied after the weighted sum (``sum_j p_j v_h,j = W_uv[h] sum_j p_j c_j``), which is the same
 arithmetic regrouped.  Portions of few rows and decoded tokens run this form.  For a portion of many rows it
-costs several times the arithmetic of plain attention (every score is as wide as the latent); without a rotated
-part and a sink, and with sizes the tcgen05 kernel takes, such a portion gathers its cached latents, expands
-them into keys and values by one product and runs that kernel over them.
+costs several times the arithmetic of plain attention (every score is as wide as the latent); with sizes the tcgen05
+kernel takes, such a portion gathers its cached rows, expands their latents into keys and values by one product and
+runs that kernel over them.  (A rotated part goes with heads of 128, a sink or an elementwise gate only beside one, a
+gate a head only without; a window keeps the folded form.)
 Norms, rotation angles, scores and softmax are 32-bit in both modes.
 
 Variants by parameter: `q_rank` None - the queries are one product of the layer's input, ``q = W_q h``, without
@@ -137,9 +138,10 @@ class LatentAttention(Mixer):
         if cache.append:
             kernels.latent_append(proj, q_cols, R, Dr, self.kv_norm, self.eps, inv_freq, rot, ctx,
                                   cache.pages, cache.block_table, cache.page_size)
-        if (not Dr and not self.has_sink and not self.window and not (self.has_gate and not self.gate_per_head)
-                and kernels.can_expand_latent(q, H, self.dim, self.value_dim, R, ctx)):
-            return self._forward_expanded(q, proj, q_cols + R, ctx, cache)
+        per_head, elementwise = (self.has_gate and self.gate_per_head), (self.has_gate and not self.gate_per_head)
+        if (not self.window and (not per_head if Dr else not self.has_sink and not elementwise)
+                and kernels.can_expand_latent(q, H, self.dim, self.value_dim, R, ctx, Dr)):
+            return self._forward_expanded(q, proj, q_cols + R + Dr, ctx, cache)
         o = self._folded(q, proj, q_cols + R + Dr, ctx, cache.pages, cache.block_table, cache.page_size)
         return kernels.linear(o, self.w_o)
 
@@ -147,8 +149,14 @@ class LatentAttention(Mixer):
         """The segments of several rows over expanded keys and values, those of one row in the folded form."""
         H = self.heads
         o = torch.empty((q.shape[0], H * self.value_dim), dtype=q.dtype, device=q.device)
-        kernels.expanded_latent_attention(q, self.w_kv, H, self.dim, cache.pages, cache.block_table, cache.page_size, ctx,
-                                          self.scale, o, proj if self.has_gate else None, gate_col0)
+        if self.rot_dim:
+            kernels.expanded_latent_attention(q, self.w_kv, H, self.dim, cache.pages, cache.block_table, cache.page_size, ctx,
+                                              self.scale, o, Dr=self.rot_dim, sink=self.sink)
+            if self.has_gate:
+                o = kernels.sigmoid_gate_rows(o, proj, gate_col0)
+        else:
+            kernels.expanded_latent_attention(q, self.w_kv, H, self.dim, cache.pages, cache.block_table, cache.page_size, ctx,
+                                              self.scale, o, proj if self.has_gate else None, gate_col0)
         sub = ctx.single_rows_context()
         if sub is not None:
             rows, _ = ctx.single_rows()
