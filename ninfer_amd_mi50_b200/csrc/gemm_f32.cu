@@ -6,13 +6,15 @@
 // A tile is BM rows x BN features, k in steps of 32; a stage's rows lie in shared memory as they do in memory, 144 bytes
 // apart, so that eight lanes' 16-byte reads of eight features meet no bank conflict and rows are broadcast.  What bounds
 // a product depends on the rows that share a weight matrix, and so does the tile:
-//   up to 4 rows    4 x 32, one warp: a stream of weights; many small CTAs keep enough bytes in flight even where a
-//                   projection has few features
-//   up to 16        16 x 64, two warps with 8 x 2 sums a thread: still the weights' stream (16 rows of products a weight
-//                   take less than the 23 bytes a clock that an SM gets from memory)
-//   up to 64        32 x 64 and, beyond 32 rows, 64 x 64 with 4 x 4 sums a thread: 64 products for 8 reads
-//   more            128 x 64 with 8 x 4 sums a thread, bound by the products themselves
-// Requests of 257 tokens and four decoded ones through two layers of Qwen1.5-MoE-A2.7B's sizes: 36.0 -> 14.6 ms; three
+//   few rows        4 x 32, one warp: a stream of weights; many small CTAs keep enough bytes in flight even where a
+//                   projection has few features.  Rows beyond four read the weights again, from L2: 20 rows of one
+//                   matrix (6144 x 2048) 40 us, with the next tile 52; 33 rows 70 and 53.  Beside one another the groups
+//                   fill the device by themselves: 4.3 rows a group 148 us and 204, 8.5 rows 228 and 212 (60 x 2048 x 1408)
+//   up to 64        16 x 64, two warps with 8 x 2 sums a thread (34 rows a group 472 us, with the next tile 518)
+//   up to 128       32 x 64 with 4 x 4 sums a thread: 100 rows 112 us, with the tile before 152, with the one behind 140
+//   more            64 x 64 with 8 x 4 sums a thread (gated 4 x 4), bound by the products themselves: 256 rows 184 us,
+//                   32 x 64 210, 128 x 64 243; twice the CTAs of 128 x 64 leave less of the last round empty
+// Requests of 257 tokens and four decoded ones through two layers of Qwen1.5-MoE-A2.7B's sizes: 36.0 -> 12.9 ms; three
 // short ones through a model of width 256: 2.09 -> 1.43 ms.
 #define NF_CHAIN_CLASS 0x40
 #include "common.cuh"
@@ -161,11 +163,13 @@ int gf_dispatch(const GfCall& c, cudaStream_t stream) {
     const int n = c.groups > 1 && usual < most ? usual : most;
     return n < 65535 ? n : 65535;
   };
-  if (rows <= 4) return gf_launch<4, GATED ? 64 : 32, 4, GATED ? 2 : 1, 6, GATED>(c, tiles(4), stream);
-  if (rows <= 16) return gf_launch<16, 64, 8, 2, 4, GATED>(c, tiles(16), stream);
-  if (rows <= 32) return gf_launch<32, 64, 4, 4, 4, GATED>(c, tiles(32), stream);
-  if (rows <= 64 || c.groups > 1) return gf_launch<64, 64, 4, 4, 3, GATED>(c, tiles(64), stream);
-  return gf_launch<128, 64, 8, 4, 3, GATED>(c, tiles(128), stream);
+  // (the lines lie between the measured sizes at which the tile below and the one above were the faster)
+  const bool alone = c.groups == 1;
+  if (rows <= (alone ? 24 : 5)) return gf_launch<4, GATED ? 64 : 32, 4, GATED ? 2 : 1, 6, GATED>(c, tiles(4), stream);
+  if (rows <= 64) return gf_launch<16, 64, 8, 2, 4, GATED>(c, tiles(16), stream);
+  if (rows <= 128) return gf_launch<32, 64, 4, 4, 4, GATED>(c, tiles(32), stream);
+  if (GATED) return gf_launch<64, 64, 4, 4, 3, GATED>(c, tiles(64), stream);
+  return gf_launch<64, 64, 8, 4, 3, GATED>(c, tiles(64), stream);
 }
 
 }  // namespace
