@@ -27,14 +27,17 @@ __global__ void add_layernorm_kernel(float* __restrict__ h, const T* __restrict_
   extern __shared__ __align__(16) float row[];      // [hidden]
   __shared__ float red[33];
   const int r = blockIdx.x;
+  constexpr int W = VEC ? 4 : 1;
+  const int units = hidden / W;
   chain_release_if_small();
+  // the weights of this thread's first run (all of them up to 4 * blockDim numbers) are asked for before the wait
+  float4 w_first = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (VEC && (int)threadIdx.x < units) w_first = *reinterpret_cast<const float4*>(w + threadIdx.x * 4);
   chain_wait(h, delta, rows, y, inv, wts);
   const int src = GATHER ? rows[r] : r;
   float* hr = h + (size_t)src * hidden;
   const T* dr = delta ? delta + (size_t)src * hidden : nullptr;
   T* o = out + (size_t)r * hidden;
-  constexpr int W = VEC ? 4 : 1;
-  const int units = hidden / W;
   float s = 0.f;
   for (int u = threadIdx.x; u < units; u += blockDim.x) {
     const int i = u * W;
@@ -85,7 +88,7 @@ __global__ void add_layernorm_kernel(float* __restrict__ h, const T* __restrict_
   for (int u = threadIdx.x; u < units; u += blockDim.x) {
     const int i = u * W;
     if constexpr (VEC) {
-      const float4 wv = *reinterpret_cast<const float4*>(w + i);
+      const float4 wv = u == (int)threadIdx.x ? w_first : *reinterpret_cast<const float4*>(w + i);
       const float ov[4] = {(row[i] - mean) * rstd * wv.x, (row[i + 1] - mean) * rstd * wv.y,
                            (row[i + 2] - mean) * rstd * wv.z, (row[i + 3] - mean) * rstd * wv.w};
       store4(o + i, ov);
@@ -176,6 +179,84 @@ add_group_rmsnorm_kernel(float* __restrict__ h, const T* __restrict__ d1, const 
 }
 
 // out[t, 0:n] = x[t, col0:col0+n] * rsqrt(mean(x^2) + eps) * w   (w may be null: weight 1)
+// The row-wise norms below in their wide form: a thread owns R runs of four consecutive elements of a row's part, keeps
+// them in registers between the two passes and asks for the weights, which no kernel writes, before the wait.  In a decode
+// step such a kernel is a chain of trips to memory (rows of 2,048 and 4,096 read element by element, twice, with the weight
+// last, took 6 to 10 us), in a prompt it moves each row once.  Four layers of 2,048, prompts of 900 to 2,048 tokens and 16
+// decoded ones: latent attention and scans 5.43 -> 5.09 ms, linear and windowed attention 6.93 -> 6.28, attention beside
+// scans and delta rules 10.87 -> 10.55.
+// MODE 0: out = x / rms(x) * w.  1: x = y * silu(z), out = x / rms(x) * w.  2, 3: out = y / rms(y) * w * act(z), act the
+// silu or the sigmoid.  blockIdx.y: the part of the row.
+template <typename TY, typename TZ, typename T, int R, int MODE>
+__global__ void __launch_bounds__(512)
+part_norm_vec_kernel(const TY* __restrict__ y, int ldy, int ycol0, const TZ* __restrict__ zsrc, int ldz, int zcol0,
+                     const float* __restrict__ w, float eps, T* __restrict__ out, int ldo, int n) {
+  __shared__ float red[33];
+  const int t = blockIdx.x, c0 = blockIdx.y * n;
+  chain_release_if_small();
+  float wk[R][4], v[R][4], z[R][4];
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { wk[c][e] = 1.f; v[c][e] = z[c][e] = 0.f; }
+    if (w && i < n) load4(w + c0 + i, wk[c]);
+  }
+  chain_wait(y, zsrc);
+  const TY* yr = y + (size_t)t * ldy + ycol0 + c0;
+  const TZ* zr = MODE ? zsrc + (size_t)t * ldz + zcol0 + c0 : nullptr;
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+    if (i < n) {
+      load4(yr + i, v[c]);
+      if (MODE) load4(zr + i, z[c]);
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < R; ++c)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (MODE) {
+        const float sg = 1.f / (1.f + expf(-z[c][e]));
+        if (MODE == 1) v[c][e] *= z[c][e] * sg;
+        else z[c][e] = MODE == 3 ? sg : z[c][e] * sg;
+      }
+      ss += v[c][e] * v[c][e];
+    }
+  const float inv = rsqrtf(block_sum(ss, red) / (float)n + eps);
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+    if (i >= n) continue;
+    float o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = v[c][e] * inv * wk[c][e] * (MODE >= 2 ? z[c][e] : 1.f);
+    store4(out + (size_t)t * ldo + c0 + i, o);
+  }
+}
+// Whether rows of `n` numbers at `p` (first column `col0`, `ld` apart, `el` bytes a number) can be moved four at a time.
+static inline bool runs_of_four(const void* p, size_t el, long ld, long col0) {
+  return ld % 4 == 0 && col0 % 4 == 0 && (uintptr_t)p % (4 * el) == 0;
+}
+// 0: not in the wide form
+template <typename TY, typename TZ, typename T, int MODE>
+static int part_norm_vec(const void* y, int ldy, int ycol0, const void* z, int ldz, int zcol0, const float* w, float eps,
+                         void* out, int ldo, int R, int n, int parts, cudaStream_t stream) {
+  if (n % 4 || n > 8192 || parts > 65535 || !runs_of_four(y, sizeof(TY), ldy, ycol0) || !runs_of_four(out, sizeof(T), ldo, 0) ||
+      (MODE && !runs_of_four(z, sizeof(TZ), ldz, zcol0)) || (uintptr_t)w % 16)
+    return 0;
+  const int units = n / 4, runs = units <= 512 ? 1 : (units <= 1024 ? 2 : 4);
+  const int th = ((units + runs - 1) / runs + 31) / 32 * 32;
+#define NF_PN(RR)                                                                                                        \
+  launch_chained(part_norm_vec_kernel<TY, TZ, T, RR, MODE>, dim3(R, parts), dim3(th), 0, stream, (const TY*)y, ldy, ycol0, \
+                 (const TZ*)z, ldz, zcol0, w, eps, (T*)out, ldo, n)
+  if (runs == 1) NF_PN(1); else if (runs == 2) NF_PN(2); else NF_PN(4);
+#undef NF_PN
+  return 1;
+}
+
 template <typename T>
 __global__ void rms_norm_slice_kernel(const T* __restrict__ x, int ldx, int col0, int n,
                                       const float* __restrict__ w, float eps, T* __restrict__ out, int ldo) {
@@ -229,6 +310,25 @@ __global__ void add_row_vector_kernel(float* __restrict__ h, const float* __rest
 
 // out[t, hd * n + i] = v[hd, t, i] * sigmoid(g[t, gcol0 + hd * n + i]):  v is laid out head by head
 // ([heads, T, n], what a batched product over heads leaves), out token by token.
+// Runs of four (n a multiple of 4, rows aligned), one a thread: see heads_sigmoid_gate_kernel.
+template <typename T>
+__global__ void __launch_bounds__(256)
+heads_sigmoid_gate_vec_kernel(const T* __restrict__ v, const T* __restrict__ g, int ldg, int gcol0, T* __restrict__ out, int rows,
+                              int heads, int n, int per_head) {
+  const int t = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * 4;
+  chain_release_if_small();
+  chain_wait(v, g);
+  if (c >= heads * n) return;
+  const int hd = c / n, i = c - hd * n;
+  float x[4], gv[4];
+  load4(v + ((size_t)hd * rows + t) * n + i, x);
+  if (per_head) gv[0] = gv[1] = gv[2] = gv[3] = to_float(g[(size_t)t * ldg + gcol0 + hd]);
+  else load4(g + (size_t)t * ldg + gcol0 + c, gv);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) x[e] *= 1.f / (1.f + expf(-gv[e]));
+  store4(out + (size_t)t * heads * n + c, x);
+}
+
 template <typename T>
 __global__ void heads_sigmoid_gate_kernel(const T* __restrict__ v, const T* __restrict__ g, int ldg, int gcol0,
                                           T* __restrict__ out, int rows, int heads, int n, int per_head) {
@@ -340,6 +440,9 @@ extern "C" int nf_rms_norm_slice(const void* x, int ldx, int col0, int n, const 
                                  int ldo, int R, int dtype, cudaStream_t stream) {
   if (R == 0) return 0;
   NF_REQUIRE(R > 0 && n > 0 && col0 >= 0 && col0 + n <= ldx && ldo >= n, "rms_norm_slice: bad sizes");
+  if (dtype == kF32 ? part_norm_vec<float, float, float, 0>(x, ldx, col0, nullptr, 0, 0, w, eps, out, ldo, R, n, 1, stream)
+                    : part_norm_vec<__nv_bfloat16, float, __nv_bfloat16, 0>(x, ldx, col0, nullptr, 0, 0, w, eps, out, ldo, R, n, 1, stream))
+    return check_launch("rms_norm_slice");
   if (dtype == kF32)
     launch_chained(rms_norm_slice_kernel<float>, dim3(R), dim3(128), 0, stream, (const float*)x, ldx, col0, n, w, eps, (float*)out, ldo);
   else
@@ -351,6 +454,9 @@ extern "C" int nf_gated_group_rmsnorm(const float* y, const void* z, int ldz, in
                                       void* out, int R, int inner, int parts, int dtype, cudaStream_t stream) {
   if (R == 0) return 0;
   NF_REQUIRE(R > 0 && inner > 0 && parts > 0 && inner % parts == 0, "gated_group_rmsnorm: %d does not split into %d parts", inner, parts);
+  if (dtype == kF32 ? part_norm_vec<float, float, float, 1>(y, inner, 0, z, ldz, zcol0, w, eps, out, inner, R, inner / parts, parts, stream)
+                    : part_norm_vec<float, __nv_bfloat16, __nv_bfloat16, 1>(y, inner, 0, z, ldz, zcol0, w, eps, out, inner, R, inner / parts, parts, stream))
+    return check_launch("gated_group_rmsnorm");
   const size_t smem = (size_t)(inner / parts) * sizeof(float);
   NF_REQUIRE(smem <= 160 * 1024, "gated_group_rmsnorm: a part of %d does not fit shared memory", inner / parts);
 #define NF_GN(T)                                                                                               \
@@ -376,6 +482,13 @@ extern "C" int nf_heads_sigmoid_gate(const void* v, const void* g, int ldg, int 
                                      int n, int per_head, int dtype, cudaStream_t stream) {
   if (R == 0) return 0;
   NF_REQUIRE(heads > 0 && n > 0 && gcol0 >= 0 && gcol0 + heads * (per_head ? 1 : n) <= ldg, "heads_sigmoid_gate: bad sizes");
+  const size_t el = dtype == kF32 ? 4 : 2;
+  if (n % 4 == 0 && runs_of_four(v, el, 0, 0) && runs_of_four(out, el, 0, 0) && (per_head || runs_of_four(g, el, ldg, gcol0))) {
+    const dim3 grid(R, (heads * n / 4 + 255) / 256);
+    if (dtype == kF32) launch_chained(heads_sigmoid_gate_vec_kernel<float>, grid, dim3(256), 0, stream, (const float*)v, (const float*)g, ldg, gcol0, (float*)out, R, heads, n, per_head);
+    else launch_chained(heads_sigmoid_gate_vec_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, (const __nv_bfloat16*)v, (const __nv_bfloat16*)g, ldg, gcol0, (__nv_bfloat16*)out, R, heads, n, per_head);
+    return check_launch("heads_sigmoid_gate");
+  }
   if (dtype == kF32)
     launch_chained(heads_sigmoid_gate_kernel<float>, dim3(R), dim3(256), 0, stream, (const float*)v, (const float*)g, ldg, gcol0, (float*)out, R, heads, n, per_head);
   else
@@ -428,6 +541,56 @@ __global__ void scaled_norm_add_kernel(float* __restrict__ h, const TD* __restri
     v += hr[i];
     hr[i] = v;
     if (out) out[(size_t)r * hidden + i] = from_float<TO>(v);
+  }
+}
+
+// The wide form (see part_norm_vec_kernel): runs of four, the row in registers, weights before the wait.
+template <typename TD, typename TO, int R>
+__global__ void __launch_bounds__(512)
+scaled_norm_add_vec_kernel(float* __restrict__ h, const TD* __restrict__ delta, const float* __restrict__ bias,
+                           const float* __restrict__ w, const float* __restrict__ ls, float eps, TO* __restrict__ out, int hidden) {
+  __shared__ float red[33];
+  const int r = blockIdx.x;
+  chain_release_if_small();
+  float wk[R][4], lk[R][4], bk[R][4], d[R][4], v[R][4];
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { wk[c][e] = lk[c][e] = 1.f; bk[c][e] = d[c][e] = v[c][e] = 0.f; }
+    if (i < hidden) {
+      load4(w + i, wk[c]);
+      if (ls) load4(ls + i, lk[c]);
+      if (bias) load4(bias + i, bk[c]);
+    }
+  }
+  chain_wait(h, delta);
+  float* hr = h + (size_t)r * hidden;
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+    if (i < hidden) {
+      load4(delta + (size_t)r * hidden + i, d[c]);
+      load4(hr + i, v[c]);
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < R; ++c)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      d[c][e] += bk[c][e];
+      ss += d[c][e] * d[c][e];
+    }
+  const float inv = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+    if (i >= hidden) continue;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[c][e] += d[c][e] * inv * wk[c][e] * lk[c][e];
+    store4(hr + i, v[c]);
+    if (out) store4(out + (size_t)r * hidden + i, v[c]);
   }
 }
 
@@ -498,6 +661,56 @@ __global__ void mean_of_rmsnorms_kernel(NormedInputs in, float eps, float* __res
   }
 }
 
+// The wide form for two inputs: both rows in registers, their sums of squares meet in one pass over the block.
+template <typename T, int R>
+__global__ void __launch_bounds__(512)
+mean_of_two_rmsnorms_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, const float* __restrict__ wa,
+                                const float* __restrict__ wb, float eps, float* __restrict__ out, int hidden) {
+  __shared__ float2 red[17];
+  const int r = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  chain_release_if_small();
+  float wk[2][R][4], v[2][R][4];
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) wk[0][c][e] = wk[1][c][e] = v[0][c][e] = v[1][c][e] = 0.f;
+    if (i < hidden) { load4(wa + i, wk[0][c]); load4(wb + i, wk[1][c]); }
+  }
+  chain_wait(a, b);
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+    if (i < hidden) { load4(a + (size_t)r * hidden + i, v[0][c]); load4(b + (size_t)r * hidden + i, v[1][c]); }
+  }
+  float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+  for (int c = 0; c < R; ++c)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { s0 += v[0][c][e] * v[0][c][e]; s1 += v[1][c][e] * v[1][c][e]; }
+  s0 = warp_sum(s0);
+  s1 = warp_sum(s1);
+  if (lane == 0) red[warp] = make_float2(s0, s1);
+  __syncthreads();
+  if (warp == 0) {
+    const float2 x = lane < nwarp ? red[lane] : make_float2(0.f, 0.f);
+    s0 = warp_sum(x.x);
+    s1 = warp_sum(x.y);
+    if (lane == 0) red[16] = make_float2(s0, s1);
+  }
+  __syncthreads();
+  const float i0 = rsqrtf(red[16].x / (float)hidden + eps), i1 = rsqrtf(red[16].y / (float)hidden + eps);
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+    if (i >= hidden) continue;
+    float o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = (v[0][c][e] * i0 * wk[0][c][e] + v[1][c][e] * i1 * wk[1][c][e]) * 0.5f;
+    store4(out + (size_t)r * hidden + i, o);
+  }
+}
+
 // out[t, c] = y[t, c] / rms(part of c) * w[c] * act(z[t, zcol0 + c]): an RMS norm in `parts` equal
 // parts of a row (w null: no weight), then a gate.  act 0: silu, 1: sigmoid.  y is float32; z is of the
 // output's type or float32 sums.
@@ -539,11 +752,20 @@ extern "C" int nf_scaled_norm_add(float* h, const void* delta, int delta_dtype, 
   if (R == 0) return 0;
   NF_REQUIRE(R > 0 && hidden > 0 && h && delta && w, "scaled_norm_add: bad arguments R=%d hidden=%d", R, hidden);
   const dim3 grid(R), block(norm_threads(hidden));
-#define NF_SNA(TD, TO) \
-  launch_chained(scaled_norm_add_kernel<TD, TO>, grid, block, 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden)
+  const bool vec = hidden % 4 == 0 && hidden <= 8192 && runs_of_four(h, 4, 0, 0) && runs_of_four(delta, delta_dtype == kF32 ? 4 : 2, 0, 0) &&
+                   runs_of_four(out, out_dtype == kF32 ? 4 : 2, 0, 0) && ((uintptr_t)w | (uintptr_t)ls | (uintptr_t)bias) % 16 == 0;
+  const int units = hidden / 4, runs = units <= 512 ? 1 : (units <= 1024 ? 2 : 4), th = ((units + runs - 1) / runs + 31) / 32 * 32;
+#define NF_SNV(TD, TO, RR) \
+  launch_chained(scaled_norm_add_vec_kernel<TD, TO, RR>, grid, dim3(th), 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden)
+#define NF_SNA(TD, TO)                                                                                                     \
+  do {                                                                                                                     \
+    if (vec) { if (runs == 1) NF_SNV(TD, TO, 1); else if (runs == 2) NF_SNV(TD, TO, 2); else NF_SNV(TD, TO, 4); }          \
+    else launch_chained(scaled_norm_add_kernel<TD, TO>, grid, block, 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden); \
+  } while (0)
   if (delta_dtype == kF32) { if (out_dtype == kF32) NF_SNA(float, float); else NF_SNA(float, __nv_bfloat16); }
   else { if (out_dtype == kF32) NF_SNA(__nv_bfloat16, float); else NF_SNA(__nv_bfloat16, __nv_bfloat16); }
 #undef NF_SNA
+#undef NF_SNV
   return check_launch("scaled_norm_add");
 }
 
@@ -577,6 +799,16 @@ extern "C" int nf_mean_of_rmsnorms(const void* const* xs, const float* const* ws
   NormedInputs in;
   in.n = n;
   for (int m = 0; m < 4; ++m) { in.x[m] = m < n ? xs[m] : nullptr; in.w[m] = m < n ? ws[m] : nullptr; }
+  const size_t el = dtype == kF32 ? 4 : 2;
+  if (n == 2 && hidden % 4 == 0 && hidden <= 4096 && runs_of_four(in.x[0], el, 0, 0) && runs_of_four(in.x[1], el, 0, 0) &&
+      ((uintptr_t)in.w[0] | (uintptr_t)in.w[1] | (uintptr_t)out) % 16 == 0) {
+    const int units = hidden / 4, runs = units <= 512 ? 1 : 2, th = ((units + runs - 1) / runs + 31) / 32 * 32;
+#define NF_MR(TT, RR) launch_chained(mean_of_two_rmsnorms_vec_kernel<TT, RR>, dim3(R), dim3(th), 0, stream, (const TT*)in.x[0], (const TT*)in.x[1], in.w[0], in.w[1], eps, out, hidden)
+    if (dtype == kF32) { if (runs == 1) NF_MR(float, 1); else NF_MR(float, 2); }
+    else { if (runs == 1) NF_MR(__nv_bfloat16, 1); else NF_MR(__nv_bfloat16, 2); }
+#undef NF_MR
+    return check_launch("mean_of_rmsnorms");
+  }
   if (dtype == kF32) launch_chained(mean_of_rmsnorms_kernel<float>, dim3(R), dim3(norm_threads(hidden)), 0, stream, in, eps, out, hidden);
   else launch_chained(mean_of_rmsnorms_kernel<__nv_bfloat16>, dim3(R), dim3(norm_threads(hidden)), 0, stream, in, eps, out, hidden);
   return check_launch("mean_of_rmsnorms");
@@ -591,7 +823,13 @@ extern "C" int nf_group_rmsnorm_gate(const float* y, const void* z, int ldz, int
              "group_rmsnorm_gate: %d does not split into %d parts", inner, parts);
   NF_REQUIRE(act == 0 || act == 1, "group_rmsnorm_gate: gate %d (0 silu, 1 sigmoid)", act);
   NF_REQUIRE(z_dtype == dtype || z_dtype == kF32, "group_rmsnorm_gate: the gate is of the output's type or float32");
-  const dim3 grid(R, parts), block(norm_threads(inner / parts));
+  const int n = inner / parts;
+#define NF_GV(TZ, T) (act == 1 ? part_norm_vec<float, TZ, T, 3>(y, inner, 0, z, ldz, zcol0, w, eps, out, inner, R, n, parts, stream) \
+                               : part_norm_vec<float, TZ, T, 2>(y, inner, 0, z, ldz, zcol0, w, eps, out, inner, R, n, parts, stream))
+  if (dtype == kF32 ? NF_GV(float, float) : (z_dtype == kF32 ? NF_GV(float, __nv_bfloat16) : NF_GV(__nv_bfloat16, __nv_bfloat16)))
+    return check_launch("group_rmsnorm_gate");
+#undef NF_GV
+  const dim3 grid(R, parts), block(norm_threads(n));
   if (dtype == kF32) launch_chained(group_rmsnorm_gate_kernel<float>, grid, block, 0, stream, y, (const float*)z, ldz, zcol0, w, eps, (float*)out, inner, parts, act);
   else if (z_dtype == kF32) launch_chained(group_rmsnorm_gate_kernel<__nv_bfloat16, float>, grid, block, 0, stream, y, (const float*)z, ldz, zcol0, w, eps, (__nv_bfloat16*)out, inner, parts, act);
   else launch_chained(group_rmsnorm_gate_kernel<__nv_bfloat16>, grid, block, 0, stream, y, (const __nv_bfloat16*)z, ldz, zcol0, w, eps, (__nv_bfloat16*)out, inner, parts, act);
