@@ -1,6 +1,7 @@
 // The recurrences  S_t = a_t S_{t-1} + w_t k_t v_t^T,  o_t = S_t^T q_t  of prompt portions on tensor cores (bfloat16
 // engines): the selective scan of ssm.cu (k = B, q = C, v = x, w = dt) and the linear attention of
-// linear_attention.cu (w = 1, a constant decay a head).  S is V x D per head, float32.
+// linear_attention.cu (w = 1, a constant decay a head); and the gated delta rule of delta_rule.cu (further down).
+// S is V x D per head, float32.
 //
 // Walking the rows one by one is bound by the chain from row to row (a prompt of 2,048 tokens, 64 heads of
 // 128 x 64: 771 us, about 1 % of the arithmetic's own time).  Over a chunk of Q rows the recurrence is three products:
@@ -18,11 +19,12 @@
 // products whose weight is at least 2^-16 of the leading one are all taken (three where one operand is bfloat16, six
 // where both are float32) with float32 sums.
 //
-// One prompt of 2,048 tokens, before (row by row) and after: scan of 64 heads of 128 x 64 755 -> 172 us (the outputs take
-// 100 of it, the chunks' states 45, the chain over 16 chunks, which moves 67 MB, the rest), 32 heads of 64 x 64 394 -> 75;
-// linear attention of 16 heads of 128 x 128 with float32 q, k and v 499 -> 205 (six products each: bound by the tensor
-// pipe), 64 x 128 with bfloat16 values 347 -> 93.  Chunks of 128 rows halve the states' traffic where the operands are
-// bfloat16; with three parts of each operand in shared memory 64 rows fit.
+// One prompt of 2,048 tokens, before (row by row) and after: scan of 64 heads of 128 x 64 755 -> 177 us (the outputs take
+// 100 of it, the chunks' states 45, the chain over 16 chunks, which moves 67 MB, the rest), 32 heads of 64 x 64 394 -> 77;
+// linear attention of 16 heads of 128 x 128 with float32 q, k and v 499 -> 218 (six products each: bound by the tensor
+// pipe), 64 x 128 with bfloat16 values 347 -> 97; the delta rule of 16 heads of 128 x 128 431 -> 198, of 8 heads
+// 421 -> 138.  Chunks of 128 rows halve the states' traffic where the operands are bfloat16; with three parts of each
+// operand in shared memory 64 rows fit.
 #define NF_CHAIN_CLASS 2
 #include "common.cuh"
 
@@ -32,18 +34,20 @@ namespace {
 constexpr int kCrThreads = 256;
 constexpr int kCrPad = 8;               // elements of padding a shared-memory row: ldmatrix then meets no bank conflict
 
-enum CrMode : int { kCrScan = 0, kCrDecay = 1 };
+enum CrMode : int { kCrScan = 0, kCrDecay = 1, kCrDelta = 2 };
 
 struct CrArgs {
   const __nv_bfloat16 *q, *k, *v;       // rows of `ld` elements, columns from q0, k0, v0 on (q and k: a head group's D)
   int ld, q0, k0, v0;
   const float* prepared;                // float32 q and k [T, 2, H, D] instead
   int v_silu;
-  int H, heads_per_group;
+  int H, heads_per_group, V;
   const __nv_bfloat16* dt;              // scan: raw step sizes
   int ld_dt, dt0;
   const float *dt_bias, *A_log, *skip;
   const float* decay;                   // a decay a head
+  const float* values;                  // delta rule: float32 values [T, H * V] (u), and [T, H, 4] of (decay, factor on
+  const float* gates;                   // the row's key, factor on its output, -)
   const int* chunks;                    // [n][3]: segment, first row, rows
   const int* runs;                      // [m][3]: segment, first chunk, chunks
   const int* seg_slot;
@@ -68,8 +72,8 @@ __device__ __forceinline__ void cr_mma(float (&c)[4], const unsigned (&a)[4], un
 // The tensor cores cut a sum off where float32 arithmetic rounds it, always towards zero: over the 48 products that a sum
 // of 128 terms in parts takes this adds up (linear attention of 64 rows, D = 128: 9.7e-7 of the results, row by row in
 // float32 1.6e-7).  So the products of one step of 16 terms start from zero, the smallest parts first, and their sum is
-// added to the running one in float32: 1.5e-7, and over 2,048 rows 3.0e-7 against 8.0e-7 row by row.  It costs a scan 3 %, 128 x 128 with
-// six products a step 16 %.
+// added to the running one in float32: 1.5e-7, and over 2,048 rows 3.0e-7 against 8.0e-7 row by row.  It
+// costs a scan 3 %, 128 x 128 with six products a step 16 %.
 template <int N>
 __device__ __forceinline__ void cr_zero(float (&t)[N][4]) {
 #pragma unroll
@@ -116,9 +120,13 @@ __device__ __forceinline__ void cr_row_gates(const CrArgs& a, int head, int row,
     const float v = to_float(a.dt[(size_t)row * a.ld_dt + a.dt0 + head]) + a.dt_bias[head];
     weight = v > 20.f ? v : log1pf(expf(v));
     decay = expf(-expf(a.A_log[head]) * weight);
-  } else {
+  } else if (MODE == kCrDecay) {
     decay = a.decay[head];
     weight = 1.f;
+  } else {
+    const float2 g = *reinterpret_cast<const float2*>(a.gates + ((size_t)row * a.H + head) * 4);
+    decay = g.x;
+    weight = g.y;
   }
 }
 
@@ -143,6 +151,21 @@ __device__ __forceinline__ void cr_load_qk(const CrArgs& a, bool keys, int head,
       cr_store_parts<PARTS>(dst + r * (D + kCrPad) + c, plane, x);
     }
   }
+}
+// Row t's decays inside its sixteen, from the chunk's in `decay`: the product up to it, after it, and to every later row
+// (diag[t / 16][t % 16][u]; 0 before it).
+template <int N>
+__device__ __forceinline__ void cr_decay_table(const float* decay, int t, float* upto, float* after, float (&diag)[N][16][17]) {
+  const int b = t & ~15;
+  float run = 1.f;
+  for (int s = b; s <= t; ++s) run *= decay[s];
+  upto[t] = run;
+  run = 1.f;
+  for (int u = 0; u < 16; ++u) {
+    if (b + u > t) run *= decay[b + u];
+    diag[t >> 4][t & 15][u] = b + u < t ? 0.f : run;
+  }
+  after[t] = run;
 }
 __device__ __forceinline__ float cr_value(float x, int silu) { return silu ? x / (1.f + expf(-x)) : x; }
 
@@ -300,8 +323,8 @@ chunk_chain_kernel(const CrArgs args, int entries) {
 }
 
 // ---- (3) a chunk's outputs --------------------------------------------------------------------------------------------
-// A warp owns 16 rows and V / (8 / (Q / 16)) columns.  Shared memory holds the queries throughout; beside them first the
-// state at the chunk's start, then the keys and values, SUB rows at a time.
+// A CTA has V of a head's a.V columns, a warp 16 rows and V / (8 / (Q / 16)) columns.  Shared memory holds the queries
+// throughout; beside them first the state at the chunk's start, then the keys and values, SUB rows at a time.
 template <int D, int V, int Q, int SUB, int QKP, int VP, int MODE>
 __global__ void __launch_bounds__(kCrThreads, 2)
 chunk_output_kernel(const CrArgs args) {
@@ -315,16 +338,16 @@ chunk_output_kernel(const CrArgs args) {
   __nv_bfloat16* Vs = Ks + (size_t)QKP * SUB * KS;                           // [VP][SUB][VS]
   __shared__ float s_decay[Q], s_weight[Q], s_upto[Q], s_after[Q];
   __shared__ float s_diag[WQ][16][17];                                       // [.][s][t]: D(s, t) inside a sixteen
-  const int chunk = blockIdx.x, head = blockIdx.y;
+  const int chunk = blockIdx.x, head = blockIdx.y, tile0 = blockIdx.z * V;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   CrArgs a = args;
-  chain_wait(a.q, a.k, a.v, a.dt, a.prepared, a.chunk_state);
+  chain_wait(a.q, a.k, a.v, a.dt, a.prepared, a.chunk_state, a.values, a.gates);
   const int row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
   if (threadIdx.x < Q)
     cr_row_gates<MODE>(a, head, row0 + threadIdx.x, (int)threadIdx.x < live, s_decay[threadIdx.x], s_weight[threadIdx.x]);
   cr_load_qk<D, QKP>(a, false, head, row0, Q, live, Qs, (size_t)Q * KS);
   {
-    const float* src = a.chunk_state + ((size_t)chunk * a.H + head) * V * D;
+    const float* src = a.chunk_state + (((size_t)chunk * a.H + head) * a.V + tile0) * D;
     for (int i = threadIdx.x; i < V * (D / 4); i += kCrThreads) {
       const int r = i / (D / 4), c = (i - r * (D / 4)) * 4;
       float x[4];
@@ -333,18 +356,7 @@ chunk_output_kernel(const CrArgs args) {
     }
   }
   __syncthreads();
-  if (threadIdx.x < Q) {                 // a row's decays inside its sixteen: up to it, after it, from it to later rows
-    const int t = threadIdx.x, b = t & ~15;
-    float run = 1.f;
-    for (int s = b; s <= t; ++s) run *= s_decay[s];
-    s_upto[t] = run;
-    run = 1.f;
-    for (int u = 0; u < 16; ++u) {
-      if (b + u > t) run *= s_decay[b + u];
-      s_diag[t >> 4][t & 15][u] = b + u < t ? 0.f : run;
-    }
-    s_after[t] = run;
-  }
+  if (threadIdx.x < Q) cr_decay_table(s_decay, threadIdx.x, s_upto, s_after, s_diag);
   __syncthreads();
   const int rb = warp % WQ, n0 = (warp / WQ) * (V / WV);       // this warp's sixteen and first column
   const int g = lane >> 2, t4 = lane & 3, mat = lane >> 3, r8 = lane & 7;
@@ -399,7 +411,7 @@ chunk_output_kernel(const CrArgs args) {
     __syncthreads();                     // everyone is done with the state, or with the rows before
     cr_load_qk<D, QKP>(a, true, head, row0 + sub, SUB, live - sub, Ks, (size_t)SUB * KS);
     {
-      const __nv_bfloat16* src = a.v + a.v0 + (size_t)head * V;
+      const __nv_bfloat16* src = a.v + a.v0 + (size_t)head * a.V + tile0;
       if (VP == 1) {
         for (int i = threadIdx.x; i < SUB * (V / 8); i += kCrThreads) {
           const int r = i / (V / 8), c = (i - r * (V / 8)) * 8;
@@ -412,9 +424,13 @@ chunk_output_kernel(const CrArgs args) {
           const int r = i / (V / 4), c = (i - r * (V / 4)) * 4;
           float x[4] = {0.f, 0.f, 0.f, 0.f};
           if (sub + r < live) {
-            load4(src + (size_t)(row0 + sub + r) * a.ld + c, x);
+            if (MODE == kCrDelta) {
+              load4(a.values + (size_t)(row0 + sub + r) * a.H * a.V + (size_t)head * a.V + tile0 + c, x);
+            } else {
+              load4(src + (size_t)(row0 + sub + r) * a.ld + c, x);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) x[e] = cr_value(x[e], a.v_silu);
+              for (int e = 0; e < 4; ++e) x[e] = cr_value(x[e], a.v_silu);
+            }
           }
           cr_store_parts<VP>(Vs + r * VS + c, (size_t)SUB * VS, x);
         }
@@ -511,12 +527,13 @@ chunk_output_kernel(const CrArgs args) {
     const int r = rb * 16 + g + 8 * hi;
     if (r >= live) continue;
     const size_t row = (size_t)(row0 + r);
-    const float skip = MODE == kCrScan ? a.skip[head] : 0.f;
-    float* dst = a.out + row * a.H * V + (size_t)head * V + n0 + t4 * 2;
-    const __nv_bfloat16* x = a.v + row * a.ld + a.v0 + (size_t)head * V + n0 + t4 * 2;
+    const float skip = MODE == kCrScan ? a.skip[head] : 0.f, factor = MODE == kCrDelta ? a.gates[(row * a.H + head) * 4 + 2] : 1.f;
+    float* dst = a.out + row * a.H * a.V + (size_t)head * a.V + tile0 + n0 + t4 * 2;
+    const __nv_bfloat16* x = a.v + row * a.ld + a.v0 + (size_t)head * a.V + tile0 + n0 + t4 * 2;
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       float y0 = acc[n][2 * hi], y1 = acc[n][2 * hi + 1];
+      if (MODE == kCrDelta) { y0 *= factor; y1 *= factor; }
       if (MODE == kCrScan) {
         const __nv_bfloat162 xx = *reinterpret_cast<const __nv_bfloat162*>(x + n * 8);
         y0 = fmaf(skip, __low2float(xx), y0);
@@ -527,24 +544,392 @@ chunk_output_kernel(const CrArgs args) {
   }
 }
 
-template <int D, int V, int Q, int SUB, int QKP, int VP, int MODE>
-static int launch_chunks(const CrArgs& a, int n_chunks, int n_runs, cudaStream_t stream) {
-  constexpr size_t smem1 = ((size_t)QKP * Q * (D + kCrPad) + 3 * (size_t)Q * (V + kCrPad)) * 2;
-  constexpr size_t part_s = 3 * (size_t)V * (D + kCrPad), part_kv = (size_t)QKP * SUB * (D + kCrPad) + (size_t)VP * SUB * (V + kCrPad);
-  constexpr size_t smem3 = ((size_t)QKP * Q * (D + kCrPad) + (part_s > part_kv ? part_s : part_kv)) * 2;
-  static_assert(smem1 <= 220 * 1024 && smem3 <= 220 * 1024, "shared memory of a chunk");
+// VT: columns of a head an output CTA has.
+template <int D, int VT, int Q, int SUB, int QKP, int VP, int MODE>
+int launch_outputs(const CrArgs& a, int n_chunks, cudaStream_t stream) {
+  constexpr size_t part_s = 3 * (size_t)VT * (D + kCrPad), part_kv = (size_t)QKP * SUB * (D + kCrPad) + (size_t)VP * SUB * (VT + kCrPad);
+  constexpr size_t smem = ((size_t)QKP * Q * (D + kCrPad) + (part_s > part_kv ? part_s : part_kv)) * 2;
+  static_assert(smem <= 220 * 1024, "shared memory of a chunk");
   static bool set = false;                // (the attribute is the function's: set twice by two threads, it is the same)
   if (!set) {
-    cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<D, V, Q, QKP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(chunk_output_kernel<D, V, Q, SUB, QKP, VP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
-    NF_REQUIRE(e == cudaSuccess, "chunk recurrence: cannot have %zu and %zu bytes of shared memory: %s", smem1, smem3, cudaGetErrorString(e));
+    const cudaError_t e = cudaFuncSetAttribute(chunk_output_kernel<D, VT, Q, SUB, QKP, VP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    NF_REQUIRE(e == cudaSuccess, "chunk recurrence: cannot have %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     set = true;
   }
-  launch_chained(chunk_state_kernel<D, V, Q, QKP, MODE>, dim3(n_chunks, a.H), dim3(kCrThreads), smem1, stream, a);
-  launch_chained(chunk_chain_kernel, dim3(n_runs, a.H, (V * D / 4 + kCrThreads - 1) / kCrThreads), dim3(kCrThreads), 0, stream, a, V * D);
-  launch_chained(chunk_output_kernel<D, V, Q, SUB, QKP, VP, MODE>, dim3(n_chunks, a.H), dim3(kCrThreads), smem3, stream, a);
+  launch_chained(chunk_output_kernel<D, VT, Q, SUB, QKP, VP, MODE>, dim3(n_chunks, a.H, a.V / VT), dim3(kCrThreads), smem, stream, a);
   return check_launch("chunk_recurrence");
+}
+
+template <int D, int V, int VT, int Q, int SUB, int QKP, int VP, int MODE>
+int launch_chunks(const CrArgs& a, int n_chunks, int n_runs, cudaStream_t stream) {
+  constexpr size_t smem = ((size_t)QKP * Q * (D + kCrPad) + 3 * (size_t)Q * (V + kCrPad)) * 2;
+  static_assert(smem <= 220 * 1024, "shared memory of a chunk");
+  static bool set = false;
+  if (!set) {
+    const cudaError_t e = cudaFuncSetAttribute(chunk_state_kernel<D, V, Q, QKP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    NF_REQUIRE(e == cudaSuccess, "chunk recurrence: cannot have %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    set = true;
+  }
+  launch_chained(chunk_state_kernel<D, V, Q, QKP, MODE>, dim3(n_chunks, a.H), dim3(kCrThreads), smem, stream, a);
+  launch_chained(chunk_chain_kernel, dim3(n_runs, a.H, (V * D / 4 + kCrThreads - 1) / kCrThreads), dim3(kCrThreads), 0, stream, a, V * D);
+  return launch_outputs<D, VT, Q, SUB, QKP, VP, MODE>(a, n_chunks, stream);
+}
+
+// ---- the gated delta rule -------------------------------------------------------------------------------------------
+//
+//   S <- g_t S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T;  o_t = S^T q_t        (k_t, q_t unit vectors)
+//
+// Over a chunk, with A_t and D(s, t) as above and the chunk's inner products m_ts = beta_t D(s, t) k_s.k_t (s < t), the u
+// solve a triangular system: U = T (V - [A_t k_t^T S_0]_t), T = (1 + m)^-1 diag(beta).  T depends on the keys and gates
+// alone, so (1) makes it for all chunks and heads at once; (2) walks the chunks, a CTA a head and 16 value columns, with
+// three products a chunk; (3) is the output kernel above with U for the values.  What the rows' norms scale (k and q are
+// bfloat16 numbers over their norm) goes into the float32 factors, so that products with k and q stay exact.
+
+constexpr int kDcRows = 64;               // rows a chunk
+
+struct DcArgs {
+  const __nv_bfloat16 *qkv, *ab;
+  int ld, q0, k0, v0, ld_ab, a0, b0;
+  const float *dt_bias, *A_log;
+  float q_scale;
+  int H, heads_per_group, V;
+  const int *chunks, *runs, *seg_slot;
+  float* state;
+  long slot_stride;
+  __nv_bfloat16* solve;                   // T as three parts: [n][H][3][64][64]
+  float* coef;                            // [n][H][64][2]: A_t / |k_t|, D(t, end) / |k_t|
+  float* gates;                           // [T][H][4]: g, 1 / |k|, q_scale / |q|, 0
+  float* chunk_state;                     // [n][H][V][D]
+  float* chunk_decay;                     // [n][H]
+  float* u;                               // [T][H * V]
+};
+
+__device__ __forceinline__ void cr_cp16(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(cr_smem(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cr_ldm2t(unsigned addr, unsigned& r0, unsigned& r1) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr) : "memory");
+}
+
+template <int D>
+__global__ void __launch_bounds__(kCrThreads)
+delta_chunk_solve_kernel(const DcArgs args) {
+  constexpr int Q = kDcRows, KS = D + kCrPad, MS = Q + 4;
+  extern __shared__ __align__(16) unsigned char cr_raw[];
+  __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(cr_raw);              // [Q][KS]
+  float* M = reinterpret_cast<float*>(Ks + Q * KS);                          // [Q][MS]
+  __shared__ float s_g[Q], s_beta[Q], s_ik[Q], s_upto[Q], s_after[Q];
+  __shared__ float s_diag[Q / 16][16][17];
+  const int chunk = blockIdx.x, head = blockIdx.y, grp = head / args.heads_per_group;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  DcArgs a = args;
+  chain_wait(a.qkv, a.ab);
+  const int row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
+  const __nv_bfloat16* kr = a.qkv + a.k0 + (size_t)grp * D;
+  const __nv_bfloat16* qr = a.qkv + a.q0 + (size_t)grp * D;
+  for (int r = warp; r < Q; r += kCrThreads / 32) {      // a warp a row: the key to shared memory, both norms
+    float kk = 0.f, qq = 0.f;
+    for (int c = lane * 4; c < D; c += 128) {
+      float k[4] = {0.f, 0.f, 0.f, 0.f}, q[4] = {0.f, 0.f, 0.f, 0.f};
+      uint2 raw = make_uint2(0, 0);
+      if (r < live) {
+        raw = *reinterpret_cast<const uint2*>(kr + (size_t)(row0 + r) * a.ld + c);
+        load4(reinterpret_cast<const __nv_bfloat16*>(&raw), k);
+        load4(qr + (size_t)(row0 + r) * a.ld + c, q);
+      }
+      *reinterpret_cast<uint2*>(Ks + r * KS + c) = raw;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { kk = fmaf(k[e], k[e], kk); qq = fmaf(q[e], q[e], qq); }
+    }
+    kk = warp_sum(kk);
+    qq = warp_sum(qq);
+    if (lane == 0) {
+      float g = 1.f, beta = 0.f, ik = 0.f;
+      if (r < live) {
+        const __nv_bfloat16* ab = a.ab + (size_t)(row0 + r) * a.ld_ab;
+        const float x = to_float(ab[a.a0 + head]) + a.dt_bias[head];
+        g = expf(-expf(a.A_log[head]) * (fmaxf(x, 0.f) + log1pf(expf(-fabsf(x)))));
+        beta = 1.f / (1.f + expf(-to_float(ab[a.b0 + head])));
+        ik = 1.f / sqrtf(kk + 1e-6f);
+        *reinterpret_cast<float4*>(a.gates + ((size_t)(row0 + r) * a.H + head) * 4) = make_float4(g, ik, a.q_scale / sqrtf(qq + 1e-6f), 0.f);
+      }
+      s_g[r] = g;
+      s_beta[r] = beta;
+      s_ik[r] = ik;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < Q) cr_decay_table(s_g, threadIdx.x, s_upto, s_after, s_diag);
+  __syncthreads();
+  if (threadIdx.x < Q) {
+    const int t = threadIdx.x, b = t >> 4;
+    float before = 1.f, past = s_after[t];
+    for (int x = 0; x < b; ++x) before *= s_upto[16 * x + 15];
+    for (int x = b + 1; x < Q / 16; ++x) past *= s_upto[16 * x + 15];
+    const float upto = before * s_upto[t];
+    *reinterpret_cast<float2*>(a.coef + (((size_t)chunk * a.H + head) * Q + t) * 2) = make_float2(upto * s_ik[t], past * s_ik[t]);
+    if (t == Q - 1) a.chunk_decay[(size_t)chunk * a.H + head] = upto;
+  }
+  {  // m_ts: warp w has rows 16 (w % 4) .. and columns 32 (w / 4) ..
+    const int rb = warp & 3, c0 = (warp >> 2) * 32, g = lane >> 2, t4 = lane & 3, mat = lane >> 3, r8 = lane & 7;
+    float p[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) p[n][e] = 0.f;
+    const unsigned ka = cr_smem(Ks + (rb * 16 + (mat & 1) * 8 + r8) * KS + (mat >> 1) * 8);
+    const unsigned kb = cr_smem(Ks + (c0 + (mat >> 1) * 8 + r8) * KS + (mat & 1) * 8);
+    if (c0 <= rb * 16 + 15) {
+#pragma unroll
+      for (int k0 = 0; k0 < D; k0 += 16) {
+        unsigned A[4], B[4];
+        cr_ldm4(ka + k0 * 2, A);
+#pragma unroll
+        for (int n = 0; n < 4; n += 2) {
+          cr_ldm4(kb + (n * 8 * KS + k0) * 2, B);
+          float t[2][4];
+          cr_zero(t);
+          cr_mma(t[0], A, B[0], B[1]);
+          cr_mma(t[1], A, B[2], B[3]);
+          cr_add(p[n], t[0]);
+          cr_add(p[n + 1], t[1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int s = c0 + n * 8 + t4 * 2 + (e & 1), t = rb * 16 + g + (e >> 1) * 8, b = s >> 4;
+        float d = 0.f;
+        if (s < t) {
+          if (b == rb) d = s_diag[rb][s & 15][t & 15];
+          else {
+            d = s_after[s] * s_upto[t];
+            for (int x = b + 1; x < rb; ++x) d *= s_upto[16 * x + 15];
+          }
+          d *= s_ik[s] * s_ik[t] * s_beta[t];
+        }
+        M[t * MS + s] = d == 0.f ? 0.f : d * p[n][e];
+      }
+  }
+  __syncthreads();
+  if (threadIdx.x < Q) {                 // thread j: column j of (1 + m)^-1 by forward substitution, times beta_j
+    const int j = threadIdx.x;
+    const float beta = s_beta[j];
+    __nv_bfloat16* out = a.solve + ((size_t)chunk * a.H + head) * 3 * Q * Q + j;
+    float x[Q];
+#pragma unroll
+    for (int t = 0; t < Q; ++t) x[t] = 0.f;
+#pragma unroll
+    for (int t = 0; t < Q; ++t) {
+      float r[4] = {t == j ? 1.f : 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int s = 0; s < t; s += 4) {
+        float m[4];
+        load4(M + t * MS + s, m);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[e] = fmaf(-m[e], x[s + e], r[e]);
+      }
+      x[t] = (r[0] + r[1]) + (r[2] + r[3]);
+      float v = x[t] * beta;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(v);
+        out[(size_t)(i * Q + t) * Q] = h;
+        v = isinf(__bfloat162float(h)) || isnan(__bfloat162float(h)) ? 0.f : v - __bfloat162float(h);
+      }
+    }
+  }
+}
+
+// Two numbers' three parts to a place of three planes.
+__device__ __forceinline__ void cr_put3(__nv_bfloat16* dst, size_t plane, float x, float y) {
+  unsigned p[3];
+  cr_split<3>(x, y, p);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) *reinterpret_cast<unsigned*>(dst + i * plane) = p[i];
+}
+
+template <int D>
+__global__ void __launch_bounds__(kCrThreads)
+delta_chunk_chain_kernel(const DcArgs args) {
+  constexpr int Q = kDcRows, KS = D + kCrPad, TS = Q + kCrPad, XS = 16 + kCrPad, NT = D / 64;
+  extern __shared__ __align__(16) unsigned char cr_raw[];
+  __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(cr_raw);              // [2][Q][KS]
+  __nv_bfloat16* Ts = Ks + 2 * Q * KS;                                       // [2][3][Q][TS]
+  __nv_bfloat16* Vs = Ts + 2 * 3 * Q * TS;                                   // [2][Q][16]
+  __nv_bfloat16* Ss = Vs + 2 * Q * 16;                                       // [3][16][KS]
+  __nv_bfloat16* Xs = Ss + 3 * 16 * KS;                                      // [3][Q][XS]
+  __nv_bfloat16* Us = Xs + 3 * Q * XS;                                       // [3][Q][XS]
+  float* coef = reinterpret_cast<float*>(Us + 3 * Q * XS);                   // [2][Q][2]
+  const int run = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * 16, grp = head / args.heads_per_group;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t4 = lane & 3, mat = lane >> 3, r8 = lane & 7;
+  DcArgs a = args;
+  chain_wait(a.qkv, a.solve, a.coef, a.chunk_decay, a.state);
+  const int seg = a.runs[3 * run], first = a.runs[3 * run + 1], n = a.runs[3 * run + 2];
+  auto fetch = [&](int c) {
+    if (c < n) {
+      const int b = c & 1, chunk = first + c, row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
+      const __nv_bfloat16* kr = a.qkv + (size_t)row0 * a.ld + a.k0 + (size_t)grp * D;
+#pragma unroll
+      for (int i = threadIdx.x; i < Q * (D / 8); i += kCrThreads) {
+        const int r = i / (D / 8), col = (i % (D / 8)) * 8;
+        cr_cp16(Ks + (b * Q + r) * KS + col, r < live ? kr + (size_t)r * a.ld + col : a.qkv, r < live);
+      }
+      const __nv_bfloat16* tp = a.solve + ((size_t)chunk * a.H + head) * 3 * Q * Q;
+#pragma unroll
+      for (int i = threadIdx.x; i < 3 * Q * (Q / 8); i += kCrThreads)
+        cr_cp16(Ts + (b * 3 * Q + i / (Q / 8)) * TS + (i % (Q / 8)) * 8, tp + (size_t)i * 8, true);
+      if (threadIdx.x < Q * 2) {
+        const int r = threadIdx.x >> 1, col = (threadIdx.x & 1) * 8;
+        const __nv_bfloat16* vr = a.qkv + (size_t)(row0 + r) * a.ld + a.v0 + (size_t)head * a.V + v0 + col;
+        cr_cp16(Vs + (b * Q + r) * 16 + col, r < live ? vr : a.qkv, r < live);
+      } else if (threadIdx.x < Q * 2 + Q / 2) {
+        const int i = threadIdx.x - Q * 2;
+        cr_cp16(coef + b * Q * 2 + i * 4, a.coef + ((size_t)chunk * a.H + head) * Q * 2 + i * 4, true);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0);
+  // the state: value columns g and g + 8 of the sixteen, key dimensions of this warp's D / 8
+  const int d0 = warp * (D / 8) + 2 * t4;
+  float* slot = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + ((size_t)head * a.V + v0 + g) * D + d0;
+  float s[NT][4];
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    const float2 x = *reinterpret_cast<const float2*>(slot + 8 * i), y = *reinterpret_cast<const float2*>(slot + 8 * D + 8 * i);
+    s[i][0] = x.x; s[i][1] = x.y; s[i][2] = y.x; s[i][3] = y.y;
+    cr_put3(Ss + g * KS + d0 + 8 * i, 16 * KS, s[i][0], s[i][1]);
+    cr_put3(Ss + (g + 8) * KS + d0 + 8 * i, 16 * KS, s[i][2], s[i][3]);
+  }
+  const int mt = warp & 3, nt = warp >> 2;           // rows 16 mt .., columns 8 nt .. of the first two products
+  const int tr = mt * 16 + g, col = nt * 8 + 2 * t4;
+  for (int c = 0; c < n; ++c) {
+    const int b = c & 1, chunk = first + c, row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
+    const float decay = a.chunk_decay[(size_t)chunk * a.H + head];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                 // the chunk is in; the state's parts are written; the rest is free
+    fetch(c + 1);
+    float* start = a.chunk_state + (((size_t)chunk * a.H + head) * a.V + v0 + g) * D + d0;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      *reinterpret_cast<float2*>(start + 8 * i) = make_float2(s[i][0], s[i][1]);
+      *reinterpret_cast<float2*>(start + 8 * D + 8 * i) = make_float2(s[i][2], s[i][3]);
+    }
+    const __nv_bfloat16* K = Ks + b * Q * KS;
+    {  // x_t = v_t - A_t S^T k_t
+      float y[1][4];
+      cr_zero(y);
+      const unsigned ka = cr_smem(K + (mt * 16 + (mat & 1) * 8 + r8) * KS + (mat >> 1) * 8);
+      const unsigned sb = cr_smem(Ss + (nt * 8 + r8) * KS + mat * 8);
+#pragma unroll
+      for (int k0 = 0; k0 < D; k0 += 32) {
+        unsigned A0[4], A1[4], B[4];
+        cr_ldm4(ka + k0 * 2, A0);
+        cr_ldm4(ka + (k0 + 16) * 2, A1);
+        float t[2][4];
+        cr_zero(t);
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+          cr_ldm4(sb + (i * 16 * KS + k0) * 2, B);
+          cr_mma(t[0], A0, B[0], B[1]);
+          cr_mma(t[1], A1, B[2], B[3]);
+        }
+        cr_add(y[0], t[0]);
+        cr_add(y[0], t[1]);
+      }
+      const float c0 = coef[(b * Q + tr) * 2], c1 = coef[(b * Q + tr + 8) * 2];
+      const __nv_bfloat162 va = *reinterpret_cast<const __nv_bfloat162*>(Vs + (b * Q + tr) * 16 + col);
+      const __nv_bfloat162 vb = *reinterpret_cast<const __nv_bfloat162*>(Vs + (b * Q + tr + 8) * 16 + col);
+      cr_put3(Xs + tr * XS + col, Q * XS, __low2float(va) - c0 * y[0][0], __high2float(va) - c0 * y[0][1]);
+      cr_put3(Xs + (tr + 8) * XS + col, Q * XS, __low2float(vb) - c1 * y[0][2], __high2float(vb) - c1 * y[0][3]);
+    }
+    __syncthreads();
+    {  // U = T X
+      float u[1][4];
+      cr_zero(u);
+      const unsigned ta = cr_smem(Ts + (b * 3 * Q + mt * 16 + (mat & 1) * 8 + r8) * TS + (mat >> 1) * 8);
+      const unsigned xb = cr_smem(Xs + (lane & 15) * XS + nt * 8);
+      for (int ks = 0; ks <= mt; ++ks) {
+        unsigned A[3][4], B[3][2];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          cr_ldm4(ta + (i * Q * TS + ks * 16) * 2, A[i]);
+          cr_ldm2t(xb + ((i * Q + ks * 16) * XS) * 2, B[i][0], B[i][1]);
+        }
+        float t[3][4];                             // (three chains side by side: this is the walk from chunk to chunk)
+        cr_zero(t);
+        cr_mma(t[2], A[0], B[2][0], B[2][1]);
+        cr_mma(t[1], A[0], B[1][0], B[1][1]);
+        cr_mma(t[0], A[0], B[0][0], B[0][1]);
+        cr_mma(t[2], A[1], B[1][0], B[1][1]);
+        cr_mma(t[1], A[1], B[0][0], B[0][1]);
+        cr_mma(t[2], A[2], B[0][0], B[0][1]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) u[0][e] += t[0][e] + (t[1][e] + t[2][e]);
+      }
+      float* dst = a.u + (size_t)(row0 + tr) * a.H * a.V + (size_t)head * a.V + v0 + col;
+      if (tr < live) *reinterpret_cast<float2*>(dst) = make_float2(u[0][0], u[0][1]);
+      if (tr + 8 < live) *reinterpret_cast<float2*>(dst + (size_t)8 * a.H * a.V) = make_float2(u[0][2], u[0][3]);
+      const float c0 = coef[(b * Q + tr) * 2 + 1], c1 = coef[(b * Q + tr + 8) * 2 + 1];
+      cr_put3(Us + tr * XS + col, Q * XS, u[0][0] * c0, u[0][1] * c0);
+      cr_put3(Us + (tr + 8) * XS + col, Q * XS, u[0][2] * c1, u[0][3] * c1);
+    }
+    __syncthreads();
+    {  // S = A S + sum_t D(t, end) u_t k_t^T
+      float w[NT][4];
+      cr_zero(w);
+      const unsigned ua = cr_smem(Us + ((mat >> 1) * 8 + r8) * XS + (mat & 1) * 8);
+      const unsigned kb = cr_smem(K + ((mat & 1) * 8 + r8) * KS + warp * (D / 8) + (NT == 2 ? (mat >> 1) * 8 : 0));
+#pragma unroll
+      for (int ks = 0; ks < Q / 16; ++ks) {
+        unsigned A[3][4], B[4];
+        float t[NT][4];
+        cr_zero(t);
+        cr_ldm4t(kb + ks * 16 * KS * 2, B);          // (one column tile: the third and fourth repeat the first two)
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+          cr_ldm4t(ua + (i * Q + ks * 16) * XS * 2, A[i]);
+#pragma unroll
+          for (int j = 0; j < NT; ++j) cr_mma(t[j], A[i], B[2 * j], B[2 * j + 1]);
+        }
+#pragma unroll
+        for (int j = 0; j < NT; ++j) cr_add(w[j], t[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[j][e] = fmaf(decay, s[j][e], w[j][e]);
+        cr_put3(Ss + g * KS + d0 + 8 * j, 16 * KS, s[j][0], s[j][1]);
+        cr_put3(Ss + (g + 8) * KS + d0 + 8 * j, 16 * KS, s[j][2], s[j][3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    *reinterpret_cast<float2*>(slot + 8 * i) = make_float2(s[i][0], s[i][1]);
+    *reinterpret_cast<float2*>(slot + 8 * D + 8 * i) = make_float2(s[i][2], s[i][3]);
+  }
+}
+
+template <int D>
+int launch_delta(const DcArgs& d, const CrArgs& a, int n_chunks, int n_runs, cudaStream_t stream) {
+  constexpr int Q = kDcRows;
+  constexpr size_t smem1 = (size_t)Q * (D + kCrPad) * 2 + (size_t)Q * (Q + 4) * 4;
+  constexpr size_t smem2 = ((size_t)2 * Q * (D + kCrPad) + 6 * Q * (Q + kCrPad) + 2 * Q * 16 + 3 * 16 * (D + kCrPad) + 6 * Q * (16 + kCrPad)) * 2 + 2 * Q * 2 * 4;
+  static bool set = false;
+  if (!set) {
+    cudaError_t e = cudaFuncSetAttribute(delta_chunk_solve_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_chain_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    NF_REQUIRE(e == cudaSuccess, "delta rule: cannot have %zu and %zu bytes of shared memory: %s", smem1, smem2, cudaGetErrorString(e));
+    set = true;
+  }
+  launch_chained(delta_chunk_solve_kernel<D>, dim3(n_chunks, d.H), dim3(kCrThreads), smem1, stream, d);
+  launch_chained(delta_chunk_chain_kernel<D>, dim3(n_runs, d.H, d.V / 16), dim3(kCrThreads), smem2, stream, d);
+  return launch_outputs<D, 64, Q, 32, 1, 3, kCrDelta>(a, n_chunks, stream);
 }
 
 }  // namespace
@@ -573,14 +958,14 @@ extern "C" int nf_chunk_scan(const void* xbc, int ldx, int x0, int b0, int c0, c
   CrArgs a = {};
   a.q = a.k = a.v = (const __nv_bfloat16*)xbc;
   a.ld = ldx; a.q0 = c0; a.k0 = b0; a.v0 = x0;
-  a.H = heads; a.heads_per_group = heads / groups;
+  a.H = heads; a.heads_per_group = heads / groups; a.V = P;
   a.dt = (const __nv_bfloat16*)dt; a.ld_dt = ld_dt; a.dt0 = dt0;
   a.dt_bias = dt_bias; a.A_log = A_log; a.skip = skip;
   a.chunks = chunks; a.runs = runs; a.seg_slot = seg_slot;
   a.state = state; a.slot_stride = (long)slot_stride;
   a.chunk_state = chunk_state; a.chunk_decay = chunk_decay; a.out = out;
-  if (N == 128) return launch_chunks<128, 64, 128, 64, 1, 1, kCrScan>(a, n_chunks, n_runs, stream);
-  return launch_chunks<64, 64, 128, 64, 1, 1, kCrScan>(a, n_chunks, n_runs, stream);
+  if (N == 128) return launch_chunks<128, 64, 64, 128, 64, 1, 1, kCrScan>(a, n_chunks, n_runs, stream);
+  return launch_chunks<64, 64, 64, 128, 64, 1, 1, kCrScan>(a, n_chunks, n_runs, stream);
 }
 
 // Linear attention of the listed chunks: prepared float32 [T, 2, H, D] (q and k), v bfloat16 [T, ld] from v0 on
@@ -596,13 +981,45 @@ extern "C" int nf_chunk_linear_attention(const float* prepared, const void* v, i
   CrArgs a = {};
   a.v = (const __nv_bfloat16*)v;
   a.ld = ld; a.v0 = v0; a.v_silu = v_silu; a.prepared = prepared;
-  a.H = H; a.heads_per_group = 1;
+  a.H = H; a.heads_per_group = 1; a.V = V;
   a.decay = decay;
   a.chunks = chunks; a.runs = runs; a.seg_slot = seg_slot;
   a.state = state; a.slot_stride = (long)slot_stride;
   a.chunk_state = chunk_state; a.chunk_decay = chunk_decay; a.out = out;
-  if (D == 128) return v_silu ? launch_chunks<128, 128, 64, 32, 3, 3, kCrDecay>(a, n_chunks, n_runs, stream)
-                              : launch_chunks<128, 128, 64, 32, 3, 1, kCrDecay>(a, n_chunks, n_runs, stream);
-  return v_silu ? launch_chunks<64, 128, 64, 32, 3, 3, kCrDecay>(a, n_chunks, n_runs, stream)
-                : launch_chunks<64, 128, 64, 32, 3, 1, kCrDecay>(a, n_chunks, n_runs, stream);
+  if (D == 128) return v_silu ? launch_chunks<128, 128, 64, 64, 32, 3, 3, kCrDecay>(a, n_chunks, n_runs, stream)
+                              : launch_chunks<128, 128, 64, 64, 32, 3, 1, kCrDecay>(a, n_chunks, n_runs, stream);
+  return v_silu ? launch_chunks<64, 128, 128, 64, 32, 3, 3, kCrDecay>(a, n_chunks, n_runs, stream)
+                : launch_chunks<64, 128, 128, 64, 32, 3, 1, kCrDecay>(a, n_chunks, n_runs, stream);
+}
+
+extern "C" int nf_chunk_delta_rule_rows(int D, int V) { return (D == 64 || D == 128) && V % 64 == 0 ? kDcRows : 0; }
+
+// The gated delta rule of the listed chunks; arguments as nf_delta_rule's (bfloat16).  Scratch: solve bfloat16
+// [n_chunks, H, 3, 64, 64], coef float32 [n_chunks, H, 64, 2], gates float32 [T, H, 4], u float32 [T, H * V], chunk_state
+// float32 [n_chunks, H, V, D], chunk_decay float32 [n_chunks, H].
+extern "C" int nf_chunk_delta_rule(const void* qkv, int ld, int q0, int k0, int v0, const void* ab, int ld_ab, int a0, int b0,
+                                   const float* dt_bias, const float* A_log, float q_scale, float* state, long long slot_stride,
+                                   const int* seg_slot, const int* chunks, int n_chunks, const int* runs, int n_runs, void* solve,
+                                   float* coef, float* gates, float* u, float* chunk_state, float* chunk_decay, float* out,
+                                   int H, int G, int D, int V, cudaStream_t stream) {
+  if (n_chunks == 0) return 0;
+  NF_REQUIRE(nf_chunk_delta_rule_rows(D, V) > 0 && G > 0 && H > 0 && H % G == 0 && H <= 65535, "chunk delta rule: sizes D=%d V=%d H=%d G=%d", D, V, H, G);
+  NF_REQUIRE(ld % 8 == 0 && q0 % 8 == 0 && k0 % 8 == 0 && v0 % 8 == 0 && (uintptr_t)qkv % 16 == 0 && slot_stride % 4 == 0 &&
+             (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0, "chunk delta rule: rows and states must be 16-byte aligned");
+  DcArgs d = {};
+  d.qkv = (const __nv_bfloat16*)qkv; d.ab = (const __nv_bfloat16*)ab;
+  d.ld = ld; d.q0 = q0; d.k0 = k0; d.v0 = v0; d.ld_ab = ld_ab; d.a0 = a0; d.b0 = b0;
+  d.dt_bias = dt_bias; d.A_log = A_log; d.q_scale = q_scale;
+  d.H = H; d.heads_per_group = H / G; d.V = V;
+  d.chunks = chunks; d.runs = runs; d.seg_slot = seg_slot;
+  d.state = state; d.slot_stride = (long)slot_stride;
+  d.solve = (__nv_bfloat16*)solve; d.coef = coef; d.gates = gates;
+  d.chunk_state = chunk_state; d.chunk_decay = chunk_decay; d.u = u;
+  CrArgs a = {};
+  a.q = a.k = d.qkv;
+  a.ld = ld; a.q0 = q0; a.k0 = k0;
+  a.H = H; a.heads_per_group = H / G; a.V = V;
+  a.values = u; a.gates = gates;
+  a.chunks = chunks; a.chunk_state = chunk_state; a.out = out;
+  return D == 128 ? launch_delta<128>(d, a, n_chunks, n_runs, stream) : launch_delta<64>(d, a, n_chunks, n_runs, stream);
 }

@@ -48,13 +48,13 @@ __global__ void __launch_bounds__(32 * kDrChunk)
 delta_rule_prepare_kernel(const T* __restrict__ qkv, int ld, int q_col0, int k_col0, const T* __restrict__ ab, int ld_ab,
                           int a_col0, int b_col0, const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                           float q_scale, const int* __restrict__ seg_row0, float* __restrict__ vectors,
-                          float* __restrict__ records, int H, int G, int D, int DP) {
+                          float* __restrict__ records, int H, int G, int D, int DP, int skip_rows) {
   extern __shared__ float sm[];                  // [chunk][q: D + 1 | k: D + 1], dots [chunk][2][chunk], decays [chunk][heads a group]
   const int c0 = blockIdx.x * kDrChunk, seg = blockIdx.y, grp = blockIdx.z;
   chain_release_if_small();
   chain_wait(qkv, ab);
   const int row0 = seg_row0[seg], n = min(kDrChunk, seg_row0[seg + 1] - row0 - c0);
-  if (n <= 0) return;
+  if (n <= 0 || seg_row0[seg + 1] - row0 >= skip_rows) return;      // (a segment that chunk_recurrence.cu serves)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = H / G;
   const int stride = D + 1;
   float* sq = sm;
@@ -167,7 +167,7 @@ template <typename T, int EPL, int LANES, int CP>        // D <= EPL * LANES
 __global__ void __launch_bounds__(kDrThreads / CP)
 delta_rule_chunks_kernel(const float* __restrict__ vectors, const float* __restrict__ records, const T* __restrict__ vsrc,
                          int ld, int v_col0, float* __restrict__ state, long slot_stride, const int* __restrict__ seg_row0,
-                         const int* __restrict__ seg_slot, float* __restrict__ out, int H, int G, int D, int V) {
+                         const int* __restrict__ seg_slot, float* __restrict__ out, int H, int G, int D, int V, int skip_rows) {
   constexpr int NTH = kDrThreads / CP;
   constexpr int COLS = kDrThreads / LANES;
   constexpr int DPAD = EPL * LANES;
@@ -185,7 +185,7 @@ delta_rule_chunks_kernel(const float* __restrict__ vectors, const float* __restr
   chain_release_if_small();
   chain_wait(vectors, records, vsrc, state);
   const int row0 = seg_row0[seg], rows = seg_row0[seg + 1] - row0;
-  if (rows <= 0) return;
+  if (rows <= 0 || rows >= skip_rows) return;
   float* slot = state + (size_t)seg_slot[seg] * slot_stride + (size_t)head * V * D;
   const bool vec = D % 4 == 0 && slot_stride % 4 == 0 && (uintptr_t)state % 16 == 0;
   float S[CP][EPL];
@@ -386,7 +386,8 @@ template <typename T>
 static int run_delta_rule(const void* qkv, int ld, int q0, int k0, int v0, const void* ab, int ld_ab, int a0, int b0,
                           const float* dt_bias, const float* A_log, float q_scale, float* state, long slot_stride,
                           const int* seg_row0, const int* seg_slot, float* vectors, float* records, float* out, int S,
-                          int max_rows, int H, int G, int D, int DP, int V, cudaStream_t stream) {
+                          int max_rows, int H, int G, int D, int DP, int V, int skip_rows, cudaStream_t stream) {
+  if (skip_rows < max_rows) max_rows = skip_rows;
   if (max_rows == 1) {
     const int vec_in = D % 4 == 0 && ld % 4 == 0 && q0 % 4 == 0 && k0 % 4 == 0 && (uintptr_t)qkv % (4 * sizeof(T)) == 0;
 #define NF_DR(E, L)                                                                                                   \
@@ -400,7 +401,7 @@ static int run_delta_rule(const void* qkv, int ld, int q0, int k0, int v0, const
   const size_t smem = (size_t)(2 * kDrChunk * (D + 1) + 2 * kDrChunk * kDrChunk + kDrChunk * (H / G)) * sizeof(float);
   launch_chained(delta_rule_prepare_kernel<T>, dim3((max_rows + kDrChunk - 1) / kDrChunk, S, G), dim3(32 * kDrChunk), smem, stream,
                  (const T*)qkv, ld, q0, k0, (const T*)ab, ld_ab, a0, b0, dt_bias, A_log, q_scale, seg_row0, vectors, records,
-                 H, G, D, DP);
+                 H, G, D, DP, skip_rows);
   if (int rc = check_launch("delta_rule_prepare")) return rc;
   // two columns a thread once there are CTAs enough (one prompt of 2,048 tokens, heads of 128 x 128: with 16 heads 433 us
   // with one column, 523 with two; with 28 heads 675 and 581)
@@ -410,7 +411,7 @@ static int run_delta_rule(const void* qkv, int ld, int q0, int k0, int v0, const
 #define NF_DR_C(E, L, CC)                                                                                             \
   launch_chained(delta_rule_chunks_kernel<T, E, L, CC>, dim3(S, H, (V + kDrThreads / L - 1) / (kDrThreads / L)),      \
                  dim3(kDrThreads / CC), 0, stream, (const float*)vectors, (const float*)records, (const T*)qkv, ld, v0, \
-                 state, slot_stride, seg_row0, seg_slot, out, H, G, D, V)
+                 state, slot_stride, seg_row0, seg_slot, out, H, G, D, V, skip_rows)
   if (D <= 32) NF_DR(4, 8); else if (D <= 64) NF_DR(8, 8); else if (D <= 128) NF_DR(16, 8); else NF_DR(16, 16);
 #undef NF_DR
   return check_launch("delta_rule_chunks");
@@ -428,12 +429,14 @@ extern "C" int nf_delta_rule_row(int D) { return D <= 32 ? 32 : (D <= 64 ? 64 : 
 // qkv [T, ld]: q (G x D) at q0, k (G x D) at k0, v (H x V) at v0; ab [T, ld_ab]: a (H) at a0, b (H) at b0; all of
 // `dtype`.  dt_bias, A_log float32 [H]; state float32, slot s at state + s * slot_stride: [H][V][D]; out float32
 // [T, H * V].  max_rows: the most rows a segment brings; 1: steps of single rows.  Otherwise vectors float32
-// [T, G, 2, nf_delta_rule_row(D)] and records float32 [T, H, nf_delta_rule_record()] are scratch.
+// [T, G, 2, nf_delta_rule_row(D)] and records float32 [T, H, nf_delta_rule_record()] are scratch.  skip_rows > 0: segments
+// of that many rows or more are left alone.
 extern "C" int nf_delta_rule(const void* qkv, int ld, int q0, int k0, int v0, const void* ab, int ld_ab, int a0, int b0,
                              const float* dt_bias, const float* A_log, float q_scale, float* state, long long slot_stride,
                              const int* seg_row0, const int* seg_slot, float* vectors, float* records, float* out, int S,
-                             int max_rows, int H, int G, int D, int V, int dtype, cudaStream_t stream) {
+                             int max_rows, int H, int G, int D, int V, int dtype, int skip_rows, cudaStream_t stream) {
   if (S == 0) return 0;
+  if (skip_rows <= 0) skip_rows = 0x7fffffff;
   NF_REQUIRE(S > 0 && max_rows > 0 && H > 0 && G > 0 && H % G == 0 && D > 0 && D <= 256 && V > 0, "delta rule: bad sizes S=%d H=%d G=%d D=%d V=%d", S, H, G, D, V);
   NF_REQUIRE(H <= 65535 && (V + 7) / 8 <= 65535 && S <= 65535 && H / G <= 512, "delta rule: too many heads, columns or requests");
   NF_REQUIRE(q0 >= 0 && k0 >= 0 && v0 >= 0 && q0 + G * D <= ld && k0 + G * D <= ld && v0 + H * V <= ld && a0 >= 0 && b0 >= 0 &&
@@ -441,6 +444,6 @@ extern "C" int nf_delta_rule(const void* qkv, int ld, int q0, int k0, int v0, co
   const int DP = nf_delta_rule_row(D);
   NF_REQUIRE(max_rows == 1 || (vectors && records && (uintptr_t)vectors % 16 == 0 && (uintptr_t)records % 16 == 0), "delta rule: prompt portions need their scratch");
   if (dtype == kF32)
-    return run_delta_rule<float>(qkv, ld, q0, k0, v0, ab, ld_ab, a0, b0, dt_bias, A_log, q_scale, state, (long)slot_stride, seg_row0, seg_slot, vectors, records, out, S, max_rows, H, G, D, DP, V, stream);
-  return run_delta_rule<__nv_bfloat16>(qkv, ld, q0, k0, v0, ab, ld_ab, a0, b0, dt_bias, A_log, q_scale, state, (long)slot_stride, seg_row0, seg_slot, vectors, records, out, S, max_rows, H, G, D, DP, V, stream);
+    return run_delta_rule<float>(qkv, ld, q0, k0, v0, ab, ld_ab, a0, b0, dt_bias, A_log, q_scale, state, (long)slot_stride, seg_row0, seg_slot, vectors, records, out, S, max_rows, H, G, D, DP, V, skip_rows, stream);
+  return run_delta_rule<__nv_bfloat16>(qkv, ld, q0, k0, v0, ab, ld_ab, a0, b0, dt_bias, A_log, q_scale, state, (long)slot_stride, seg_row0, seg_slot, vectors, records, out, S, max_rows, H, G, D, DP, V, skip_rows, stream);
 }

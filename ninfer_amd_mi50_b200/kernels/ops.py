@@ -46,9 +46,11 @@ TUNING = {
     # recurrences over prompt portions: segments of at least this many rows run as chunks on tensor cores (three launches
     # that fill the device with a few hundred rows, where walking the rows costs the same each: the selective scan of 64
     # heads takes 44 us against 55 at 128 rows, 32 against 32 at 64; linear attention of 16 heads of 128 x 128 takes 62
-    # against 134 at 512 rows, 57 against 44 at 128); a huge number leaves every row to the kernels that walk them
+    # against 134 at 512 rows, 57 against 44 at 128; the delta rule of 16 heads of 128 x 128 takes 68 against 118 at 512
+    # rows, 52 against 40 at 128); a huge number leaves every row to the kernels that walk them
     "chunk_scan_min_rows": 96,
     "chunk_linear_min_rows": 192,
+    "chunk_delta_min_rows": 192,
     "chunk_recurrence_max_mb": 512,      # scratch for the chunks' states; a longer step's chunks run group after group
     "qkv_rope_fused": True,       # few bfloat16 rows: rotation and cache append in the projection's epilogue
     "router_tensor_min_rows": 128,   # router logits of more rows than this use tensor cores
@@ -1523,15 +1525,17 @@ LINEAR_ATTENTION_MAX_DIM = 256
 
 
 def _recurrence_chunks(ctx, src: torch.Tensor, columns: Sequence[int], state: torch.Tensor, state_off: int, heads: int, D: int,
-                       V: int, scan: bool):
+                       V: int, kind: str):
     """What `ctx.recurrence_chunks` says for a step whose long segments the chunked recurrences (chunk_recurrence.cu) are to
     serve, else None: bfloat16 rows and states that can be read 16 bytes at a time, sizes that those kernels have, and a
     segment of at least as many rows as `TUNING` says."""
-    min_rows = TUNING["chunk_scan_min_rows" if scan else "chunk_linear_min_rows"]
+    min_rows = TUNING[f"chunk_{kind}_min_rows"]
     if (src.dtype != torch.bfloat16 or getattr(ctx, "seg_len_host", None) is None or getattr(ctx, "graph_mode", False)
             or ctx.max_rows_per_seg < min_rows or not hasattr(ctx, "recurrence_chunks")):
         return None
-    rows = int(_lib.load().nf_chunk_recurrence_rows(c_int(D), c_int(V), c_int(1 if scan else 0)))
+    lib = _lib.load()
+    rows = int(lib.nf_chunk_delta_rule_rows(c_int(D), c_int(V)) if kind == "delta" else
+               lib.nf_chunk_recurrence_rows(c_int(D), c_int(V), c_int(1 if kind == "scan" else 0)))
     if (not rows or any(c % 8 for c in columns) or src.shape[1] % 8 or src.data_ptr() % 16 or state.stride(0) % 4
             or (state.data_ptr() + 4 * state_off) % 16):
         return None
@@ -1573,7 +1577,7 @@ def decay_linear_attention(src: torch.Tensor, q_col0: int, k_col0: int, v_col0: 
         _lib.call("nf_linear_attention_prepare", _p(src), c_int(src.shape[1]), c_int(q_col0), c_int(k_col0),
                   _p(inv_freq) if rot else None, c_int(rot), c_float(k_scale), c_int(1 if silu else 0), _p(ctx.positions),
                   _p(prepared), c_int(T), c_int(heads), c_int(D), c_int(_dt(src)), c_float(q_scale), _stream())
-    chunked = (_recurrence_chunks(ctx, src, (v_col0,), state, 0, heads, D, V, scan=False)
+    chunked = (_recurrence_chunks(ctx, src, (v_col0,), state, 0, heads, D, V, "linear")
                if prepared is not None and gates is None else None)
     skip_rows = 0
     if chunked is not None:
@@ -1637,15 +1641,32 @@ def delta_rule(qkv: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, ab: tor
     T = qkv.shape[0]
     out = torch.empty((T, heads * V), dtype=torch.float32, device=qkv.device)
     vectors = records = None
-    rows = int(ctx.max_rows_per_seg)
+    rows, skip_rows = int(ctx.max_rows_per_seg), 0
+    state_p = c_void_p(state.data_ptr() + 4 * state_off)
+    chunked = _recurrence_chunks(ctx, qkv, (q_col0, k_col0, v_col0), state, state_off, heads, D, V, "delta")
+    if chunked is not None:
+        lists, others = chunked
+        states, decays = _chunk_scratch(lists, heads, D, V, qkv.device)
+        n = states.shape[0]
+        floats = lambda *shape: torch.empty(shape, dtype=torch.float32, device=qkv.device)
+        solve = torch.empty((n, heads, 3, 64, 64), dtype=qkv.dtype, device=qkv.device)
+        coef, gates, u = floats(n, heads, 64, 2), floats(T, heads, 4), floats(T, heads * V)
+        for chunks, n, runs, m in lists:
+            _lib.call("nf_chunk_delta_rule", _p(qkv), c_int(qkv.shape[1]), c_int(q_col0), c_int(k_col0), c_int(v_col0), _p(ab),
+                      c_int(ab.shape[1]), c_int(a_col0), c_int(b_col0), _p(dt_bias), _p(A_log), c_float(q_scale), state_p,
+                      c_longlong(state.stride(0)), _p(ctx.seg_slot), _p(chunks), c_int(n), _p(runs), c_int(m), _p(solve), _p(coef),
+                      _p(gates), _p(u), _p(states), _p(decays), _p(out), c_int(heads), c_int(kv_heads), c_int(D), c_int(V), _stream())
+        if not others:
+            return out
+        skip_rows = TUNING["chunk_delta_min_rows"]
     if rows > 1:
         vectors = torch.empty((T, kv_heads, 2, int(_lib.load().nf_delta_rule_row(c_int(D)))), dtype=torch.float32, device=qkv.device)
         records = torch.empty((T, heads, int(_lib.load().nf_delta_rule_record())), dtype=torch.float32, device=qkv.device)
     _lib.call("nf_delta_rule", _p(qkv), c_int(qkv.shape[1]), c_int(q_col0), c_int(k_col0), c_int(v_col0), _p(ab),
               c_int(ab.shape[1]), c_int(a_col0), c_int(b_col0), _p(dt_bias), _p(A_log), c_float(q_scale),
-              c_void_p(state.data_ptr() + 4 * state_off), c_longlong(state.stride(0)), _p(ctx.seg_row0), _p(ctx.seg_slot),
+              state_p, c_longlong(state.stride(0)), _p(ctx.seg_row0), _p(ctx.seg_slot),
               _p(vectors), _p(records), _p(out), c_int(ctx.S), c_int(rows), c_int(heads), c_int(kv_heads), c_int(D), c_int(V),
-              c_int(_dt(qkv)), _stream())
+              c_int(_dt(qkv)), c_int(skip_rows), _stream())
     return out
 
 
@@ -1688,7 +1709,7 @@ def ssd_scan(xbc: torch.Tensor, x_col0: int, b_col0: int, c_col0: int, dt_src: t
     T = xbc.shape[0]
     y = torch.empty((T, heads * P), dtype=torch.float32, device=xbc.device)
     state_p = c_void_p(state.data_ptr() + 4 * state_off)
-    chunked = _recurrence_chunks(ctx, xbc, (x_col0, b_col0, c_col0), state, state_off, heads, N, P, scan=True)
+    chunked = _recurrence_chunks(ctx, xbc, (x_col0, b_col0, c_col0), state, state_off, heads, N, P, "scan")
     skip_rows = 0
     if chunked is not None:
         lists, others = chunked
