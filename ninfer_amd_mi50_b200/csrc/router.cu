@@ -13,34 +13,87 @@
 
 namespace nf {
 
+// n numbers of x as float32 into shared memory, 16 bytes of x a thread and step where alignment allows, several steps in
+// flight: the rows are one trip to L2.
+template <typename T>
+__device__ __forceinline__ void stage_rows(const T* __restrict__ x, float* xs, int total) {
+  constexpr int PER = 16 / (int)sizeof(T);
+  if (((uintptr_t)x & 15) == 0 && total % PER == 0) {
+    constexpr int U = 8;
+    const int step = blockDim.x * PER;
+    for (int i0 = threadIdx.x * PER; i0 < total; i0 += step * U) {
+      uint4 raw[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * step < total) raw[u] = *reinterpret_cast<const uint4*>(x + i0 + u * step);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (i0 + u * step < total) {
+          const T* v = reinterpret_cast<const T*>(&raw[u]);
+          // 16-byte stores: scalar ones would put the lanes 8 floats apart, 8 to a bank
+#pragma unroll
+          for (int j = 0; j < PER; j += 4)
+            *reinterpret_cast<float4*>(xs + i0 + u * step + j) =
+                make_float4(to_float(v[j]), to_float(v[j + 1]), to_float(v[j + 2]), to_float(v[j + 3]));
+        }
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < total; i += blockDim.x) xs[i] = to_float(x[i]);
+  }
+}
+
 // Router logits: out[t, e] = x[t] . wr[e] in float32, for the E router rows and `extra`
 // further rows (the shared expert's gate).  A block takes TT tokens and 8 rows of wr, one
 // warp per row; a lane sums its strided share of the hidden dimension and the warp adds the
 // 32 shares in a fixed tree, so the value for (t, e) is the same whatever TT is and
-// whatever else is in the batch.
-template <typename T, int TT>
+// whatever else is in the batch.  PRE > 0: rows of up to 128 PRE numbers; a lane's share of the
+// weights, which no kernel writes, is in registers before the wait for x (the sums run in lane_dot's
+// order exactly).
+template <typename T, int TT, int PRE>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const T* __restrict__ x, const float* __restrict__ wr, int n_tokens, int hidden,
                      int rows, float* __restrict__ out) {
-  extern __shared__ float xs[];        // [TT][hidden]
+  extern __shared__ __align__(16) float xs[];        // [TT][hidden]
   const int t0 = blockIdx.y * TT;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nt = min(TT, n_tokens - t0);
-  for (int i = threadIdx.x; i < nt * hidden; i += blockDim.x) {
-    const int tt = i / hidden, c = i - tt * hidden;
-    xs[tt * hidden + c] = to_float(x[(size_t)(t0 + tt) * hidden + c]);
-  }
-  __syncthreads();
   const int e = blockIdx.x * 8 + warp;
+  const float* w = wr + (size_t)min(e, rows - 1) * hidden;
+  float4 wv[PRE > 0 ? PRE : 1];
+  if constexpr (PRE > 0) {
+#pragma unroll
+    for (int j = 0; j < PRE; ++j) {
+      const int i = lane * 4 + j * 128;
+      wv[j] = i < hidden ? *reinterpret_cast<const float4*>(w + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  chain_wait(x);
+  stage_rows(x + (size_t)t0 * hidden, xs, nt * hidden);
+  __syncthreads();
   if (e >= rows) return;
-  const float* w = wr + (size_t)e * hidden;
-  float acc[TT];
+#pragma unroll 2
+  for (int tt = 0; tt < nt; ++tt) {
+    const float* xt = xs + (size_t)tt * hidden;
+    float v;
+    if constexpr (PRE > 0) {
+      float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
-  for (int tt = 0; tt < TT; ++tt) acc[tt] = lane_dot(xs + tt * hidden, w, hidden, lane);
-#pragma unroll
-  for (int tt = 0; tt < TT; ++tt) {
-    const float v = warp_sum(acc[tt]);
-    if (lane == 0 && tt < nt) out[(size_t)(t0 + tt) * rows + e] = v;
+      for (int j = 0; j < PRE; ++j) {
+        const int i = lane * 4 + j * 128;
+        if (i < hidden) {
+          const float4 xv = *reinterpret_cast<const float4*>(xt + i);
+          s0 = fmaf(xv.x, wv[j].x, s0);
+          s1 = fmaf(xv.y, wv[j].y, s1);
+          s2 = fmaf(xv.z, wv[j].z, s2);
+          s3 = fmaf(xv.w, wv[j].w, s3);
+        }
+      }
+      v = warp_sum((s0 + s1) + (s2 + s3));
+    } else {
+      v = warp_sum(lane_dot(xt, w, hidden, lane));
+    }
+    if (lane == 0) out[(size_t)(t0 + tt) * rows + e] = v;
   }
 }
 
@@ -87,14 +140,13 @@ __global__ void identity_expert_rows_kernel(const U* __restrict__ x, const int* 
   for (int i = threadIdx.x; i < pieces; i += blockDim.x) dst[i] = src[i];
 }
 
-template <bool STAGED>
 __global__ void __launch_bounds__(1024)
-moe_plan_kernel(const int* __restrict__ topk_idx, int n, int E, int* __restrict__ offsets,
-                int* __restrict__ order, int* __restrict__ inv, int* __restrict__ active,
-                int n_active_max) {
-  extern __shared__ int counts[];      // [E + 1], then (STAGED) n experts as 16-bit
-  plan_block<STAGED>(topk_idx, n, E, offsets, order, inv, counts,
-                     reinterpret_cast<unsigned short*>(counts + E + 1), active, n_active_max);
+moe_plan_kernel(const int* __restrict__ topk_idx, int n, int E, int* __restrict__ offsets, int* __restrict__ order,
+                int* __restrict__ inv, int warps, int* __restrict__ active, int n_active_max) {
+  extern __shared__ int counts[];      // [E + 1], then the warps' counts [warps][E]
+  chain_release_if_small();
+  chain_wait(topk_idx);
+  plan_block(topk_idx, n, E, offsets, order, inv, counts, counts + E + 1, warps, active, n_active_max);
 }
 
 // Few tokens (decode steps): logits, selection and plan in one launch.  Blocks (8 router rows,
@@ -109,7 +161,7 @@ router_fused_kernel(const T* __restrict__ x, const float* __restrict__ wr, int n
                     int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ inv,
                     int* __restrict__ active, int n_active_max, int* __restrict__ ticket,
                     const float* __restrict__ bias) {
-  extern __shared__ float xs[];        // [hidden]; the last block reuses it
+  extern __shared__ __align__(16) float xs[];        // [hidden]; the last block reuses it
   __shared__ int s_last;
   const int rows = E + extra;
   const int t = blockIdx.y;
@@ -130,7 +182,7 @@ router_fused_kernel(const T* __restrict__ x, const float* __restrict__ wr, int n
     }
   }
   chain_wait(x);
-  for (int i = threadIdx.x; i < hidden; i += blockDim.x) xs[i] = to_float(x[(size_t)t * hidden + i]);
+  stage_rows(x + (size_t)t * hidden, xs, hidden);
   __syncthreads();
   if (e < rows) {
     float v;
@@ -166,9 +218,8 @@ router_fused_kernel(const T* __restrict__ x, const float* __restrict__ wr, int n
                  extra_out, lane, nullptr, bias);
   __threadfence_block();
   __syncthreads();
-  int* counts = reinterpret_cast<int*>(xs);         // [E + 1], then the pairs' experts
-  plan_block<true>(topk_idx, n_tokens * k, E, offsets, order, inv, counts,
-                   reinterpret_cast<unsigned short*>(counts + E + 1), active, n_active_max);
+  int* counts = reinterpret_cast<int*>(xs);         // [E + 1], then the warps' counts
+  plan_block(topk_idx, n_tokens * k, E, offsets, order, inv, counts, counts + E + 1, 8, active, n_active_max);
   if (threadIdx.x == 0) *ticket = 0;
 }
 
@@ -235,34 +286,7 @@ router_cluster_kernel(const T* __restrict__ x, const float* __restrict__ wr, int
     }
   }
   chain_wait(x);
-  {
-    // x -> float32 in shared memory, 16 bytes of x a thread a step where alignment allows
-    const int total = n_tokens * hidden;
-    constexpr int PER = 16 / (int)sizeof(T);
-    if (((uintptr_t)x & 15) == 0 && total % PER == 0) {
-      constexpr int U = 8;                       // loads in flight a thread: the rows are one trip to L2, not one each
-      const int step = blockDim.x * PER;
-      for (int i0 = threadIdx.x * PER; i0 < total; i0 += step * U) {
-        uint4 raw[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (i0 + u * step < total) raw[u] = *reinterpret_cast<const uint4*>(x + i0 + u * step);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (i0 + u * step < total) {
-            const T* v = reinterpret_cast<const T*>(&raw[u]);
-            // 16-byte stores: scalar ones would put the lanes 8 floats apart, 8 to a bank
-#pragma unroll
-            for (int j = 0; j < PER; j += 4)
-              *reinterpret_cast<float4*>(xs + i0 + u * step + j) =
-                  make_float4(to_float(v[j]), to_float(v[j + 1]), to_float(v[j + 2]), to_float(v[j + 3]));
-          }
-        }
-      }
-    } else {
-      for (int i = threadIdx.x; i < total; i += blockDim.x) xs[i] = to_float(x[i]);
-    }
-  }
+  stage_rows(x, xs, n_tokens * hidden);
   __syncthreads();
   bool met = false;                      // this thread has seen every CTA of the cluster running
   for (int e = e0; e < rows; e += 8 * kRouterCluster) {
@@ -357,95 +381,40 @@ router_cluster_kernel(const T* __restrict__ x, const float* __restrict__ wr, int
   }
 }
 
-// The same plan for many pairs, spread over the device.  Block e ranks the pairs of expert e
-// (in pair order, so token order is kept) and counts them; the second kernel turns counts into
-// offsets and scatters.
-__global__ void __launch_bounds__(1024)
-moe_rank_kernel(const int* __restrict__ topk_idx, int n, int* __restrict__ counts, int* __restrict__ inv) {
-  // warp w takes the contiguous chunk w of the pairs: count, prefix over warps, then rank
-  __shared__ int warp_tot[32];
-  const int e = blockIdx.x;
-  chain_release_if_small();
-  chain_wait(topk_idx);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-  const int chunk = ((n + nwarp - 1) / nwarp + 31) & ~31;
-  const int lo = warp * chunk, hi = min(n, lo + chunk);
-  int cnt = 0;
-  for (int base = lo; base < hi; base += 32) {
-    const int i = base + lane;
-    cnt += __popc(__ballot_sync(0xffffffffu, i < hi && topk_idx[i] == e));
-  }
-  if (lane == 0) warp_tot[warp] = cnt;
-  __syncthreads();
-  int running = 0;
-  for (int w = 0; w < warp; ++w) running += warp_tot[w];
-  for (int base = lo; base < hi; base += 32) {
-    const int i = base + lane;
-    const bool mine = i < hi && topk_idx[i] == e;
-    const unsigned b = __ballot_sync(0xffffffffu, mine);
-    if (mine) inv[i] = running + __popc(b & ((1u << lane) - 1u));
-    running += __popc(b);
-  }
-  if (threadIdx.x == blockDim.x - 1) counts[e] = running;
-}
-
-__global__ void __launch_bounds__(256)
-moe_scatter_kernel(const int* __restrict__ topk_idx, int n, int E, const int* __restrict__ counts,
-                   int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ inv,
-                   int* __restrict__ active, int n_active_max) {
-  extern __shared__ int off[];        // [E + 1]
-  chain_release_if_small();
-  chain_wait(topk_idx, counts);
-  if (threadIdx.x == 0) {
-    int run = 0, na = 0;
-    const bool list = active && blockIdx.x == 0;
-    for (int e = 0; e < E; ++e) {
-      off[e] = run;
-      if (list && counts[e] > 0 && na < n_active_max) active[na++] = e;
-      run += counts[e];
-    }
-    off[E] = run;
-    if (list)
-      for (; na < n_active_max; ++na) active[na] = -1;
-  }
-  __syncthreads();
-  if (blockIdx.x == 0)
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = off[e];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int e = topk_idx[i];
-  if (e < 0 || e >= E) return;
-  const int p = off[e] + inv[i];
-  inv[i] = p;
-  order[p] = i;
-}
-
 }  // namespace nf
 
 using namespace nf;
 
-template <typename T, int TT>
+template <typename T, int TT, int PRE>
 static int launch_logits(const void* x, const float* wr, int T_, int hidden, int rows, float* logits,
                          cudaStream_t stream) {
   const size_t smem = (size_t)TT * hidden * sizeof(float);
   static size_t allowed = 48 * 1024;      // raised once per size, outside any stream capture
   if (smem > allowed) {
-    cudaFuncSetAttribute(router_logits_kernel<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(router_logits_kernel<T, TT, PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     allowed = smem;
   }
   dim3 grid((rows + 7) / 8, (T_ + TT - 1) / TT);
   NF_REQUIRE(grid.y <= 65535, "router: too many tokens in one call (%d)", T_);
-  router_logits_kernel<T, TT><<<grid, 256, smem, stream>>>((const T*)x, wr, T_, hidden, rows, logits);
+  launch_chained(router_logits_kernel<T, TT, PRE>, grid, dim3(256), smem, stream, (const T*)x, wr, T_, hidden, rows, logits);
   return check_launch("router_logits");
 }
-
+template <typename T, int PRE>
+static int launch_logits_p(const void* x, const float* wr, int T_, int hidden, int rows, float* logits,
+                           cudaStream_t stream) {
+  // tokens per block: as many as fit shared memory, to read the router matrix fewer times, while the blocks fill the
+  // device (61 rows of 2,048 numbers, 64 tokens: two tokens a block, read one number at a time,
+  // took 25 us; with the shorter plan a pass of 64 short requests over 12 layers went from 52.4 to 51.1 ms)
+  if (T_ > 128 && (size_t)8 * hidden * 4 <= 160 * 1024) return launch_logits<T, 8, PRE>(x, wr, T_, hidden, rows, logits, stream);
+  if (T_ > 16 && (size_t)4 * hidden * 4 <= 160 * 1024) return launch_logits<T, 4, PRE>(x, wr, T_, hidden, rows, logits, stream);
+  return launch_logits<T, 1, PRE>(x, wr, T_, hidden, rows, logits, stream);
+}
 template <typename T>
 static int launch_logits_t(const void* x, const float* wr, int T_, int hidden, int rows, float* logits,
                            cudaStream_t stream) {
-  // tokens per block: as many as fit shared memory, to read the router matrix fewer times
-  if (T_ > 128 && (size_t)8 * hidden * 4 <= 160 * 1024) return launch_logits<T, 8>(x, wr, T_, hidden, rows, logits, stream);
-  if (T_ > 8 && (size_t)2 * hidden * 4 <= 160 * 1024) return launch_logits<T, 2>(x, wr, T_, hidden, rows, logits, stream);
-  return launch_logits<T, 1>(x, wr, T_, hidden, rows, logits, stream);
+  if (hidden % 4 == 0 && (uintptr_t)wr % 16 == 0 && hidden <= 16 * 128) return launch_logits_p<T, 16>(x, wr, T_, hidden, rows, logits, stream);
+  if (hidden % 4 == 0 && (uintptr_t)wr % 16 == 0 && hidden <= 32 * 128) return launch_logits_p<T, 32>(x, wr, T_, hidden, rows, logits, stream);
+  return launch_logits_p<T, 0>(x, wr, T_, hidden, rows, logits, stream);
 }
 
 // logits: float32 scratch [T, E + extra], also an output (the raw router logits).  Here and below: bias float32 [E] or
@@ -460,11 +429,12 @@ extern "C" int nf_router_topk(const void* x, const float* wr, int T, int hidden,
   int rc = dtype == kF32 ? launch_logits_t<float>(x, wr, T, hidden, E + extra, logits, stream)
                          : launch_logits_t<__nv_bfloat16>(x, wr, T, hidden, E + extra, logits, stream);
   if (rc) return rc;
-  router_select_kernel<<<(T + 3) / 4, 128, (size_t)4 * E * sizeof(float), stream>>>(logits, E + extra, 1, T, E, extra, k, norm_topk, topk_idx, topk_w, extra_out, bias);
+  launch_chained(router_select_kernel, dim3((T + 3) / 4), dim3(128), (size_t)4 * E * sizeof(float), stream, (const float*)logits,
+                 (long)(E + extra), 1l, T, E, extra, k, norm_topk, topk_idx, topk_w, extra_out, bias);
   return check_launch("router_select");
 }
 
-// Few tokens: logits + selection + plan in one launch.  Needs max(hidden, 8 * E, E + 1 + T * k / 2 + 1)
+// Few tokens: logits + selection + plan in one launch.  Needs max(hidden, 9 * E + 1)
 // floats of shared memory; `ticket` is a zeroed int that the kernel leaves zeroed.
 extern "C" int nf_router_fused(const void* x, const float* wr, int T, int hidden, int E, int extra, int k,
                                int norm_topk, float* logits, int* topk_idx, float* topk_w,
@@ -473,8 +443,7 @@ extern "C" int nf_router_fused(const void* x, const float* wr, int T, int hidden
   if (T == 0) return 0;
   NF_REQUIRE(T > 0 && T <= 65535 && hidden > 0 && E > 0 && k > 0 && k <= E && extra >= 0, "router: bad sizes T=%d hidden=%d E=%d k=%d", T, hidden, E, k);
   size_t words = (size_t)hidden;
-  if ((size_t)8 * E > words) words = (size_t)8 * E;
-  if ((size_t)E + 2 + (size_t)T * k / 2 > words) words = (size_t)E + 2 + (size_t)T * k / 2;
+  if ((size_t)9 * E + 1 > words) words = (size_t)9 * E + 1;
   const size_t smem = words * sizeof(float);
   NF_REQUIRE(smem <= 160 * 1024 && E < 65536, "router: sizes too large for the fused kernel");
   static size_t allowed_f = 48 * 1024, allowed_b = 48 * 1024;
@@ -560,28 +529,24 @@ extern "C" int nf_router_select(const float* logits, long long tok_stride, long 
   return check_launch("router_select");
 }
 
-// counts: int32 scratch [E] (may be null: then one block does everything).
 // active / n_active_max: optional list of the experts that have pairs (ascending, -1 padded).
-extern "C" int nf_moe_plan(const int* topk_idx, int n, int E, int* offsets, int* order, int* inv,
-                           int* counts, int* active, int n_active_max, cudaStream_t stream) {
+extern "C" int nf_moe_plan(const int* topk_idx, int n, int E, int* offsets, int* order, int* inv, int* active,
+                           int n_active_max, cudaStream_t stream) {
   NF_REQUIRE(n >= 0 && E > 0 && E <= 8192, "moe_plan: bad sizes n=%d E=%d", n, E);
-  if (n > 2048 && counts) {
-    launch_chained(moe_rank_kernel, dim3(E), dim3(1024), 0, stream, topk_idx, n, counts, inv);
-    if (int rc = check_launch("moe_rank")) return rc;
-    launch_chained(moe_scatter_kernel, dim3((n + 255) / 256), dim3(256), (E + 1) * sizeof(int), stream, topk_idx, n, E, (const int*)counts, offsets, order, inv, active, n_active_max);
-    return check_launch("moe_scatter");
+  // warps that count: no more than there are runs of 32 pairs, than 160 KB of counts hold, than a block has
+  int warps = (n + 31) / 32;
+  const int hold = (40 * 1024 - (E + 1)) / E;
+  if (warps > hold) warps = hold;
+  if (warps > 32) warps = 32;
+  if (warps < 1) warps = 1;
+  const size_t smem = (size_t)(E + 1 + warps * E) * sizeof(int);
+  static size_t allowed = 48 * 1024;
+  if (smem > allowed) {
+    cudaFuncSetAttribute(moe_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allowed = smem;
   }
-  const size_t staged = (size_t)(E + 1) * sizeof(int) + (size_t)n * sizeof(unsigned short);
-  if (E < 65536 && staged <= 160 * 1024) {
-    static size_t allowed = 48 * 1024;
-    if (staged > allowed) {
-      cudaFuncSetAttribute(moe_plan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staged);
-      allowed = staged;
-    }
-    moe_plan_kernel<true><<<1, 1024, staged, stream>>>(topk_idx, n, E, offsets, order, inv, active, n_active_max);
-  } else {
-    moe_plan_kernel<false><<<1, 1024, (E + 1) * sizeof(int), stream>>>(topk_idx, n, E, offsets, order, inv, active, n_active_max);
-  }
+  const int threads = 32 * warps > 256 ? 32 * warps : 256;
+  launch_chained(moe_plan_kernel, dim3(1), dim3(threads), smem, stream, topk_idx, n, E, offsets, order, inv, warps, active, n_active_max);
   return check_launch("moe_plan");
 }
 

@@ -236,51 +236,77 @@ __device__ __forceinline__ void select_token_ruled(const float* __restrict__ row
   __syncwarp();
 }
 
-// Plan by one block: stable counting sort of the n pairs by expert, and (if `active` is
-// given) the list of experts that have pairs, ascending, padded with -1 to n_active_max.  `counts` is E + 1 ints
-// of shared memory; with STAGED, `ex` holds n 16-bit expert ids so that the E passes over the
-// pairs do not go to global memory.
-template <bool STAGED>
-__device__ __forceinline__ void plan_block(const int* __restrict__ topk_idx, int n, int E,
-                                           int* __restrict__ offsets, int* __restrict__ order,
-                                           int* __restrict__ inv, int* counts, unsigned short* ex,
+// Plan by one block: stable counting sort of the n pairs by expert, and (if `active` is given) the list of experts that
+// have pairs, ascending, padded with -1 to n_active_max.  The first `warps` warps take consecutive runs of the pairs, 32
+// pairs at a time: lanes that hold the same expert find one another by a match, and a warp keeps its counts so far in its
+// row of `hist` [warps][E]; the rows are then added up over the warps and the experts.  (Every expert walking all pairs,
+// as this did before, costs E / 32 passes over them: 13 us for 2,048 pairs of 60 experts, 6 us for 256.)
+// counts: E + 1 ints of shared memory.
+__device__ __forceinline__ void plan_block(const int* __restrict__ topk_idx, int n, int E, int* __restrict__ offsets,
+                                           int* __restrict__ order, int* __restrict__ inv, int* counts, int* hist, int warps,
                                            int* __restrict__ active, int n_active_max) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-  if (STAGED) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ex[i] = (unsigned short)__ldcg(topk_idx + i);
-    __syncthreads();
-  }
-  for (int e = warp; e < E; e += nwarp) {
-    int running = 0;
-    for (int base = 0; base < n; base += 32) {
-      const int i = base + lane;
-      const bool mine = i < n && (STAGED ? (int)ex[i] : topk_idx[i]) == e;
-      const unsigned b = __ballot_sync(0xffffffffu, mine);
-      if (mine) inv[i] = running + __popc(b & ((1u << lane) - 1u));   // rank inside the expert
-      running += __popc(b);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunk = ((n + warps - 1) / warps + 31) & ~31;
+  const int lo = warp < warps ? warp * chunk : n, hi = min(n, lo + chunk);
+  int* mine = hist + warp * E;
+  for (int i = threadIdx.x; i < warps * E; i += blockDim.x) hist[i] = 0;
+  __syncthreads();
+  for (int base = lo; base < hi; base += 32) {
+    const int i = base + lane;
+    int e = i < hi ? __ldcg(topk_idx + i) : -1;
+    if (e < 0 || e >= E) e = -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, e);
+    const unsigned before = peers & ((1u << lane) - 1u);
+    const int so_far = e >= 0 ? mine[e] : 0;
+    __syncwarp();
+    if (e >= 0) {
+      inv[i] = so_far + __popc(before);                  // rank among this warp's pairs of the expert
+      if (before == 0) mine[e] = so_far + __popc(peers);
     }
-    if (lane == 0) counts[e] = running;
+    __syncwarp();
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0, na = 0;
-    for (int e = 0; e < E; ++e) {
-      const int c = counts[e];
-      if (c > 0 && active && na < n_active_max) active[na++] = e;
-      counts[e] = run;
-      offsets[e] = run;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int run = 0;
+    for (int w = 0; w < warps; ++w) {
+      const int c = hist[w * E + e];
+      hist[w * E + e] = run;
       run += c;
     }
-    counts[E] = run;
-    offsets[E] = run;
-    if (active)
-      for (; na < n_active_max; ++na) active[na] = -1;
+    counts[e] = run;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int e = STAGED ? (int)ex[i] : topk_idx[i];
+  if (warp == 0) {                       // 32 experts a round: exclusive prefix of the counts, list of those with pairs
+    int run = 0, na = 0;
+    for (int base = 0; base <= E; base += 32) {
+      const int e = base + lane;
+      const int c = e < E ? counts[e] : 0;
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      if (e <= E) {
+        counts[e] = run + incl - c;
+        offsets[e] = run + incl - c;
+      }
+      run += __shfl_sync(0xffffffffu, incl, 31);
+      const unsigned b = __ballot_sync(0xffffffffu, c > 0);
+      if (active) {
+        const int at = na + __popc(b & ((1u << lane) - 1u));
+        if (c > 0 && at < n_active_max) active[at] = e;
+      }
+      na += __popc(b);
+    }
+    if (active)
+      for (int i = min(na, n_active_max) + lane; i < n_active_max; i += 32) active[i] = -1;
+  }
+  __syncthreads();
+  for (int i = lo + lane; i < hi; i += 32) {
+    const int e = __ldcg(topk_idx + i);
     if (e < 0 || e >= E) continue;
-    const int p = counts[e] + inv[i];
+    const int p = counts[e] + mine[e] + inv[i];
     inv[i] = p;
     order[p] = i;
   }
