@@ -13,6 +13,9 @@
 //
 // All query heads of a group share the CTA, so keys and values are read once per kv head.
 //
+// Few rows of up to eight blocks (a context bound of 1,024 keys) take one launch: a row's blocks are a thread-block
+// cluster, and what the second kernel does is done there, out of the CTAs' shared memory (same sums in the same order).
+//
 // Further forms.  SIGMOID: a key weighs sigmoid(score + sig_bias[h]), not normalised over keys - blocks carry the
 // maximum 0 and simply add.  CAPPED: the softmax over cap * tanh(score / cap).  Turned values: the merge turns the first `turn_dims` numbers of a head's result by minus
 // the row's position (what turn_back in qk_norm_append.cu does in a pass of its own, here on the float32 sum).
@@ -64,7 +67,21 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
 // weighted sum of values are tensor-core products with the keys (values) as the 16-row
 // operand and up to 8 query heads of the group as the 8-column operand; softmax stays in
 // float32 in between.  Warp w owns keys [32 w, 32 w + 32) of the block.
-template <int D, int FORM>
+__device__ __forceinline__ float ld_cluster_f32(const float* local, unsigned cta) {
+  unsigned remote;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(cta));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+constexpr int kClusterSplits = 8;  // most key blocks of a row that one cluster takes (the portable cluster size)
+constexpr int kClusterCtas = 256;  // most CTAs of such a launch (see launch_split)
+
+template <int D, int FORM, bool CLUSTER>
 __global__ void __launch_bounds__(128)
 decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_stride,
                               const __nv_bfloat16* __restrict__ pages,
@@ -89,6 +106,7 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
   const int RH = min(G, HC);                                        // heads kept per pass
   float* red = sc + G * kSplit;                                     // [4 warps][RH][D]
   float* ml = red + 4 * RH * D;                                     // [G][2]
+  float* part = ml + 2 * G;                                         // CLUSTER: [G][D] this block's sums
   // wi: the row's place in this launch (workspace, counters); t: the row itself
   const int wi = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -106,7 +124,10 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
   const int k_base = split * kSplit;
   const int k_begin = max(lo, k_base);
   const int k_end = min(pos + 1, k_base + kSplit);
-  if (k_begin >= k_end) return;
+  const bool empty = k_begin >= k_end;
+  if (!CLUSTER && empty) return;
+  if (empty) chain_wait();             // (its CTA still meets the others, and may write a part of the result)
+  if (!empty) {
   const int seg = row_seg[t];
   const int* bt = block_table + (size_t)seg * bt_width;
   const size_t head_stride = (size_t)page_size * D;
@@ -270,10 +291,41 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
 #pragma unroll
       for (int w = 0; w < 4; ++w) s += red[(w * RH + hh) * D + d];
       const int hq = kvh * G + h0 + hh;
-      ws_acc[(((size_t)wi * Hq + hq) * nsplit + split) * D + d] = s;
+      if (CLUSTER) part[(h0 + hh) * D + d] = s;
+      else ws_acc[(((size_t)wi * Hq + hq) * nsplit + split) * D + d] = s;
     }
     __syncthreads();
   }
+  }
+  if constexpr (CLUSTER) {
+    cluster_meet();                    // every block's sums stand in its CTA's shared memory
+    const int s0 = lo / kSplit, n = pos / kSplit - s0 + 1;
+    for (int i = split * blockDim.x + threadIdx.x; i < G * D; i += nsplit * blockDim.x) {
+      const int hh = i / D;
+      float bm[kClusterSplits], bl[kClusterSplits], ba[kClusterSplits];
+#pragma unroll
+      for (int s = 0; s < kClusterSplits; ++s)
+        if (s < n) {
+          bm[s] = ld_cluster_f32(ml + 2 * hh, s0 + s);
+          bl[s] = ld_cluster_f32(ml + 2 * hh + 1, s0 + s);
+          ba[s] = ld_cluster_f32(part + i, s0 + s);
+        }
+      float m = -INFINITY, l = 0.f, o = 0.f;
+#pragma unroll
+      for (int s = 0; s < kClusterSplits; ++s)
+        if (s < n) m = fmaxf(m, bm[s]);
+#pragma unroll
+      for (int s = 0; s < kClusterSplits; ++s)
+        if (s < n) {
+          const float w = expf(bm[s] - m);
+          l += bl[s] * w;
+          o += ba[s] * w;
+        }
+      const float inv = SIGMOID ? 1.f : (l > 0.f ? 1.f / l : 0.f);
+      out[((size_t)t * Hq + (size_t)kvh * G) * D + i] = __float2bfloat16_rn(o * inv);
+    }
+    cluster_meet();                    // nobody leaves while its shared memory is being read
+  } else {
   for (int h = threadIdx.x; h < G; h += blockDim.x) {
     const int hq = kvh * G + h;
     float* o = ws_ml + (((size_t)wi * Hq + hq) * nsplit + split) * 2;
@@ -310,6 +362,7 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
       for (int s = s0; s <= s1; ++s) o += __ldcg(accp + (size_t)s * D + d) * expf(__ldcg(mlp + 2 * s) - m);
       out[((size_t)t * Hq + hq) * D + d] = __float2bfloat16_rn(o * inv_l);
     }
+  }
   }
 }
 
@@ -422,18 +475,35 @@ static int launch_split(const void* qkv, int q_row_stride, const void* pages, co
                         int bt_width, const int* positions, const int* row_seg, float* ws_acc,
                         float* ws_ml, int T, int Hq, int Hkv, int page_size, int num_pages, int window,
                         float scale, int nsplit, int* counters, void* out, const int* row_list, const float* sig_bias,
-                        float softcap, cudaStream_t stream) {
+                        float softcap, bool* merged, cudaStream_t stream) {
   const int G = Hq / Hkv;
   const size_t smem = (size_t)2 * kSplit * (D + 8) * sizeof(__nv_bfloat16) +
                       ((size_t)G * kSplit + 4 * (G < 8 ? G : 8) * D + 2 * G) * sizeof(float);
   NF_REQUIRE(smem <= 200 * 1024, "decode attention: %d query heads per kv head need too much shared memory", G);
+  dim3 grid(T, Hkv, nsplit);
+  const size_t smem_c = smem + (size_t)G * D * sizeof(float);
+  // At most 256 CTAs: one row of 16 key heads 14.4 -> 12.4 us for all launches of the attention, two rows of eight blocks
+  // 14.6 -> 12.6; but four rows (512 CTAs) 14.6 both ways, eight 15.2 -> 23 and 16 of four key heads 14.6 -> 19: clusters
+  // start as a whole, with three CTAs' shared memory on an SM, where single CTAs trickle in and empty ones leave at once.
+  if (*merged && nsplit <= kClusterSplits && smem_c <= 100 * 1024 && (long long)T * Hkv * nsplit <= kClusterCtas) {
+    static size_t allowed_c = 48 * 1024;
+    if (smem_c > allowed_c) {
+      cudaFuncSetAttribute(decode_attention_split_kernel<D, FORM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c);
+      allowed_c = smem_c;
+    }
+    launch_chained_clusters(decode_attention_split_kernel<D, FORM, true>, grid, dim3(128), smem_c, stream, dim3(1, 1, nsplit),
+                             (const __nv_bfloat16*)qkv, q_row_stride, (const __nv_bfloat16*)pages, block_table, bt_width,
+                             positions, row_seg, ws_acc, ws_ml, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters,
+                             (__nv_bfloat16*)out, row_list, sig_bias, softcap);
+    return check_launch("decode_attention_cluster");
+  }
+  *merged = false;
   static size_t allowed = 48 * 1024;
   if (smem > allowed) {
-    cudaFuncSetAttribute(decode_attention_split_kernel<D, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(decode_attention_split_kernel<D, FORM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     allowed = smem;
   }
-  dim3 grid(T, Hkv, nsplit);
-  launch_chained(decode_attention_split_kernel<D, FORM>, grid, dim3(128), smem, stream,
+  launch_chained(decode_attention_split_kernel<D, FORM, false>, grid, dim3(128), smem, stream,
                  (const __nv_bfloat16*)qkv, q_row_stride, (const __nv_bfloat16*)pages, block_table, bt_width,
                  positions, row_seg, ws_acc, ws_ml, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters,
                  (__nv_bfloat16*)out, row_list, sig_bias, softcap);
@@ -451,6 +521,7 @@ int decode_attention_stream(const void* qkv, int q_row_stride, const void* pages
                             int nsplit, const int* row_list, const float* sig_bias, float softcap, cudaStream_t stream);
 int decode_attention_stream_status();
 int g_decode_stream = 1;
+int g_decode_cluster = 1;
 }  // namespace nf
 
 using namespace nf;
@@ -473,6 +544,12 @@ extern "C" int nf_set_decode_stream(int on) {
   return 0;
 }
 
+// 0: a row's blocks are always merged by a second kernel; 1 (default): by their cluster where they fit one.
+extern "C" int nf_set_decode_cluster(int on) {
+  g_decode_cluster = on ? 1 : 0;
+  return 0;
+}
+
 // bfloat16 only; head_dim in {16, 32, 64, 128, 256}.  `nsplit` >= ceil(max context / 128) of
 // the rows in this call.  Workspace: ws_acc float32 [T, Hq, nsplit, D], ws_ml [T, Hq, nsplit, 2].
 static int decode_attention_impl(const void* qkv, int q_row_stride, const void* pages,
@@ -486,14 +563,16 @@ static int decode_attention_impl(const void* qkv, int q_row_stride, const void* 
   NF_REQUIRE(T > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && nsplit > 0, "decode attention: bad sizes T=%d Hq=%d Hkv=%d nsplit=%d", T, Hq, Hkv, nsplit);
   NF_REQUIRE(Hkv <= 65535 && nsplit <= kMaxMergeSplits, "decode attention: too many kv heads or key blocks (context beyond %d keys)", kMaxMergeSplits * kSplit);
   int rc;
+  bool merged = g_decode_cluster && !counters && !turn_freq;      // asked for; then: whether the launch merged its blocks itself
   // The persistent kernel pays a start-up (every CTA lists the rows' blocks) that only many
   // blocks repay: measured on B200, it wins from about a thousand blocks on.
   if (g_decode_stream && !counters && (long long)T * Hkv * nsplit >= 1024 &&
       decode_attention_stream_fits(T, Hq, Hkv, D, page_size)) {
+    merged = false;
     rc = decode_attention_stream(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, ws_acc, ws_ml,
                                  T, Hq, Hkv, D, page_size, num_pages, window, scale, nsplit, row_list, sig_bias, softcap, stream);
   } else
-#define NF_DA_CALL(DD, SG) launch_split<DD, SG>(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, ws_acc, ws_ml, T, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters, out, row_list, sig_bias, softcap, stream)
+#define NF_DA_CALL(DD, SG) launch_split<DD, SG>(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, ws_acc, ws_ml, T, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters, out, row_list, sig_bias, softcap, &merged, stream)
 #define NF_DA(DD) case DD: rc = sig_bias ? NF_DA_CALL(DD, kFormSigmoid) : (softcap > 0.f ? NF_DA_CALL(DD, kFormCapped) : NF_DA_CALL(DD, kFormSoftmax)); break;
   switch (D) {
     NF_DA(16)
@@ -507,7 +586,7 @@ static int decode_attention_impl(const void* qkv, int q_row_stride, const void* 
   }
 #undef NF_DA
 #undef NF_DA_CALL
-  if (rc || counters) return rc;      // with counters the split kernel's last CTAs have merged
+  if (rc || counters || merged) return rc;      // with counters the split kernel's last CTAs have merged
   dim3 grid(T, Hq);
   int dthreads = 32;
   while (dthreads < D && dthreads < 256) dthreads <<= 1;

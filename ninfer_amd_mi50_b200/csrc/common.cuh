@@ -95,10 +95,10 @@ inline void launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size
                                                   // did not keep it as its last error
 }
 
-// The same with the CTAs launched as clusters of `cluster_x` consecutive blocks of grid.x.
+// The same with the CTAs launched as clusters of the given shape.
 template <typename... KArgs, typename... Args>
-inline void launch_chained_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                   int cluster_x, Args... args) {
+inline void launch_chained_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    dim3 cluster, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -106,15 +106,20 @@ inline void launch_chained_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 blo
   cfg.stream = stream;
   cudaLaunchAttribute attrs[2];
   attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = cluster_x;
-  attrs[0].val.clusterDim.y = 1;
-  attrs[0].val.clusterDim.z = 1;
+  attrs[0].val.clusterDim.x = cluster.x;
+  attrs[0].val.clusterDim.y = cluster.y;
+  attrs[0].val.clusterDim.z = cluster.z;
   attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attrs[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attrs;
   cfg.numAttrs = chain_this_launch(NF_CHAIN_CLASS, stream) ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
   if (e != cudaSuccess) note_launch_error(e);
+}
+template <typename... KArgs, typename... Args>
+inline void launch_chained_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                   int cluster_x, Args... args) {
+  launch_chained_clusters(kernel, grid, block, smem, stream, dim3(cluster_x), args...);
 }
 
 #define NF_REQUIRE(cond, ...)            \
