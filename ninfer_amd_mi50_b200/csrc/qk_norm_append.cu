@@ -62,6 +62,83 @@ qk_whole_norm_append_kernel(const float* __restrict__ proj, int ld, int q_col0, 
 }
 
 
+// The wide form: rows of up to 2,048 R numbers, a thread has R runs of four of q and of k in registers between the two
+// passes; biases, weights and the page, which the kernel before does not write, are asked for before the wait.  (One row of
+// 2 x 2,048 numbers read element by element twice took 12 us in a decode step.)
+template <typename T, int R>
+__global__ void __launch_bounds__(512)
+qk_whole_norm_append_vec_kernel(const float* __restrict__ proj, int ld, int q_col0, int k_col0,
+                                const float* __restrict__ bias_q, const float* __restrict__ bias_k,
+                                const float* __restrict__ wq, const float* __restrict__ wk, float eps,
+                                const int* __restrict__ positions, const int* __restrict__ row_seg, T* __restrict__ q_out,
+                                int Hq, int Hkv, int D, T* __restrict__ pages, const int* __restrict__ block_table, int bt_width,
+                                int page_size, int num_pages, int append) {
+  __shared__ float red[33];
+  const int t = blockIdx.x;
+  const int width[2] = {Hq * D, Hkv * D};
+  chain_release_if_small();
+  T* kdst = nullptr;
+  if (append) {
+    const int pos = positions[t], lp = pos / page_size;
+    const int page = (lp >= 0 && lp < bt_width) ? block_table[(size_t)row_seg[t] * bt_width + lp] : -1;
+    if (page >= 0 && page < num_pages)                       // no page reserved: never write out of bounds
+      kdst = pages + ((size_t)page * 2 * Hkv * page_size + (size_t)(pos - lp * page_size)) * D;
+  }
+  float b[2][R][4], w[2][R][4], v[2][R][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+      const int i = (c * 512 + threadIdx.x) * 4;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) b[m][c][e] = w[m][c][e] = v[m][c][e] = 0.f;
+      if (i < width[m]) {
+        const float* bias = m ? bias_k : bias_q;
+        if (bias) load4(bias + i, b[m][c]);
+        load4((m ? wk : wq) + i, w[m][c]);
+      }
+    }
+  chain_wait(proj);
+  const float* row = proj + (size_t)t * ld;
+  float ss[2] = {0.f, 0.f};
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+      const int i = (c * 512 + threadIdx.x) * 4;
+      if (i < width[m]) load4(row + (m ? k_col0 : q_col0) + i, v[m][c]);
+    }
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int c = 0; c < R; ++c)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        v[m][c][e] += b[m][c][e];
+        ss[m] += v[m][c][e] * v[m][c][e];
+      }
+  const float inv_q = rsqrtf(block_sum(ss[0], red) / (float)width[0] + eps);
+  const float inv_k = rsqrtf(block_sum(ss[1], red) / (float)width[1] + eps);
+  const size_t head_stride = (size_t)page_size * D;
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * 512 + threadIdx.x) * 4;
+    float o[4];
+    if (i < width[0]) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = v[0][c][e] * inv_q * w[0][c][e];
+      store4(q_out + (size_t)t * width[0] + i, o);
+    }
+    if (kdst && i < width[1]) {
+      const int head = i / D, d = i - head * D;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = v[1][c][e] * inv_k * w[1][c][e];
+      store4(kdst + (size_t)head * head_stride + d, o);
+      store4(kdst + (size_t)(Hkv + head) * head_stride + d, v[1][c]);
+    }
+  }
+}
+
 // The same stage for an attention with values of their own and a rotation: biases; q and k each over
 // the root mean square of the WHOLE projection times a weight of the projection's width; then the first
 // `rot` dimensions of every q and k head turned by the row's position (pair (i, i + rot/2), angle
@@ -77,8 +154,10 @@ qk_whole_norm_append_kernel(const float* __restrict__ proj, int ld, int q_col0, 
 // The row's normed values wait in shared memory (float32) between the two passes.
 // VEC: all sizes are multiples of 4 (the turned halves too): runs of four elements an access, and the norm's
 // factors are applied where the values are read for the second time.
+// Steps that leave SMs idle (up to one row each) give a row 512 threads instead of 256: the kernel is a chain of trips to
+// memory there, and half as many follow one another.
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(512)
 whole_norm_rope_append_kernel(const float* __restrict__ proj, int ld, int q_col0, int k_col0, int v_col0,
                               const float* __restrict__ bias_q, const float* __restrict__ bias_k,
                               const float* __restrict__ bias_v, const float* __restrict__ wq,
@@ -98,8 +177,27 @@ whole_norm_rope_append_kernel(const float* __restrict__ proj, int ld, int q_col0
   float* vcs_s = sn_s + half;
   float* vsn_s = vcs_s + Dv / 2;
   chain_release_if_small();
-  // the angles depend on the position alone (a step's input, not the kernel before's output): all heads share them
+  // the angles and the page depend on the step's inputs alone, not on the kernel before's output: all heads share them
   const int pos = positions[t];
+  T* krow = nullptr;                           // where head 0's key of this token starts
+  size_t k_head_stride = 0, v_head_stride = 0;
+  T* vrow = nullptr;
+  if (Hkv > 0) {
+    const int lp = pos / page_size;
+    const int page = (lp >= 0 && lp < bt_width) ? block_table[(size_t)row_seg[t] * bt_width + lp] : -1;
+    if (page >= 0 && page < num_pages) {       // no page reserved: never write out of bounds
+      const int in_page = pos - lp * page_size;
+      if (rows_layout) {
+        krow = pages + ((size_t)page * page_size + in_page) * ((size_t)Hkv * (D + Dv));
+        vrow = krow + (size_t)Hkv * D;
+        k_head_stride = D; v_head_stride = Dv;
+      } else {
+        krow = pages + ((size_t)page * 2 * Hkv * page_size + in_page) * P;
+        k_head_stride = v_head_stride = (size_t)page_size * P;
+        vrow = krow + (size_t)Hkv * k_head_stride;
+      }
+    }
+  }
   for (int u = threadIdx.x; u < half; u += blockDim.x) {
     float sn, cs;
     sincosf((float)pos * inv_freq[u], &sn, &cs);
@@ -155,25 +253,6 @@ whole_norm_rope_append_kernel(const float* __restrict__ proj, int ld, int q_col0
     for (int i = threadIdx.x; i < KW; i += blockDim.x) y[QW + i] = y[QW + i] * inv_k * wk[i];
   }
   __syncthreads();
-  T* krow = nullptr;                           // where head 0's key of this token starts
-  size_t k_head_stride = 0, v_head_stride = 0;
-  T* vrow = nullptr;
-  if (Hkv > 0) {
-    const int lp = pos / page_size;
-    const int page = (lp >= 0 && lp < bt_width) ? block_table[(size_t)row_seg[t] * bt_width + lp] : -1;
-    if (page >= 0 && page < num_pages) {       // no page reserved: never write out of bounds
-      const int in_page = pos - lp * page_size;
-      if (rows_layout) {
-        krow = pages + ((size_t)page * page_size + in_page) * ((size_t)Hkv * (D + Dv));
-        vrow = krow + (size_t)Hkv * D;
-        k_head_stride = D; v_head_stride = Dv;
-      } else {
-        krow = pages + ((size_t)page * 2 * Hkv * page_size + in_page) * P;
-        k_head_stride = v_head_stride = (size_t)page_size * P;
-        vrow = krow + (size_t)Hkv * k_head_stride;
-      }
-    }
-  }
   // a unit is a turned pair (u, u + rot/2) of a head, whose angle is worked out once, or a single dimension beyond
   const int units = D - half;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
@@ -399,6 +478,17 @@ extern "C" int nf_qk_whole_norm_append(const float* proj, int ld, int q_col0, in
   NF_REQUIRE(T > 0 && Hq > 0 && Hkv > 0 && D > 0 && wq && wk, "qk_whole_norm_append: bad arguments");
   NF_REQUIRE(q_col0 >= 0 && k_col0 >= 0 && q_col0 + Hq * D <= ld && k_col0 + Hkv * D <= ld,
              "qk_whole_norm_append: the column ranges leave the projection");
+  const size_t el = dtype == kF32 ? 4 : 2;
+  const int widest = (Hq > Hkv ? Hq : Hkv) * D;
+  if (((D | ld | q_col0 | k_col0) & 3) == 0 && widest <= 4 * 2048 && (uintptr_t)proj % 16 == 0 && (uintptr_t)q_out % (4 * el) == 0 &&
+      (uintptr_t)pages % (4 * el) == 0 && ((uintptr_t)bias_q | (uintptr_t)bias_k | (uintptr_t)wq | (uintptr_t)wk) % 16 == 0) {
+#define NF_QV(TT, RR) launch_chained(qk_whole_norm_append_vec_kernel<TT, RR>, dim3(T), dim3(512), 0, stream, proj, ld, q_col0, k_col0, bias_q, bias_k, wq, wk, eps, positions, row_seg, (TT*)q_out, Hq, Hkv, D, (TT*)pages, block_table, bt_width, page_size, num_pages, append)
+#define NF_QV_R(TT) do { if (widest <= 2048) NF_QV(TT, 1); else if (widest <= 4096) NF_QV(TT, 2); else NF_QV(TT, 4); } while (0)
+    if (dtype == kF32) NF_QV_R(float); else NF_QV_R(__nv_bfloat16);
+#undef NF_QV_R
+#undef NF_QV
+    return check_launch("qk_whole_norm_append");
+  }
   if (dtype == kF32)
     launch_chained(qk_whole_norm_append_kernel<float>, dim3(T), dim3(256), 0, stream, proj, ld, q_col0, k_col0, bias_q, bias_k, wq, wk, eps, positions, row_seg, (float*)q_out, Hq, Hkv, D, (float*)pages, block_table, bt_width, page_size, num_pages, append);
   else
@@ -436,7 +526,7 @@ extern "C" int nf_whole_norm_rope_append(const float* proj, int ld, int q_col0, 
 #define NF_WN(TT, VE)                                                                                                  \
   do {                                                                                                                \
     if (smem > 48 * 1024) cudaFuncSetAttribute(whole_norm_rope_append_kernel<TT, VE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    launch_chained(whole_norm_rope_append_kernel<TT, VE>, dim3(T), dim3(256), smem, stream, proj, ld, q_col0, k_col0, \
+    launch_chained(whole_norm_rope_append_kernel<TT, VE>, dim3(T), dim3(T <= 148 ? 512 : 256), smem, stream, proj, ld, q_col0, k_col0, \
                    v_col0, bias_q, bias_k, bias_v, wq, wk, eps, inv_freq, rot, mag, positions, row_seg, (TT*)q_out,   \
                    Hq, Hkv, D, Dv, (TT*)pages, block_table, bt_width, page_size, num_pages, rows_layout, P,           \
                    interleaved, v_freq);                                                                              \

@@ -41,6 +41,42 @@ __global__ void causal_conv_silu_kernel(const T* __restrict__ src, int lds, int 
   const int seg = row_seg[t];
   const int r0 = seg_row0[seg];
   float* st = state + (size_t)seg_slot[seg] * slot_stride;            // [K - 1][C]
+  // A single row of few taps, all of whose columns lie on 16 bytes: every operand is asked for at once, four numbers an
+  // access.  (Tap by tap, number by number, a decode step of 8 rows of 8,192 channels spent 8 us on this.)
+  if (SINGLE && VE > 1 && K >= 2 && K <= 4 && (slot_stride | (long)C) % 4 == 0 && ((uintptr_t)state | (uintptr_t)taps) % 16 == 0) {
+    float w[4][VE], u[4][VE], b[VE];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < K) {
+#pragma unroll
+        for (int e = 0; e < VE; e += 4) {
+          load4(taps + (size_t)j * C + c + e, w[j] + e);
+          if (j < K - 1) load4(st + (size_t)j * C + c + e, u[j] + e);
+        }
+        if (j == K - 1) {
+          if (VE == 8) load8(reinterpret_cast<const __nv_bfloat16*>(src) + (size_t)t * lds + col0 + c, u[j]);
+          else load4(reinterpret_cast<const float*>(src) + (size_t)t * lds + col0 + c, u[j]);
+        }
+      }
+#pragma unroll
+    for (int e = 0; e < VE; ++e) b[e] = bias ? bias[c + e] : 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < K) {
+#pragma unroll
+        for (int e = 0; e < VE; ++e) b[e] = fmaf(w[j][e], u[j][e], b[e]);
+        if (j > 0) {
+#pragma unroll
+          for (int e = 0; e < VE; e += 4) store4(st + (size_t)(j - 1) * C + c + e, u[j] + e);
+        }
+      }
+    T* o = out + (size_t)t * C + c;
+#pragma unroll
+    for (int e = 0; e < VE; ++e) b[e] = b[e] / (1.f + expf(-b[e]));
+#pragma unroll
+    for (int e = 0; e < VE; e += 4) store4(o + e, b + e);
+    return;
+  }
   float acc[VE];
 #pragma unroll
   for (int e = 0; e < VE; ++e) acc[e] = bias ? bias[c + e] : 0.f;
