@@ -240,7 +240,7 @@ __device__ __forceinline__ float gated_act(float g, float u, int kind, float lim
 }
 // Forms of the attention kernels: the softmax, weights sigmoid(score + bias) that are not normalised over keys, and
 // the softmax over scores that were capped, score <- cap * tanh(score / cap).
-enum AttentionForm : int { kFormSoftmax = 0, kFormSigmoid = 1, kFormCapped = 2 };
+enum AttentionForm : int { kFormSoftmax = 0, kFormSigmoid = 1, kFormCapped = 2, kFormBiased = 3 };
 // cap * tanh(x * scale / cap) as cap - 2 cap / (1 + 2^(x * in2)) with in2 = 2 log2(e) scale / cap: the error is a few
 // float32 roundings of cap itself.
 __device__ __forceinline__ float cap_score(float x, float cap, float in2) { return cap - __fdividef(2.f * cap, 1.f + exp2f(x * in2)); }

@@ -761,12 +761,17 @@ def biased_window_attention(q: torch.Tensor, Hq: int, Hkv: int, D: int, pages: t
             if singles is not None and n_single:
                 flash(singles, n_single, int(_lib.load().nf_prefill_attention_shares(c_int(window), c_int(int(ctx.max_context)))))
             if not ctx.all_single and (
-                    sigmoid_bias is not None and gate is None and T >= TUNING["prefill_attention_tc_min_rows"]
+                    (sigmoid_bias is None or gate is None) and T >= TUNING["prefill_attention_tc_min_rows"]
                     and _lib.load().nf_prefill_attention_tc_fits(c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size),
                                                                 c_longlong(pages.shape[0]))):
                 # tcgen05 / TMEM / TMA: tiles of 128 rows, blocks of 128 keys
                 tiles, n_tiles = _tiles(ctx, 128, window, 128, False, 2 if n_single else 1)
-                if n_tiles:
+                if n_tiles and sigmoid_bias is None:
+                    _lib.call("nf_biased_attention_tc", _p(q), c_longlong(T), c_int(q.shape[1]), _p(pages), _p(block_table),
+                              c_int(block_table.shape[1]), _p(ctx.positions), _p(ctx.seg_row0), _p(tiles), c_int(n_tiles),
+                              _p(out), c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size), c_int(pages.shape[0]), c_int(window),
+                              c_float(scale), _p(slopes), c_int(keep), gate_p, c_int(gate_ld), _stream())
+                elif n_tiles:
                     _lib.call("nf_sigmoid_attention_tc", _p(q), c_longlong(T), c_int(q.shape[1]), _p(pages), _p(block_table),
                               c_int(block_table.shape[1]), _p(ctx.positions), _p(ctx.seg_row0), _p(tiles), c_int(n_tiles),
                               _p(out), c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size), c_int(pages.shape[0]), c_int(window),

@@ -1,0 +1,55 @@
+"""The forms of the tcgen05 prefill attention (csrc/attention_prefill_tc.cu) at the edges of a tile and of a window."""
+
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import _step_context, make_cache_case, tol
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D,page", [(64, 32), (128, 64)])
+@pytest.mark.parametrize("window", [0, 1, 129, 200])
+@pytest.mark.parametrize("form", ["softmax", "capped", "sigmoid", "biased"])
+def test_forms_at_the_edges(D, page, window, form, monkeypatch):
+    from ninfer_amd_mi50_b200 import kernels
+    dtype, Hq, Hkv, scale = torch.bfloat16, 4, 2, 1 / math.sqrt(D)
+    seg_lens, pos0s = [2, 127, 128, 129, 255, 256, 257, 385], [700, 0, 5, 127, 0, 128, 63, 300]
+    n_pages = sum((p + n + page - 1) // page for p, n in zip(pos0s, seg_lens)) + 2
+    pages, bt, c, qkv = make_cache_case(dtype, Hq, Hkv, D, page, seg_lens, pos0s, n_pages, 7 + window)
+    bias = torch.linspace(-1.0, 1.0, Hq, device="cuda")
+    gate = torch.linspace(-3.0, 3.0, qkv.shape[0] * (Hq + 1), device="cuda").view(-1, Hq + 1)
+    keep = 5 if window != 129 else 150                # (150: kept keys that reach into a second block)
+
+    def attend(rows, lens, at, table, how):
+        for k, v in how.items():
+            monkeypatch.setitem(kernels.TUNING, k, v)
+        part = type(c)(positions=c.positions[rows], row_seg=torch.repeat_interleave(
+            torch.arange(len(lens), device="cuda"), torch.tensor(lens, device="cuda")).int())
+        ctx = _step_context(part, lens, at, dtype, 1024)
+        q = qkv[rows].contiguous()
+        if form == "sigmoid":
+            return kernels.biased_window_attention(q[:, :Hq * D].contiguous(), Hq, Hkv, D, pages, table, page, ctx, window, 0,
+                                                   scale, None, sigmoid_bias=bias)
+        if form == "biased":
+            return kernels.biased_window_attention(q[:, :Hq * D].contiguous(), Hq, Hkv, D, pages, table, page, ctx, window, keep,
+                                                   scale, 0.01 * (bias + 1.0), gate[rows].contiguous(), 1)
+        return kernels.paged_attention(q, Hq, Hkv, D, pages, table, page, ctx, window, scale,
+                                       softcap=20.0 if form == "capped" else 0.0)
+
+    fast = {"prefill_attention_tc_min_rows": 1, "bf16_attention": "auto"}
+    every = list(range(sum(seg_lens)))
+    out = attend(every, seg_lens, pos0s, bt, fast)
+    assert kernels.tensor_core_status() == 0
+    ref = attend(every, seg_lens, pos0s, bt, {"bf16_attention": "generic"})
+    # sigmoid weights are not normalised: up to 685 of them below 1, each rounded to 2^-9, on values of unit size miss by
+    # 2^-9 / sqrt(3) sqrt(685 / 3) = 0.017 on average, six times that at most
+    torch.testing.assert_close(out.float(), ref.float(), **tol(dtype, 6.4 if form == "sigmoid" else 1.0))
+    # the longest segment again, in portions that begin elsewhere in a tile: a row's sums depend on its position alone
+    first, n, p0 = sum(seg_lens[:-1]), seg_lens[-1], pos0s[-1]
+    for a, b in ((0, 130), (130, n)):
+        rows = list(range(first + a, first + b))
+        again = attend(rows, [b - a], [p0 + a], bt[-1:].contiguous(), fast)
+        assert torch.equal(again, out[rows])
