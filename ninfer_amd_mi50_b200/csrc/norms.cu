@@ -182,7 +182,7 @@ add_group_rmsnorm_kernel(float* __restrict__ h, const T* __restrict__ d1, const 
 // The row-wise norms below in their wide form: a thread owns R runs of four consecutive elements of a row's part, keeps
 // them in registers between the two passes and asks for the weights, which no kernel writes, before the wait.  In a decode
 // step such a kernel is a chain of trips to memory (rows of 2,048 and 4,096 read element by element, twice, with the weight
-// last, took 6 to 10 us), in a prompt it moves each row once.  Four layers of 2,048, prompts of 900 to 2,048 tokens and 16
+// last, took 6 to 10 us, now 3 to 5), in a prompt it moves each row once.  Four layers of 2,048, prompts of 900 to 2,048 tokens and 16
 // decoded ones: latent attention and scans 5.43 -> 5.09 ms, linear and windowed attention 6.93 -> 6.28, attention beside
 // scans and delta rules 10.87 -> 10.55.
 // MODE 0: out = x / rms(x) * w.  1: x = y * silu(z), out = x / rms(x) * w.  2, 3: out = y / rms(y) * w * act(z), act the

