@@ -333,7 +333,20 @@ router_cluster_kernel(const T* __restrict__ x, const float* __restrict__ wr, int
     select_token<false>(lg_all + (size_t)tt * rows, 1, sel + warp * E, tt, E, extra, k, norm_topk, topk_idx, topk_w,
                         extra_out, lane, chosen, bias);
   __syncthreads();
-  for (int e = warp; e < E; e += 8) {
+  // up to 32 pairs: one warp ranks them by a match and goes on to the offsets without meeting the others again
+  const bool few = n <= 32;
+  if (few && warp > 0) return;
+  int my_e = -1, my_rank = 0;
+  if (few) {
+    for (int e = lane; e < E; e += 32) counts[e] = 0;
+    if (lane < n) my_e = (int)chosen[lane];
+    const unsigned peers = __match_any_sync(0xffffffffu, my_e);
+    my_rank = __popc(peers & ((1u << lane) - 1u));
+    __syncwarp();
+    if (my_e >= 0 && my_rank == 0) counts[my_e] = __popc(peers);
+    __syncwarp();
+  }
+  for (int e = few ? E : warp; e < E; e += 8) {
     int running = 0;
     for (int base = 0; base < n; base += 32) {
       const int i = base + lane;
@@ -344,7 +357,7 @@ router_cluster_kernel(const T* __restrict__ x, const float* __restrict__ wr, int
     }
     if (lane == 0) counts[e] = running;
   }
-  __syncthreads();
+  if (!few) __syncthreads();
   if (warp == 0) {
     // one warp, 32 experts a round: exclusive prefix of the counts (-> offsets) and the list of
     // the experts that have pairs, ascending, then -1
@@ -372,6 +385,15 @@ router_cluster_kernel(const T* __restrict__ x, const float* __restrict__ wr, int
     }
     if (active)
       for (int i = min(na, n_active_max) + lane; i < n_active_max; i += 32) active[i] = -1;
+  }
+  if (few) {
+    __syncwarp();
+    if (my_e >= 0) {
+      const int p = counts[my_e] + my_rank;
+      inv[lane] = p;
+      order[p] = lane;
+    }
+    return;
   }
   __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) {

@@ -99,6 +99,17 @@ __device__ __forceinline__ void select_token(const float* row, long exp_stride, 
   if (bad) sum = 1.f;
   __syncwarp();
   float sel_sum = 0.f;
+  // Up to 128 experts: a lane's four in registers, as integers in the probabilities' order plus one (0: taken or none), so
+  // that a choice is two reductions of the warp (the largest, then its lowest expert) instead of ten shuffles in a chain.
+  // Four of 60 experts for one row: the whole routing 7.3 -> 5.6 us, eight rows 10.8 -> 9.3.
+  constexpr int kOwn = 4;
+  const bool own = E <= 32 * kOwn;
+  unsigned key[kOwn];
+#pragma unroll
+  for (int c = 0; c < kOwn; ++c) {
+    const int e = lane + 32 * c;
+    key[c] = own && e < E ? __float_as_uint(lg[e]) + 1u : 0u;
+  }
   for (int j0 = 0; j0 < k; j0 += 32) {
     // lane j - j0 keeps the weight of choice j until the sum of the selected is known
     float mine = 0.f;
@@ -106,21 +117,33 @@ __device__ __forceinline__ void select_token(const float* row, long exp_stride, 
     for (int j = j0; j < j1; ++j) {
       float best = -1.f;
       int best_e = 0x7fffffff;
-      for (int e = lane; e < E; e += 32) {
-        const float p = lg[e];
-        if (p > best) { best = p; best_e = e; }     // ascending e: first maximum wins
-      }
+      if (own) {
+        const unsigned top = __reduce_max_sync(0xffffffffu, max(max(key[0], key[1]), max(key[2], key[3])));
+        best = __uint_as_float(top - 1u);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-        if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
+        for (int c = kOwn - 1; c >= 0; --c)
+          if (key[c] == top) best_e = lane + 32 * c;
+        best_e = __reduce_min_sync(0xffffffffu, best_e);
+#pragma unroll
+        for (int c = 0; c < kOwn; ++c)
+          if (best_e == lane + 32 * c) key[c] = 0u;
+      } else {
+        for (int e = lane; e < E; e += 32) {
+          const float p = lg[e];
+          if (p > best) { best = p; best_e = e; }     // ascending e: first maximum wins
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+          const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
+          if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
+        }
       }
       // (k <= E and every probability is >= 0 > -1, and a taken one is -2: best_e is a valid expert)
       if (lane == 0) {
         if (topk_idx) topk_idx[(size_t)t * k + j] = best_e;
         if (chosen) chosen[(size_t)t * k + j] = (unsigned short)best_e;
-        lg[best_e] = -2.f;                           // taken
+        if (!own) lg[best_e] = -2.f;                 // taken
       }
       if (lane == j - j0) mine = bad ? __int_as_float(0x7fc00000) : best / sum;
       sel_sum += best / sum;
