@@ -518,6 +518,12 @@ extern "C" int nf_scale_gather_rows(const void* x, const int* order, int div, co
 // ---------------------------------------------------------------------------------------------
 namespace nf {
 
+// One element of the update, in the kernels below to the last bit alike: (d / rms) * w (* scale) added to the stream.
+__device__ __forceinline__ float scaled_norm_sum(float d, float inv, float w, const float* ls, float scale, float h) {
+  const float t = d * inv;
+  return ls ? fmaf(t * w, scale, h) : fmaf(t, w, h);
+}
+
 template <typename TD, typename TO>
 __global__ void scaled_norm_add_kernel(float* __restrict__ h, const TD* __restrict__ delta,
                                        const float* __restrict__ bias, const float* __restrict__ w,
@@ -531,66 +537,62 @@ __global__ void scaled_norm_add_kernel(float* __restrict__ h, const TD* __restri
   float ss = 0.f;
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
     const float d = to_float(dr[i]) + (bias ? bias[i] : 0.f);
-    ss += d * d;
+    ss = fmaf(d, d, ss);
   }
   const float inv = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
     const float d = to_float(dr[i]) + (bias ? bias[i] : 0.f);
-    float v = d * inv * w[i];
-    if (ls) v *= ls[i];
-    v += hr[i];
+    const float v = scaled_norm_sum(d, inv, w[i], ls, ls ? ls[i] : 1.f, hr[i]);
     hr[i] = v;
     if (out) out[(size_t)r * hidden + i] = from_float<TO>(v);
   }
 }
 
-// The wide form (see part_norm_vec_kernel): runs of four, the row in registers, weights before the wait.
+// Rows of up to R numbers a thread: the same sums in the same order, with the row in registers between the two passes, all
+// its numbers asked for at once and the weights, which no kernel writes, before the wait (see part_norm_vec_kernel).
 template <typename TD, typename TO, int R>
 __global__ void __launch_bounds__(512)
-scaled_norm_add_vec_kernel(float* __restrict__ h, const TD* __restrict__ delta, const float* __restrict__ bias,
-                           const float* __restrict__ w, const float* __restrict__ ls, float eps, TO* __restrict__ out, int hidden) {
+scaled_norm_add_regs_kernel(float* __restrict__ h, const TD* __restrict__ delta, const float* __restrict__ bias,
+                            const float* __restrict__ w, const float* __restrict__ ls, float eps, TO* __restrict__ out, int hidden) {
   __shared__ float red[33];
   const int r = blockIdx.x;
   chain_release_if_small();
-  float wk[R][4], lk[R][4], bk[R][4], d[R][4], v[R][4];
+  float wk[R], lk[R], d[R], hk[R];
 #pragma unroll
   for (int c = 0; c < R; ++c) {
-    const int i = (c * blockDim.x + threadIdx.x) * 4;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) { wk[c][e] = lk[c][e] = 1.f; bk[c][e] = d[c][e] = v[c][e] = 0.f; }
+    const int i = c * blockDim.x + threadIdx.x;
+    wk[c] = lk[c] = 1.f;
+    d[c] = hk[c] = 0.f;
     if (i < hidden) {
-      load4(w + i, wk[c]);
-      if (ls) load4(ls + i, lk[c]);
-      if (bias) load4(bias + i, bk[c]);
+      wk[c] = w[i];
+      if (ls) lk[c] = ls[i];
+      if (bias) d[c] = bias[i];
     }
   }
   chain_wait(h, delta);
   float* hr = h + (size_t)r * hidden;
+  const TD* dr = delta + (size_t)r * hidden;
+  TD raw[R];
 #pragma unroll
   for (int c = 0; c < R; ++c) {
-    const int i = (c * blockDim.x + threadIdx.x) * 4;
-    if (i < hidden) {
-      load4(delta + (size_t)r * hidden + i, d[c]);
-      load4(hr + i, v[c]);
-    }
+    const int i = c * blockDim.x + threadIdx.x;
+    if (i < hidden) { raw[c] = dr[i]; hk[c] = hr[i]; }
   }
   float ss = 0.f;
 #pragma unroll
   for (int c = 0; c < R; ++c)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      d[c][e] += bk[c][e];
-      ss += d[c][e] * d[c][e];
+    if (c * (int)blockDim.x + (int)threadIdx.x < hidden) {
+      d[c] = to_float(raw[c]) + d[c];
+      ss = fmaf(d[c], d[c], ss);
     }
   const float inv = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
 #pragma unroll
   for (int c = 0; c < R; ++c) {
-    const int i = (c * blockDim.x + threadIdx.x) * 4;
+    const int i = c * blockDim.x + threadIdx.x;
     if (i >= hidden) continue;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) v[c][e] += d[c][e] * inv * wk[c][e] * lk[c][e];
-    store4(hr + i, v[c]);
-    if (out) store4(out + (size_t)r * hidden + i, v[c]);
+    const float v = scaled_norm_sum(d[c], inv, wk[c], ls, lk[c], hk[c]);
+    hr[i] = v;
+    if (out) out[(size_t)r * hidden + i] = from_float<TO>(v);
   }
 }
 
@@ -615,14 +617,12 @@ __global__ void routed_scaled_norm_add_kernel(float* __restrict__ h, const T* __
     }
     const float d = to_float(from_float<T>(acc));
     row[i] = d;
-    ss += d * d;
+    ss = fmaf(d, d, ss);
   }
   const float invr = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
   float* hr = h + (size_t)r * hidden;
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-    float v = row[i] * invr * w[i];
-    if (ls) v *= ls[i];
-    v += hr[i];
+    const float v = scaled_norm_sum(row[i], invr, w[i], ls, ls ? ls[i] : 1.f, hr[i]);
     hr[i] = v;
     if (out) out[(size_t)r * hidden + i] = from_float<TO>(v);
   }
@@ -752,14 +752,12 @@ extern "C" int nf_scaled_norm_add(float* h, const void* delta, int delta_dtype, 
   if (R == 0) return 0;
   NF_REQUIRE(R > 0 && hidden > 0 && h && delta && w, "scaled_norm_add: bad arguments R=%d hidden=%d", R, hidden);
   const dim3 grid(R), block(norm_threads(hidden));
-  const bool vec = hidden % 4 == 0 && hidden <= 8192 && runs_of_four(h, 4, 0, 0) && runs_of_four(delta, delta_dtype == kF32 ? 4 : 2, 0, 0) &&
-                   runs_of_four(out, out_dtype == kF32 ? 4 : 2, 0, 0) && ((uintptr_t)w | (uintptr_t)ls | (uintptr_t)bias) % 16 == 0;
-  const int units = hidden / 4, runs = units <= 512 ? 1 : (units <= 1024 ? 2 : 4), th = ((units + runs - 1) / runs + 31) / 32 * 32;
+  const int each = (hidden + (int)block.x - 1) / (int)block.x;
 #define NF_SNV(TD, TO, RR) \
-  launch_chained(scaled_norm_add_vec_kernel<TD, TO, RR>, grid, dim3(th), 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden)
+  launch_chained(scaled_norm_add_regs_kernel<TD, TO, RR>, grid, block, 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden)
 #define NF_SNA(TD, TO)                                                                                                     \
   do {                                                                                                                     \
-    if (vec) { if (runs == 1) NF_SNV(TD, TO, 1); else if (runs == 2) NF_SNV(TD, TO, 2); else NF_SNV(TD, TO, 4); }          \
+    if (each <= 4) NF_SNV(TD, TO, 4); else if (each <= 8) NF_SNV(TD, TO, 8); else if (each <= 16) NF_SNV(TD, TO, 16);      \
     else launch_chained(scaled_norm_add_kernel<TD, TO>, grid, block, 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden); \
   } while (0)
   if (delta_dtype == kF32) { if (out_dtype == kF32) NF_SNA(float, float); else NF_SNA(float, __nv_bfloat16); }
