@@ -283,6 +283,7 @@ def work_models(s: dict, prompt: int, batch: int, context: int, design: str = ""
             "nf_pair_hash_embed": (T * W * (2 + 4 + 4), 0.0),
             "nf_latent_attention_generic": (rows_ctx * Wl * 2 + 2 * T * H * R * 2, 2.0 * H * (Wl + R) * pairs),
             "nf_latent_attention_mma": (rows_ctx * Wl * 2 + 2 * T * H * R * 2, 2.0 * H * (Wl + R) * pairs),
+            "nf_dense_rot_attention_tc": (rows_ctx * (2 * H * D + Dr) * 2 + T * H * (2 * D + Dr) * 2, 2.0 * H * (2 * D + Dr) * pairs),
             "nf_prefill_attention_tc": (rows_ctx * 2 * H * D * 2 + 2 * T * H * D * 2, 4.0 * H * D * pairs),
             "nf_prefill_attention": (rows_ctx * 2 * H * D * 2 + 2 * T * H * D * 2, 4.0 * H * D * pairs),
             "nf_decode_attention": (rows_ctx * 2 * H * D * 2 + 2 * T * H * D * 2, 4.0 * H * D * pairs),
@@ -302,6 +303,11 @@ def work_models(s: dict, prompt: int, batch: int, context: int, design: str = ""
             "nf_gather_rows": (T * s["top"] * W * 4, 0.0),
         }
         table.update(own)
+        # prompt forms of the same work: recurrences in chunks, windowed attention on the tcgen05 kernel
+        for entry, like in (("nf_chunk_scan", "nf_ssd_scan"), ("nf_chunk_linear_attention", "nf_decay_linear_attention"),
+                            ("nf_chunk_delta_rule", "nf_delta_rule"), ("nf_biased_attention_tc", "nf_prefill_attention_biased")):
+            if like in table:
+                table[entry] = table[like]
         return table
 
     keep = 0 if design == "pudizen" else KEEP_FIRST
