@@ -79,7 +79,7 @@ __device__ __forceinline__ void cluster_meet() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 constexpr int kClusterSplits = 8;  // most key blocks of a row that one cluster takes (the portable cluster size)
-constexpr int kClusterCtas = 256;  // most CTAs of such a launch (see launch_split)
+constexpr int kClusterCtas = 148;  // most CTAs of such a launch (see launch_split)
 
 template <int D, int FORM, bool CLUSTER>
 __global__ void __launch_bounds__(128)
@@ -482,10 +482,12 @@ static int launch_split(const void* qkv, int q_row_stride, const void* pages, co
   NF_REQUIRE(smem <= 200 * 1024, "decode attention: %d query heads per kv head need too much shared memory", G);
   dim3 grid(T, Hkv, nsplit);
   const size_t smem_c = smem + (size_t)G * D * sizeof(float);
-  // At most 256 CTAs: one row of 16 key heads 14.4 -> 12.4 us for all launches of the attention, two rows of eight blocks
-  // 14.6 -> 12.6; but four rows (512 CTAs) 14.6 both ways, eight 15.2 -> 23 and 16 of four key heads 14.6 -> 19: clusters
-  // start as a whole, with three CTAs' shared memory on an SM, where single CTAs trickle in and empty ones leave at once.
-  if (*merged && nsplit <= kClusterSplits && smem_c <= 100 * 1024 && (long long)T * Hkv * nsplit <= kClusterCtas) {
+  // At most one CTA a SM (in a chain of such calls: one row of 16 key heads 5.5 -> 4.2 us, of 1,000 keys 6.4 -> 4.8, eight
+  // rows of one block 6.1 -> 4.6): clusters start as a whole, where single CTAs trickle in and empty ones leave at once
+  // (256 CTAs: two rows of eight blocks 5.8 -> 7.4; 512: four rows 5.9 -> 13.7).  And enough CTAs a row for its heads: a
+  // thread adds up at most four numbers (28 heads on four key heads, one block: 6.5 -> 7.1, in four blocks 6.5 -> 5.6).
+  if (*merged && nsplit <= kClusterSplits && smem_c <= 100 * 1024 && (long long)T * Hkv * nsplit <= kClusterCtas &&
+      G * D <= 4 * 128 * nsplit) {
     static size_t allowed_c = 48 * 1024;
     if (smem_c > allowed_c) {
       cudaFuncSetAttribute(decode_attention_split_kernel<D, FORM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c);
