@@ -278,8 +278,20 @@ __device__ __forceinline__ void ms_route(const MsArgs& p, float* scratch, int* s
         select_token(p.logits + (size_t)tt * rows, 1, lg + warp * p.E, tt, p.E, p.extra, p.k, p.norm_topk, nullptr,
                      sw, p.extra > 0 ? sext : nullptr, lane, chosen, p.rbias);
       consumers_sync();
-      // stable counting sort of the pairs by expert
-      for (int e2 = warp; e2 < p.E; e2 += kMsConsumers) {
+      // stable counting sort of the pairs by expert: up to 32 of them by one warp, which goes on without meeting
+      // the others (eight requests' decoded tokens over 12 layers 60.0 -> 59.6 ms)
+      const bool few = n <= 32;
+      if (few && warp == 0) {
+        for (int e2 = lane; e2 < p.E; e2 += 32) counts[e2] = 0;
+        const int mine = lane < n ? (int)chosen[lane] : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, mine);
+        const int before = __popc(peers & ((1u << lane) - 1u));
+        if (mine >= 0) rank[lane] = (unsigned short)before;
+        __syncwarp();
+        if (mine >= 0 && before == 0) counts[mine] = __popc(peers);
+        __syncwarp();
+      }
+      for (int e2 = few ? p.E : warp; e2 < p.E; e2 += kMsConsumers) {
         int running = 0;
         for (int base = 0; base < n; base += 32) {
           const int i = base + lane;
@@ -290,7 +302,7 @@ __device__ __forceinline__ void ms_route(const MsArgs& p, float* scratch, int* s
         }
         if (lane == 0) counts[e2] = running;
       }
-      consumers_sync();
+      if (!few) consumers_sync();
       if (warp == 0) {
         // 32 experts a round: offsets (exclusive prefix of the counts), the experts that have pairs,
         // and their rows eight at a time
