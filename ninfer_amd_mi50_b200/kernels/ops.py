@@ -43,6 +43,10 @@ TUNING = {
     # take at most `latent_expand_max_mb`; a huge number keeps every row on the latent kernel
     "latent_expand_min_rows": 128,
     "latent_expand_max_mb": 1024,
+    # ... with a rotated part from this many operations of the folded form on (it runs them at 160 TFLOP/s, and expanding
+    # costs a layer some 80 us of launches and copies: 29 short prompts on 8 heads, 1.5e9 a step, took 6.4 ms expanded and
+    # 5.6 folded; a prompt of 2,048 rows on 16 heads, 73e9, 455 us folded and 39 beside its expansion)
+    "latent_expand_rotated_min_ops": 12e9,
     # recurrences over prompt portions: segments of at least this many rows run as chunks on tensor cores (three launches
     # that fill the device with a few hundred rows, where walking the rows costs the same each: the selective scan of 64
     # heads takes 44 us against 55 at 128 rows, 32 against 32 at 64; linear attention of 16 heads of 128 x 128 takes 62
@@ -1818,6 +1822,10 @@ def can_expand_latent(q: torch.Tensor, heads: int, D: int, Dv: int, R: int, ctx,
         return False
     rows = sum(n for n in ctx.seg_len_host if n > 1)
     held = sum(p + n for p, n in zip(ctx.seg_pos0_host, ctx.seg_len_host) if n > 1)
+    if Dr:
+        pairs = sum(n * p + n * (n + 1) // 2 for p, n in zip(ctx.seg_pos0_host, ctx.seg_len_host) if n > 1)
+        if 2 * heads * (2 * R + Dr) * pairs < TUNING["latent_expand_rotated_min_ops"]:
+            return False
     return rows >= TUNING["latent_expand_min_rows"] and held * 2 * heads * D * 2 <= TUNING["latent_expand_max_mb"] << 20
 
 
