@@ -51,10 +51,12 @@ TUNING = {
     # that fill the device with a few hundred rows, where walking the rows costs the same each: the selective scan of 64
     # heads takes 44 us against 55 at 128 rows, 32 against 32 at 64; linear attention of 16 heads of 128 x 128 takes 62
     # against 134 at 512 rows, 57 against 44 at 128; the delta rule of 16 heads of 128 x 128 takes 68 against 118 at 512
-    # rows, 52 against 40 at 128); a huge number leaves every row to the kernels that walk them
-    "chunk_scan_min_rows": 96,
-    "chunk_linear_min_rows": 192,
-    "chunk_delta_min_rows": 192,
+    # rows, 52 against 40 at 128); a huge number leaves every row to the kernels that walk them.
+    # Between 96 and 256 rows a single segment gains a little, but a step of many such segments, which the walking kernels
+    # serve side by side, pays for the further launches: 29 prompts of 35 to 279 rows 6.1 ms against 5.6)
+    "chunk_scan_min_rows": 256,
+    "chunk_linear_min_rows": 256,
+    "chunk_delta_min_rows": 256,
     "chunk_recurrence_max_mb": 512,      # scratch for the chunks' states; a longer step's chunks run group after group
     "qkv_rope_fused": True,       # few bfloat16 rows: rotation and cache append in the projection's epilogue
     "router_tensor_min_rows": 128,   # router logits of more rows than this use tensor cores
