@@ -14,6 +14,10 @@
 // chunks and heads at once.  Chunks are counted from a segment's first row of the step.  Decays are products, never
 // quotients or differences of logarithms, so a decay near zero does no harm.
 //
+// A row's result holds what the rows up to it hold and nothing of the later ones, whatever their numbers are: a zero weight
+// is no protection from an infinity or a NaN (0 * inf), so on the diagonal the scores of later keys are left out by a
+// choice, and a product there that came out other than finite is done again without the values that are not.
+//
 // Everything beyond the activations stays float32 in what it carries: a float32 operand goes to the bfloat16 tensor
 // cores as three bfloat16 parts (8 + 8 + 8 bits: the number itself), a bfloat16 one as it is, and the partial
 // products whose weight is at least 2^-16 of the leading one are all taken (three where one operand is bfloat16, six
@@ -84,6 +88,15 @@ __device__ __forceinline__ void cr_zero(float (&t)[N][4]) {
 __device__ __forceinline__ void cr_add(float (&c)[4], const float (&t)[4]) {
 #pragma unroll
   for (int e = 0; e < 4; ++e) c[e] += t[e];
+}
+__device__ __forceinline__ bool cr_finite(const float (&t)[4]) {
+  return fabsf(t[0]) < INFINITY && fabsf(t[1]) < INFINITY && fabsf(t[2]) < INFINITY && fabsf(t[3]) < INFINITY;
+}
+// A packed pair with zeros for what is not finite.
+__device__ __forceinline__ unsigned cr_finite_only(unsigned x) {
+  if ((x & 0x7f800000u) == 0x7f800000u) x &= 0x0000ffffu;
+  if ((x & 0x00007f80u) == 0x00007f80u) x &= 0xffff0000u;
+  return x;
 }
 // Two neighbouring numbers as PARTS packed pairs of bfloat16 that add up to them.  What has no remainder (an infinity,
 // a NaN) stands in the first part alone.
@@ -473,8 +486,8 @@ chunk_output_kernel(const CrArgs args) {
         for (int n = 0; n < 2; ++n)
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const int s = n * 8 + t4 * 2 + (e & 1);
-            p[n][e] *= s_diag[rb][s][g + (e >> 1) * 8] * s_weight[b * 16 + s];
+            const int s = n * 8 + t4 * 2 + (e & 1), t = g + (e >> 1) * 8;
+            p[n][e] = s > t ? 0.f : p[n][e] * (s_diag[rb][s][t] * s_weight[b * 16 + s]);
           }
       } else {
         float between = 1.f;
@@ -514,6 +527,39 @@ chunk_output_kernel(const CrArgs args) {
           for (int i = 2 - j; i >= 0; --i) {
             cr_mma(t[0], P[i], B[0], B[1]);
             cr_mma(t[1], P[i], B[2], B[3]);
+          }
+        }
+        if (b == rb && __any_sync(0xffffffffu, !cr_finite(t[0]) || !cr_finite(t[1]))) {
+          // a value that is not finite met the zero weight of an earlier row: once more without such values, which then
+          // go to their own row and the later ones
+          cr_zero(t);
+#pragma unroll
+          for (int j = VP - 1; j >= 0; --j) {
+            unsigned B[4];
+            cr_ldm4t(vb + ((j * SUB + sb) * VS + n * 8) * 2, B);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) B[i] = cr_finite_only(B[i]);
+#pragma unroll
+            for (int i = 2 - j; i >= 0; --i) {
+              cr_mma(t[0], P[i], B[0], B[1]);
+              cr_mma(t[1], P[i], B[2], B[3]);
+            }
+          }
+#pragma unroll 1
+          for (int s = 0; s < 16; ++s) {
+            const float x0 = s & 8 ? (s & 1 ? p[1][1] : p[1][0]) : (s & 1 ? p[0][1] : p[0][0]);
+            const float x1 = s & 8 ? (s & 1 ? p[1][3] : p[1][2]) : (s & 1 ? p[0][3] : p[0][2]);
+            const float w0 = __shfl_sync(0xffffffffu, x0, (lane & 28) | ((s & 7) >> 1));
+            const float w1 = __shfl_sync(0xffffffffu, x1, (lane & 28) | ((s & 7) >> 1));
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const float v = __bfloat162float(Vs[(size_t)(sb + s) * VS + n0 + (n + j) * 8 + t4 * 2 + e]);
+                if (fabsf(v) < INFINITY) continue;
+                if (s <= g) t[j][e] = fmaf(w0, v, t[j][e]);
+                if (s <= g + 8) t[j][e + 2] = fmaf(w1, v, t[j][e + 2]);
+              }
           }
         }
         cr_add(acc[n], t[0]);
@@ -732,7 +778,7 @@ delta_chunk_solve_kernel(const DcArgs args) {
         for (int e = 0; e < 4; ++e) r[e] = fmaf(-m[e], x[s + e], r[e]);
       }
       x[t] = (r[0] + r[1]) + (r[2] + r[3]);
-      float v = x[t] * beta;
+      float v = t < j ? 0.f : x[t] * beta;     // (also where beta is not a number)
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
         const __nv_bfloat16 h = __float2bfloat16_rn(v);
@@ -853,12 +899,17 @@ delta_chunk_chain_kernel(const DcArgs args) {
       cr_zero(u);
       const unsigned ta = cr_smem(Ts + (b * 3 * Q + mt * 16 + (mat & 1) * 8 + r8) * TS + (mat >> 1) * 8);
       const unsigned xb = cr_smem(Xs + (lane & 15) * XS + nt * 8);
-      for (int ks = 0; ks <= mt; ++ks) {
+      // u += the sixteen ks of T times X; apart: the values of X that are not finite are left out
+      auto add_sixteen = [&](int ks, bool apart) {
         unsigned A[3][4], B[3][2];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
           cr_ldm4(ta + (i * Q * TS + ks * 16) * 2, A[i]);
           cr_ldm2t(xb + ((i * Q + ks * 16) * XS) * 2, B[i][0], B[i][1]);
+          if (apart) {
+            B[i][0] = cr_finite_only(B[i][0]);
+            B[i][1] = cr_finite_only(B[i][1]);
+          }
         }
         float t[3][4];                             // (three chains side by side: this is the walk from chunk to chunk)
         cr_zero(t);
@@ -870,6 +921,25 @@ delta_chunk_chain_kernel(const DcArgs args) {
         cr_mma(t[2], A[2], B[0][0], B[0][1]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) u[0][e] += t[0][e] + (t[1][e] + t[2][e]);
+      };
+      for (int ks = 0; ks <= mt; ++ks) add_sixteen(ks, false);
+      if (__any_sync(0xffffffffu, !cr_finite(u[0]))) {                       // (see the outputs)
+        cr_zero(u);
+#pragma unroll 1
+        for (int ks = 0; ks <= mt; ++ks) add_sixteen(ks, ks == mt);
+        auto whole = [&](const __nv_bfloat16* x) {
+          return (__bfloat162float(x[0]) + __bfloat162float(x[Q * TS])) + __bfloat162float(x[2 * Q * TS]);
+        };
+        const __nv_bfloat16* tp = Ts + ((size_t)b * 3 * Q + tr) * TS + mt * 16;
+#pragma unroll 1
+        for (int j = 0; j < 16; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float x = __bfloat162float(Xs[(mt * 16 + j) * XS + col + e]);
+            if (fabsf(x) < INFINITY) continue;
+            if (j <= g) u[0][e] = fmaf(whole(tp + j), x, u[0][e]);
+            if (j <= g + 8) u[0][e + 2] = fmaf(whole(tp + 8 * TS + j), x, u[0][e + 2]);
+          }
       }
       float* dst = a.u + (size_t)(row0 + tr) * a.H * a.V + (size_t)head * a.V + v0 + col;
       if (tr < live) *reinterpret_cast<float2*>(dst) = make_float2(u[0][0], u[0][1]);

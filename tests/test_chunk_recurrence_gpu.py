@@ -155,3 +155,50 @@ def test_delta_rule_in_chunks(lens, D, V, alike, monkeypatch):
     for slot in (0, len(lens) + 1):
         assert torch.equal(state[slot].double(), before[slot])
     assert torch.equal(state[:, :off].double(), before[:, :off])
+
+
+@pytest.mark.parametrize("kind", ["scan", "linear", "delta"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [5, 70, 139])
+def test_what_is_not_finite_stays_behind_its_row(kind, bad, at, monkeypatch):
+    """A query, key, value or gate that is not a number, or infinite, leaves the rows before it as they were, bit for bit;
+    a value also every other column of its head."""
+    from ninfer_amd_mi50_b200 import kernels
+    monkeypatch.setitem(kernels.TUNING, f"chunk_{kind}_min_rows", 63)
+    lens, g = [141, 64], torch.Generator(device="cuda").manual_seed(at)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ctx, T = context(lens), sum(lens)
+    H, G, D, V = 4, 2, 128, 64 if kind == "scan" else 128
+    keys = H if kind == "linear" else G                       # heads that q and k have
+    src, gates = rand(T, 2 * keys * D + H * V).bfloat16(), rand(T, 2 * H).bfloat16()
+    q0, k0, v0 = 0, keys * D, 2 * keys * D
+    bias, rate, first = rand(H), rand(H), rand(len(lens) + 2, H * V * D)
+
+    def run(src, gates):
+        state = first.clone()
+        if kind == "scan":
+            out = kernels.ssd_scan(src, v0, k0, q0, gates, 0, bias, rate, bias, state, 0, ctx, H, V, D, G)
+        elif kind == "linear":
+            out = kernels.decay_linear_attention(src, q0, k0, v0, torch.sigmoid(bias), None, 0, 1.0, False, state, ctx, H, D, V)
+        else:
+            out = kernels.delta_rule(src, q0, k0, v0, gates, 0, H, bias, rate, 0.1, state, 0, ctx, H, G, D, V)
+        return out.view(T, H, V), state.view(-1, H, V, D)
+
+    want, end = run(src, gates)
+    assert want.isfinite().all() and end.isfinite().all()
+    for col, of_row in ((q0 + 3, True), (k0 + 3, False), (v0 + 7, False)) + (((None, False),) if kind != "linear" else ()):
+        s, ga = src.clone(), gates.clone()
+        (ga if col is None else s)[at, 0 if col is None else col] = bad
+        if col is None and bad > 0 and kind == "scan":
+            continue                                          # (an infinite step size: a decay of nothing, fine to walk over)
+        out, state = run(s, ga)
+        assert torch.equal(out[:at], want[:at]), (col, "rows before")
+        assert torch.equal(out[lens[0]:], want[lens[0]:]) and torch.equal(state[1], end[1]), (col, "the other request")
+        if col == v0 + 7:
+            assert not out[at:lens[0], 0, 7].isfinite().any() and not state[2, 0, 7].isfinite().all()
+            others = torch.arange(V, device="cuda") != 7
+            assert torch.equal(out[:, 0, others], want[:, 0, others]) and torch.equal(out[:, 1:], want[:, 1:])
+        elif of_row:
+            assert not out[at, 0].isfinite().any() and torch.equal(out[at + 1:], want[at + 1:]) and torch.equal(state, end)
+        elif not (col is None and bad > 0):                   # (an infinite gate of the delta rule forgets everything)
+            assert not out[at, 0].isfinite().any()
