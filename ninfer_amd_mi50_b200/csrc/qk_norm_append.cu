@@ -154,10 +154,9 @@ qk_whole_norm_append_vec_kernel(const float* __restrict__ proj, int ld, int q_co
 // The row's normed values wait in shared memory (float32) between the two passes.
 // VEC: all sizes are multiples of 4 (the turned halves too): runs of four elements an access, and the norm's
 // factors are applied where the values are read for the second time.
-// Steps that leave SMs idle (up to one row each) give a row 512 threads instead of 256: the kernel is a chain of trips to
-// memory there, and half as many follow one another.
+// 256 threads a row whatever the step holds: the order of the norms' sums hangs on the number of threads.
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(256)
 whole_norm_rope_append_kernel(const float* __restrict__ proj, int ld, int q_col0, int k_col0, int v_col0,
                               const float* __restrict__ bias_q, const float* __restrict__ bias_k,
                               const float* __restrict__ bias_v, const float* __restrict__ wq,
@@ -526,7 +525,7 @@ extern "C" int nf_whole_norm_rope_append(const float* proj, int ld, int q_col0, 
 #define NF_WN(TT, VE)                                                                                                  \
   do {                                                                                                                \
     if (smem > 48 * 1024) cudaFuncSetAttribute(whole_norm_rope_append_kernel<TT, VE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    launch_chained(whole_norm_rope_append_kernel<TT, VE>, dim3(T), dim3(T <= 148 ? 512 : 256), smem, stream, proj, ld, q_col0, k_col0, \
+    launch_chained(whole_norm_rope_append_kernel<TT, VE>, dim3(T), dim3(256), smem, stream, proj, ld, q_col0, k_col0, \
                    v_col0, bias_q, bias_k, bias_v, wq, wk, eps, inv_freq, rot, mag, positions, row_seg, (TT*)q_out,   \
                    Hq, Hkv, D, Dv, (TT*)pages, block_table, bt_width, page_size, num_pages, rows_layout, P,           \
                    interleaved, v_freq);                                                                              \

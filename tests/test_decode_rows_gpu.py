@@ -57,3 +57,25 @@ def test_norm_over_whole_rows(Hq, Hkv, D, with_bias, dtype):
         held = pages[table[t, 0], :, :, 7 * t]
         assert near(held[0].reshape(-1), (rms(k) * wk.double())[t]) and near(held[1].reshape(-1), k[t])
     assert int((pages != 0).any(-1).sum()) == 2 * Hkv * T
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_row_normed_in_steps_of_any_size(dtype):
+    """The norm over whole rows before a rotation: a row's bits do not hang on how many rows the step has."""
+    from ninfer_amd_mi50_b200 import kernels
+    Hq, Hkv, D, page, n = 17, 3, 64, 16, 149
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    proj, wq, wk, freq = rand(n, (Hq + 2 * Hkv) * D), rand(Hq * D), rand(Hkv * D), rand(16)
+    seen = []
+    for T in (1, 148, 149):
+        ctx = context([1] * T)
+        ctx.positions = torch.arange(T, dtype=torch.int32, device="cuda") % page
+        pages = torch.zeros(n, 2, Hkv, page, D, dtype=dtype, device="cuda")
+        table = torch.arange(T, dtype=torch.int32, device="cuda").view(T, 1)
+        q = kernels.whole_norm_rope_append(proj[:T], 0, Hq * D, (Hq + Hkv) * D, None, None, None, wq, wk, 1e-5, freq, 32, 1.0,
+                                           Hq, Hkv, D, D, ctx, pages, table, page, dtype)
+        seen.append((q, pages))
+    for q, pages in seen[:2]:
+        T = q.shape[0]
+        assert torch.equal(q, seen[2][0][:T]) and torch.equal(pages[:T], seen[2][1][:T])
