@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import ctypes
 from dataclasses import dataclass
-from typing import Optional, Sequence, Tuple
+from typing import List, Optional, Sequence, Tuple
 
 import torch
 
@@ -43,10 +43,13 @@ TUNING = {
     # take at most `latent_expand_max_mb`; a huge number keeps every row on the latent kernel
     "latent_expand_min_rows": 128,
     "latent_expand_max_mb": 1024,
-    # ... with a rotated part from this many operations of the folded form on (it runs them at 160 TFLOP/s, and expanding
-    # costs a layer some 80 us of launches and copies: 29 short prompts on 8 heads, 1.5e9 a step, took 6.4 ms expanded and
-    # 5.6 folded; a prompt of 2,048 rows on 16 heads, 73e9, 455 us folded and 39 beside its expansion)
-    "latent_expand_rotated_min_ops": 12e9,
+    # ... with a rotated part a segment by itself, from this many operations of its folded form on (it runs them at 160
+    # TFLOP/s; the rows beside it keep that form, so that a step's host has both forms' launches to make).  Steps of four
+    # layers, two of them with latents, folded and expanded: one decoded row beside 1,024 rows on 8 heads (4.8e9) 1.10 and
+    # 1.18 ms, beside segments of 992, 375 and 538 rows of which the first is expanded 1.47 and 1.91; 8 decoded rows beside
+    # 768 rows on 16 heads (1.04e10) 1.66 and 1.48, beside 512 rows behind 2,048 on 8 (1.1e10) 1.49 and 1.40, beside 2,000
+    # rows on 8 (1.8e10) 2.55 and 2.22; 2,000 rows on 16 and nothing else 3.42 and 2.18
+    "latent_expand_rotated_min_ops": 10e9,
     # recurrences over prompt portions: segments of at least this many rows run as chunks on tensor cores (three launches
     # that fill the device with a few hundred rows, where walking the rows costs the same each: the selective scan of 64
     # heads takes 44 us against 55 at 128 rows, 32 against 32 at 64; linear attention of 16 heads of 128 x 128 takes 62
@@ -1347,12 +1350,17 @@ def add_row_vector(h: torch.Tensor, vec: torch.Tensor) -> None:
     _lib.call("nf_add_row_vector", _p(h), _p(vec), c_int(h.shape[0]), c_int(h.shape[1]), _stream())
 
 
-def heads_sigmoid_gate(v: torch.Tensor, g_src: torch.Tensor, g_col0: int, per_head: bool = False) -> torch.Tensor:
-    """v [heads, T, n] (head-major) times sigmoid(g_src[:, g_col0 + head * n + i]) -> [T, heads * n]; `per_head`: the
-    gate has one number a head, g_src[:, g_col0 + head]."""
+def heads_sigmoid_gate(v: torch.Tensor, g_src: torch.Tensor, g_col0: int, per_head: bool = False,
+                       out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """v [heads, T, n] (head-major) times sigmoid(g_src[:, g_col0 + head * n + i]) -> [T, heads * n] (into `out` if
+    given); `per_head`: the gate has one number a head, g_src[:, g_col0 + head]."""
     _chk(v, "v"); _chk(g_src, "g_src", v.dtype)
     heads, T, n = v.shape
-    out = torch.empty((T, heads * n), dtype=v.dtype, device=v.device)
+    if out is None:
+        out = torch.empty((T, heads * n), dtype=v.dtype, device=v.device)
+    _chk(out, "out", v.dtype)
+    if out.shape != (T, heads * n):
+        raise ValueError("heads_sigmoid_gate: out does not have the result's shape")
     _lib.call("nf_heads_sigmoid_gate", _p(v), _p(g_src), c_int(g_src.shape[1]), c_int(g_col0), _p(out), c_int(T),
               c_int(heads), c_int(n), c_int(1 if per_head else 0), c_int(_dt(v)), _stream())
     return out
@@ -1815,43 +1823,64 @@ def latent_attention(q_abs: torch.Tensor, q: torch.Tensor, head_stride: int, rot
     return out
 
 
-def can_expand_latent(q: torch.Tensor, heads: int, D: int, Dv: int, R: int, ctx, Dr: int = 0) -> bool:
-    """Whether `expanded_latent_attention` serves the step's segments of several rows; `Dr`: rotated dimensions behind
-    every query's D and every cached row's R."""
+def can_expand_latent(q: torch.Tensor, heads: int, D: int, Dv: int, R: int, ctx, Dr: int = 0) -> List[Tuple[int, ...]]:
+    """The step's segments that `expanded_latent_attention` serves, in groups, a call each (none: the folded form serves
+    them all); `Dr`: rotated dimensions behind every query's D and every cached row's R.
+
+    With a rotated part a segment's own rows and positions decide, so that its bits do not hang on what else the step
+    holds; a group is as many of them as `latent_expand_max_mb` has room for.  Without one it is all segments of several
+    rows or none."""
     if not (q.is_cuda and q.dtype == torch.bfloat16 and TUNING["bf16_attention"] != "generic" and D == Dv
             and (D in (64, 128) if Dr == 0 else (D, Dr) == (128, 64)) and R % 8 == 0 and q.shape[1] % 8 == 0 and q.is_contiguous()
             and ctx.seg_len_host is not None and ctx.seg_pos0_host is not None):
-        return False
-    rows = sum(n for n in ctx.seg_len_host if n > 1)
-    held = sum(p + n for p, n in zip(ctx.seg_pos0_host, ctx.seg_len_host) if n > 1)
-    if Dr:
-        pairs = sum(n * p + n * (n + 1) // 2 for p, n in zip(ctx.seg_pos0_host, ctx.seg_len_host) if n > 1)
-        if 2 * heads * (2 * R + Dr) * pairs < TUNING["latent_expand_rotated_min_ops"]:
-            return False
-    return rows >= TUNING["latent_expand_min_rows"] and held * 2 * heads * D * 2 <= TUNING["latent_expand_max_mb"] << 20
+        return []
+    most = (TUNING["latent_expand_max_mb"] << 20) // (2 * heads * D * 2)
+    key = ("expanded", most, Dr, heads * (2 * R + Dr))                # (asked for by every layer)
+    if key not in ctx._tiles:
+        ctx._tiles[key] = _expanded_segments(ctx, most, Dr, 2 * heads * (2 * R + Dr))
+    return ctx._tiles[key]
+
+
+def _expanded_segments(ctx, most: int, Dr: int, pair_ops: int) -> List[Tuple[int, ...]]:
+    several = [(s, n, p) for s, (n, p) in enumerate(zip(ctx.seg_len_host, ctx.seg_pos0_host)) if n > 1]
+    if Dr == 0:
+        fits = sum(n for _, n, _ in several) >= TUNING["latent_expand_min_rows"] and sum(n + p for _, n, p in several) <= most
+        return [tuple(s for s, _, _ in several)] if fits else []
+    groups, held = [], 0
+    for s, n, p in several:
+        if (n < TUNING["latent_expand_min_rows"] or p + n > most
+                or pair_ops * (n * p + n * (n + 1) // 2) < TUNING["latent_expand_rotated_min_ops"]):
+            continue
+        if not groups or held + p + n > most:
+            groups.append(())
+            held = 0
+        groups[-1] += (s,)
+        held += p + n
+    return groups
 
 
 def expanded_latent_attention(q: torch.Tensor, w_kv: torch.Tensor, heads: int, D: int, pages: torch.Tensor,
                               block_table: torch.Tensor, page_size: int, ctx, scale: float, out: torch.Tensor,
                               gate: Optional[torch.Tensor] = None, gate_col0: int = 0, Dr: int = 0,
-                              sink: Optional[torch.Tensor] = None) -> None:
-    """Causal softmax attention of the step's segments of several rows over a latent cache, by expanding it: the
+                              sink: Optional[torch.Tensor] = None, segments: Optional[Tuple[int, ...]] = None) -> None:
+    """Causal softmax attention of the given segments (None: all of several rows) over a latent cache, by expanding it: the
     segments' cached rows c (pages [n, page_size, R]) are gathered, one product with w_kv [2 * heads * D, R] (keys of
     all heads, then values) gives every token's keys and values, and the tcgen05 kernel runs over those.  q [T, ld]
     holds the queries in its first heads * D columns; head h's output times sigmoid(gate[t, gate_col0 + h]) (bfloat16)
-    goes to out [T, heads * D], whose rows of single-row segments are left as they are.
+    goes to out [T, heads * D], whose rows of other segments are left as they are.
 
     With `Dr` the cached rows are [c | Dr rotated dimensions that all heads share], the queries heads * (D + Dr), and
     exp(sink[h]) joins the softmax's denominator (no gate then: it is the caller's)."""
     _chk(q, "q", torch.bfloat16); _chk(w_kv, "w_kv", q.dtype); _chk(pages, "pages", q.dtype); _chk(out, "out", q.dtype)
     R = w_kv.shape[1]
-    base, total = ctx.context_rows(2)
+    if segments is None:
+        segments = tuple(s for s, n in enumerate(ctx.seg_len_host) if n > 1)
+    base, total, tiles, n_tiles = ctx.whole_contexts(segments, 128)
     c = torch.empty((total, R + Dr), dtype=q.dtype, device=q.device)
     _lib.call("nf_gather_cached_rows", _p(pages), _p(block_table), c_int(block_table.shape[1]), _p(ctx.seg_pos0),
               _p(ctx.seg_row0), _p(base), _p(c), c_int(ctx.S), c_int((R + Dr) * 2), c_int(page_size), c_int(pages.shape[0]),
               c_int(int(ctx.max_context)), c_int(total), _stream())
     kv = linear(c, w_kv) if Dr == 0 else torch.mm(c[:, :R], w_kv.t())        # (a product over the rows' first part)
-    tiles, n_tiles = ctx.paired_query_tiles(128, 0, 128, pair=False, min_rows=2)
     if Dr:
         if sink is not None:
             _chk(sink, "sink", torch.float32)

@@ -253,26 +253,36 @@ class StepContext:
         self._tiles["single"] = out
         return out
 
-    def single_rows_context(self) -> Optional["StepContext"]:
-        """The segments that bring exactly one row as a step of their own (rows in `single_rows` order), for a
-        kernel that takes whole steps; None if there are none.  Built on the host; not in graph mode."""
-        if "single_ctx" not in self._tiles:
-            rows, n = self.single_rows()
-            sub = None
-            if n:
-                segs = [s for s, m in enumerate(self.seg_len_host) if m == 1]
-                idx = self.row_seg.index_select(0, rows)
-                count = torch.arange(n + 1, dtype=torch.int32, device=self.device)
-                pos0 = [self.seg_pos0_host[s] for s in segs]
-                sub = StepContext(
-                    dtype=self.dtype, device=self.device, T=n, S=n, token_ids=self.token_ids.index_select(0, rows),
-                    positions=self.positions.index_select(0, rows), row_seg=count[:n], seg_row0=count,
-                    seg_pos0=self.seg_pos0.index_select(0, idx), seg_slot=self.seg_slot.index_select(0, idx),
-                    logit_rows=count[:0], block_tables={g: t.index_select(0, idx) for g, t in self.block_tables.items()},
-                    seg_len_host=[1] * n, seg_pos0_host=pos0, max_rows_per_seg=1, max_context=max(pos0) + 1)
-                sub.scratch["segments"] = idx
-            self._tiles["single_ctx"] = sub
-        return self._tiles["single_ctx"]
+    def segments_context(self, segments: Tuple[int, ...]) -> Tuple[object, object, "StepContext"]:
+        """The given segments as a step of their own, for a kernel that takes whole steps: (their rows, their numbers, the
+        step); rows and numbers index this step's, as slices where the segments are its first ones (what decoded rows
+        are: nothing is copied then), else as int32 tensors.  Built on the host; not in graph mode."""
+        key = ("segments", segments)
+        if key not in self._tiles:
+            segments = tuple(sorted(segments))
+            S, T = len(segments), sum(self.seg_len_host[s] for s in segments)
+            if segments == tuple(range(S)):
+                rows, numbers, row_seg, row0 = slice(0, T), slice(0, S), self.row_seg[:T], self.seg_row0[:S + 1]
+                pick = lambda t, at: t[at]
+            else:
+                flat, of, first, starts = [], [], [0], [0]
+                for n in self.seg_len_host:
+                    starts.append(starts[-1] + n)
+                for i, s in enumerate(segments):
+                    flat += range(starts[s], starts[s + 1])
+                    of += [i] * self.seg_len_host[s]
+                    first.append(len(flat))
+                rows, row_seg, row0, numbers = self._ints(flat + of + first + list(segments)).split([T, T, S + 1, S])
+                pick = lambda t, at: t.index_select(0, at)
+            lens, pos0 = ([v[s] for s in segments] for v in (self.seg_len_host, self.seg_pos0_host))
+            sub = StepContext(
+                dtype=self.dtype, device=self.device, T=T, S=S, token_ids=pick(self.token_ids, rows),
+                positions=pick(self.positions, rows), row_seg=row_seg, seg_row0=row0, seg_pos0=pick(self.seg_pos0, numbers),
+                seg_slot=pick(self.seg_slot, numbers), logit_rows=self.logit_rows[:0],
+                block_tables={g: pick(t, numbers) for g, t in self.block_tables.items()}, seg_len_host=lens,
+                seg_pos0_host=pos0, max_rows_per_seg=max(lens), max_context=max(p + n for p, n in zip(pos0, lens)))
+            self._tiles[key] = (rows, numbers, sub)
+        return self._tiles[key]
 
     def recurrence_chunks(self, rows_per_chunk: int, min_rows: int, max_chunks: int
                           ) -> Tuple[List[Tuple[torch.Tensor, int, torch.Tensor, int]], bool]:
@@ -303,17 +313,23 @@ class StepContext:
             self._tiles[key] = (lists, others)
         return self._tiles[key]
 
-    def context_rows(self, min_rows: int) -> Tuple[torch.Tensor, int]:
-        """Where each segment's whole context (what it held and what it brings) starts in a matrix that holds the
-        contexts of all segments of at least `min_rows` rows one after the other: (int32 [S], -1 for the others;
-        rows in all).  Built on the host; not in graph mode."""
-        key = ("context_rows", min_rows)
+    def whole_contexts(self, segments: Tuple[int, ...], rows_per_tile: int) -> Tuple[torch.Tensor, int, torch.Tensor, int]:
+        """For attention over a matrix that holds the whole contexts (what was held and what the step brings) of the given
+        segments one after the other: int32 [S] of where each starts in it, -1 for the other segments; its rows; query
+        tiles of those segments, one to a CTA, heaviest first, as `paired_query_tiles` gives them; their number.  Built on
+        the host; not in graph mode."""
+        key = ("whole_contexts", segments, rows_per_tile)
         if key not in self._tiles:
-            base, total = [], 0
-            for n, p in zip(self.seg_len_host, self.seg_pos0_host):
-                base.append(total if n >= min_rows else -1)
-                total += p + n if n >= min_rows else 0
-            self._tiles[key] = (self._ints(base), total)
+            base, total, chosen, tiles, row = [], 0, set(segments), [], 0
+            for s, (n, p) in enumerate(zip(self.seg_len_host, self.seg_pos0_host)):
+                base.append(total if s in chosen else -1)
+                if s in chosen:
+                    total += p + n
+                    tiles += [(-(p + min(r + rows_per_tile, n)), s, row + r) for r in range(0, n, rows_per_tile)]
+                row += n
+            tiles.sort()
+            flat = self._ints(base + [-1] * (-len(base) % 4) + [v for _, s, r in tiles for v in (s, r, -1, -1)])
+            self._tiles[key] = (flat[:len(base)], total, flat[len(flat) - 4 * len(tiles):], len(tiles))
         return self._tiles[key]
 
     def paired_query_tiles(self, rows_per_tile: int, window: int, keys_per_block: int,

@@ -139,37 +139,42 @@ class LatentAttention(Mixer):
             kernels.latent_append(proj, q_cols, R, Dr, self.kv_norm, self.eps, inv_freq, rot, ctx,
                                   cache.pages, cache.block_table, cache.page_size)
         per_head, elementwise = (self.has_gate and self.gate_per_head), (self.has_gate and not self.gate_per_head)
-        if (not self.window and (not per_head if Dr else not self.has_sink and not elementwise)
-                and kernels.can_expand_latent(q, H, self.dim, self.value_dim, R, ctx, Dr)):
-            return self._forward_expanded(q, proj, q_cols + R + Dr, ctx, cache)
+        groups = []
+        if not self.window and (not per_head if Dr else not self.has_sink and not elementwise):
+            groups = kernels.can_expand_latent(q, H, self.dim, self.value_dim, R, ctx, Dr)
+        if groups:
+            return self._forward_expanded(q, proj, q_cols + R + Dr, ctx, cache, groups)
         o = self._folded(q, proj, q_cols + R + Dr, ctx, cache.pages, cache.block_table, cache.page_size)
         return kernels.linear(o, self.w_o)
 
-    def _forward_expanded(self, q, proj, gate_col0: int, ctx: StepContext, cache: CacheView) -> torch.Tensor:
-        """The segments of several rows over expanded keys and values, those of one row in the folded form."""
+    def _forward_expanded(self, q, proj, gate_col0: int, ctx: StepContext, cache: CacheView, groups) -> torch.Tensor:
+        """The segments of `groups` over expanded keys and values, the others in the folded form."""
         H = self.heads
         o = torch.empty((q.shape[0], H * self.value_dim), dtype=q.dtype, device=q.device)
-        if self.rot_dim:
+        gate = proj if self.has_gate and not self.rot_dim else None
+        for segments in groups:
             kernels.expanded_latent_attention(q, self.w_kv, H, self.dim, cache.pages, cache.block_table, cache.page_size, ctx,
-                                              self.scale, o, Dr=self.rot_dim, sink=self.sink)
-            if self.has_gate:
-                o = kernels.sigmoid_gate_rows(o, proj, gate_col0)
-        else:
-            kernels.expanded_latent_attention(q, self.w_kv, H, self.dim, cache.pages, cache.block_table, cache.page_size, ctx,
-                                              self.scale, o, proj if self.has_gate else None, gate_col0)
-        sub = ctx.single_rows_context()
-        if sub is not None:
-            rows, _ = ctx.single_rows()
-            own = proj is q
-            q_s = q.index_select(0, rows)
-            proj_s = q_s if own else proj.index_select(0, rows)
-            table = cache.block_table.index_select(0, sub.scratch["segments"])
-            o.index_copy_(0, rows.long(), self._folded(q_s, proj_s, gate_col0, sub, cache.pages, table, cache.page_size))
+                                              self.scale, o, gate, gate_col0 if gate is not None else 0, self.rot_dim, self.sink,
+                                              segments)
+        if self.has_gate and self.rot_dim:
+            o = kernels.sigmoid_gate_rows(o, proj, gate_col0)
+        taken = {s for segments in groups for s in segments}
+        others = tuple(s for s in range(ctx.S) if s not in taken)
+        if others:
+            rows, numbers, sub = ctx.segments_context(others)
+            if isinstance(rows, slice):
+                self._folded(q[rows], proj[rows], gate_col0, sub, cache.pages, cache.block_table[numbers], cache.page_size, o[rows])
+            else:
+                q_s = q.index_select(0, rows)
+                proj_s = q_s if proj is q else proj.index_select(0, rows)
+                table = cache.block_table.index_select(0, numbers)
+                o.index_copy_(0, rows.long(), self._folded(q_s, proj_s, gate_col0, sub, cache.pages, table, cache.page_size))
         return kernels.linear(o, self.w_o)
 
-    def _folded(self, q, proj, gate_col0: int, ctx: StepContext, pages, block_table, page_size: int) -> torch.Tensor:
-        """Gated outputs [T, H * vdim] with the key projection folded into the query and the value projection
-        applied after the weighted sum."""
+    def _folded(self, q, proj, gate_col0: int, ctx: StepContext, pages, block_table, page_size: int,
+                out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """Gated outputs [T, H * vdim] (in `out` if given) with the key projection folded into the query and the value
+        projection applied after the weighted sum."""
         H, T = self.heads, q.shape[0]
         # the key projection folded into the query: [H, T, dim] x [H, dim, R]
         q_heads = q[:, :H * self.q_head].unflatten(1, (H, self.q_head))
@@ -178,5 +183,6 @@ class LatentAttention(Mixer):
                                          self.sink, self.scale, self.window or 0)
         v = kernels.heads_linear(o_lat, self.w_uv)                            # [H, T, vdim]
         if self.has_gate:
-            return kernels.heads_sigmoid_gate(v, proj, gate_col0, per_head=self.gate_per_head)
-        return v.transpose(0, 1).reshape(T, H * self.value_dim)
+            return kernels.heads_sigmoid_gate(v, proj, gate_col0, per_head=self.gate_per_head, out=out)
+        v = v.transpose(0, 1)
+        return v.reshape(T, H * self.value_dim) if out is None else out.view(T, H, self.value_dim).copy_(v)

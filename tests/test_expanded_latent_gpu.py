@@ -61,3 +61,43 @@ def test_expanded_against_folded(lens, sharp, monkeypatch):
     # that takes over may not be further off (a tenth is what the few rows of a segment of two scatter by)
     new, old = (torch.stack(e).square().mean().sqrt().item() for e in off)
     assert new <= 1.1 * old, (new, old)
+
+
+def test_a_segment_decides_for_itself():
+    """A short portion with rotated dimensions keeps the folded form beside a long one that is expanded: beside decoded
+    rows or behind the long one (its rows are then picked out), it gives what it gives alone."""
+    from ninfer_amd_mi50_b200 import kernels
+    from ninfer_amd_mi50_b200.config.model_config import PartSpec
+    from ninfer_amd_mi50_b200.parts.base import CacheView
+    from ninfer_amd_mi50_b200.parts.latent_attention import LatentAttention
+    heads, R, width, short, long = 16, 512, 256, 40, 1024
+    part = LatentAttention(width, heads, D, DR, D, R, None, (D + DR) ** -0.5, 1e-5, PartSpec.make("rotary_half_split", head_dim=DR, theta=1e4),
+                           "x.")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    shapes = {t.name: (t.shape, t.role) for t in part.tensor_specs()}
+    part.load(lambda name: rand(*shapes[name][0]) if shapes[name][1] == "vector" else
+              (rand(*shapes[name][0]) * shapes[name][0][1] ** -0.5).bfloat16())
+    rows = {n: rand(n, width).bfloat16() for n in (short, long, 1)}
+
+    def run(lens):
+        ctx = context(lens)
+        ctx.seg_pos0_host, ctx.seg_pos0 = [0] * len(lens), torch.zeros_like(ctx.seg_pos0)
+        ctx.positions, ctx.max_context = torch.cat([torch.arange(n, dtype=torch.int32, device="cuda") for n in lens]), max(lens)
+        per = (max(lens) + PAGE - 1) // PAGE
+        table = torch.arange(len(lens) * per, dtype=torch.int32, device="cuda").view(len(lens), per)
+        pages = torch.zeros(len(lens) * per, PAGE, R + DR, dtype=torch.bfloat16, device="cuda")
+        out = part.forward(torch.cat([rows[n] for n in lens]), ctx, CacheView(part.cache_spec(), pages, table, PAGE), None)
+        kernels.check_status("latent attention")
+        q = torch.empty(ctx.T, heads * (D + DR), dtype=torch.bfloat16, device="cuda")
+        at = sum(lens[:lens.index(short)])
+        return out[at:at + short].double(), kernels.can_expand_latent(q, heads, D, D, R, ctx, DR)
+
+    alone, expanded = run([short])
+    assert not expanded
+    for lens in ([short, long], [1, short, long], [long, short], [1, long, short, 1]):
+        # products of other row counts may round a few numbers the other way (2^-9 of each); the expanded form rounds all of
+        # them at other places, 4e-3
+        got, expanded = run(lens)
+        assert ((got - alone).norm() / alone.norm()).item() <= 1e-3, lens
+        assert expanded == [(lens.index(long),)]
