@@ -40,6 +40,59 @@ constexpr int kCrPad = 8;               // elements of padding a shared-memory r
 
 enum CrMode : int { kCrScan = 0, kCrDecay = 1, kCrDelta = 2 };
 
+// Which chunks a launch serves: those of the segments of at least min_rows rows, counted over all of them, from chunk
+// `first` on, and of these segments those from number `first_run` on.  Where they lie is worked out on the device from the
+// step's own index of rows: lists of chunks and runs made on the host cost a step of few rows, which waits for its host,
+// more than the recurrence itself (one scan of 256 rows: 24 us to build and send them).
+struct CrChunks {
+  const int* seg_row0;
+  int S, min_rows, first, n, first_run;
+};
+struct CrPlace {
+  int seg, row0, rows, chunk;           // a segment, its first row, its rows, the number of its first chunk
+};
+// The segment of chunk `c`, or (RUN) the segment of number `c`; a warp's lanes look at 32 segments at a time.  The index is
+// a step's input, complete before the step's kernels began.
+template <int Q, bool RUN>
+__device__ __forceinline__ CrPlace cr_find(const CrChunks& at, int c) {
+  const int lane = threadIdx.x & 31;
+  int chunks = 0, runs = 0;
+  for (int s0 = 0; s0 < at.S; s0 += 32) {
+    const int s = s0 + lane, row0 = s < at.S ? at.seg_row0[s] : 0, rows = s < at.S ? at.seg_row0[s + 1] - row0 : 0;
+    const bool mine = rows >= at.min_rows;
+    const int k = mine ? (rows + Q - 1) / Q : 0;
+    int incl = k;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, mine);
+    const int number = runs + __popc(b & ((1u << lane) - 1u)), first = chunks + incl - k;
+    const unsigned hit = __ballot_sync(0xffffffffu, mine && (RUN ? number == c : c >= first && c < first + k));
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      return {s0 + src, __shfl_sync(0xffffffffu, row0, src), __shfl_sync(0xffffffffu, rows, src), __shfl_sync(0xffffffffu, first, src)};
+    }
+    chunks += __shfl_sync(0xffffffffu, incl, 31);
+    runs += __popc(b);
+  }
+  return {0, 0, 0, 0};                  // (no such chunk: no rows)
+}
+// First row and rows of chunk `c` of the launch.
+template <int Q>
+__device__ __forceinline__ int2 cr_rows(const CrChunks& at, int c) {
+  const CrPlace p = cr_find<Q, false>(at, at.first + c);
+  const int off = (at.first + c - p.chunk) * Q;
+  return make_int2(p.row0 + off, max(0, min(Q, p.rows - off)));
+}
+// Of a segment's chunks those in the launch: x the first one's number in the launch, y how many, z its number in the segment.
+template <int Q>
+__device__ __forceinline__ int3 cr_run(const CrChunks& at, const CrPlace& p) {
+  const int lo = max(p.chunk, at.first), hi = min(p.chunk + (p.rows + Q - 1) / Q, at.first + at.n);
+  return make_int3(lo - at.first, max(0, hi - lo), lo - p.chunk);
+}
+
 struct CrArgs {
   const __nv_bfloat16 *q, *k, *v;       // rows of `ld` elements, columns from q0, k0, v0 on (q and k: a head group's D)
   int ld, q0, k0, v0;
@@ -52,8 +105,7 @@ struct CrArgs {
   const float* decay;                   // a decay a head
   const float* values;                  // delta rule: float32 values [T, H * V] (u), and [T, H, 4] of (decay, factor on
   const float* gates;                   // the row's key, factor on its output, -)
-  const int* chunks;                    // [n][3]: segment, first row, rows
-  const int* runs;                      // [m][3]: segment, first chunk, chunks
+  CrChunks at;
   const int* seg_slot;
   float* state;
   long slot_stride;
@@ -197,8 +249,9 @@ chunk_state_kernel(const CrArgs args) {
   const int chunk = blockIdx.x, head = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   CrArgs a = args;
+  const int2 place = cr_rows<Q>(a.at, chunk);
+  const int row0 = place.x, live = place.y;
   chain_wait(a.q, a.k, a.v, a.dt, a.prepared);
-  const int row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
   float weight = 0.f;
   if (threadIdx.x < Q) {
     float decay;
@@ -293,14 +346,17 @@ chunk_state_kernel(const CrArgs args) {
 
 // ---- (2) the chain over a segment's chunks --------------------------------------------------------------------------
 // A thread carries four of a head's V D state entries through the segment's chunks; loads run four chunks ahead.
+template <int Q>
 __global__ void __launch_bounds__(kCrThreads)
 chunk_chain_kernel(const CrArgs args, int entries) {
   constexpr int AHEAD = 4;
   const int run = blockIdx.x, head = blockIdx.y, e = (blockIdx.z * kCrThreads + threadIdx.x) * 4;
   CrArgs a = args;
+  const CrPlace place = cr_find<Q, true>(a.at, a.at.first_run + run);
+  const int3 own = cr_run<Q>(a.at, place);
+  const int seg = place.seg, first = own.x, n = own.y;
   chain_wait(a.chunk_state, a.chunk_decay, a.state);
   if (e >= entries) return;
-  const int seg = a.runs[3 * run], first = a.runs[3 * run + 1], n = a.runs[3 * run + 2];
   float* slot = a.state + (size_t)a.seg_slot[seg] * a.slot_stride + (size_t)head * entries + e;
   float* mine = a.chunk_state + ((size_t)first * a.H + head) * entries + e;
   const float* decay = a.chunk_decay + (size_t)first * a.H + head;
@@ -354,8 +410,9 @@ chunk_output_kernel(const CrArgs args) {
   const int chunk = blockIdx.x, head = blockIdx.y, tile0 = blockIdx.z * V;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   CrArgs a = args;
+  const int2 place = cr_rows<Q>(a.at, chunk);
+  const int row0 = place.x, live = place.y;
   chain_wait(a.q, a.k, a.v, a.dt, a.prepared, a.chunk_state, a.values, a.gates);
-  const int row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
   if (threadIdx.x < Q)
     cr_row_gates<MODE>(a, head, row0 + threadIdx.x, (int)threadIdx.x < live, s_decay[threadIdx.x], s_weight[threadIdx.x]);
   cr_load_qk<D, QKP>(a, false, head, row0, Q, live, Qs, (size_t)Q * KS);
@@ -617,7 +674,7 @@ int launch_chunks(const CrArgs& a, int n_chunks, int n_runs, cudaStream_t stream
     set = true;
   }
   launch_chained(chunk_state_kernel<D, V, Q, QKP, MODE>, dim3(n_chunks, a.H), dim3(kCrThreads), smem, stream, a);
-  launch_chained(chunk_chain_kernel, dim3(n_runs, a.H, (V * D / 4 + kCrThreads - 1) / kCrThreads), dim3(kCrThreads), 0, stream, a, V * D);
+  launch_chained(chunk_chain_kernel<Q>, dim3(n_runs, a.H, (V * D / 4 + kCrThreads - 1) / kCrThreads), dim3(kCrThreads), 0, stream, a, V * D);
   return launch_outputs<D, VT, Q, SUB, QKP, VP, MODE>(a, n_chunks, stream);
 }
 
@@ -639,7 +696,8 @@ struct DcArgs {
   const float *dt_bias, *A_log;
   float q_scale;
   int H, heads_per_group, V;
-  const int *chunks, *runs, *seg_slot;
+  CrChunks at;
+  const int* seg_slot;
   float* state;
   long slot_stride;
   __nv_bfloat16* solve;                   // T as three parts: [n][H][3][64][64]
@@ -669,8 +727,9 @@ delta_chunk_solve_kernel(const DcArgs args) {
   const int chunk = blockIdx.x, head = blockIdx.y, grp = head / args.heads_per_group;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   DcArgs a = args;
+  const int2 place = cr_rows<Q>(a.at, chunk);
+  const int row0 = place.x, live = place.y;
   chain_wait(a.qkv, a.ab);
-  const int row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
   const __nv_bfloat16* kr = a.qkv + a.k0 + (size_t)grp * D;
   const __nv_bfloat16* qr = a.qkv + a.q0 + (size_t)grp * D;
   for (int r = warp; r < Q; r += kCrThreads / 32) {      // a warp a row: the key to shared memory, both norms
@@ -813,11 +872,13 @@ delta_chunk_chain_kernel(const DcArgs args) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t4 = lane & 3, mat = lane >> 3, r8 = lane & 7;
   DcArgs a = args;
+  const CrPlace place = cr_find<Q, true>(a.at, a.at.first_run + run);
+  const int3 own = cr_run<Q>(a.at, place);
+  const int seg = place.seg, first = own.x, n = own.y, seg_row = place.row0 + own.z * Q, seg_rows = place.rows - own.z * Q;
   chain_wait(a.qkv, a.solve, a.coef, a.chunk_decay, a.state);
-  const int seg = a.runs[3 * run], first = a.runs[3 * run + 1], n = a.runs[3 * run + 2];
   auto fetch = [&](int c) {
     if (c < n) {
-      const int b = c & 1, chunk = first + c, row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
+      const int b = c & 1, chunk = first + c, row0 = seg_row + c * Q, live = min(Q, seg_rows - c * Q);
       const __nv_bfloat16* kr = a.qkv + (size_t)row0 * a.ld + a.k0 + (size_t)grp * D;
 #pragma unroll
       for (int i = threadIdx.x; i < Q * (D / 8); i += kCrThreads) {
@@ -854,7 +915,7 @@ delta_chunk_chain_kernel(const DcArgs args) {
   const int mt = warp & 3, nt = warp >> 2;           // rows 16 mt .., columns 8 nt .. of the first two products
   const int tr = mt * 16 + g, col = nt * 8 + 2 * t4;
   for (int c = 0; c < n; ++c) {
-    const int b = c & 1, chunk = first + c, row0 = a.chunks[3 * chunk + 1], live = a.chunks[3 * chunk + 2];
+    const int b = c & 1, chunk = first + c, row0 = seg_row + c * Q, live = min(Q, seg_rows - c * Q);
     const float decay = a.chunk_decay[(size_t)chunk * a.H + head];
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                 // the chunk is in; the state's parts are written; the rest is free
@@ -1013,12 +1074,12 @@ extern "C" int nf_chunk_recurrence_rows(int D, int V, int scan) {
   return (D == 64 || D == 128) && V == 128 ? 64 : 0;
 }
 
-// The selective scan of the listed chunks; arguments as nf_ssd_scan's (bfloat16).  chunks int32 [n_chunks, 3] of
-// (segment, first row, rows), in order within a segment; runs int32 [n_runs, 3] of (segment, first chunk, chunks).
-// chunk_state float32 [n_chunks, heads, P, N], chunk_decay float32 [n_chunks, heads]: scratch.
+// The selective scan of chunks first_chunk .. + n_chunks of the segments of at least min_rows rows (counted over all such
+// segments, nf_chunk_recurrence_rows rows each but a segment's last); they belong to n_runs of those segments, from number
+// first_run on.  Arguments as nf_ssd_scan's (bfloat16).  chunk_state float32 [n_chunks, heads, P, N], chunk_decay float32 [n_chunks, heads]: scratch.
 extern "C" int nf_chunk_scan(const void* xbc, int ldx, int x0, int b0, int c0, const void* dt, int ld_dt, int dt0,
                              const float* dt_bias, const float* A_log, const float* skip, float* state, long long slot_stride,
-                             const int* seg_slot, const int* chunks, int n_chunks, const int* runs, int n_runs,
+                             const int* seg_slot, const int* seg_row0, int S, int min_rows, int first_chunk, int n_chunks, int first_run, int n_runs,
                              float* chunk_state, float* chunk_decay, float* out, int heads, int P, int N, int groups,
                              cudaStream_t stream) {
   if (n_chunks == 0) return 0;
@@ -1031,18 +1092,19 @@ extern "C" int nf_chunk_scan(const void* xbc, int ldx, int x0, int b0, int c0, c
   a.H = heads; a.heads_per_group = heads / groups; a.V = P;
   a.dt = (const __nv_bfloat16*)dt; a.ld_dt = ld_dt; a.dt0 = dt0;
   a.dt_bias = dt_bias; a.A_log = A_log; a.skip = skip;
-  a.chunks = chunks; a.runs = runs; a.seg_slot = seg_slot;
+  a.at = {seg_row0, S, min_rows, first_chunk, n_chunks, first_run}; a.seg_slot = seg_slot;
   a.state = state; a.slot_stride = (long)slot_stride;
   a.chunk_state = chunk_state; a.chunk_decay = chunk_decay; a.out = out;
   if (N == 128) return launch_chunks<128, 64, 64, 128, 64, 1, 1, kCrScan>(a, n_chunks, n_runs, stream);
   return launch_chunks<64, 64, 64, 128, 64, 1, 1, kCrScan>(a, n_chunks, n_runs, stream);
 }
 
-// Linear attention of the listed chunks: prepared float32 [T, 2, H, D] (q and k), v bfloat16 [T, ld] from v0 on
+// Linear attention of such chunks: prepared float32 [T, 2, H, D] (q and k), v bfloat16 [T, ld] from v0 on
 // (through SiLU with v_silu), decay float32 [H]; the rest as above.
 extern "C" int nf_chunk_linear_attention(const float* prepared, const void* v, int ld, int v0, int v_silu, const float* decay,
                                          float* state, long long slot_stride, const int* seg_slot,
-                                         const int* chunks, int n_chunks, const int* runs, int n_runs, float* chunk_state,
+                                         const int* seg_row0, int S, int min_rows, int first_chunk, int n_chunks,
+                                         int first_run, int n_runs, float* chunk_state,
                                          float* chunk_decay, float* out, int H, int D, int V, cudaStream_t stream) {
   if (n_chunks == 0) return 0;
   NF_REQUIRE(nf_chunk_recurrence_rows(D, V, 0) > 0 && H > 0 && H <= 65535 && decay, "chunk linear attention: sizes D=%d V=%d H=%d", D, V, H);
@@ -1053,7 +1115,7 @@ extern "C" int nf_chunk_linear_attention(const float* prepared, const void* v, i
   a.ld = ld; a.v0 = v0; a.v_silu = v_silu; a.prepared = prepared;
   a.H = H; a.heads_per_group = 1; a.V = V;
   a.decay = decay;
-  a.chunks = chunks; a.runs = runs; a.seg_slot = seg_slot;
+  a.at = {seg_row0, S, min_rows, first_chunk, n_chunks, first_run}; a.seg_slot = seg_slot;
   a.state = state; a.slot_stride = (long)slot_stride;
   a.chunk_state = chunk_state; a.chunk_decay = chunk_decay; a.out = out;
   if (D == 128) return v_silu ? launch_chunks<128, 128, 64, 64, 32, 3, 3, kCrDecay>(a, n_chunks, n_runs, stream)
@@ -1064,12 +1126,13 @@ extern "C" int nf_chunk_linear_attention(const float* prepared, const void* v, i
 
 extern "C" int nf_chunk_delta_rule_rows(int D, int V) { return (D == 64 || D == 128) && V % 64 == 0 ? kDcRows : 0; }
 
-// The gated delta rule of the listed chunks; arguments as nf_delta_rule's (bfloat16).  Scratch: solve bfloat16
+// The gated delta rule of such chunks; arguments as nf_delta_rule's (bfloat16).  Scratch: solve bfloat16
 // [n_chunks, H, 3, 64, 64], coef float32 [n_chunks, H, 64, 2], gates float32 [T, H, 4], u float32 [T, H * V], chunk_state
 // float32 [n_chunks, H, V, D], chunk_decay float32 [n_chunks, H].
 extern "C" int nf_chunk_delta_rule(const void* qkv, int ld, int q0, int k0, int v0, const void* ab, int ld_ab, int a0, int b0,
                                    const float* dt_bias, const float* A_log, float q_scale, float* state, long long slot_stride,
-                                   const int* seg_slot, const int* chunks, int n_chunks, const int* runs, int n_runs, void* solve,
+                                   const int* seg_slot, const int* seg_row0, int S, int min_rows, int first_chunk, int n_chunks,
+                                   int first_run, int n_runs, void* solve,
                                    float* coef, float* gates, float* u, float* chunk_state, float* chunk_decay, float* out,
                                    int H, int G, int D, int V, cudaStream_t stream) {
   if (n_chunks == 0) return 0;
@@ -1081,7 +1144,7 @@ extern "C" int nf_chunk_delta_rule(const void* qkv, int ld, int q0, int k0, int 
   d.ld = ld; d.q0 = q0; d.k0 = k0; d.v0 = v0; d.ld_ab = ld_ab; d.a0 = a0; d.b0 = b0;
   d.dt_bias = dt_bias; d.A_log = A_log; d.q_scale = q_scale;
   d.H = H; d.heads_per_group = H / G; d.V = V;
-  d.chunks = chunks; d.runs = runs; d.seg_slot = seg_slot;
+  d.at = {seg_row0, S, min_rows, first_chunk, n_chunks, first_run}; d.seg_slot = seg_slot;
   d.state = state; d.slot_stride = (long)slot_stride;
   d.solve = (__nv_bfloat16*)solve; d.coef = coef; d.gates = gates;
   d.chunk_state = chunk_state; d.chunk_decay = chunk_decay; d.u = u;
@@ -1090,6 +1153,6 @@ extern "C" int nf_chunk_delta_rule(const void* qkv, int ld, int q0, int k0, int 
   a.ld = ld; a.q0 = q0; a.k0 = k0;
   a.H = H; a.heads_per_group = H / G; a.V = V;
   a.values = u; a.gates = gates;
-  a.chunks = chunks; a.chunk_state = chunk_state; a.out = out;
+  a.at = d.at; a.chunk_state = chunk_state; a.out = out;
   return D == 128 ? launch_delta<128>(d, a, n_chunks, n_runs, stream) : launch_delta<64>(d, a, n_chunks, n_runs, stream);
 }

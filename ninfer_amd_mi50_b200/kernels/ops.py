@@ -50,16 +50,24 @@ TUNING = {
     # 768 rows on 16 heads (1.04e10) 1.66 and 1.48, beside 512 rows behind 2,048 on 8 (1.1e10) 1.49 and 1.40, beside 2,000
     # rows on 8 (1.8e10) 2.55 and 2.22; 2,000 rows on 16 and nothing else 3.42 and 2.18
     "latent_expand_rotated_min_ops": 10e9,
-    # recurrences over prompt portions: segments of at least this many rows run as chunks on tensor cores (three launches
-    # that fill the device with a few hundred rows, where walking the rows costs the same each: the selective scan of 64
-    # heads takes 44 us against 55 at 128 rows, 32 against 32 at 64; linear attention of 16 heads of 128 x 128 takes 62
-    # against 134 at 512 rows, 57 against 44 at 128; the delta rule of 16 heads of 128 x 128 takes 68 against 118 at 512
-    # rows, 52 against 40 at 128); a huge number leaves every row to the kernels that walk them.
-    # Between 96 and 256 rows a single segment gains a little, but a step of many such segments, which the walking kernels
-    # serve side by side, pays for the further launches: 29 prompts of 35 to 279 rows 6.1 ms against 5.6)
-    "chunk_scan_min_rows": 256,
-    "chunk_linear_min_rows": 256,
-    "chunk_delta_min_rows": 256,
+    # recurrences over prompt portions run as chunks on tensor cores (three launches that fill the device with a few hundred
+    # rows; walking the rows costs the same each) in steps whose longest segment has at least `chunk_*_min_rows` rows, or
+    # whose segments of `chunk_beside_rows` and more bring at least `chunk_min_work` rows x state numbers together; all
+    # segments of `chunk_beside_rows` and more then run so, the others are walked.  On the device chunks win much earlier
+    # (the scan of 64 heads at 96 rows: 29 us against 37), but they cost the host of a step some 20 us a recurrence, which
+    # is what a step of few rows waits for.  Steps of four layers one after the other, walked and in chunks: scans of 64
+    # heads of 128 x 64 beside latent attention, 512 rows (2.7e8) 1.00 and 1.01 ms, 768 (4.0e8) 1.04 and 0.88, 16 x 100 rows
+    # (8.4e8) 1.92 and 1.89, segments of 31 to 279 rows (9.8e8) 2.43 and 1.91; linear attention of 16 heads of 128 x 128 and
+    # 64 x 128, 512 rows 1.16 and 1.24, 1,024 1.66 and 1.33, segments of 31 to 279 (4.9e8 and 2.4e8) 2.52 and 2.24; the same
+    # on 8 heads, 1,024 rows 1.26 and 1.31 (waited for 1.49 and 1.31), 2,000 2.18 and 1.46, segments of 31 to 279 (2.4e8 and
+    # 1.2e8) 1.88 and 1.97; scans and delta rules of 8 heads, 1,024 rows 1.54 and 1.63 (8 decoded rows beside them 2.23 and
+    # 1.91).  Segments below 64 rows in chunks: a delta rule of 32 segments of 32 rows 233 us walked, 426 in chunks, of 64
+    # rows 217 and 247.  A huge number leaves every row to the kernels that walk them
+    "chunk_scan_min_rows": 1024,
+    "chunk_linear_min_rows": 1024,
+    "chunk_delta_min_rows": 1024,
+    "chunk_beside_rows": 64,
+    "chunk_min_work": 3.2e8,
     "chunk_recurrence_max_mb": 512,      # scratch for the chunks' states; a longer step's chunks run group after group
     "qkv_rope_fused": True,       # few bfloat16 rows: rotation and cache append in the projection's epilogue
     "router_tensor_min_rows": 128,   # router logits of more rows than this use tensor cores
@@ -1544,12 +1552,13 @@ LINEAR_ATTENTION_MAX_DIM = 256
 
 def _recurrence_chunks(ctx, src: torch.Tensor, columns: Sequence[int], state: torch.Tensor, state_off: int, heads: int, D: int,
                        V: int, kind: str):
-    """What `ctx.recurrence_chunks` says for a step whose long segments the chunked recurrences (chunk_recurrence.cu) are to
-    serve, else None: bfloat16 rows and states that can be read 16 bytes at a time, sizes that those kernels have, and a
-    segment of at least as many rows as `TUNING` says."""
-    min_rows = TUNING[f"chunk_{kind}_min_rows"]
-    if (src.dtype != torch.bfloat16 or getattr(ctx, "seg_len_host", None) is None or getattr(ctx, "graph_mode", False)
-            or ctx.max_rows_per_seg < min_rows or not hasattr(ctx, "recurrence_chunks")):
+    """For a step whose longer segments the chunked recurrences (chunk_recurrence.cu) are to serve: (least rows of such a
+    segment, the groups and the longest of the others that `ctx.recurrence_chunks` gives), else None: bfloat16 rows and
+    states that can be read 16 bytes at a time, sizes that those kernels have, and a step as `TUNING` says."""
+    longest = TUNING[f"chunk_{kind}_min_rows"]
+    least, work = min(longest, TUNING["chunk_beside_rows"]), TUNING["chunk_min_work"] / (heads * D * V)
+    if (src.dtype != torch.bfloat16 or ctx.max_rows_per_seg < least or (ctx.max_rows_per_seg < longest and ctx.T < work)
+            or getattr(ctx, "seg_len_host", None) is None or getattr(ctx, "graph_mode", False) or not hasattr(ctx, "recurrence_chunks")):
         return None
     lib = _lib.load()
     rows = int(lib.nf_chunk_delta_rule_rows(c_int(D), c_int(V)) if kind == "delta" else
@@ -1557,14 +1566,20 @@ def _recurrence_chunks(ctx, src: torch.Tensor, columns: Sequence[int], state: to
     if (not rows or any(c % 8 for c in columns) or src.shape[1] % 8 or src.data_ptr() % 16 or state.stride(0) % 4
             or (state.data_ptr() + 4 * state_off) % 16):
         return None
-    return ctx.recurrence_chunks(rows, min_rows, max(1, (TUNING["chunk_recurrence_max_mb"] << 20) // (heads * D * V * 4)))
+    groups, others, total = ctx.recurrence_chunks(rows, least, max(1, (TUNING["chunk_recurrence_max_mb"] << 20) // (heads * D * V * 4)))
+    return (least, groups, others) if groups and (ctx.max_rows_per_seg >= longest or total >= work) else None
 
 
-def _chunk_scratch(lists, heads: int, D: int, V: int, device) -> Tuple[torch.Tensor, torch.Tensor]:
+def _chunk_scratch(groups, heads: int, D: int, V: int, device) -> Tuple[torch.Tensor, torch.Tensor]:
     """Float32 scratch for the largest group of chunks: their states, their decays."""
-    n = max(g[1] for g in lists)
-    return (torch.empty((n, heads, V, D), dtype=torch.float32, device=device),
-            torch.empty((n, heads), dtype=torch.float32, device=device))
+    n = max(g[1] for g in groups)
+    flat = torch.empty(n * heads * (V * D + 1), dtype=torch.float32, device=device)
+    return flat, flat[n * heads * V * D:]
+
+
+def _chunk_place(ctx, least: int, group) -> tuple:
+    first, n, first_run, runs = group
+    return (_p(ctx.seg_slot), _p(ctx.seg_row0), c_int(ctx.S), c_int(least), c_int(first), c_int(n), c_int(first_run), c_int(runs))
 
 
 def decay_linear_attention(src: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, decay: torch.Tensor,
@@ -1599,15 +1614,14 @@ def decay_linear_attention(src: torch.Tensor, q_col0: int, k_col0: int, v_col0: 
                if prepared is not None and gates is None else None)
     skip_rows = 0
     if chunked is not None:
-        lists, others = chunked
-        states, decays = _chunk_scratch(lists, heads, D, V, src.device)
-        for chunks, n, runs, m in lists:
+        skip_rows, runs, others = chunked
+        states, decays = _chunk_scratch(runs, heads, D, V, src.device)
+        for group in runs:
             _lib.call("nf_chunk_linear_attention", _p(prepared), _p(src), c_int(src.shape[1]), c_int(v_col0), c_int(1 if silu else 0),
-                      _p(decay), _p(state), c_longlong(state.stride(0)), _p(ctx.seg_slot), _p(chunks), c_int(n),
-                      _p(runs), c_int(m), _p(states), _p(decays), _p(out), c_int(heads), c_int(D), c_int(V), _stream())
+                      _p(decay), _p(state), c_longlong(state.stride(0)), *_chunk_place(ctx, skip_rows, group),
+                      _p(states), _p(decays), _p(out), c_int(heads), c_int(D), c_int(V), _stream())
         if not others:
             return out
-        skip_rows = TUNING["chunk_linear_min_rows"]
     _lib.call("nf_decay_linear_attention", _p(src), c_int(src.shape[1]), c_int(q_col0), c_int(k_col0), c_int(v_col0),
               _p(decay), _p(inv_freq) if rot else None, c_int(rot), c_float(k_scale), c_int(1 if silu else 0),
               _p(state), c_longlong(state.stride(0)), _p(ctx.seg_row0), _p(ctx.seg_slot), _p(ctx.seg_pos0), _p(out),
@@ -1663,20 +1677,20 @@ def delta_rule(qkv: torch.Tensor, q_col0: int, k_col0: int, v_col0: int, ab: tor
     state_p = c_void_p(state.data_ptr() + 4 * state_off)
     chunked = _recurrence_chunks(ctx, qkv, (q_col0, k_col0, v_col0), state, state_off, heads, D, V, "delta")
     if chunked is not None:
-        lists, others = chunked
-        states, decays = _chunk_scratch(lists, heads, D, V, qkv.device)
-        n = states.shape[0]
+        skip_rows, runs, others = chunked
+        states, decays = _chunk_scratch(runs, heads, D, V, qkv.device)
+        n = max(g[1] for g in runs)
         floats = lambda *shape: torch.empty(shape, dtype=torch.float32, device=qkv.device)
         solve = torch.empty((n, heads, 3, 64, 64), dtype=qkv.dtype, device=qkv.device)
         coef, gates, u = floats(n, heads, 64, 2), floats(T, heads, 4), floats(T, heads * V)
-        for chunks, n, runs, m in lists:
+        for group in runs:
             _lib.call("nf_chunk_delta_rule", _p(qkv), c_int(qkv.shape[1]), c_int(q_col0), c_int(k_col0), c_int(v_col0), _p(ab),
                       c_int(ab.shape[1]), c_int(a_col0), c_int(b_col0), _p(dt_bias), _p(A_log), c_float(q_scale), state_p,
-                      c_longlong(state.stride(0)), _p(ctx.seg_slot), _p(chunks), c_int(n), _p(runs), c_int(m), _p(solve), _p(coef),
+                      c_longlong(state.stride(0)), *_chunk_place(ctx, skip_rows, group), _p(solve), _p(coef),
                       _p(gates), _p(u), _p(states), _p(decays), _p(out), c_int(heads), c_int(kv_heads), c_int(D), c_int(V), _stream())
         if not others:
             return out
-        skip_rows = TUNING["chunk_delta_min_rows"]
+        rows = max(others, 2)                     # (the kernels of single rows serve steps without others)
     if rows > 1:
         vectors = torch.empty((T, kv_heads, 2, int(_lib.load().nf_delta_rule_row(c_int(D)))), dtype=torch.float32, device=qkv.device)
         records = torch.empty((T, heads, int(_lib.load().nf_delta_rule_record())), dtype=torch.float32, device=qkv.device)
@@ -1730,16 +1744,15 @@ def ssd_scan(xbc: torch.Tensor, x_col0: int, b_col0: int, c_col0: int, dt_src: t
     chunked = _recurrence_chunks(ctx, xbc, (x_col0, b_col0, c_col0), state, state_off, heads, N, P, "scan")
     skip_rows = 0
     if chunked is not None:
-        lists, others = chunked
-        states, decays = _chunk_scratch(lists, heads, N, P, xbc.device)
-        for chunks, n, runs, m in lists:
+        skip_rows, runs, others = chunked
+        states, decays = _chunk_scratch(runs, heads, N, P, xbc.device)
+        for group in runs:
             _lib.call("nf_chunk_scan", _p(xbc), c_int(xbc.shape[1]), c_int(x_col0), c_int(b_col0), c_int(c_col0), _p(dt_src),
                       c_int(dt_src.shape[1]), c_int(dt_col0), _p(dt_bias), _p(A_log), _p(D), state_p, c_longlong(state.stride(0)),
-                      _p(ctx.seg_slot), _p(chunks), c_int(n), _p(runs), c_int(m), _p(states), _p(decays), _p(y), c_int(heads),
+                      *_chunk_place(ctx, skip_rows, group), _p(states), _p(decays), _p(y), c_int(heads),
                       c_int(P), c_int(N), c_int(groups), _stream())
         if not others:
             return y
-        skip_rows = TUNING["chunk_scan_min_rows"]
     _lib.call("nf_ssd_scan", _p(xbc), c_int(xbc.shape[1]), c_int(x_col0), c_int(b_col0), c_int(c_col0), _p(dt_src),
               c_int(dt_src.shape[1]), c_int(dt_col0), _p(dt_bias), _p(A_log), _p(D),
               state_p, c_longlong(state.stride(0)), _p(ctx.seg_row0), _p(ctx.seg_slot), _p(y), c_int(ctx.S), c_int(heads),

@@ -12,6 +12,8 @@ function; here the same stages are objects chosen layer by layer.
 
 from __future__ import annotations
 
+import bisect
+import itertools
 from dataclasses import dataclass, field
 from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
@@ -285,32 +287,21 @@ class StepContext:
         return self._tiles[key]
 
     def recurrence_chunks(self, rows_per_chunk: int, min_rows: int, max_chunks: int
-                          ) -> Tuple[List[Tuple[torch.Tensor, int, torch.Tensor, int]], bool]:
-        """Chunks of `rows_per_chunk` rows, counted from the first row, of the segments that bring at least `min_rows`
-        rows: a list of groups of at most `max_chunks` of them, to be run one after the other, each as (int32 [n, 3] of
-        (segment, first row, rows), n, int32 [m, 3] of the segments' runs in it as (segment, first chunk, chunks), m);
-        and whether other segments are left.  Built on the host; not available in graph mode."""
+                          ) -> Tuple[List[Tuple[int, int, int, int]], int, int]:
+        """Chunks of `rows_per_chunk` rows of the segments that bring at least `min_rows` rows, counted over those
+        segments: groups of at most `max_chunks` of them, to be run one after the other, each as (first chunk, chunks,
+        number of the first segment it has a part of among those segments, such segments); the most rows that another
+        segment brings; and the rows of those segments.  Not available in graph mode."""
         key = ("recurrence_chunks", rows_per_chunk, min_rows, max_chunks)
         if key not in self._tiles:
-            groups, row, others = [], 0, False
-            for s, n in enumerate(self.seg_len_host):
-                others = others or n < min_rows
-                for r in range(0, n if n >= min_rows else 0, rows_per_chunk):
-                    if not groups or len(groups[-1][0]) == max_chunks:
-                        groups.append(([], []))
-                    chunks, runs = groups[-1]
-                    if not runs or runs[-1][0] != s:
-                        runs.append([s, len(chunks), 0])
-                    runs[-1][2] += 1
-                    chunks.append([s, row + r, min(rows_per_chunk, n - r)])
-                row += n
-            flat = self._ints([v for chunks, runs in groups for part in (chunks, runs) for c in part for v in c])
-            lists, at = [], 0
-            for chunks, runs in groups:
-                mid, end = at + 3 * len(chunks), at + 3 * (len(chunks) + len(runs))
-                lists.append((flat[at:mid], len(chunks), flat[mid:end], len(runs)))
-                at = end
-            self._tiles[key] = (lists, others)
+            ends = list(itertools.accumulate((n + rows_per_chunk - 1) // rows_per_chunk for n in self.seg_len_host if n >= min_rows))
+            others = max((n for n in self.seg_len_host if n < min_rows), default=0)
+            groups = []
+            for first in range(0, ends[-1] if ends else 0, max_chunks):
+                last = min(ends[-1], first + max_chunks) - 1
+                run = bisect.bisect_right(ends, first)
+                groups.append((first, last + 1 - first, run, bisect.bisect_right(ends, last) + 1 - run))
+            self._tiles[key] = (groups, others, sum(n for n in self.seg_len_host if n >= min_rows))
         return self._tiles[key]
 
     def whole_contexts(self, segments: Tuple[int, ...], rows_per_tile: int) -> Tuple[torch.Tensor, int, torch.Tensor, int]:

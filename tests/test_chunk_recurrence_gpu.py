@@ -6,8 +6,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 # segments at the edges of a chunk (64 and 128 rows) and of its sixteens, beside short ones that the row-by-row kernel
-# keeps; the last entry is several groups of chunks when the scratch is small
-LENGTHS = [[64], [65, 1, 63], [127, 128, 129], [80, 3, 257], [700]]
+# keeps, and more than a warp's lanes of them; the last two are several groups of chunks when the scratch is small
+LENGTHS = [[64], [65, 1, 63], [127, 128, 129], [80, 3, 257], [1] * 33 + [70, 2, 200], [700], [300, 2, 130, 200, 70]]
 
 
 def context(lens):
@@ -47,7 +47,7 @@ def test_scan_in_chunks(lens, N, slow, monkeypatch):
     from ninfer_amd_mi50_b200 import kernels
     monkeypatch.setitem(kernels.TUNING, "chunk_scan_min_rows", 63)
     H, P, G = 6, 64, 2
-    if lens == [700]:
+    if sum(lens) >= 700:
         monkeypatch.setitem(kernels.TUNING, "chunk_recurrence_max_mb", 1)
     g = torch.Generator(device="cuda").manual_seed(sum(lens) + N)
     rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
@@ -82,7 +82,7 @@ def test_linear_attention_in_chunks(lens, D, silu, monkeypatch):
     from ninfer_amd_mi50_b200 import kernels
     monkeypatch.setitem(kernels.TUNING, "chunk_linear_min_rows", 63)
     H, V = 5, 128
-    if lens == [700]:
+    if sum(lens) >= 700:
         monkeypatch.setitem(kernels.TUNING, "chunk_recurrence_max_mb", 1)
     g = torch.Generator(device="cuda").manual_seed(sum(lens) + D)
     rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
@@ -117,7 +117,7 @@ def test_delta_rule_in_chunks(lens, D, V, alike, monkeypatch):
     from ninfer_amd_mi50_b200 import kernels
     monkeypatch.setitem(kernels.TUNING, "chunk_delta_min_rows", 63)
     H, G, off = 4, 2, 8
-    if lens == [700]:
+    if sum(lens) >= 700:
         monkeypatch.setitem(kernels.TUNING, "chunk_recurrence_max_mb", 1)
     g = torch.Generator(device="cuda").manual_seed(sum(lens) + D)
     rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
@@ -202,3 +202,23 @@ def test_what_is_not_finite_stays_behind_its_row(kind, bad, at, monkeypatch):
             assert not out[at, 0].isfinite().any() and torch.equal(out[at + 1:], want[at + 1:]) and torch.equal(state, end)
         elif not (col is None and bad > 0):                   # (an infinite gate of the delta rule forgets everything)
             assert not out[at, 0].isfinite().any()
+
+
+@pytest.mark.parametrize("lens,heads,chunks,walk", [
+    ([128], 64, False, True),                          # too little for three launches more
+    ([279, 162, 202, 244, 254, 40], 8, False, True),   # neither long nor much: one form, not both
+    ([279, 162, 202, 244, 254, 64], 64, True, False),  # much work together
+    ([1024], 4, True, False),                          # a long chain
+    ([1, 1024, 63, 64], 4, True, True),                # what is too short for a chunk is walked beside it
+    ([1] * 64, 64, False, True)])
+def test_which_form_a_step_takes(lens, heads, chunks, walk, monkeypatch):
+    from ninfer_amd_mi50_b200 import kernels
+    from ninfer_amd_mi50_b200.kernels import ops
+    P, N, G, called, call = 64, 128, 1, [], ops._lib.call
+    monkeypatch.setattr(ops._lib, "call", lambda name, *a: (called.append(name), call(name, *a))[1])
+    ctx, T = context(lens), sum(lens)
+    xbc, dt = (torch.zeros(T, c, dtype=torch.bfloat16, device="cuda") for c in (heads * P + 2 * G * N, heads))
+    one = torch.ones(heads, device="cuda")
+    state = torch.zeros(len(lens) + 2, heads * P * N, device="cuda")
+    kernels.ssd_scan(xbc, 0, heads * P, heads * P + G * N, dt, 0, one, one, one, state, 0, ctx, heads, P, N, G)
+    assert called == ["nf_chunk_scan"] * chunks + ["nf_ssd_scan"] * walk
