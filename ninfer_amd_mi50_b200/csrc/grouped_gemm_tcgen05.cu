@@ -376,21 +376,22 @@ extern "C" int nf_set_grouped_gemm_pair(int on, int min_rows) {
 }
 
 // out[p, :n_features] for sorted rows p of every group.  X holds the rows in sorted order
-// ([total_rows, K], already gathered).  Wp holds the groups' weights packed as
+// ([total_rows, ldx], of which the first K columns count, already gathered; ldx 0: K).  Wp holds the groups' weights packed as
 // [groups][ceil(n_features / 128)][ceil(K / 64)][128 or 256 rows][64], each tile in the
 // 128-byte-swizzled image (SwiGLU: 128 gate rows then the 128 matching up rows per tile),
 // zero-padded.  Needs K % 8 == 0 and a 16-byte aligned X (TMA).
-extern "C" int nf_grouped_gemm_tc(const void* X, long long total_rows, const void* Wp, int groups,
+extern "C" int nf_grouped_gemm_tc(const void* X, long long total_rows, int ldx, const void* Wp, int groups,
                                   int n_features, int K, const int* offsets, void* out, int ldo,
                                   int swiglu, float act_limit, float act_alpha, cudaStream_t stream) {
   if (total_rows == 0) return 0;
   NF_REQUIRE(total_rows > 0 && groups > 0 && n_features > 0 && K > 0, "grouped_gemm_tc: bad sizes");
   NF_REQUIRE(K % 8 == 0, "grouped_gemm_tc: K=%d must be a multiple of 8 (16-byte rows for TMA)", K);
+  NF_REQUIRE(ldx == 0 || (ldx >= K && ldx % 8 == 0), "grouped_gemm_tc: rows %d apart for K=%d", ldx, K);
   NF_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)Wp % 16 == 0), "grouped_gemm_tc: operands must be 16-byte aligned");
   NF_REQUIRE(groups <= kMaxGroupsTc, "grouped_gemm_tc: %d groups, at most %d", groups, kMaxGroupsTc);
   CUtensorMap mx, mx_half;
-  if (int rc = make_map(&mx, X, total_rows, K, kXBox)) return rc;
-  if (int rc = make_map(&mx_half, X, total_rows, K, kXBox / 2)) return rc;
+  if (int rc = make_map(&mx, X, total_rows, K, kXBox, ldx)) return rc;
+  if (int rc = make_map(&mx_half, X, total_rows, K, kXBox / 2, ldx)) return rc;
   NF_REQUIRE(swiglu >= 0 && swiglu <= 3, "grouped_gemm_tc: epilogue %d (0 none, 1 silu-gated, 2 capped, 3 ungated GELU)", swiglu);
   const GatedActParams act{swiglu, act_limit, act_alpha};
   if (swiglu == kActSilu || swiglu == kActCapped) return launch_tc<true, false>(Wp, mx, mx_half, offsets, out, ldo, n_features, K, groups, act, stream);

@@ -1047,7 +1047,7 @@ def moe_gemm1(x: torch.Tensor, w13, plan: MoePlan, k: int, gathered: Optional[to
             # rows in sorted order, then one tensor-core launch over all experts
             xp = gathered if gathered is not None else moe_gather(x, plan, k)
             kind, limit, alpha = _act(True, act)
-            _lib.call("nf_grouped_gemm_tc", _p(xp), c_longlong(T * k), _p(w13.data), c_int(E),
+            _lib.call("nf_grouped_gemm_tc", _p(xp), c_longlong(T * k), c_int(0), _p(w13.data), c_int(E),
                       c_int(inner), c_int(H), _p(plan.offsets), _p(out), c_int(inner), c_int(kind),
                       c_float(limit), c_float(alpha), _stream())
         return out
@@ -1092,7 +1092,7 @@ def moe_gemm2(act: torch.Tensor, w2, plan: MoePlan, plan_is_older: bool = False,
             _skinny(act, inner, w2.data, w2.group_stride, y, n, H, inner, E, plan.num_tokens, plan.offsets,
                     None, 1, False, packed=True, group_map=plan.active, early_index=plan_is_older)
         else:
-            _lib.call("nf_grouped_gemm_tc", _p(act), c_longlong(n), _p(w2.data), c_int(E), c_int(H),
+            _lib.call("nf_grouped_gemm_tc", _p(act), c_longlong(n), c_int(0), _p(w2.data), c_int(E), c_int(H),
                       c_int(inner), _p(plan.offsets), _p(y), c_int(H), c_int(3 if gelu else 0), c_float(0.0),
                       c_float(0.0), _stream())
             return y
@@ -1875,7 +1875,8 @@ def _expanded_segments(ctx, most: int, Dr: int, pair_ops: int) -> List[Tuple[int
 def expanded_latent_attention(q: torch.Tensor, w_kv: torch.Tensor, heads: int, D: int, pages: torch.Tensor,
                               block_table: torch.Tensor, page_size: int, ctx, scale: float, out: torch.Tensor,
                               gate: Optional[torch.Tensor] = None, gate_col0: int = 0, Dr: int = 0,
-                              sink: Optional[torch.Tensor] = None, segments: Optional[Tuple[int, ...]] = None) -> None:
+                              sink: Optional[torch.Tensor] = None, segments: Optional[Tuple[int, ...]] = None,
+                              packed: Optional[PackedWeights] = None) -> None:
     """Causal softmax attention of the given segments (None: all of several rows) over a latent cache, by expanding it: the
     segments' cached rows c (pages [n, page_size, R]) are gathered, one product with w_kv [2 * heads * D, R] (keys of
     all heads, then values) gives every token's keys and values, and the tcgen05 kernel runs over those.  q [T, ld]
@@ -1883,17 +1884,24 @@ def expanded_latent_attention(q: torch.Tensor, w_kv: torch.Tensor, heads: int, D
     goes to out [T, heads * D], whose rows of other segments are left as they are.
 
     With `Dr` the cached rows are [c | Dr rotated dimensions that all heads share], the queries heads * (D + Dr), and
-    exp(sink[h]) joins the softmax's denominator (no gate then: it is the caller's)."""
+    exp(sink[h]) joins the softmax's denominator (no gate then: it is the caller's).  `packed`, w_kv as `pack_weights`
+    lays it out, lets the experts' tcgen05 product read the latents where they lie in those rows (2,048 rows, 16 heads,
+    latents of 512: 17 us; a library product of the same 11)."""
     _chk(q, "q", torch.bfloat16); _chk(w_kv, "w_kv", q.dtype); _chk(pages, "pages", q.dtype); _chk(out, "out", q.dtype)
     R = w_kv.shape[1]
     if segments is None:
         segments = tuple(s for s, n in enumerate(ctx.seg_len_host) if n > 1)
-    base, total, tiles, n_tiles = ctx.whole_contexts(segments, 128)
+    base, total, tiles, n_tiles, ends = ctx.whole_contexts(segments, 128)
     c = torch.empty((total, R + Dr), dtype=q.dtype, device=q.device)
     _lib.call("nf_gather_cached_rows", _p(pages), _p(block_table), c_int(block_table.shape[1]), _p(ctx.seg_pos0),
               _p(ctx.seg_row0), _p(base), _p(c), c_int(ctx.S), c_int((R + Dr) * 2), c_int(page_size), c_int(pages.shape[0]),
               c_int(int(ctx.max_context)), c_int(total), _stream())
-    kv = linear(c, w_kv) if Dr == 0 else torch.mm(c[:, :R], w_kv.t())        # (a product over the rows' first part)
+    if packed is not None:
+        kv = torch.empty((total, 2 * heads * D), dtype=q.dtype, device=q.device)
+        _lib.call("nf_grouped_gemm_tc", _p(c), c_longlong(total), c_int(R + Dr), _p(packed.data), c_int(1), c_int(2 * heads * D),
+                  c_int(R), _p(ends), _p(kv), c_int(2 * heads * D), c_int(0), c_float(0.0), c_float(0.0), _stream())
+    else:
+        kv = linear(c[:, :R].contiguous(), w_kv)
     if Dr:
         if sink is not None:
             _chk(sink, "sink", torch.float32)

@@ -304,11 +304,12 @@ class StepContext:
             self._tiles[key] = (groups, others, sum(n for n in self.seg_len_host if n >= min_rows))
         return self._tiles[key]
 
-    def whole_contexts(self, segments: Tuple[int, ...], rows_per_tile: int) -> Tuple[torch.Tensor, int, torch.Tensor, int]:
+    def whole_contexts(self, segments: Tuple[int, ...], rows_per_tile: int
+                       ) -> Tuple[torch.Tensor, int, torch.Tensor, int, torch.Tensor]:
         """For attention over a matrix that holds the whole contexts (what was held and what the step brings) of the given
         segments one after the other: int32 [S] of where each starts in it, -1 for the other segments; its rows; query
-        tiles of those segments, one to a CTA, heaviest first, as `paired_query_tiles` gives them; their number.  Built on
-        the host; not in graph mode."""
+        tiles of those segments, one to a CTA, heaviest first, as `paired_query_tiles` gives them; their number; and int32
+        (0, rows of the matrix).  Built on the host; not in graph mode."""
         key = ("whole_contexts", segments, rows_per_tile)
         if key not in self._tiles:
             base, total, chosen, tiles, row = [], 0, set(segments), [], 0
@@ -319,8 +320,9 @@ class StepContext:
                     tiles += [(-(p + min(r + rows_per_tile, n)), s, row + r) for r in range(0, n, rows_per_tile)]
                 row += n
             tiles.sort()
-            flat = self._ints(base + [-1] * (-len(base) % 4) + [v for _, s, r in tiles for v in (s, r, -1, -1)])
-            self._tiles[key] = (flat[:len(base)], total, flat[len(flat) - 4 * len(tiles):], len(tiles))
+            n = len(base)
+            flat = self._ints(base + [0, total] + [v for _, s, r in tiles for v in (s, r, -1, -1)])
+            self._tiles[key] = (flat[:n], total, flat[n + 2:], len(tiles), flat[n:n + 2])
         return self._tiles[key]
 
     def paired_query_tiles(self, rows_per_tile: int, window: int, keys_per_block: int,

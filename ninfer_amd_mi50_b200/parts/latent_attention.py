@@ -63,7 +63,7 @@ class LatentAttention(Mixer):
         self.q_head = self.dim + self.rot_dim
         self.names = dict(self.DEFAULT_NAMES)
         self.names.update(dict(tensor_names or ()))
-        self.w_in = self.w_uq = self.w_uk = self.w_uv = self.w_o = None
+        self.w_in = self.w_uq = self.w_uk = self.w_uv = self.w_o = self.w_kv_packed = None
         self.q_norm = self.kv_norm = self.sink = None
 
     def _n(self, what: str) -> str:
@@ -104,6 +104,9 @@ class LatentAttention(Mixer):
         self.w_kv = torch.cat([fetch(self._n("uk")), fetch(self._n("uv"))], dim=0).contiguous()
         self.w_uk = self.w_kv[:H * self.dim].view(H, self.dim, self.kv_rank)                               # q_plain_h @ W_uk[h]
         self.w_uv = self.w_kv[H * self.dim:].view(H, self.value_dim, self.kv_rank).transpose(1, 2)          # o_h @ W_uv[h]^T
+        if (self.w_kv.is_cuda and self.w_kv.dtype == torch.bfloat16 and kernels.can_pack(self.w_kv.shape[0], self.kv_rank)
+                and (self.dim, self.value_dim, self.rot_dim) == (128, 128, 64) and not self.window):
+            self.w_kv_packed = kernels.pack_weights(self.w_kv[None], swiglu=False)     # to expand rows [c | rotated]
         self.q_norm = fetch(self._n("dq_norm")) if self.q_rank else None
         self.kv_norm = fetch(self._n("dkv_norm"))
         self.sink = fetch(self._n("sink")) if self.has_sink else None
@@ -111,6 +114,7 @@ class LatentAttention(Mixer):
     def weight_bytes(self) -> int:
         el = self.w_in.element_size()
         n = sum(t.numel() for t in (self.w_in, self.w_uq, self.w_uk, self.w_uv, self.w_o) if t is not None) * el
+        n += self.w_kv_packed.data.numel() * el if self.w_kv_packed is not None else 0
         return n + 4 * ((self.q_rank or 0) + self.kv_rank + (self.heads if self.has_sink else 0))
 
     # ---- cache ------------------------------------------------------------------------
@@ -155,7 +159,7 @@ class LatentAttention(Mixer):
         for segments in groups:
             kernels.expanded_latent_attention(q, self.w_kv, H, self.dim, cache.pages, cache.block_table, cache.page_size, ctx,
                                               self.scale, o, gate, gate_col0 if gate is not None else 0, self.rot_dim, self.sink,
-                                              segments)
+                                              segments, self.w_kv_packed)
         if self.has_gate and self.rot_dim:
             o = kernels.sigmoid_gate_rows(o, proj, gate_col0)
         taken = {s for segments in groups for s in segments}

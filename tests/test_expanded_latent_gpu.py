@@ -101,3 +101,28 @@ def test_a_segment_decides_for_itself():
         got, expanded = run(lens)
         assert ((got - alone).norm() / alone.norm()).item() <= 1e-3, lens
         assert expanded == [(lens.index(long),)]
+
+
+@pytest.mark.parametrize("lens", [[2], [63, 1, 64], [257], [500, 300]])
+@pytest.mark.parametrize("rank", [64, 72, 512])
+def test_expanded_by_the_packed_product(lens, rank):
+    """The latents read where they lie in the cached rows, by the experts' product, against the plain one."""
+    from ninfer_amd_mi50_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(sum(lens) + rank)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ctx = context(lens)
+    T, per = sum(lens), (ctx.max_context + PAGE - 1) // PAGE
+    table = torch.arange(len(lens) * per, dtype=torch.int32, device="cuda").flip(0).contiguous().view(len(lens), per)
+    pages = rand(len(lens) * per, PAGE, rank + DR).bfloat16()
+    q, w_kv = rand(T, H * (D + DR)).bfloat16(), (rand(2 * H * D, rank) * rank ** -0.5).bfloat16()
+    outs = []
+    for packed in (None, kernels.pack_weights(w_kv[None], swiglu=False)):
+        out = torch.zeros((T, H * D), dtype=q.dtype, device="cuda")
+        kernels.expanded_latent_attention(q, w_kv, H, D, pages, table, PAGE, ctx, (D + DR) ** -0.5, out, Dr=DR, packed=packed)
+        kernels.check_status("expanded latent attention")
+        assert kernels.tensor_core_status() == 0
+        outs.append(out.double())
+    # the same bfloat16 keys and values but where two orders of a float32 sum fall on either side of a rounding: such a
+    # number is off by 2^-8 of itself, one in some hundreds
+    assert ((outs[0] - outs[1]).norm() / outs[0].norm()).item() <= 1e-3
+    assert outs[0].abs().sum() > 0
