@@ -9,7 +9,10 @@
 //   few rows        4 x 32, one warp: a stream of weights; many small CTAs keep enough bytes in flight even where a
 //                   projection has few features.  Rows beyond four read the weights again, from L2: 20 rows of one
 //                   matrix (6144 x 2048) 40 us, with the next tile 52; 33 rows 70 and 53.  Beside one another the groups
-//                   fill the device by themselves: 4.3 rows a group 148 us and 204, 8.5 rows 228 and 212 (60 x 2048 x 1408)
+//                   fill the device by themselves: 4.3 rows a group 148 us and 204, 8.5 rows 228 and 212 (60 x 2048 x 1408).
+//                   A matrix beyond L2 they read from memory: a head of 151936 x 2048 with 5 rows 431 us, with the next
+//                   tile 320, 16 rows 843 and 328, 24 rows 1247 and 671 (4 rows 236 and 320); 32000 x 2048 with 5 rows 115
+//                   and 88; half of 12288 x 4096 is still in L2: 8 rows 74 and 93, 12 rows 100 and 95
 //   up to 64        16 x 64, two warps with 8 x 2 sums a thread (34 rows a group 472 us, with the next tile 518)
 //   up to 128       32 x 64 with 4 x 4 sums a thread: 100 rows 112 us, with the tile before 152, with the one behind 140
 //   more            64 x 64 with 8 x 4 sums a thread (gated 4 x 4), bound by the products themselves: 256 rows 184 us,
@@ -22,6 +25,7 @@
 namespace nf {
 namespace {
 
+constexpr size_t kGfL2 = 126u << 20, kGfFar = 230u << 20;    // bytes of a matrix: beyond L2; with next to nothing left in it
 constexpr int kGfK = 32;                  // k a stage
 constexpr int kGfRow = kGfK + 4;          // floats between two rows of a stage
 
@@ -165,7 +169,8 @@ int gf_dispatch(const GfCall& c, cudaStream_t stream) {
   };
   // (the lines lie between the measured sizes at which the tile below and the one above were the faster)
   const bool alone = c.groups == 1;
-  if (rows <= (alone ? 24 : 5)) return gf_launch<4, GATED ? 64 : 32, 4, GATED ? 2 : 1, 6, GATED>(c, tiles(4), stream);
+  const size_t matrix = (size_t)c.N * (GATED ? 2 : 1) * c.K * sizeof(float);
+  if (rows <= (!alone ? 5 : matrix > kGfFar ? 4 : matrix > kGfL2 ? 10 : 24)) return gf_launch<4, GATED ? 64 : 32, 4, GATED ? 2 : 1, 6, GATED>(c, tiles(4), stream);
   if (rows <= 64) return gf_launch<16, 64, 8, 2, 4, GATED>(c, tiles(16), stream);
   if (rows <= 128) return gf_launch<32, 64, 4, 4, 4, GATED>(c, tiles(32), stream);
   if (GATED) return gf_launch<64, 64, 4, 4, 3, GATED>(c, tiles(64), stream);

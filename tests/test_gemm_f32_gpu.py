@@ -45,3 +45,20 @@ def test_experts(T, E, k):
     e = idx.long()
     gate, up = torch.einsum("tkih,th->tki", w13.double()[e], x.double()).split(inner, 2)
     close(got, torch.einsum("tkhi,tki->tkh", w2.double()[e], torch.nn.functional.silu(gate) * up), 4 * (H + inner))
+
+
+@pytest.mark.parametrize("N,K", [(32800, 2048), (20000, 2048)])
+def test_matrices_beyond_l2(N, K):
+    """More than twice L2 and more than once: other tiles for few rows, the same bits."""
+    from ninfer_amd_mi50_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(N)
+    wide = torch.randn(N * K + 1, generator=g, device="cuda")
+    moved = wide[1:].view(N, K)                                # one element on: the kernel for rows that are not aligned
+    w = moved.clone()
+    for M in (4, 5, 10, 11, 24, 25):
+        x = torch.randn(M, K, generator=g, device="cuda")
+        got = kernels.linear(x, w)
+        assert torch.equal(got, kernels.linear(x, moved)), M
+        if M == 11:
+            close(got, x.double() @ w.double().T, K)
+            assert torch.equal(kernels.linear_swiglu(x, w), kernels.linear_swiglu(x, moved))
