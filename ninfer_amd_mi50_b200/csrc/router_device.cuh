@@ -263,8 +263,7 @@ __device__ __forceinline__ void select_token_ruled(const float* __restrict__ row
 // have pairs, ascending, padded with -1 to n_active_max.  The first `warps` warps take consecutive runs of the pairs, 32
 // pairs at a time: lanes that hold the same expert find one another by a match, and a warp keeps its counts so far in its
 // row of `hist` [warps][E]; the rows are then added up over the warps and the experts.  (Every expert walking all pairs,
-// as this did before, costs E / 32 passes over them: 13 us for 2,048 pairs of 60 experts, now 5; two
-// kernels of 20 us together for 8,192, now one of 13.)
+// as this did before, costs E / 32 passes over them: 14 us for 2,048 pairs of 60 experts, now 6.)
 // counts: E + 1 ints of shared memory.
 __device__ __forceinline__ void plan_block(const int* __restrict__ topk_idx, int n, int E, int* __restrict__ offsets,
                                            int* __restrict__ order, int* __restrict__ inv, int* counts, int* hist, int warps,

@@ -644,6 +644,19 @@ def test_moe_plan(K, T, k, E):
     assert torch.equal(plan.active, ref.active)
 
 
+@pytest.mark.parametrize("T,k,E", [(6143, 2, 8), (6144, 2, 8), (2175, 8, 256), (2176, 8, 256), (3481, 10, 512), (3482, 10, 512),
+                                   (4400, 8, 513)])
+def test_moe_plan_spread_over_the_device(K, T, k, E):
+    """Both sides of the sizes from which every expert has a block of its own; half of the experts get no pairs."""
+    g = torch.Generator().manual_seed(24)
+    idx = (torch.stack([torch.randperm(E // 2, generator=g)[:min(k, E // 2)] for _ in range(64)]) * 2).to(torch.int32).cuda()
+    idx = idx.repeat((T + 63) // 64, 1)[:T].contiguous()
+    plan = K.moe_plan(idx, E)
+    ref = P.moe_plan(idx, E)
+    for name in ("offsets", "order", "inv", "active"):
+        assert torch.equal(getattr(plan, name), getattr(ref, name)), name
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T,H,I,E,k", [(1, 200, 72, 6, 3), (50, 96, 100, 16, 4), (130, 256, 33, 8, 2),
                                        (64, 512, 136, 60, 4), (8, 2048, 1408, 60, 4)])
