@@ -13,13 +13,16 @@
 //
 // All query heads of a group share the CTA, so keys and values are read once per kv head.
 //
-// Few rows of up to eight blocks (a context bound of 1,024 keys) take one launch: a row's blocks are a thread-block
-// cluster, and what the second kernel does is done there, out of the CTAs' shared memory (same sums in the same order).
+// Few rows of up to eight blocks (a context bound of 1,024 keys, at most 148 CTAs, CTAs enough for a row's heads: see
+// launch_split) take one launch: a row's blocks are a thread-block cluster, and what the second kernel does is done there,
+// out of the CTAs' shared memory (same sums in the same order).
 //
 // Further forms.  SIGMOID: a key weighs sigmoid(score + sig_bias[h]), not normalised over keys - blocks carry the
 // maximum 0 and simply add.  CAPPED: the softmax over cap * tanh(score / cap).  Turned values: the merge turns the first `turn_dims` numbers of a head's result by minus
 // the row's position (what turn_back in qk_norm_append.cu does in a pass of its own, here on the float32 sum).
 #define NF_CHAIN_CLASS 8
+#include <atomic>
+
 #include "common.cuh"
 #include "decode_range.cuh"
 
@@ -61,12 +64,6 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   return *reinterpret_cast<unsigned*>(&v);
 }
 
-// Workspace per (row, q head, split): D floats of unnormalised output, and (m, l) apart.
-// The CTA first asks for all of its keys and values (asynchronous copies into shared
-// memory, so that all 2 * 128 * D * 2 bytes are in flight at once).  Scores and the
-// weighted sum of values are tensor-core products with the keys (values) as the 16-row
-// operand and up to 8 query heads of the group as the 8-column operand; softmax stays in
-// float32 in between.  Warp w owns keys [32 w, 32 w + 32) of the block.
 __device__ __forceinline__ float ld_cluster_f32(const float* local, unsigned cta) {
   unsigned remote;
   float v;
@@ -80,7 +77,16 @@ __device__ __forceinline__ void cluster_meet() {
 }
 constexpr int kClusterSplits = 8;  // most key blocks of a row that one cluster takes (the portable cluster size)
 constexpr int kClusterCtas = 148;  // most CTAs of such a launch (see launch_split)
+constexpr size_t kClusterSmem = 100 * 1024;   // most shared memory of such a CTA, so that two fit a SM: heads of 256 have more
+constexpr bool cluster_fits(int D) { return (size_t)2 * kSplit * (D + 8) * sizeof(__nv_bfloat16) <= kClusterSmem; }
+std::atomic<int> g_cluster_launches{0};
 
+// Workspace per (row, q head, split): D floats of unnormalised output, and (m, l) apart.
+// The CTA first asks for all of its keys and values (asynchronous copies into shared
+// memory, so that all 2 * 128 * D * 2 bytes are in flight at once).  Scores and the
+// weighted sum of values are tensor-core products with the keys (values) as the 16-row
+// operand and up to 8 query heads of the group as the 8-column operand; softmax stays in
+// float32 in between.  Warp w owns keys [32 w, 32 w + 32) of the block.
 template <int D, int FORM, bool CLUSTER>
 __global__ void __launch_bounds__(128)
 decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_stride,
@@ -486,18 +492,21 @@ static int launch_split(const void* qkv, int q_row_stride, const void* pages, co
   // rows of one block 6.1 -> 4.6): clusters start as a whole, where single CTAs trickle in and empty ones leave at once
   // (256 CTAs: two rows of eight blocks 5.8 -> 7.4; 512: four rows 5.9 -> 13.7).  And enough CTAs a row for its heads: a
   // thread adds up at most four numbers (28 heads on four key heads, one block: 6.5 -> 7.1, in four blocks 6.5 -> 5.6).
-  if (*merged && nsplit <= kClusterSplits && smem_c <= 100 * 1024 && (long long)T * Hkv * nsplit <= kClusterCtas &&
-      G * D <= 4 * 128 * nsplit) {
-    static size_t allowed_c = 48 * 1024;
-    if (smem_c > allowed_c) {
-      cudaFuncSetAttribute(decode_attention_split_kernel<D, FORM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c);
-      allowed_c = smem_c;
+  if constexpr (cluster_fits(D)) {
+    if (*merged && nsplit <= kClusterSplits && smem_c <= kClusterSmem && (long long)T * Hkv * nsplit <= kClusterCtas &&
+        G * D <= 4 * 128 * nsplit) {
+      static size_t allowed_c = 48 * 1024;
+      if (smem_c > allowed_c) {
+        cudaFuncSetAttribute(decode_attention_split_kernel<D, FORM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c);
+        allowed_c = smem_c;
+      }
+      launch_chained_clusters(decode_attention_split_kernel<D, FORM, true>, grid, dim3(128), smem_c, stream, dim3(1, 1, nsplit),
+                               (const __nv_bfloat16*)qkv, q_row_stride, (const __nv_bfloat16*)pages, block_table, bt_width,
+                               positions, row_seg, ws_acc, ws_ml, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters,
+                               (__nv_bfloat16*)out, row_list, sig_bias, softcap);
+      g_cluster_launches.fetch_add(1, std::memory_order_relaxed);
+      return check_launch("decode_attention_cluster");
     }
-    launch_chained_clusters(decode_attention_split_kernel<D, FORM, true>, grid, dim3(128), smem_c, stream, dim3(1, 1, nsplit),
-                             (const __nv_bfloat16*)qkv, q_row_stride, (const __nv_bfloat16*)pages, block_table, bt_width,
-                             positions, row_seg, ws_acc, ws_ml, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters,
-                             (__nv_bfloat16*)out, row_list, sig_bias, softcap);
-    return check_launch("decode_attention_cluster");
   }
   *merged = false;
   static size_t allowed = 48 * 1024;
@@ -551,6 +560,9 @@ extern "C" int nf_set_decode_cluster(int on) {
   g_decode_cluster = on ? 1 : 0;
   return 0;
 }
+
+// How many launches merged their blocks in clusters since the last call.
+extern "C" int nf_decode_cluster_launches() { return g_cluster_launches.exchange(0); }
 
 // bfloat16 only; head_dim in {16, 32, 64, 128, 256}.  `nsplit` >= ceil(max context / 128) of
 // the rows in this call.  Workspace: ws_acc float32 [T, Hq, nsplit, D], ws_ml [T, Hq, nsplit, 2].
