@@ -284,7 +284,7 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q_abs, const __nv_
 }
 
 // out[h, t, :] = (sum_s e^{m_s - M} O_s) / (sum_s e^{m_s - M} l_s + e^{sink_h - M}),  M the maximum of
-// the m_s and the sink; splits in ascending order.
+// the m_s and the sink; the outputs' splits in ascending order, the denominator's a lane's strided share and then the warp's.
 // The splits' weights are worked out once a (row, head), a warp's lanes side by side, and the sums run with their loads in
 // flight, four numbers a thread: one split after the other, each asking for its maximum and then for its numbers, was
 // 21 us of a decode step (37 splits of 512 numbers), now 6.
@@ -306,8 +306,9 @@ latent_attention_merge_kernel(const float* __restrict__ ws_o, const float* __res
     float l = 0.f;
     for (int s = threadIdx.x; s < nsplit; s += 32) {
       const float2 ml = *reinterpret_cast<const float2*>(ws_ml + (base + s) * 2);
-      const float w = ml.x != -INFINITY ? __expf(ml.x - M) : 0.f;
-      wt[s] = w;
+      const bool seen = ml.x != -INFINITY;               // (or the split has no key that the row sees: left out below,
+      const float w = seen ? __expf(ml.x - M) : 0.f;     // whatever its sums hold - zero times a later row's NaN, say)
+      wt[s] = seen ? w : -1.f;
       l += w * ml.y;
     }
     l = warp_sum(l) + (sink ? __expf(sk - M) : 0.f);
@@ -322,7 +323,7 @@ latent_attention_merge_kernel(const float* __restrict__ ws_o, const float* __res
       load4(ws_o + (base + s) * R + d, x);
       const float w = wt[s];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[e] = fmaf(w, x[e], acc[e]);
+      for (int e = 0; e < 4; ++e) acc[e] = w < 0.f ? acc[e] : fmaf(w, x[e], acc[e]);
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[e] *= s_inv;

@@ -126,3 +126,23 @@ def test_expanded_by_the_packed_product(lens, rank):
     # number is off by 2^-8 of itself, one in some hundreds
     assert ((outs[0] - outs[1]).norm() / outs[0].norm()).item() <= 1e-3
     assert outs[0].abs().sum() > 0
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_folded_rows_before_a_split_that_is_not_finite(bad):
+    """A cached row that is not finite leaves alone the rows of the portion that see no key of its key block (64 keys), a
+    split of its own here: the merge leaves out what such a split adds up."""
+    from ninfer_amd_mi50_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(9)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    heads, p, n = 2, 56, 16                                  # positions 56 to 71
+    ctx = context([n])
+    ctx.seg_pos0_host, ctx.seg_pos0, ctx.max_context = [p], ctx.seg_pos0 + p, p + n
+    ctx.positions = ctx.positions + p
+    pages, table = rand(2, PAGE, R + DR).bfloat16(), torch.tensor([[1, 0]], dtype=torch.int32, device="cuda")
+    q, q_abs = rand(n, heads * (D + DR)).bfloat16(), rand(heads, n, R).bfloat16()
+    run = lambda: kernels.latent_attention(q_abs, q, D + DR, D, DR, pages, table, PAGE, ctx, None, 0.1)
+    want = run()
+    pages[0, 5, 3] = bad                                     # position 69
+    got = run()
+    assert torch.equal(got[:, :64 - p], want[:, :64 - p]) and not got[:, 69 - p:].isfinite().all()
