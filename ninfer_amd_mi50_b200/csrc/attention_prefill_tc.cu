@@ -55,7 +55,9 @@
 //
 // Contract on the cache: rows of a page that lie beyond a request's position are read (whole
 // pages are copied) and multiplied by zero, so they must hold finite numbers; the cache manager
-// creates its pool zero-filled and only kernels write to it.
+// creates its pool zero-filled and only kernels write to it.  The DENSE form's blocks reach into the next request's rows,
+// which are under no such contract: there the softmax warps put zeros in the place of the values behind a tile's last
+// position.
 #include "tcgen05.cuh"
 
 namespace nf {
@@ -481,6 +483,16 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           sum += ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
         }
         l_run += sum;
+        if constexpr (DENSE) {
+          const int own_keys = t.pos_last + 1 - kb;
+          if (own_keys < kKeys) {                                // the tile's last block
+            if (!mbar_wait(&bars->v_full[gs % STAGES], (gs / STAGES) & 1, stop, 11, &g_fa_error)) { ok = false; break; }
+            unsigned char* vst = KV + (size_t)(gs % STAGES) * (QB + VB) + QB;
+            for (int i = own_keys * 8 + (threadIdx.x & 255); i < kKeys * 8; i += 256)
+#pragma unroll
+              for (int a = 0; a < ATOMS; ++a) reinterpret_cast<uint4*>(vst + a * kAtom)[i] = make_uint4(0, 0, 0, 0);
+          }
+        }
         fence_async_smem();
         tc_fence_before();
         __syncwarp();
@@ -687,7 +699,7 @@ extern "C" int nf_dense_rot_attention_tc(const void* q, long long T, int q_row_s
 }
 
 // 0 if no tensor-core attention kernel has given up on a wait since the last call; else the code
-// of the first wait that did (1-2 producer, 3-7 MMA issuer, 8-10 softmax).  Synchronises.
+// of the first wait that did (1-2 producer, 3-7 MMA issuer, 8-11 softmax).  Synchronises.
 extern "C" int nf_prefill_attention_tc_status() {
   int v = 0, zero = 0;
   if (cudaMemcpyFromSymbol(&v, g_fa_error, sizeof(int)) != cudaSuccess) return -1;

@@ -146,3 +146,30 @@ def test_folded_rows_before_a_split_that_is_not_finite(bad):
     pages[0, 5, 3] = bad                                     # position 69
     got = run()
     assert torch.equal(got[:, :64 - p], want[:, :64 - p]) and not got[:, 69 - p:].isfinite().all()
+
+
+@pytest.mark.parametrize("rotated", [0, DR])
+@pytest.mark.parametrize("lens", [[257, 40], [2, 129, 130], [100, 1, 28]])
+def test_requests_do_not_meet_in_a_block(lens, rotated):
+    """Requests lie one after the other in the expanded matrix, and a block of 128 keys reaches from one into the next: what
+    is not finite there stays behind."""
+    from ninfer_amd_mi50_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    ctx = context(lens)
+    per = (ctx.max_context + PAGE - 1) // PAGE
+    table = torch.arange(len(lens) * per, dtype=torch.int32, device="cuda").view(len(lens), per)
+    pages = rand(len(lens) * per, PAGE, R + rotated).bfloat16()
+    q, w_kv = rand(sum(lens), H * (D + rotated)).bfloat16(), (rand(2 * H * D, R) * R ** -0.5).bfloat16()
+
+    def attend():
+        out = torch.zeros((sum(lens), H * D), dtype=q.dtype, device="cuda")
+        kernels.expanded_latent_attention(q, w_kv, H, D, pages, table, PAGE, ctx, 0.1, out, Dr=rotated)
+        assert kernels.tensor_core_status() == 0
+        return out
+
+    want, before = attend(), sum(lens[:-1])
+    pages[(len(lens) - 1) * per:, :, ::2] = float("inf")     # the last request's rows
+    pages[(len(lens) - 1) * per:, :, 1] = float("nan")
+    got = attend()
+    assert torch.equal(got[:before], want[:before]) and not got[before:].isfinite().any()
