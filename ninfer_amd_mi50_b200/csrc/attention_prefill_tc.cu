@@ -56,8 +56,8 @@
 // Contract on the cache: rows of a page that lie beyond a request's position are read (whole
 // pages are copied) and multiplied by zero, so they must hold finite numbers; the cache manager
 // creates its pool zero-filled and only kernels write to it.  The DENSE form's blocks reach into the next request's rows,
-// which are under no such contract: there the softmax warps put zeros in the place of the values behind a tile's last
-// position.
+// which are under no such contract, and the BIASED form stands in for a kernel that does not read such rows: there the
+// softmax warps put zeros in the place of the values behind a tile's last position.
 #include "tcgen05.cuh"
 
 namespace nf {
@@ -483,7 +483,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           sum += ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
         }
         l_run += sum;
-        if constexpr (DENSE) {
+        if constexpr (DENSE || BIASED) {
           const int own_keys = t.pos_last + 1 - kb;
           if (own_keys < kKeys) {                                // the tile's last block
             if (!mbar_wait(&bars->v_full[gs % STAGES], (gs / STAGES) & 1, stop, 11, &g_fa_error)) { ok = false; break; }

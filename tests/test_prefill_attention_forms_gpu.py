@@ -53,3 +53,30 @@ def test_forms_at_the_edges(D, page, window, form, monkeypatch):
         rows = list(range(first + a, first + b))
         again = attend(rows, [b - a], [p0 + a], bt[-1:].contiguous(), fast)
         assert torch.equal(again, out[rows])
+
+
+@pytest.mark.parametrize("D,page", [(64, 32), (128, 64)])
+@pytest.mark.parametrize("window", [0, 300])
+def test_biased_form_leaves_out_what_a_page_held_before(D, page, window, monkeypatch):
+    """Rows of a request's last page behind its end, which hold another's infinities and NaN: the same bits."""
+    from ninfer_amd_mi50_b200 import kernels
+    dtype, Hq, Hkv = torch.bfloat16, 4, 2
+    seg_lens, pos0s = [2, 127, 129, 250], [700, 0, 5, 130]
+    ends = [p + n for p, n in zip(pos0s, seg_lens)]
+    n_pages = sum((e + page - 1) // page for e in ends) + 2
+    pages, bt, c, qkv = make_cache_case(dtype, Hq, Hkv, D, page, seg_lens, pos0s, n_pages, 3)
+    monkeypatch.setitem(kernels.TUNING, "prefill_attention_tc_min_rows", 1)
+    ctx, q = _step_context(c, seg_lens, pos0s, dtype, 1024), qkv[:, :Hq * D].contiguous()
+    slopes = torch.linspace(0.0, 0.02, Hq, device="cuda")
+
+    def attend():
+        out = kernels.biased_window_attention(q, Hq, Hkv, D, pages, bt, page, ctx, window, 5, 0.1, slopes)
+        assert kernels.tensor_core_status() == 0
+        return out
+
+    want = attend()
+    for s, e in enumerate(ends):
+        if e % page:
+            pages[bt[s, e // page], :, :, e % page:] = float("nan")
+            pages[bt[s, e // page], :, :, e % page:, ::2] = float("inf")
+    assert torch.equal(attend(), want) and want.isfinite().all()
