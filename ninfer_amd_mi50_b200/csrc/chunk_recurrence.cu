@@ -4,7 +4,7 @@
 // S is V x D per head, float32.
 //
 // Walking the rows one by one is bound by the chain from row to row (a prompt of 2,048 tokens, 64 heads of
-// 128 x 64: 771 us, about 1 % of the arithmetic's own time).  Over a chunk of Q rows the recurrence is three products:
+// 128 x 64: 755 us, about 1 % of the arithmetic's own time).  Over a chunk of Q rows the recurrence is three products:
 //
 //   o_t  = A_t S_0^T q_t + sum_{s <= t} (D(s, t) w_s q_t.k_s) v_s      A_t = a_1 ... a_t, D(s, t) = a_{s+1} ... a_t
 //   S_Q  = A_Q S_0 + sum_s D(s, Q) w_s k_s v_s^T

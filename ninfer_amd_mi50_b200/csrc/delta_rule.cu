@@ -24,6 +24,8 @@
 //    so the sums over D of all its rows are taken of the same registers, independent of one another, and only the
 //    short triangle in u is sequential.  Chunk c + 1's vectors and records are on their way (cp.async) meanwhile.
 //
+// The long segments of bfloat16 engines' larger steps run in chunks of 64 rows instead (chunk_recurrence.cu).
+//
 // A step of single rows is one kernel: every group of LANES lanes takes the vectors' norms itself, along with the
 // state's products (the norms are factors of those sums).
 //

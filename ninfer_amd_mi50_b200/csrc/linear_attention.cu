@@ -18,7 +18,8 @@
 // memory lies under the arithmetic.  A lane reads its entries of k and q as 16-byte pieces (rows
 // padded by 4 floats every EPL, which keeps the lanes of a column on different banks); the sum
 // over a column is log2(LANES) shuffles.  A token's result depends on earlier tokens only
-// through S, which holds the same bits however the request was cut.
+// through S, which these kernels leave with the same bits however the request was cut.  The long segments of bfloat16
+// engines' larger steps run in chunks instead (chunk_recurrence.cu): there the cut shows, by float32 roundings.
 //
 // The state of a slot is laid out [head][value column][D]: a column's entries are contiguous, so
 // the lanes of a column read and write whole 32-byte sectors.

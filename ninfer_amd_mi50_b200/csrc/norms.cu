@@ -178,7 +178,6 @@ add_group_rmsnorm_kernel(float* __restrict__ h, const T* __restrict__ d1, const 
   }
 }
 
-// out[t, 0:n] = x[t, col0:col0+n] * rsqrt(mean(x^2) + eps) * w   (w may be null: weight 1)
 // The row-wise norms below in their wide form: a thread owns R runs of four consecutive elements of a row's part, keeps
 // them in registers between the two passes and asks for the weights, which no kernel writes, before the wait.  In a decode
 // step such a kernel is a chain of trips to memory (rows of 2,048 and 4,096 read element by element, twice, with the weight
@@ -257,6 +256,7 @@ static int part_norm_vec(const void* y, int ldy, int ycol0, const void* z, int l
   return 1;
 }
 
+// out[t, 0:n] = x[t, col0:col0+n] * rsqrt(mean(x^2) + eps) * w   (w may be null: weight 1)
 template <typename T>
 __global__ void rms_norm_slice_kernel(const T* __restrict__ x, int ldx, int col0, int n,
                                       const float* __restrict__ w, float eps, T* __restrict__ out, int ldo) {

@@ -13,8 +13,9 @@
 //    request and walks that request's rows of the step in order; a column's N states are spread
 //    over a warp's lanes (registers), so y's sum over N is a shuffle reduction in a fixed order.  The
 //    step's B, C, x and dt are staged through shared memory sixteen tokens at a time.  A token's
-//    result depends on the tokens before it only through S, which is the same bits however the
-//    request was cut into steps.
+//    result depends on the tokens before it only through S, which this kernel leaves with the same bits
+//    however the request was cut into steps.  The long segments of bfloat16 engines' larger steps run in chunks instead
+//    (chunk_recurrence.cu): there the cut shows, by float32 roundings.
 //
 // Decays, step sizes, the state and the sums are float32; x, B, C come as the activations' type.
 #define NF_CHAIN_CLASS 2

@@ -13,8 +13,9 @@ without softmax or denominator.  Two designs of it are served by parameters:
   times a weight; times ``sigmoid(W_g x)``; out-projection.
 
 What a request keeps between steps is S for every head, float32, of fixed size (`state_spec`), so
-prompts cut into portions, decoded tokens and mixed batches all run the same kernel
-(``csrc/linear_attention.cu``), which continues from the slot and leaves it updated.  Decays,
+prompts cut into portions, decoded tokens and mixed batches run the same kernel
+(``csrc/linear_attention.cu``), which continues from the slot and leaves it updated, but for the long segments of a
+bfloat16 engine's larger steps, which run in chunks (``csrc/chunk_recurrence.cu``).  Decays,
 angles, the turned and scaled vectors, S and the sums are 32-bit in both modes; the projections
 (and their SiLU's argument) are in the engine's type.  The projections that read x (q, k, v and
 the gate) are one matrix, fused at load.

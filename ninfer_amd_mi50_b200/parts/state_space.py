@@ -14,7 +14,8 @@ square), multiplied by a weight, and projected out.  The gate comes before the n
 What a request keeps between steps is of fixed size: the convolution's last ``taps - 1`` inputs
 and S for every head, both float32, side by side in one slot (`state_spec`).  A step's rows of
 one request continue from the slot and leave it updated, so prompts cut into portions, decoded
-tokens and mixed batches all run the same two kernels (``csrc/ssm.cu``).  Decays, step sizes and
+tokens and mixed batches run the same two kernels (``csrc/ssm.cu``), but for the long segments of a bfloat16
+engine's larger steps, whose scan runs in chunks (``csrc/chunk_recurrence.cu``).  Decays, step sizes and
 the state are 32-bit in both modes; the projections, the convolution's output and the gate are in
 the engine's type.
 """
