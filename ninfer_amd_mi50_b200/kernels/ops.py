@@ -637,12 +637,26 @@ def paged_attention(qkv: torch.Tensor, Hq: int, Hkv: int, D: int, pages: torch.T
                   c_int(n_tiles), _p(out), c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size),
                   c_int(pages.shape[0]), c_int(window), c_float(scale), _stream())
         return out
-    _lib.call("nf_paged_attention_generic", _p(qkv), c_int(qkv.shape[1]), _p(pages),
-              _p(block_table), c_int(block_table.shape[1]), _p(ctx.positions), _p(ctx.row_seg),
-              _p(out), c_int(T), c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size),
-              c_int(pages.shape[0]), c_int(window), c_float(scale), c_int(_dt(qkv)), None, c_int(0), None,
-              c_int(0), None, c_float(softcap), _stream())
+    _plain_attention(qkv, Hq, Hkv, D, pages, block_table, page_size, ctx, window, scale, out, softcap=softcap)
     return out
+
+
+def _plain_attention(q, Hq, Hkv, D, pages, block_table, page_size, ctx, window, scale, out, slopes=None, keep=0, gate_p=None,
+                     gate_ld=0, sigmoid_bias=None, softcap=0.0) -> None:
+    """The kernels that sum in float32 on CUDA cores: in float32 one whose CTAs share the keys among the rows of a
+    segment, where rows are whole 16-byte pieces; else one warp a row and head.  Same sums in both."""
+    T = q.shape[0]
+    if q.dtype == torch.float32 and D % 4 == 0 and D <= 256 and pages.data_ptr() % 16 == 0 and hasattr(ctx, "seg_row0"):
+        _lib.call("nf_paged_attention_f32", _p(q), c_int(q.shape[1]), _p(pages), _p(block_table), c_int(block_table.shape[1]),
+                  _p(ctx.positions), _p(ctx.row_seg), _p(ctx.seg_row0), c_int(ctx.seg_row0.shape[0] - 1),
+                  c_int(ctx.max_rows_per_seg), _p(out), c_int(T), c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size),
+                  c_int(pages.shape[0]), c_int(window), c_float(scale), _p(slopes), c_int(keep), gate_p, c_int(gate_ld),
+                  _p(sigmoid_bias), c_float(softcap), _stream())
+        return
+    _lib.call("nf_paged_attention_generic", _p(q), c_int(q.shape[1]), _p(pages), _p(block_table),
+              c_int(block_table.shape[1]), _p(ctx.positions), _p(ctx.row_seg), _p(out), c_int(T), c_int(Hq),
+              c_int(Hkv), c_int(D), c_int(page_size), c_int(pages.shape[0]), c_int(window), c_float(scale),
+              c_int(_dt(q)), _p(slopes), c_int(keep), gate_p, c_int(gate_ld), _p(sigmoid_bias), c_float(softcap), _stream())
 
 
 def qk_whole_norm_append(proj: torch.Tensor, q_col0: int, k_col0: int, bias_q: Optional[torch.Tensor],
@@ -798,10 +812,8 @@ def biased_window_attention(q: torch.Tensor, Hq: int, Hkv: int, D: int, pages: t
                 if n_tiles:
                     flash(tiles, n_tiles, 0)
             return out
-    _lib.call("nf_paged_attention_generic", _p(q), c_int(q.shape[1]), _p(pages), _p(block_table),
-              c_int(block_table.shape[1]), _p(ctx.positions), _p(ctx.row_seg), _p(out), c_int(T), c_int(Hq),
-              c_int(Hkv), c_int(D), c_int(page_size), c_int(pages.shape[0]), c_int(window), c_float(scale),
-              c_int(_dt(q)), _p(slopes), c_int(keep), gate_p, c_int(gate_ld), _p(sigmoid_bias), c_float(0.0), _stream())
+    _plain_attention(q, Hq, Hkv, D, pages, block_table, page_size, ctx, window, scale, out, slopes=slopes, keep=keep,
+                     gate_p=gate_p, gate_ld=gate_ld, sigmoid_bias=sigmoid_bias)
     return out
 
 

@@ -1,0 +1,127 @@
+"""Kernels of decode steps and of the all-32-bit path at the sizes where they can go wrong: float32 attention that shares
+its keys among a segment's rows."""
+
+import math
+from dataclasses import replace
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from ninfer_amd_mi50_b200 import kernels
+    kernels.load()
+    return kernels
+
+
+def ints(values):
+    return torch.tensor(list(values), dtype=torch.int32, device="cuda")
+
+
+def make_step(dtype, lens, pos0s, Hkv, D, page, seed):
+    from ninfer_amd_mi50_b200.parts.base import StepContext
+    g = torch.Generator().manual_seed(seed)
+    need = [(p + n + page - 1) // page for p, n in zip(pos0s, lens)]
+    order, at = torch.randperm(sum(need), generator=g).tolist(), 0
+    bt = torch.full((len(lens), max(need) + 1), -1, dtype=torch.int32)
+    for s, n in enumerate(need):
+        bt[s, :n] = torch.tensor(order[at:at + n])
+        at += n
+    pages = torch.randn((sum(need), 2, Hkv, page, D), generator=g).to(dtype).cuda()
+    positions = [p + i for p, n in zip(pos0s, lens) for i in range(n)]
+    row_seg = [s for s, n in enumerate(lens) for _ in range(n)]
+    row0 = [0]
+    for n in lens:
+        row0.append(row0[-1] + n)
+    ctx = StepContext(dtype=dtype, device=torch.device("cuda"), T=len(positions), S=len(lens), token_ids=ints([0] * len(positions)),
+                      positions=ints(positions), row_seg=ints(row_seg), seg_row0=ints(row0), seg_pos0=ints(pos0s),
+                      seg_slot=ints(range(len(lens))), logit_rows=ints([]), seg_len_host=list(lens), seg_pos0_host=list(pos0s),
+                      max_rows_per_seg=max(lens), max_context=max(p + n for p, n in zip(pos0s, lens)))
+    return pages, bt.cuda(), ctx, positions, row_seg, g
+
+
+def exact_attention(q, pages, bt, positions, row_seg, Hq, page, window, keep, scale, slopes=None, gate=None, sig=None, cap=0.0):
+    """Row by row in 64 bits; q [T, Hq, D]."""
+    out = torch.zeros_like(q, dtype=torch.float64)
+    Hkv = pages.shape[2]
+    for t, (p, s) in enumerate(zip(positions, row_seg)):
+        j = torch.arange(p + 1, device="cuda")
+        kv = pages[bt[s, j // page].long(), :, :, j % page].double()          # [keys, 2, Hkv, D]
+        k, v = (kv[:, i].repeat_interleave(Hq // Hkv, 1) for i in (0, 1))
+        x = torch.einsum("hd,jhd->hj", q[t].double(), k) * scale
+        if cap:
+            x = cap * torch.tanh(x / cap)
+        if slopes is not None:
+            x = x - slopes.double()[:, None] * (p - j)
+        seen = (j > p - window) | (j < keep) if window else torch.ones_like(j, dtype=torch.bool)
+        if sig is not None:
+            w = torch.sigmoid(x + sig.double()[:, None]) * seen
+        else:
+            w = torch.softmax(x.masked_fill(~seen, -math.inf), -1)
+        out[t] = torch.einsum("hj,jhd->hd", w, v)
+        if gate is not None:
+            out[t] *= torch.sigmoid(gate[t].double())[:, None]
+    return out
+
+
+STEPS = [([37, 1, 16, 2, 1, 17], [0, 130, 61, 5, 0, 250]), ([1, 1, 1], [0, 127, 400]), ([130], [129])]
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,page", [(6, 2, 48, 16), (4, 1, 128, 64), (3, 3, 256, 32), (4, 2, 64, 16), (5, 1, 20, 24),
+                                          (40, 2, 32, 16)])
+@pytest.mark.parametrize("lens,pos0s", STEPS)
+@pytest.mark.parametrize("form", ["plain", "window", "kept", "cap", "sigmoid"])
+def test_float32_attention_that_shares_keys(K, Hq, Hkv, D, page, lens, pos0s, form):
+    """Against 64 bits, against the kernel of one warp a row (the same bits where no window shifts its blocks), and with
+    a step's rows sent one by one (the same bits always)."""
+    pages, bt, ctx, positions, row_seg, g = make_step(torch.float32, lens, pos0s, Hkv, D, page, 5)
+    T = ctx.T
+    q = torch.randn((T, Hq * D), generator=g).cuda()
+    scale = D ** -0.5
+    window = 70 if form in ("window", "kept") else 0
+    keep = 5 if form == "kept" else 0
+    slopes = torch.tensor([0.3 / (i + 1) for i in range(Hq)]).cuda() if form == "kept" else None
+    gate = torch.randn((T, Hq), generator=g).cuda() if form == "kept" else None
+    sig = torch.linspace(-1, 1, Hq).cuda() if form == "sigmoid" else None
+    cap = 2.0 if form == "cap" else 0.0
+
+    def run(ctx, rows=slice(None)):
+        if form in ("plain", "cap", "window"):
+            qkv = torch.cat([q[rows], torch.zeros((len(q[rows]), 2 * Hkv * D), device="cuda")], 1)
+            return K.paged_attention(qkv, Hq, Hkv, D, pages, bt, page, ctx, window, scale, softcap=cap)
+        return K.biased_window_attention(q[rows].contiguous(), Hq, Hkv, D, pages, bt, page, ctx, window, keep, scale, slopes,
+                                         None if gate is None else gate[rows].contiguous(), 0, sig)
+
+    out = run(ctx)
+    want = exact_attention(q.view(T, Hq, D), pages, bt, positions, row_seg, Hq, page, window, keep, scale, slopes, gate, sig, cap)
+    # sums of up to 401 products of 256 and of 401 weights, float32: some 2^-24 * sqrt(657) of the terms' size, times four
+    bound = 6e-6 * max(1.0, want.abs().max().item())
+    assert (out.view(T, Hq, D) - want).abs().max() <= bound
+    # without the segments' rows: one warp a row and head
+    warp = run(SimpleNamespace(positions=ctx.positions, row_seg=ctx.row_seg))
+    if window == 0:
+        assert torch.equal(out, warp)
+    else:
+        assert (out - warp).abs().max() <= bound
+    at = 0
+    for s, n in enumerate(lens):
+        for i in (0, n - 1):
+            one = replace(ctx, T=1, S=1, positions=ints([pos0s[s] + i]), row_seg=ints([s]), seg_row0=ints([0, 1]), seg_len_host=[1],
+                          max_rows_per_seg=1, _tiles={})
+            assert torch.equal(run(one, slice(at + i, at + i + 1))[0], out[at + i])
+        at += n
+
+
+def test_float32_attention_keeps_a_number_that_is_not_finite_behind_its_row(K):
+    """Later rows of a segment hold NaN: rows before them see nothing of it."""
+    pages, bt, ctx, positions, row_seg, g = make_step(torch.float32, [40], [3], 2, 64, 16, 6)
+    q = torch.randn((40, 4 * 64 + 2 * 2 * 64), generator=g).cuda()
+    good = K.paged_attention(q, 4, 2, 64, pages, bt, 16, ctx, 0, 0.125)
+    page, slot = int(bt[0, 23 // 16]), 23 % 16
+    pages[page, :, :, slot] = math.nan                        # position 23, row 20
+    bad = K.paged_attention(q, 4, 2, 64, pages, bt, 16, ctx, 0, 0.125)
+    assert torch.equal(bad[:20], good[:20]) and bad[20:].isnan().any(1).all()
