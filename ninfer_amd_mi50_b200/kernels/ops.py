@@ -1769,7 +1769,8 @@ def ssd_scan(xbc: torch.Tensor, x_col0: int, b_col0: int, c_col0: int, dt_src: t
     _lib.call("nf_ssd_scan", _p(xbc), c_int(xbc.shape[1]), c_int(x_col0), c_int(b_col0), c_int(c_col0), _p(dt_src),
               c_int(dt_src.shape[1]), c_int(dt_col0), _p(dt_bias), _p(A_log), _p(D),
               state_p, c_longlong(state.stride(0)), _p(ctx.seg_row0), _p(ctx.seg_slot), _p(y), c_int(ctx.S), c_int(heads),
-              c_int(P), c_int(N), c_int(groups), c_int(_dt(xbc)), c_int(skip_rows), _stream())
+              c_int(P), c_int(N), c_int(groups), c_int(_dt(xbc)), c_int(skip_rows),
+              c_int(1 if getattr(ctx, "all_single", False) else 0), _stream())
     return y
 
 

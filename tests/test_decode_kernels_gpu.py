@@ -1,5 +1,5 @@
 """Kernels of decode steps and of the all-32-bit path at the sizes where they can go wrong: float32 attention that shares
-its keys among a segment's rows."""
+its keys among a segment's rows, the scan of single rows."""
 
 import math
 from dataclasses import replace
@@ -125,3 +125,22 @@ def test_float32_attention_keeps_a_number_that_is_not_finite_behind_its_row(K):
     pages[page, :, :, slot] = math.nan                        # position 23, row 20
     bad = K.paged_attention(q, 4, 2, 64, pages, bt, 16, ctx, 0, 0.125)
     assert torch.equal(bad[:20], good[:20]) and bad[20:].isnan().any(1).all()
+
+
+@pytest.mark.parametrize("heads,P,N,groups", [(8, 64, 128, 2), (6, 20, 64, 3), (3, 7, 16, 1), (4, 33, 200, 4), (2, 64, 256, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_scan_of_single_rows_has_the_walking_kernels_bits(K, heads, P, N, groups, dtype):
+    _, _, ctx, _, _, g = make_step(dtype, [1, 1, 1], [0, 5, 9], 1, 16, 16, 8)
+    ctx.seg_slot = ints([2, 0, 3])
+    C = heads * P + 2 * groups * N
+    xbc = torch.randn((3, C), generator=g).to(dtype).cuda()
+    dt = torch.randn((3, heads + 5), generator=g).to(dtype).cuda()
+    bias, rate, D = (torch.randn((heads,), generator=g).cuda() for _ in range(3))
+    state = torch.randn((4, 10 + heads * P * N), generator=g).cuda()
+    results = []
+    for bound in (1, 2):                                      # 2: a bound of two rows a segment, so that rows are walked
+        st = state.clone()
+        y = K.ssd_scan(xbc, 0, heads * P, heads * P + groups * N, dt, 5, bias, rate, D, st, 10,
+                       replace(ctx, max_rows_per_seg=bound, _tiles={}), heads, P, N, groups)
+        results.append((y, st))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
