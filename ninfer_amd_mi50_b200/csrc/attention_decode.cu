@@ -17,6 +17,11 @@
 // launch_split) take one launch: a row's blocks are a thread-block cluster, and what the second kernel does is done there,
 // out of the CTAs' shared memory (same sums in the same order).
 //
+// BIASED: slopes[h] * (pos - j) off a key's score, a window that keeps the request's first keys visible, and a gate a head
+// (in the merge).  A row's blocks are then those of the kept keys that lie before the window's first block, and the
+// window's; the workspace holds these alone, in ascending order, however long the context (a window of 1,024 keys and one
+// row of 16 heads: 21 us a layer while such rows took shares of four blocks of 64 keys of attention_prefill.cu's kernel).
+//
 // Further forms.  SIGMOID: a key weighs sigmoid(score + sig_bias[h]), not normalised over keys - blocks carry the
 // maximum 0 and simply add.  CAPPED: the softmax over cap * tanh(score / cap).  Turned values: the merge turns the first `turn_dims` numbers of a head's result by minus
 // the row's position (what turn_back in qk_norm_append.cu does in a pass of its own, here on the float32 sum).
@@ -96,8 +101,9 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
                               float* __restrict__ ws_acc, float* __restrict__ ws_ml, int Hq, int Hkv,
                               int page_size, int num_pages, int window, float scale, int nsplit,
                               int* __restrict__ counters, __nv_bfloat16* __restrict__ out,
-                              const int* __restrict__ row_list, const float* __restrict__ sig_bias, float softcap) {
-  constexpr bool SIGMOID = FORM == kFormSigmoid, CAPPED = FORM == kFormCapped;
+                              const int* __restrict__ row_list, const float* __restrict__ sig_bias, float softcap,
+                              const float* __restrict__ slopes, int keep_first) {
+  constexpr bool SIGMOID = FORM == kFormSigmoid, CAPPED = FORM == kFormCapped, BIASED = FORM == kFormBiased;
   constexpr int LPR = D / 8;            // 16-byte pieces of one key row
   constexpr int RPL = 32 / LPR;         // key rows a warp copies at once
   constexpr int DS = D + 8;             // shared-memory row stride: 16 bytes of padding keep
@@ -125,11 +131,18 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
   const int t = row_list ? row_list[wi] : wi;
   const int newest = positions[t];
   int pos = newest, lo;
-  if (decode_key_range(pos, lo, window, nsplit, kSplit) && kvh == 0 && split == 0 && threadIdx.x == 0)
+  int block = split, kept = 0;          // which block of keys; keys below `kept` are seen without the window
+  if constexpr (BIASED) {
+    const KeptRange range = kept_key_range(pos, window, keep_first, kSplit);
+    lo = range.lo, kept = range.kept;
+    if (range.blocks > nsplit && kvh == 0 && split == 0 && threadIdx.x == 0) atomicCAS(&g_decode_split_range_error, 0, 1 + t);
+    block = split < range.blocks ? range.block(split) : -1;
+  } else if (decode_key_range(pos, lo, window, nsplit, kSplit) && kvh == 0 && split == 0 && threadIdx.x == 0) {
     atomicCAS(&g_decode_split_range_error, 0, 1 + t);
-  const int k_base = split * kSplit;
-  const int k_begin = max(lo, k_base);
-  const int k_end = min(pos + 1, k_base + kSplit);
+  }
+  const int k_base = block * kSplit;
+  const int k_begin = BIASED && k_base < kept ? k_base : max(lo, k_base);
+  const int k_end = BIASED && block < 0 ? k_begin : min(BIASED && k_base + kSplit <= lo ? kept : pos + 1, k_base + kSplit);
   const bool empty = k_begin >= k_end;
   if (!CLUSTER && empty) return;
   if (empty) chain_wait();             // (its CTA still meets the others, and may write a part of the result)
@@ -154,7 +167,7 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
       const int j = k_base + myrow;
       const int lp = j / page_size;
       const int page = lp < bt_width ? bt[lp] : -1;
-      if (page >= 0 && page < num_pages)
+      if (page >= 0 && page < num_pages && (!BIASED || j >= lo || j < kept))
         my_src = pages + (size_t)page * page_stride + (size_t)kvh * head_stride + (size_t)(j - lp * page_size) * D;
     }
 #pragma unroll
@@ -227,7 +240,15 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
       for (int i = 0; i < 4; ++i) {
         const int r = warp * 32 + m * 16 + g + (i >> 1) * 8;
         const int h = h0 + 2 * tq + (i & 1);
-        if (h < G && r >= n0 && r < n1) sc[h * kSplit + r] = CAPPED ? cap_score(c[m][i], softcap, in2) : c[m][i] * scale;
+        if (h < G && r >= n0 && r < n1) {
+          float v = CAPPED ? cap_score(c[m][i], softcap, in2) : c[m][i] * scale;
+          if constexpr (BIASED) {
+            const int j = k_base + r;
+            if (slopes) v = fmaf(-slopes[kvh * G + h], (float)(pos - j), v);
+            if (j < lo && j >= kept) v = -INFINITY;      // between the kept keys and the window
+          }
+          sc[h * kSplit + r] = v;
+        }
       }
   }
   __syncthreads();
@@ -385,7 +406,8 @@ __global__ void decode_attention_merge_kernel(const float* __restrict__ ws_acc,
                                               const int* __restrict__ positions, T* __restrict__ out,
                                               int Hq, int D, int window, int nsplit, int dthreads,
                                               const int* __restrict__ row_list, int normalise,
-                                              const float* __restrict__ turn_freq, int turn_dims, int interleaved) {
+                                              const float* __restrict__ turn_freq, int turn_dims, int interleaved,
+                                              int keep_first, const float* __restrict__ gate, int gate_ld) {
   extern __shared__ float runs[];      // [runs of this row][D]
   __shared__ float wgt[kMaxMergeSplits], wl[kMaxMergeSplits];
   __shared__ float s_m, s_inv;
@@ -396,10 +418,15 @@ __global__ void decode_attention_merge_kernel(const float* __restrict__ ws_acc,
   // began; the partial results are the predecessor's
   const int t = row_list ? row_list[wi] : wi;
   int pos = positions[t], lo;
-  decode_key_range(pos, lo, window, nsplit, kSplit);
-  chain_wait(ws_acc, ws_ml);
-  const int s0 = lo / kSplit, s1 = pos / kSplit;                       // first and last split with keys
-  const int n = s1 - s0 + 1;
+  int s0 = 0, n;                       // the row's first block in the workspace, and how many it has
+  if (keep_first >= 0) {
+    n = min(nsplit, kept_key_range(pos, window, keep_first, kSplit).blocks);
+  } else {
+    decode_key_range(pos, lo, window, nsplit, kSplit);
+    s0 = lo / kSplit;
+    n = pos / kSplit - s0 + 1;
+  }
+  chain_wait(ws_acc, ws_ml, gate);
   const float* ml = ws_ml + (((size_t)wi * Hq + h) * nsplit + s0) * 2;
   const float* acc = ws_acc + (((size_t)wi * Hq + h) * nsplit + s0) * D;
   // every block's (m, l) in one parallel read; the serial parts below then walk shared memory
@@ -421,7 +448,9 @@ __global__ void decode_attention_merge_kernel(const float* __restrict__ ws_acc,
   if (threadIdx.x == 0) {
     float l = 0.f;
     for (int s = 0; s < n; ++s) l += wl[s] * wgt[s];                              // ascending order
-    s_inv = !normalise ? 1.f : (l > 0.f ? 1.f / l : 0.f);
+    float inv = !normalise ? 1.f : (l > 0.f ? 1.f / l : 0.f);
+    if (gate) inv *= 1.f / (1.f + expf(-gate[(size_t)t * gate_ld + h]));
+    s_inv = inv;
   }
   __syncthreads();
   // Runs of kMergeRun blocks are added by different thread groups (a long context has hundreds of
@@ -481,7 +510,7 @@ static int launch_split(const void* qkv, int q_row_stride, const void* pages, co
                         int bt_width, const int* positions, const int* row_seg, float* ws_acc,
                         float* ws_ml, int T, int Hq, int Hkv, int page_size, int num_pages, int window,
                         float scale, int nsplit, int* counters, void* out, const int* row_list, const float* sig_bias,
-                        float softcap, bool* merged, cudaStream_t stream) {
+                        float softcap, bool* merged, const float* slopes, int keep_first, cudaStream_t stream) {
   const int G = Hq / Hkv;
   const size_t smem = (size_t)2 * kSplit * (D + 8) * sizeof(__nv_bfloat16) +
                       ((size_t)G * kSplit + 4 * (G < 8 ? G : 8) * D + 2 * G) * sizeof(float);
@@ -492,7 +521,7 @@ static int launch_split(const void* qkv, int q_row_stride, const void* pages, co
   // rows of one block 6.1 -> 4.6): clusters start as a whole, where single CTAs trickle in and empty ones leave at once
   // (256 CTAs: two rows of eight blocks 5.8 -> 7.4; 512: four rows 5.9 -> 13.7).  And enough CTAs a row for its heads: a
   // thread adds up at most four numbers (28 heads on four key heads, one block: 6.5 -> 7.1, in four blocks 6.5 -> 5.6).
-  if constexpr (cluster_fits(D)) {
+  if constexpr (cluster_fits(D) && FORM != kFormBiased) {
     if (*merged && nsplit <= kClusterSplits && smem_c <= kClusterSmem && (long long)T * Hkv * nsplit <= kClusterCtas &&
         G * D <= 4 * 128 * nsplit) {
       static size_t allowed_c = 48 * 1024;
@@ -503,7 +532,7 @@ static int launch_split(const void* qkv, int q_row_stride, const void* pages, co
       launch_chained_clusters(decode_attention_split_kernel<D, FORM, true>, grid, dim3(128), smem_c, stream, dim3(1, 1, nsplit),
                                (const __nv_bfloat16*)qkv, q_row_stride, (const __nv_bfloat16*)pages, block_table, bt_width,
                                positions, row_seg, ws_acc, ws_ml, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters,
-                               (__nv_bfloat16*)out, row_list, sig_bias, softcap);
+                               (__nv_bfloat16*)out, row_list, sig_bias, softcap, slopes, keep_first);
       g_cluster_launches.fetch_add(1, std::memory_order_relaxed);
       return check_launch("decode_attention_cluster");
     }
@@ -517,7 +546,7 @@ static int launch_split(const void* qkv, int q_row_stride, const void* pages, co
   launch_chained(decode_attention_split_kernel<D, FORM, false>, grid, dim3(128), smem, stream,
                  (const __nv_bfloat16*)qkv, q_row_stride, (const __nv_bfloat16*)pages, block_table, bt_width,
                  positions, row_seg, ws_acc, ws_ml, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters,
-                 (__nv_bfloat16*)out, row_list, sig_bias, softcap);
+                 (__nv_bfloat16*)out, row_list, sig_bias, softcap, slopes, keep_first);
   return check_launch("decode_attention_split");
 }
 
@@ -572,22 +601,24 @@ static int decode_attention_impl(const void* qkv, int q_row_stride, const void* 
                                  int Hq, int Hkv, int D, int page_size, int num_pages, int window,
                                  float scale, int nsplit, int* counters, const int* row_list,
                                  cudaStream_t stream, const float* sig_bias = nullptr,
-                                 const float* turn_freq = nullptr, int turn_dims = 0, int interleaved = 0, float softcap = 0.f) {
+                                 const float* turn_freq = nullptr, int turn_dims = 0, int interleaved = 0, float softcap = 0.f,
+                                 const float* slopes = nullptr, int keep_first = -1, const float* gate = nullptr, int gate_ld = 0) {
   if (T == 0) return 0;
   NF_REQUIRE(T > 0 && Hq > 0 && Hkv > 0 && Hq % Hkv == 0 && nsplit > 0, "decode attention: bad sizes T=%d Hq=%d Hkv=%d nsplit=%d", T, Hq, Hkv, nsplit);
   NF_REQUIRE(Hkv <= 65535 && nsplit <= kMaxMergeSplits, "decode attention: too many kv heads or key blocks (context beyond %d keys)", kMaxMergeSplits * kSplit);
   int rc;
-  bool merged = g_decode_cluster && !counters && !turn_freq;      // asked for; then: whether the launch merged its blocks itself
+  const bool biased = keep_first >= 0;
+  bool merged = g_decode_cluster && !counters && !turn_freq && !biased;      // asked for; then: whether the launch merged its blocks itself
   // The persistent kernel pays a start-up (every CTA lists the rows' blocks) that only many
   // blocks repay: measured on B200, it wins from about a thousand blocks on.
-  if (g_decode_stream && !counters && (long long)T * Hkv * nsplit >= 1024 &&
+  if (g_decode_stream && !counters && !biased && (long long)T * Hkv * nsplit >= 1024 &&
       decode_attention_stream_fits(T, Hq, Hkv, D, page_size)) {
     merged = false;
     rc = decode_attention_stream(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, ws_acc, ws_ml,
                                  T, Hq, Hkv, D, page_size, num_pages, window, scale, nsplit, row_list, sig_bias, softcap, stream);
   } else
-#define NF_DA_CALL(DD, SG) launch_split<DD, SG>(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, ws_acc, ws_ml, T, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters, out, row_list, sig_bias, softcap, &merged, stream)
-#define NF_DA(DD) case DD: rc = sig_bias ? NF_DA_CALL(DD, kFormSigmoid) : (softcap > 0.f ? NF_DA_CALL(DD, kFormCapped) : NF_DA_CALL(DD, kFormSoftmax)); break;
+#define NF_DA_CALL(DD, SG) launch_split<DD, SG>(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, ws_acc, ws_ml, T, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters, out, row_list, sig_bias, softcap, &merged, slopes, keep_first, stream)
+#define NF_DA(DD) case DD: rc = biased ? NF_DA_CALL(DD, kFormBiased) : sig_bias ? NF_DA_CALL(DD, kFormSigmoid) : (softcap > 0.f ? NF_DA_CALL(DD, kFormCapped) : NF_DA_CALL(DD, kFormSoftmax)); break;
   switch (D) {
     NF_DA(16)
     NF_DA(32)
@@ -616,7 +647,7 @@ static int decode_attention_impl(const void* qkv, int q_row_stride, const void* 
   }
   launch_chained(decode_attention_merge_kernel<__nv_bfloat16>, grid, dim3(dthreads * groups), smem, stream,
                  (const float*)ws_acc, (const float*)ws_ml, positions, (__nv_bfloat16*)out, Hq, D, window, nsplit,
-                 dthreads, row_list, sig_bias ? 0 : 1, turn_freq, turn_dims, interleaved);
+                 dthreads, row_list, sig_bias ? 0 : 1, turn_freq, turn_dims, interleaved, keep_first, gate, gate_ld);
   return check_launch("decode_attention_merge");
 }
 
@@ -659,6 +690,28 @@ extern "C" int nf_decode_attention_further(const void* qkv, int q_row_stride, co
   return decode_attention_impl(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, out, ws_acc,
                                ws_ml, T, Hq, Hkv, D, page_size, num_pages, window, scale, nsplit, nullptr, row_list,
                                stream, sig_bias, turn_freq, turn_dims, interleaved, softcap);
+}
+
+// Most blocks of keys a row at a position below `max_context` has in the biased form.
+extern "C" int nf_decode_attention_biased_splits(int window, int keep_first, int max_context) {
+  if (max_context < 1) max_context = 1;
+  const int all = (max_context + kSplit - 1) / kSplit;
+  if (window <= 0 || window >= max_context) return all;
+  const int own = (window - 1 + kSplit - 1) / kSplit + 1 + (keep_first + kSplit - 1) / kSplit;    // ragged at both ends; kept
+  return own < all ? own : all;
+}
+
+// The biased form: slopes float32 [Hq] or null; keep_first >= 0 (it counts only with a window); gate float32 [rows, gate_ld]
+// (column h: head h's gate logit) or null.  nsplit: at least nf_decode_attention_biased_splits() of the longest context.
+extern "C" int nf_decode_attention_biased(const void* qkv, int q_row_stride, const void* pages, const int* block_table,
+                                          int bt_width, const int* positions, const int* row_seg, void* out, float* ws_acc,
+                                          float* ws_ml, const int* row_list, int T, int Hq, int Hkv, int D, int page_size,
+                                          int num_pages, int window, float scale, int nsplit, const float* slopes, int keep_first,
+                                          const float* gate, int gate_ld, cudaStream_t stream) {
+  NF_REQUIRE(keep_first >= 0 && (!gate || gate_ld >= Hq), "decode attention: bad options");
+  return decode_attention_impl(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, out, ws_acc, ws_ml, T, Hq,
+                               Hkv, D, page_size, num_pages, window, scale, nsplit, nullptr, row_list, stream, nullptr, nullptr, 0,
+                               0, 0.f, slopes, window > 0 ? keep_first : 0, gate, gate_ld);
 }
 
 // The same in one launch: `counters` are T * Hkv ints that are zero before the call and are left

@@ -17,4 +17,20 @@ __device__ __forceinline__ bool decode_key_range(int& pos, int& lo, int window, 
   return true;
 }
 
+// The keys of a row with a window that keeps the request's first `keep_first` keys visible: those below `kept`, and
+// lo..pos.  Its blocks, in ascending order: the `before` that hold kept keys and lie before the window's first, and the window's.
+struct KeptRange {
+  int lo, kept, before, first, blocks;
+  __device__ __forceinline__ int block(int i) const { return i < before ? i : first + i - before; }
+};
+__device__ __forceinline__ KeptRange kept_key_range(int pos, int window, int keep_first, int block) {
+  KeptRange r;
+  r.lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  r.kept = min(keep_first, r.lo);
+  r.first = r.lo / block;
+  r.before = min(r.first, (r.kept + block - 1) / block);
+  r.blocks = r.before + pos / block - r.first + 1;
+  return r;
+}
+
 }  // namespace nf

@@ -273,6 +273,7 @@ def work_models(s: dict, prompt: int, batch: int, context: int, design: str = ""
             "nf_poly_norm_act": (T * s["top"] * s["ff"] * (4 + 2), 0.0),
             "nf_embed_copies": (T * W * (2 + 4 * STREAMS), 0.0),
             "nf_prefill_attention_biased": windowed,
+            "nf_decode_attention_biased": windowed,
             "nf_paged_attention_generic": windowed,
             # two shapes share the kernel (lightning 128 x 128, retention 64 x 128): the mean of the two
             "nf_decay_linear_attention": tuple((a + b) / 2 for a, b in zip(la(D, D), la(RET_DIM, D))),

@@ -1,5 +1,5 @@
 """Kernels of decode steps and of the all-32-bit path at the sizes where they can go wrong: float32 attention that shares
-its keys among a segment's rows, the scan of single rows."""
+its keys among a segment's rows, the biased split-key attention of single rows, the scan of single rows."""
 
 import math
 from dataclasses import replace
@@ -125,6 +125,27 @@ def test_float32_attention_keeps_a_number_that_is_not_finite_behind_its_row(K):
     pages[page, :, :, slot] = math.nan                        # position 23, row 20
     bad = K.paged_attention(q, 4, 2, 64, pages, bt, 16, ctx, 0, 0.125)
     assert torch.equal(bad[:20], good[:20]) and bad[20:].isnan().any(1).all()
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,page", [(4, 4, 128, 64), (6, 2, 64, 16), (20, 2, 32, 32), (2, 1, 16, 32)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (300, 4), (128, 130), (1024, 4), (1, 1), (129, 0)])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_biased_attention_of_single_rows(K, Hq, Hkv, D, page, window, keep, mixed):
+    pos0s = [0, 127, 128, 299, 300, 428, 431, 1500, 1023, 1024, 1151, 1152]
+    lens = [1] * len(pos0s)
+    if mixed:
+        lens[2] = 9
+    pages, bt, ctx, positions, row_seg, g = make_step(torch.bfloat16, lens, pos0s, Hkv, D, page, 7)
+    T = ctx.T
+    q = torch.randn((T, Hq * D), generator=g).bfloat16().cuda()
+    slopes = torch.tensor([0.05 / (i + 1) for i in range(Hq)]).cuda()
+    gate = torch.randn((T, Hq + 3), generator=g).cuda()
+    out = K.biased_window_attention(q, Hq, Hkv, D, pages, bt, page, ctx, window, keep, D ** -0.5, slopes, gate, 3)
+    want = exact_attention(q.view(T, Hq, D), pages, bt, positions, row_seg, Hq, page, window, keep if window else 0, D ** -0.5,
+                           slopes, gate[:, 3:])
+    # weights and outputs rounded to bfloat16 once each: 2^-8 of the values' size (up to 4.5 of unit variance)
+    assert (out.view(T, Hq, D) - want).abs().max() <= 2 ** -8 * 4.5
+    K.check_status()
 
 
 @pytest.mark.parametrize("heads,P,N,groups", [(8, 64, 128, 2), (6, 20, 64, 3), (3, 7, 16, 1), (4, 33, 200, 4), (2, 64, 256, 1)])
