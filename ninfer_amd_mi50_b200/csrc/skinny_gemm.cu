@@ -343,6 +343,16 @@ skinny_gemm_kernel(const __nv_bfloat16* __restrict__ X, int ldx, const __nv_bflo
 
 static thread_local GatedActParams t_gated_act{kActNone, 0.f, 0.f};   // the current call's epilogue
 
+// Weights in flight to registers lie in the L1's part of the SM's memory until they are there; what it is not given is
+// shared memory, which these CTAs need little of but the kernels beside and around them more.  A half is the split at
+// which the chain of a decode step was fastest: with the driver's choice (the least shared memory that the CTAs of an SM
+// need) 14.0 ms for a prompt and 16 tokens over 12 layers, now 13.7; with all of it as shared memory 18.4.
+constexpr int kSharedPercent = 50;
+template <typename... KArgs>
+static void prefer_half_shared(void (*kernel)(KArgs...)) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kSharedPercent);      // (a hint: failing, it changes nothing)
+}
+
 int g_skinny_max_split = kMaxSplit;      // nf_set_skinny_max_split(): 1 turns the split over k off
 
 template <int NT, bool SWIGLU, bool PACKED, typename TC>
@@ -360,6 +370,8 @@ static int launch_nt(const void* X, int ldx, const void* W, size_t wgs, void* Y,
     const int nchunks = (K + 31) / 32;
     while (ksplit * 2 <= g_skinny_max_split && ctas * ksplit * 2 <= 4 * 148 && nchunks / (ksplit * 2) >= kWarps) ksplit *= 2;
   }
+  static const bool asked = (prefer_half_shared(skinny_gemm_kernel<NT, SWIGLU, PACKED, TC>), true);
+  (void)asked;
   if (ksplit > 1) {
     grid.x *= ksplit;
     launch_chained_cluster(skinny_gemm_kernel<NT, SWIGLU, PACKED, TC>, grid, dim3(kWarps * 32), 0, stream, ksplit,
@@ -451,6 +463,9 @@ extern "C" int nf_skinny_qkv_rope(const void* X, int ldx, const void* W, void* Y
                  Hq, Hkv, D, bt_width, page_size, num_pages, append};
   dim3 grid(1, N / 16, 1);
   NF_REQUIRE(grid.y <= 65535, "skinny_qkv_rope: too many heads");
+  static const bool asked = (prefer_half_shared(skinny_gemm_kernel<1, false, false, __nv_bfloat16, true>),
+                             prefer_half_shared(skinny_gemm_kernel<2, false, false, __nv_bfloat16, true>), true);
+  (void)asked;
   if (M <= 8)
     launch_chained(skinny_gemm_kernel<1, false, false, __nv_bfloat16, true>, grid, dim3(kWarps * 32), 0, stream,
                    (const __nv_bfloat16*)X, ldx, (const __nv_bfloat16*)W, (size_t)0, (__nv_bfloat16*)Y, ldy, M, N, K,
