@@ -195,28 +195,96 @@ __device__ __forceinline__ void cr_row_gates(const CrArgs& a, int head, int row,
   }
 }
 
-// `rows` rows of the keys (or queries) into planes [PARTS][.][D + pad]; zeros from `live` rows on.
-template <int D, int PARTS>
-__device__ __forceinline__ void cr_load_qk(const CrArgs& a, bool keys, int head, int row0, int rows, int live,
-                                           __nv_bfloat16* dst, size_t plane) {
-  if (PARTS == 1) {
-    const __nv_bfloat16* src = (keys ? a.k + a.k0 : a.q + a.q0) + (size_t)(head / a.heads_per_group) * D;
-    for (int i = threadIdx.x; i < rows * (D / 8); i += kCrThreads) {
-      const int r = i / (D / 8), c = (i - r * (D / 8)) * 8;
-      uint4 x = make_uint4(0, 0, 0, 0);
-      if (r < live) x = *reinterpret_cast<const uint4*>(src + (size_t)(row0 + r) * a.ld + c);
-      *reinterpret_cast<uint4*>(dst + r * (D + kCrPad) + c) = x;
-    }
-  } else {
-    const float* src = a.prepared + (size_t)(keys ? a.H + head : head) * D;
-    for (int i = threadIdx.x; i < rows * (D / 4); i += kCrThreads) {
-      const int r = i / (D / 4), c = (i - r * (D / 4)) * 4;
-      float x[4] = {0.f, 0.f, 0.f, 0.f};
-      if (r < live) load4(src + (size_t)(row0 + r) * 2 * a.H * D + c, x);
-      cr_store_parts<PARTS>(dst + r * (D + kCrPad) + c, plane, x);
+// What a chunk's CTA reads goes through registers in two halves: `ask` issues every load, `put` brings the numbers to
+// shared memory (in parts, where they are float32).  Between the two lies other work - gates, decay tables, the products
+// with the rows or the state before - so that a CTA, of which only two fit a SM, does not stand still for each of its reads
+// (loads and stores in one loop: 42 % of the issue slots of the output kernel lost to waiting for loads, 47 % of the
+// states').
+//
+// ROWS rows of the keys (or queries) for planes [PARTS][.][D + pad]; zeros from `live` rows on.
+template <int D, int PARTS, int ROWS>
+struct CrQkRows {
+  static constexpr int W = PARTS == 1 ? 8 : 4, N = ROWS * (D / W) / kCrThreads;
+  static_assert(ROWS * (D / W) % kCrThreads == 0, "whole rounds of loads");
+  uint4 x[N];
+  __device__ __forceinline__ void ask(const CrArgs& a, bool keys, int head, int row0, int live) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int at = threadIdx.x + i * kCrThreads, r = at / (D / W), c = (at % (D / W)) * W;
+      x[i] = make_uint4(0, 0, 0, 0);
+      if (r < live) {
+        if (PARTS == 1)
+          x[i] = *reinterpret_cast<const uint4*>((keys ? a.k + a.k0 : a.q + a.q0) + (size_t)(head / a.heads_per_group) * D + (size_t)(row0 + r) * a.ld + c);
+        else
+          x[i] = *reinterpret_cast<const uint4*>(a.prepared + (size_t)(keys ? a.H + head : head) * D + (size_t)(row0 + r) * 2 * a.H * D + c);
+      }
     }
   }
-}
+  __device__ __forceinline__ void put(__nv_bfloat16* dst, size_t plane) const {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int at = threadIdx.x + i * kCrThreads, r = at / (D / W), c = (at % (D / W)) * W;
+      if (PARTS == 1) {
+        *reinterpret_cast<uint4*>(dst + r * (D + kCrPad) + c) = x[i];
+      } else {
+        const float f[4] = {__uint_as_float(x[i].x), __uint_as_float(x[i].y), __uint_as_float(x[i].z), __uint_as_float(x[i].w)};
+        cr_store_parts<PARTS>(dst + r * (D + kCrPad) + c, plane, f);
+      }
+    }
+  }
+};
+__device__ __forceinline__ float cr_value(float x, int silu) { return silu ? x / (1.f + expf(-x)) : x; }
+// ROWS rows of V columns of a head's values from column `col` on, for planes [PARTS][.][V + pad]: bfloat16 as they are
+// (PARTS 1), through the activation and times a row's `scale` (null: 1), or (FLOATS) the float32 numbers of `values`.
+template <int V, int PARTS, int ROWS, bool FLOATS>
+struct CrValueRows {
+  static constexpr int W = PARTS == 1 ? 8 : 4, N = ROWS * (V / W) / kCrThreads;
+  static_assert(ROWS * (V / W) % kCrThreads == 0 && !(FLOATS && PARTS == 1), "whole rounds of loads");
+  uint4 x[N];
+  __device__ __forceinline__ void ask(const CrArgs& a, int head, int col, int row0, int live) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int at = threadIdx.x + i * kCrThreads, r = at / (V / W), c = (at % (V / W)) * W;
+      x[i] = make_uint4(0, 0, 0, 0);
+      if (r < live) {
+        if (FLOATS) {
+          x[i] = *reinterpret_cast<const uint4*>(a.values + (size_t)(row0 + r) * a.H * a.V + (size_t)head * a.V + col + c);
+        } else {
+          const __nv_bfloat16* src = a.v + a.v0 + (size_t)head * a.V + col + (size_t)(row0 + r) * a.ld + c;
+          if (PARTS == 1) {
+            x[i] = *reinterpret_cast<const uint4*>(src);
+          } else {
+            const uint2 half = *reinterpret_cast<const uint2*>(src);
+            x[i].x = half.x, x[i].y = half.y;
+          }
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void put(__nv_bfloat16* dst, size_t plane, int silu, const float* scale) const {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int at = threadIdx.x + i * kCrThreads, r = at / (V / W), c = (at % (V / W)) * W;
+      if (PARTS == 1) {
+        *reinterpret_cast<uint4*>(dst + r * (V + kCrPad) + c) = x[i];
+        continue;
+      }
+      float f[4] = {__uint_as_float(x[i].x), __uint_as_float(x[i].y), __uint_as_float(x[i].z), __uint_as_float(x[i].w)};
+      if (!FLOATS) {
+        const uint2 half = make_uint2(x[i].x, x[i].y);
+        load4(reinterpret_cast<const __nv_bfloat16*>(&half), f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) f[e] = cr_value(f[e], silu);
+        if (scale) {
+          const float by = scale[r];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) f[e] *= by;
+        }
+      }
+      cr_store_parts<PARTS>(dst + r * (V + kCrPad) + c, plane, f);
+    }
+  }
+};
 // Row t's decays inside its sixteen, from the chunk's in `decay`: the product up to it, after it, and to every later row
 // (diag[t / 16][t % 16][u]; 0 before it).
 template <int N>
@@ -232,12 +300,11 @@ __device__ __forceinline__ void cr_decay_table(const float* decay, int t, float*
   }
   after[t] = run;
 }
-__device__ __forceinline__ float cr_value(float x, int silu) { return silu ? x / (1.f + expf(-x)) : x; }
 
 // ---- (1) a chunk's contribution to the state: [V, D] = sum_s (w_s D(s, end) v_s) k_s^T -------------------------------
 // 8 warps: a warp owns 32 value rows and D V / 256 state columns.
 template <int D, int V, int Q, int QKP, int MODE>
-__global__ void __launch_bounds__(kCrThreads)
+__global__ void __launch_bounds__(kCrThreads, 2)
 chunk_state_kernel(const CrArgs args) {
   constexpr int WM = V / 32, WN = 8 / WM, NT = D / WN / 8;     // warps along V and D, column tiles a warp
   constexpr int KS = D + kCrPad, VS = V + kCrPad;
@@ -252,13 +319,16 @@ chunk_state_kernel(const CrArgs args) {
   const int2 place = cr_rows<Q>(a.at, chunk);
   const int row0 = place.x, live = place.y;
   chain_wait(a.q, a.k, a.v, a.dt, a.prepared);
+  CrQkRows<D, QKP, Q> keys;
+  CrValueRows<V, 3, Q, false> values;
+  keys.ask(a, true, head, row0, live);
+  values.ask(a, head, 0, row0, live);
   float weight = 0.f;
   if (threadIdx.x < Q) {
     float decay;
     cr_row_gates<MODE>(a, head, row0 + threadIdx.x, (int)threadIdx.x < live, decay, weight);
     s_decay[threadIdx.x] = decay;
   }
-  cr_load_qk<D, QKP>(a, true, head, row0, Q, live, Ks, (size_t)Q * KS);
   __syncthreads();
   if (threadIdx.x < Q) {                 // w_s D(s, end): the rows after s in its 16, then whole sixteens
     float run = 1.f;
@@ -275,21 +345,9 @@ chunk_state_kernel(const CrArgs args) {
   }
   __syncthreads();
   if (threadIdx.x < Q) s_scale[threadIdx.x] = weight;
+  keys.put(Ks, (size_t)Q * KS);
   __syncthreads();
-  {
-    const __nv_bfloat16* src = a.v + a.v0 + (size_t)head * V;
-    for (int i = threadIdx.x; i < Q * (V / 4); i += kCrThreads) {
-      const int r = i / (V / 4), c = (i - r * (V / 4)) * 4;
-      float x[4] = {0.f, 0.f, 0.f, 0.f};
-      if (r < live) {
-        load4(src + (size_t)(row0 + r) * a.ld + c, x);
-        const float f = s_scale[r];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[e] = cr_value(x[e], a.v_silu) * f;
-      }
-      cr_store_parts<3>(Vs + r * VS + c, (size_t)Q * VS, x);
-    }
-  }
+  values.put(Vs, (size_t)Q * VS, a.v_silu, s_scale);
   __syncthreads();
   const int m0 = (warp % WM) * 32, n0 = (warp / WM) * (D / WN);
   float acc[2][NT][4];
@@ -413,18 +471,28 @@ chunk_output_kernel(const CrArgs args) {
   const int2 place = cr_rows<Q>(a.at, chunk);
   const int row0 = place.x, live = place.y;
   chain_wait(a.q, a.k, a.v, a.dt, a.prepared, a.chunk_state, a.values, a.gates);
-  if (threadIdx.x < Q)
-    cr_row_gates<MODE>(a, head, row0 + threadIdx.x, (int)threadIdx.x < live, s_decay[threadIdx.x], s_weight[threadIdx.x]);
-  cr_load_qk<D, QKP>(a, false, head, row0, Q, live, Qs, (size_t)Q * KS);
+  CrQkRows<D, QKP, Q> queries;
+  constexpr int SN = V * (D / 4) / kCrThreads;
+  static_assert(V * (D / 4) % kCrThreads == 0, "whole rounds of loads");
+  float start[SN][4];                    // the state at the chunk's start
+  queries.ask(a, false, head, row0, live);
   {
     const float* src = a.chunk_state + (((size_t)chunk * a.H + head) * a.V + tile0) * D;
-    for (int i = threadIdx.x; i < V * (D / 4); i += kCrThreads) {
-      const int r = i / (D / 4), c = (i - r * (D / 4)) * 4;
-      float x[4];
-      load4(src + (size_t)i * 4, x);
-      cr_store_parts<3>(Ss + r * KS + c, (size_t)V * KS, x);
-    }
+#pragma unroll
+    for (int i = 0; i < SN; ++i) load4(src + (size_t)(threadIdx.x + i * kCrThreads) * 4, start[i]);
   }
+  if (threadIdx.x < Q)
+    cr_row_gates<MODE>(a, head, row0 + threadIdx.x, (int)threadIdx.x < live, s_decay[threadIdx.x], s_weight[threadIdx.x]);
+  queries.put(Qs, (size_t)Q * KS);
+#pragma unroll
+  for (int i = 0; i < SN; ++i) {
+    const int at = threadIdx.x + i * kCrThreads;
+    cr_store_parts<3>(Ss + (at / (D / 4)) * KS + (at % (D / 4)) * 4, (size_t)V * KS, start[i]);
+  }
+  CrQkRows<D, QKP, SUB> keys;            // the next SUB rows
+  CrValueRows<V, VP, SUB, MODE == kCrDelta> values;
+  keys.ask(a, true, head, row0, live);
+  values.ask(a, head, tile0, row0, live);
   __syncthreads();
   if (threadIdx.x < Q) cr_decay_table(s_decay, threadIdx.x, s_upto, s_after, s_diag);
   __syncthreads();
@@ -479,34 +547,13 @@ chunk_output_kernel(const CrArgs args) {
   for (int sub = 0; sub < Q; sub += SUB) {
     if (sub >= live) break;
     __syncthreads();                     // everyone is done with the state, or with the rows before
-    cr_load_qk<D, QKP>(a, true, head, row0 + sub, SUB, live - sub, Ks, (size_t)SUB * KS);
-    {
-      const __nv_bfloat16* src = a.v + a.v0 + (size_t)head * a.V + tile0;
-      if (VP == 1) {
-        for (int i = threadIdx.x; i < SUB * (V / 8); i += kCrThreads) {
-          const int r = i / (V / 8), c = (i - r * (V / 8)) * 8;
-          uint4 x = make_uint4(0, 0, 0, 0);
-          if (sub + r < live) x = *reinterpret_cast<const uint4*>(src + (size_t)(row0 + sub + r) * a.ld + c);
-          *reinterpret_cast<uint4*>(Vs + r * VS + c) = x;
-        }
-      } else {
-        for (int i = threadIdx.x; i < SUB * (V / 4); i += kCrThreads) {
-          const int r = i / (V / 4), c = (i - r * (V / 4)) * 4;
-          float x[4] = {0.f, 0.f, 0.f, 0.f};
-          if (sub + r < live) {
-            if (MODE == kCrDelta) {
-              load4(a.values + (size_t)(row0 + sub + r) * a.H * a.V + (size_t)head * a.V + tile0 + c, x);
-            } else {
-              load4(src + (size_t)(row0 + sub + r) * a.ld + c, x);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) x[e] = cr_value(x[e], a.v_silu);
-            }
-          }
-          cr_store_parts<VP>(Vs + r * VS + c, (size_t)SUB * VS, x);
-        }
-      }
-    }
+    keys.put(Ks, (size_t)SUB * KS);
+    values.put(Vs, (size_t)SUB * VS, a.v_silu, nullptr);
     __syncthreads();
+    if (sub + SUB < live) {
+      keys.ask(a, true, head, row0 + sub + SUB, live - sub - SUB);
+      values.ask(a, head, tile0, row0 + sub + SUB, live - sub - SUB);
+    }
     if (!work) continue;
 #pragma unroll 1
     for (int sb = 0; sb < SUB; sb += 16) {
