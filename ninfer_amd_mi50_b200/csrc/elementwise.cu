@@ -496,6 +496,55 @@ __global__ void gated_bias_act_kernel(const TI* __restrict__ gu, const float* __
   act[(size_t)m * inner + i] = from_float<T>(gated_act(g, u, kind, limit, alpha));
 }
 
+// The same in runs of four columns, one access each, and ROWS rows a thread, all asked for at once: the biases are read
+// once for them (rows x columns 2,048 x 5,632 of float32 sums, 115 MB: element by element 46 us).
+template <typename TI, typename T, int ROWS>
+__global__ void __launch_bounds__(256)
+gated_bias_act_x4_kernel(const TI* __restrict__ gu, const float* __restrict__ bias, T* __restrict__ act, int M, int inner, int kind,
+                         float limit, float alpha) {
+  const int m0 = blockIdx.y * ROWS, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  float bg[4] = {0.f, 0.f, 0.f, 0.f}, bu[4] = {0.f, 0.f, 0.f, 0.f};
+  if (bias && i < inner) {
+    load4(bias + i, bg);
+    load4(bias + inner + i, bu);
+  }
+  chain_wait(gu);
+  if (i >= inner) return;
+  float g[ROWS][4], u[ROWS][4];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    if (m0 + r < M) {
+      const TI* row = gu + (size_t)(m0 + r) * 2 * inner;
+      load4(row + i, g[r]);
+      load4(row + inner + i, u[r]);
+    }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    if (m0 + r < M) {
+      if (bias) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { g[r][e] += bg[e]; u[r][e] += bu[e]; }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) g[r][e] = gated_act(g[r][e], u[r][e], kind, limit, alpha);
+      store4(act + (size_t)(m0 + r) * inner + i, g[r]);
+    }
+}
+
+template <typename TI, typename T>
+static void launch_gated_bias_act(const TI* gu, const float* bias, T* act, int M, int inner, int kind, float limit, float alpha,
+                                  cudaStream_t stream) {
+  if (inner % 4 == 0 && (uintptr_t)gu % (4 * sizeof(TI)) == 0 && (uintptr_t)act % (4 * sizeof(T)) == 0 && (uintptr_t)bias % 16 == 0) {
+    const int tiles = (inner / 4 + 255) / 256;
+    if (M >= 64)      // (rows enough for every SM to have several CTAs all the same)
+      launch_chained(gated_bias_act_x4_kernel<TI, T, 4>, dim3(tiles, (M + 3) / 4), dim3(256), 0, stream, gu, bias, act, M, inner, kind, limit, alpha);
+    else
+      launch_chained(gated_bias_act_x4_kernel<TI, T, 1>, dim3(tiles, M), dim3(256), 0, stream, gu, bias, act, M, inner, kind, limit, alpha);
+  } else {
+    launch_chained(gated_bias_act_kernel<TI, T>, dim3((inner + 255) / 256, M), dim3(256), 0, stream, gu, bias, act, inner, kind, limit, alpha);
+  }
+}
+
 }  // namespace nf
 
 extern "C" int nf_pair_hash_embed(const void* table, const int* ids, const int* row_seg, const int* seg_row0,
@@ -524,14 +573,13 @@ extern "C" int nf_gated_bias_act(const void* gu, int in_dtype, const float* bias
   // rows in grid.y, 65535 at a time
   for (int m0 = 0; m0 < M; m0 += 65535) {
     const int rows = M - m0 < 65535 ? M - m0 : 65535;
-    const dim3 grid((inner + 255) / 256, rows);
     const size_t in_off = (size_t)m0 * 2 * inner, out_off = (size_t)m0 * inner;
     if (dtype == kF32)
-      launch_chained(gated_bias_act_kernel<float, float>, grid, dim3(256), 0, stream, (const float*)gu + in_off, bias, (float*)act + out_off, inner, kind, limit, alpha);
+      launch_gated_bias_act((const float*)gu + in_off, bias, (float*)act + out_off, rows, inner, kind, limit, alpha, stream);
     else if (in_dtype == kF32)
-      launch_chained(gated_bias_act_kernel<float, __nv_bfloat16>, grid, dim3(256), 0, stream, (const float*)gu + in_off, bias, (__nv_bfloat16*)act + out_off, inner, kind, limit, alpha);
+      launch_gated_bias_act((const float*)gu + in_off, bias, (__nv_bfloat16*)act + out_off, rows, inner, kind, limit, alpha, stream);
     else
-      launch_chained(gated_bias_act_kernel<__nv_bfloat16, __nv_bfloat16>, grid, dim3(256), 0, stream, (const __nv_bfloat16*)gu + in_off, bias, (__nv_bfloat16*)act + out_off, inner, kind, limit, alpha);
+      launch_gated_bias_act((const __nv_bfloat16*)gu + in_off, bias, (__nv_bfloat16*)act + out_off, rows, inner, kind, limit, alpha, stream);
   }
   return check_launch("gated_bias_act");
 }

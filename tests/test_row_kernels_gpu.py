@@ -1,0 +1,73 @@
+"""Row-wise kernels of prompt steps that move runs of four numbers: against the forms that move one at a time (which columns
+off a 16-byte boundary still take), bit for bit, at the edges of a run of rows."""
+
+import pytest
+import torch
+
+from test_decode_kernels_gpu import ints, make_step
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from ninfer_amd_mi50_b200 import kernels
+    kernels.load()
+    return kernels
+
+
+@pytest.mark.parametrize("M", [1, 63, 64, 67, 130])
+@pytest.mark.parametrize("inner", [4, 1028, 1031])
+@pytest.mark.parametrize("act", [None, (2, 7.0, 1.702)])
+def test_gated_activation_of_sums(K, M, inner, act):
+    g = torch.Generator().manual_seed(1)
+    gu, bias = torch.randn((M, 2 * inner), generator=g).cuda() * 4, torch.randn((2 * inner,), generator=g).cuda()
+    for b in (None, bias):
+        for src, dtype in ((gu, torch.bfloat16), (gu, torch.float32), (gu.bfloat16(), torch.bfloat16)):
+            out = K.gated_bias_act(src, b, act, dtype)
+            x = src.double() + (0.0 if b is None else b.double())
+            gate, up = x[:, :inner], x[:, inner:]
+            if act is None:
+                want = gate * torch.sigmoid(gate) * up
+            else:
+                gate, up = gate.clamp(max=7.0), up.clamp(-7.0, 7.0)
+                want = gate * torch.sigmoid(1.702 * gate) * (up + 1.0)
+            # float32 arithmetic of a few roundings, then one to the result's type
+            torch.testing.assert_close(out.double(), want, rtol=2 ** -8 if dtype == torch.bfloat16 else 1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("D,rot", [(128, 0), (64, 64), (64, 16), (32, 8), (20, 0)])
+@pytest.mark.parametrize("silu", [True, False])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_queries_and_keys_prepared_in_runs_of_four(K, D, rot, silu, dtype):
+    H, V = 5, 16
+    _, _, ctx, _, _, g = make_step(dtype, [19, 2], [3, 0], 1, 16, 16, 11)
+    src = torch.randn((ctx.T, H * (2 * D + V) + 4), generator=g).to(dtype).cuda()
+    shifted = torch.empty((ctx.T, src.shape[1] + 4), dtype=dtype, device="cuda")
+    shifted[:, 1:-3] = src                                    # the same columns, off a boundary
+    freq = torch.rand((max(1, rot // 2),), generator=g).cuda()
+    decay = torch.linspace(0.8, 0.99, H).cuda()
+    outs = []
+    for x, c in ((src, 0), (shifted, 1)):
+        state = torch.zeros((2, H * V * D), device="cuda")
+        outs.append((K.decay_linear_attention(x, c, c + H * D, c + 2 * H * D, decay, freq if rot else None, rot, 0.5, silu, state,
+                                              ctx, H, D, V), state))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("lens", [[64], [65, 1, 3], [15, 16, 17, 18], [1, 2, 200]])
+@pytest.mark.parametrize("C,taps", [(8, 4), (264, 2), (1032, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_convolution_with_rows_in_flight(K, lens, C, taps, dtype):
+    """Several requests in a tile of sixteen rows, tiles that end early; the row-by-row form takes the columns off a boundary."""
+    _, _, ctx, _, _, g = make_step(dtype, lens, [7] * len(lens), 1, 16, 16, 12)
+    src = torch.randn((ctx.T, C + 8), generator=g).to(dtype).cuda()
+    shifted = torch.empty((ctx.T, C + 17), dtype=dtype, device="cuda")
+    shifted[:, 1:-8] = src
+    w, b = torch.randn((taps, C), generator=g).cuda(), torch.randn((C,), generator=g).cuda()
+    state = torch.randn((len(lens), (taps - 1) * C), generator=g).cuda()
+    outs = []
+    for x, c in ((src, 8), (shifted, 9)):
+        st = state.clone()
+        outs.append((K.causal_conv_silu(x, c, C, w, b, st, ctx), st))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
