@@ -13,6 +13,10 @@
 //                   A matrix beyond L2 they read from memory: a head of 151936 x 2048 with 5 rows 431 us, with the next
 //                   tile 320, 16 rows 843 and 328, 24 rows 1247 and 671 (4 rows 236 and 320); 32000 x 2048 with 5 rows 115
 //                   and 88; half of 12288 x 4096 is still in L2: 8 rows 74 and 93, 12 rows 100 and 95
+//                   Between, where 8 x 32 tiles of two warps are few (up to 400 CTAs), those: what counts there is the chain
+//                   over k, and more CTAs beside one another (one matrix, rows x features x k: 16 x 6144 x 2048 29 us, with
+//                   the tile before 33, with the next one 42; 32 x 2048 x 5632 50, 67, 108; 32 x 2048 x 2048 20, 28, 41; 768
+//                   CTAs, 32 x 6144 x 2048: 65, 63, 48; 8 x 6144 x 2048 21, 23, 42)
 //   up to 64        16 x 64, two warps with 8 x 2 sums a thread (34 rows a group 472 us, with the next tile 518)
 //   up to 128       32 x 64 with 4 x 4 sums a thread: 100 rows 112 us, with the tile before 152, with the one behind 140
 //   more            64 x 64 with 8 x 4 sums a thread (gated 4 x 4), bound by the products themselves: 256 rows 184 us,
@@ -170,6 +174,9 @@ int gf_dispatch(const GfCall& c, cudaStream_t stream) {
   // (the lines lie between the measured sizes at which the tile below and the one above were the faster)
   const bool alone = c.groups == 1;
   const size_t matrix = (size_t)c.N * (GATED ? 2 : 1) * c.K * sizeof(float);
+  if constexpr (!GATED)
+    if (alone && rows > 4 && rows <= 32 && (c.N + 31) / 32 * ((c.max_rows + 7) / 8) <= 400 && matrix <= kGfL2)
+      return gf_launch<8, 32, 4, 1, 8, false>(c, tiles(8), stream);
   if (rows <= (!alone ? 5 : matrix > kGfFar ? 4 : matrix > kGfL2 ? 10 : 24)) return gf_launch<4, GATED ? 64 : 32, 4, GATED ? 2 : 1, 6, GATED>(c, tiles(4), stream);
   if (rows <= 64) return gf_launch<16, 64, 8, 2, 4, GATED>(c, tiles(16), stream);
   if (rows <= 128) return gf_launch<32, 64, 4, 4, 4, GATED>(c, tiles(32), stream);

@@ -71,3 +71,15 @@ def test_convolution_with_rows_in_flight(K, lens, C, taps, dtype):
         st = state.clone()
         outs.append((K.causal_conv_silu(x, c, C, w, b, st, ctx), st))
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("rows", [4, 5, 8, 9, 16, 24, 25, 32, 33])
+@pytest.mark.parametrize("n,k", [(32, 64), (100, 2048), (2048, 256), (6144, 128)])
+def test_float32_products_of_few_rows(K, rows, n, k):
+    """A row's bits are the same in every tile."""
+    g = torch.Generator().manual_seed(2)
+    x, w = torch.randn((rows, k), generator=g).cuda(), torch.randn((n, k), generator=g).cuda()
+    out = K.linear(x, w)
+    assert torch.equal(out, torch.cat([K.linear(x[r:r + 1].contiguous(), w) for r in range(rows)]))
+    # a chain of k float32 products and sums
+    assert (out - x.double() @ w.double().T).abs().max() <= 2 ** -24 * k ** 0.5 * 5 * k ** 0.5
