@@ -24,8 +24,13 @@
 //              may touch the same 32 lanes) and take 64 of its 128 scores each: ``tcgen05.ld``,
 //              mask, a reference maximum that is only raised when a score exceeds it by more than
 //              2^8 (then O's row is rescaled in tensor memory), P = 2^(s - m) as bfloat16 into
-//              shared memory in the swizzled K-major image; at the end of the tile O divided by
-//              the row sum is stored
+//              one of two buffers in tensor memory, out of which the second product reads it; at the
+//              end of the tile O divided by the row sum is stored
+//
+// What bounds a tile is the chain of its softmax, block after block.  With one buffer of P in shared memory 550 of a
+// block's 2,780 cycles were waiting for the product of the block before; 2,048 rows of 16 heads 42.5 us, now 40.5, behind
+// 6,144 further keys 183.7, now 181.4.  (A quarter or half of the exponentials as polynomials on the multiply-add units
+// instead of the special-function unit: 41.9 and 45.7, it is issue slots that are short.)
 //
 // The SIGMOID form has weights sigmoid(score + sig_bias[h]) that are not normalised over keys: no maximum, no rescaling,
 // no sum; P = 1 / (1 + 2^-(s + b)) and O is stored as it stands.
@@ -74,8 +79,8 @@ constexpr float kRaise = 8.f;    // raise the reference maximum only beyond this
 __device__ int g_fa_error = 0;
 
 struct __align__(8) FaBarriers {
-  unsigned long long q_full, q_empty, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full,
-      p_free, o_final, o_read;
+  unsigned long long q_full, q_empty, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full[2],
+      p_free[2], o_final, o_read;
   unsigned tmem_base;
   int stop;
 };
@@ -105,6 +110,14 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+
+__device__ __forceinline__ float max3(float x, float y, float z) {
+  float v;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(x), "f"(y), "f"(z));
+  return v;
+}
+// shared memory for P: none where it lives in tensor memory
+constexpr int fa_p_bytes(int parts) { return parts == 1 ? 0 : parts * 2 * kAtom; }
 
 struct TileInfo {
   int seg, row0, n_rows, pos_first, pos_last, kb_first, n_kept, n_blocks;
@@ -145,13 +158,14 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   constexpr int KATOMS = (D + ROT) / 64;          // ... across a query or key
   constexpr int QB = KATOMS * kAtom, VB = ATOMS * kAtom;   // bytes of the Q tile and of a K block; of a V block
   constexpr int STAGES = ROT ? 1 : 2, PARTS = ROT ? 2 : 1; // K and V stages; bfloat16 numbers a weight is given as
+  constexpr int PBUF = PARTS == 1 ? 2 : 1;        // buffers of P: two in tensor memory, or one in shared memory
   static_assert(!ROT || (DENSE && FORM == kFormSoftmax), "the further dimensions go with the dense softmax form");
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* Qs = smem;
   unsigned char* KV = Qs + QB;                    // [stages][K block, V block]
   unsigned char* Ps = KV + STAGES * (QB + VB);    // [parts][2 atoms][128 rows][128 bytes]
-  FaBarriers* bars = reinterpret_cast<FaBarriers*>(Ps + PARTS * 2 * kAtom);
+  FaBarriers* bars = reinterpret_cast<FaBarriers*>(Ps + fa_p_bytes(PARTS));
   float* s_rowsum = reinterpret_cast<float*>(bars + 1);      // [2 halves][128 rows]: the two threads of a row add up
   float* s_rowmax = s_rowsum + 2 * kQ;                       // [2 block parities][2 halves][128 rows]
   volatile int* stop = &bars->stop;
@@ -173,8 +187,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       mbar_init(&bars->s_full[s], 1);
       mbar_init(&bars->s_empty[s], 8);
     }
-    mbar_init(&bars->p_full, 8);
-    mbar_init(&bars->p_free, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&bars->p_full[s], 8);
+      mbar_init(&bars->p_free[s], 1);
+    }
     mbar_init(&bars->o_final, 1);
     mbar_init(&bars->o_read, 8);
     bars->stop = 0;
@@ -189,7 +205,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = bars->tmem_base;
-  const unsigned tmem_o = tmem + 2 * kKeys;       // S buffers at columns 0 and 128, O at 256
+  const unsigned tmem_o = tmem + 2 * kKeys;       // S buffers at columns 0 and 128, O at 256, P's at 384 and 448
+  const unsigned tmem_p = tmem + 3 * kKeys;
   // Launched chained: the zero-fill, the barriers and the tensor-memory allocation above touch
   // nothing outside the SM and ran while the kernel before this one drained; queries, keys and
   // values (and the first write of `out`) come after the wait.
@@ -284,23 +301,24 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       bool ok = true;
       // O += P V of the block whose values sit in stage gp % STAGES; `first`: the first block of a tile
       auto issue_pv = [&](bool first) -> bool {
-        const int vs = gp % STAGES;
+        const int vs = gp % STAGES, pb = gp % PBUF;
         if (!mbar_wait(&bars->v_full[vs], (gp / STAGES) & 1, stop, 4, &g_fa_error)) return false;
-        if (!mbar_wait(&bars->p_full, gp & 1, stop, 5, &g_fa_error)) return false;
+        if (!mbar_wait(&bars->p_full[pb], (gp / PBUF) & 1, stop, 5, &g_fa_error)) return false;
         if (first && gq > 0 && !mbar_wait(&bars->o_read, (gq - 1) & 1, stop, 6, &g_fa_error)) return false;
         tc_fence_after();
         const unsigned char* vst = KV + (size_t)vs * (QB + VB) + QB;
 #pragma unroll
         for (int kk = 0; kk < kKeys / 16; ++kk) {
           const unsigned long long b = smem_desc_mn(vst + kk * 16 * 128, kAtom);
+          if (PBUF == 2) tc_mma_ts(tmem_o, tmem_p + pb * (kKeys / 2) + 8 * kk, b, idesc_pv, (!first || kk > 0) ? 1u : 0u);
 #pragma unroll
-          for (int part = 0; part < PARTS; ++part) {
+          for (int part = 0; part < PARTS && PBUF == 1; ++part) {
             const unsigned long long a = smem_desc(Ps + (2 * part + (kk >> 2)) * kAtom) + 2 * (kk & 3);
             tc_mma(tmem_o, a, b, idesc_pv, (!first || kk > 0 || part > 0) ? 1u : 0u);
           }
         }
         tc_commit(&bars->v_empty[vs]);           // the values of this block are free ...
-        tc_commit(&bars->p_free);                // ... and so are P and O, once these have run
+        tc_commit(&bars->p_free[pb]);            // ... and so are P and O, once these have run
         ++gp;
         return true;
       };
@@ -403,7 +421,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};     // four chains, not one
           if (all_visible) {
 #pragma unroll
-            for (int i = 0; i < HK; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(u[i]));
+            for (int i = 0; i < HK; i += 2) m4[(i >> 1) & 3] = max3(m4[(i >> 1) & 3], __uint_as_float(u[i]), __uint_as_float(u[i + 1]));
           } else {
 #pragma unroll
             for (int i = 0; i < HK; ++i) {
@@ -435,9 +453,13 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           alpha = exp2f(m_ref - mx);
           m_ref = mx;
         }
-        // P and O are free once the product of the block before has run
-        if (gp > 0 && !mbar_wait(&bars->p_free, (gp - 1) & 1, stop, 9, &g_fa_error)) { ok = false; break; }
+        // This buffer of P is free once the product that read it has run; O, which only a raise touches, once the
+        // product of the block before has
+        const int pb = gp % PBUF;
+        if (gp >= PBUF && !mbar_wait(&bars->p_free[pb], (gp / PBUF - 1) & 1, stop, 9, &g_fa_error)) { ok = false; break; }
+        if (PBUF == 2) tc_fence_after();
         if (!SIGMOID && __any_sync(0xffffffffu, raise)) {                   // the whole warp, each row by its own factor
+          if (PBUF == 2 && !mbar_wait(&bars->p_free[pb ^ 1], ((gp - 1) / PBUF) & 1, stop, 9, &g_fa_error)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < HD / 32; ++c) {
@@ -456,6 +478,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // and gives 0.
         float sum = 0.f;
         unsigned char* prow = Ps + half * kAtom + r * 128;
+        unsigned pk[PBUF == 2 ? HK / 2 : 1];
 #pragma unroll
         for (int q = 0; q < HK / 8; ++q) {
           float p[8];
@@ -471,7 +494,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           w.y = *reinterpret_cast<unsigned*>(&b1);
           w.z = *reinterpret_cast<unsigned*>(&b2);
           w.w = *reinterpret_cast<unsigned*>(&b3);
-          *reinterpret_cast<uint4*>(prow + ((q ^ (r & 7)) << 4)) = w;   // piece q: keys 8 q .. 8 q + 7 of the atom
+          if constexpr (PBUF == 2) pk[4 * q] = w.x, pk[4 * q + 1] = w.y, pk[4 * q + 2] = w.z, pk[4 * q + 3] = w.w;
+          else *reinterpret_cast<uint4*>(prow + ((q ^ (r & 7)) << 4)) = w;   // piece q: keys 8 q .. 8 q + 7 of the atom
           if constexpr (PARTS == 2) {
             auto rest = [](float x, float y, __nv_bfloat162 b) {
               const __nv_bfloat162 d = __floats2bfloat162_rn(x - __low2float(b), y - __high2float(b));
@@ -483,6 +507,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           sum += ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
         }
         l_run += sum;
+        if constexpr (PBUF == 2) {
+          tc_st32(tmem_p + lane_addr + pb * (kKeys / 2) + half * (HK / 2), pk);
+          tc_wait_st();
+        }
         if constexpr (DENSE || BIASED) {
           const int own_keys = t.pos_last + 1 - kb;
           if (own_keys < kKeys) {                                // the tile's last block
@@ -493,10 +521,10 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
               for (int a = 0; a < ATOMS; ++a) reinterpret_cast<uint4*>(vst + a * kAtom)[i] = make_uint4(0, 0, 0, 0);
           }
         }
-        fence_async_smem();
+        if (PBUF == 1 || DENSE || BIASED) fence_async_smem();    // (what was written to shared memory above)
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->p_full);
+        if (lane == 0) mbar_arrive(&bars->p_full[pb]);
       }
       if (!ok) break;
       // ---- the tile's rows: O / l ---------------------------------------------------------------------
@@ -564,7 +592,7 @@ int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mkv, const CUten
                       const int* kv_base, const void* gate, int gate_ld, float softcap, const float* slopes, int keep_first,
                       cudaStream_t stream) {
   constexpr int QB = (D + ROT) / 64 * kAtom, VB = D / 64 * kAtom;
-  const size_t smem = 1024 + QB + (ROT ? 1 : 2) * (size_t)(QB + VB) + (ROT ? 4 : 2) * kAtom + sizeof(FaBarriers) + 6 * kQ * sizeof(float);
+  const size_t smem = 1024 + QB + (ROT ? 1 : 2) * (size_t)(QB + VB) + fa_p_bytes(ROT ? 2 : 1) + sizeof(FaBarriers) + 6 * kQ * sizeof(float);
   static bool set = false;
   if (!set) {
     cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<D, ROT, FORM, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
