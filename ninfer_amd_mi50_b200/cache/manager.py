@@ -22,6 +22,7 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import Dict, Hashable, List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from ..parts.base import CacheSpec, CacheView, StateSpec
@@ -52,6 +53,9 @@ class RequestEntry:
     reserved: int = 0                      # tokens for which pages are held
     # per group: logical page index -> physical page (-1 once released or never held)
     tables: List[List[int]] = field(default_factory=list)
+    # the same numbers as int32 arrays (a table's length of them count): a decode step copies a request's row of the block
+    # table as it is, instead of turning a list of a hundred numbers into an array every step
+    rows: List[np.ndarray] = field(default_factory=list)
 
 
 class CacheManager:
@@ -121,7 +125,8 @@ class CacheManager:
         slot = self._free_slots.pop()
         for slab in self.state.values():
             slab[slot].zero_()
-        self.requests[req] = RequestEntry(slot, tables=[[] for _ in self.groups])
+        self.requests[req] = RequestEntry(slot, tables=[[] for _ in self.groups],
+                                          rows=[np.full(self.max_pages_per_request, -1, np.int32) for _ in self.groups])
         return slot
 
     def close(self, req: Hashable) -> None:
@@ -171,14 +176,18 @@ class CacheManager:
         if new_length > self.max_context:
             raise OutOfPages(f"request {req!r}: {new_length} tokens exceed max_context={self.max_context}")
         need = self.pages_needed(req, new_length)
+        if not any(need):                      # (most decode steps: the pages held have room)
+            ent.reserved = max(ent.reserved, new_length)
+            return
         for n, g in zip(need, self.groups):
             if n > g.pool.num_free:
                 raise OutOfPages(f"request {req!r}: group {g.index} needs {n} pages, "
                                  f"{g.pool.num_free} free")
-        for n, g, table in zip(need, self.groups, ent.tables):
+        for n, g, table, row in zip(need, self.groups, ent.tables, ent.rows):
             first_new = len(table)
             taken, again = g.pool.take_marking_reuse(n)
             table.extend(taken)
+            row[first_new:first_new + n] = taken
             if not (again and self.clear_reused_pages and g.pages is not None):
                 continue
             # A page that is handed out again still holds its earlier owner's entries.  Kernels
@@ -205,13 +214,15 @@ class CacheManager:
         if new_length > ent.reserved:
             raise AssertionError(f"commit to {new_length} beyond the reserved {ent.reserved}")
         ent.length = new_length
-        for g, table in zip(self.groups, ent.tables):
+        for g, table, row in zip(self.groups, ent.tables, ent.rows):
+            if g.spec.kind != "window":
+                continue
             first = self._first_live_page(g, new_length)
             dead = [i for i in range(self._first_droppable_page(g), min(first, len(table))) if table[i] >= 0]
             if dead:
                 g.pool.give_back([table[i] for i in dead])
                 for i in dead:
-                    table[i] = -1
+                    table[i] = row[i] = -1
 
     def truncate(self, req: Hashable) -> None:
         """Drop a reservation that was never committed (a step that did not run)."""
@@ -225,6 +236,11 @@ class CacheManager:
 
     def block_table(self, group: int, req: Hashable) -> List[int]:
         return self.requests[req].tables[group]
+
+    def block_row(self, group: int, req: Hashable) -> np.ndarray:
+        """The same as an int32 array; a view that the next reservation or commit may change."""
+        ent = self.requests[req]
+        return ent.rows[group][:len(ent.tables[group])]
 
     # ---- what a mixer call sees ------------------------------------------------------
     def view(self, cache_slot: int, block_tables: Dict[int, torch.Tensor], append: bool

@@ -31,8 +31,10 @@ class BatchError(ValueError):
     pass
 
 
-def validate_entries(entries: Sequence[StepEntry], cache: CacheManager, vocab_size: int) -> None:
+def validate_entries(entries: Sequence[StepEntry], cache: CacheManager, vocab_size: int) -> List[np.ndarray]:
+    """Raises `BatchError` for entries that cannot be run; returns their tokens as arrays."""
     seen = set()
+    arrays: List[np.ndarray] = []
     for e in entries:
         if e.req in seen:
             raise BatchError(f"request {e.req!r} appears twice in one step")
@@ -41,18 +43,27 @@ def validate_entries(entries: Sequence[StepEntry], cache: CacheManager, vocab_si
             raise BatchError(f"request {e.req!r} is not open")
         if len(e.tokens) == 0:
             raise BatchError(f"request {e.req!r} brings no tokens")
-        toks = np.asarray(e.tokens, dtype=np.int64)     # one pass in numpy: a long portion has thousands
-        bad = np.flatnonzero((toks < 0) | (toks >= vocab_size))
-        if bad.size:
-            raise BatchError(f"request {e.req!r}: token id {int(toks[bad[0]])} outside [0, {vocab_size})")
+        if len(e.tokens) == 1 and type(e.tokens[0]) is int:
+            if not 0 <= e.tokens[0] < vocab_size:
+                raise BatchError(f"request {e.req!r}: token id {e.tokens[0]} outside [0, {vocab_size})")
+            toks = e.tokens
+        else:
+            toks = np.asarray(e.tokens, dtype=np.int64)     # one pass in numpy: a long portion has thousands
+            bad = np.flatnonzero((toks < 0) | (toks >= vocab_size))
+            if bad.size:
+                raise BatchError(f"request {e.req!r}: token id {int(toks[bad[0]])} outside [0, {vocab_size})")
         for w in e.want:
             if not 0 <= int(w) < len(e.tokens):
                 raise BatchError(f"request {e.req!r}: wanted place {w} outside its {len(e.tokens)} tokens")
+        arrays.append(toks)
+    return arrays
 
 
 def pack_step(entries: Sequence[StepEntry], cache: CacheManager, dtype: torch.dtype,
-              device: torch.device, *, table_width: Optional[int] = None) -> StepContext:
-    """Build the step's metadata.  Pages for the new tokens must be reserved already."""
+              device: torch.device, *, table_width: Optional[int] = None,
+              arrays: Optional[Sequence[np.ndarray]] = None) -> StepContext:
+    """Build the step's metadata.  Pages for the new tokens must be reserved already.  `arrays`: the entries' tokens
+    as `validate_entries` returned them (a list of thousands is turned into an array once a step)."""
     S = len(entries)
     # numpy pieces, not Python lists: a 2,048-token portion was 0.85 ms of list building here
     pieces_tok, pieces_pos, pieces_seg = [], [], []
@@ -65,7 +76,7 @@ def pack_step(entries: Sequence[StepEntry], cache: CacheManager, dtype: torch.dt
         n = len(e.tokens)
         pos0 = cache.length(e.req)
         row0 = seg_row0[-1]
-        pieces_tok.append(np.asarray(e.tokens, dtype=np.int32))
+        pieces_tok.append(np.asarray(e.tokens if arrays is None else arrays[s], dtype=np.int32))
         pieces_pos.append(np.arange(pos0, pos0 + n, dtype=np.int32))
         pieces_seg.append(np.full(n, s, dtype=np.int32))
         seg_row0.append(row0 + n)
@@ -77,7 +88,7 @@ def pack_step(entries: Sequence[StepEntry], cache: CacheManager, dtype: torch.dt
     # block tables, one per cache group, padded to a common width with -1
     tables = []
     for g in cache.groups:
-        rows = [cache.block_table(g.index, e.req) for e in entries]
+        rows = [cache.block_row(g.index, e.req) for e in entries]
         width = table_width or max(1, max(len(r) for r in rows))
         tbl = np.full((S, width), -1, dtype=np.int32)
         for i, r in enumerate(rows):

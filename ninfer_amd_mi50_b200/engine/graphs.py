@@ -40,6 +40,9 @@ def context_bucket(n: int, limit: int) -> int:
     return min((n + 511) // 512 * 512, max(limit, 1))
 
 
+STAGES = 16                          # steps of one graph whose index data may be on its way
+
+
 class DecodeGraph:
     def __init__(self, runner, rows: int, context_bound: int):
         self.runner, self.S, self.context_bound = runner, rows, context_bound
@@ -49,13 +52,15 @@ class DecodeGraph:
         sizes = [S, S, S, S + 1, S, S, S] + [S * self.width for _ in cache.groups]
         self.offsets = np.cumsum([0] + sizes)
         total = int(self.offsets[-1])
-        # Two pinned staging buffers used in turn, each with the event of its last copy: the host
-        # runs a step ahead of the device on purpose, so the copy out of a buffer may still be
-        # queued when the next step is being prepared; a buffer is rewritten only after its own
-        # last copy has finished.
-        self.hosts = [torch.empty((total,), dtype=torch.int32).pin_memory() for _ in range(2)]
+        # Pinned staging buffers used in turn, each with the event of its last copy: the host runs
+        # ahead of the device on purpose, so the copy out of a buffer may still be queued when the
+        # next steps are being prepared; a buffer is rewritten only after its own last copy has
+        # finished.  As many as STAGES steps ahead: the time that decode steps give the host is what
+        # it prepares the next prompt's eager step in (with two buffers it waited a step's length at
+        # every step: 1.4 of 5.3 ms over four prompts of 2,048 tokens and 12 decode steps).
+        self.hosts = list(torch.empty((STAGES, total), dtype=torch.int32).pin_memory().unbind(0))
         self.nps = [h.numpy() for h in self.hosts]
-        self.copied: List[Optional[torch.cuda.Event]] = [None, None]
+        self.copied: List[Optional[torch.cuda.Event]] = [None] * STAGES      # made at the first use, recorded again at every other
         self.turn = 0
         self.dev = torch.zeros((total,), dtype=torch.int32, device=dev)
         parts = [self.dev[self.offsets[i]:self.offsets[i + 1]] for i in range(len(sizes))]
@@ -113,7 +118,7 @@ class DecodeGraph:
         for gi, g in enumerate(cache.groups):
             tbl = a[o[7 + gi]:o[8 + gi]].reshape(S, self.width)
             for s, e in enumerate(entries):
-                row = cache.block_table(g.index, e.req)
+                row = cache.block_row(g.index, e.req)
                 tbl[s, :len(row)] = row
                 tbl[s, len(row):] = -1
             tbl[n:, 0] = g.null_page
@@ -125,15 +130,15 @@ class DecodeGraph:
         device) replace the entries' token ids: the tokens a step before has just drawn, which
         the host has not read yet."""
         lengths = [self.runner.cache.length(e.req) for e in entries]
-        i = self.turn & 1
+        i = self.turn % STAGES
         self.turn += 1
         if self.copied[i] is not None:
             self.copied[i].synchronize()        # the copy that last read this buffer is done
         self._fill(self.nps[i], entries, lengths)
         self.dev.copy_(self.hosts[i], non_blocking=True)
-        done = torch.cuda.Event()
-        done.record(torch.cuda.current_stream(self.dev.device))
-        self.copied[i] = done
+        if self.copied[i] is None:
+            self.copied[i] = torch.cuda.Event()
+        self.copied[i].record(torch.cuda.current_stream(self.dev.device))
         if device_tokens is not None:
             self.dev[self.offsets[0]:self.offsets[0] + len(entries)].copy_(device_tokens)
         self.graph.replay()

@@ -62,7 +62,7 @@ class ModelRunner:
         entries = list(entries)
         if not entries:
             return torch.empty((0, self.model.vocab_size), dtype=torch.float32, device=self.device)
-        validate_entries(entries, self.cache, self.model.vocab_size)
+        arrays = validate_entries(entries, self.cache, self.model.vocab_size)
         self.reserve(entries)
         try:
             if self.graphs is not None and self.graphs.eligible(entries):
@@ -70,7 +70,7 @@ class ModelRunner:
             elif device_tokens is not None:
                 raise ValueError("token ids on the device can only feed a step that is replayed from a graph")
             else:
-                ctx = pack_step(entries, self.cache, self.dtype, self.device)
+                ctx = pack_step(entries, self.cache, self.dtype, self.device, arrays=arrays)
                 logits, moved = self.run(ctx), ctx.scratch.get("h2d_bytes", 0)
         except Exception:
             for e in entries:
