@@ -169,6 +169,14 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return red[32];
 }
 
+// CTAs of a row-wise kernel with `threads` threads each: one a row as long as they find room beside one another,
+// beyond that as many, which walk the rows with the next one's numbers on their way while one is summed up and written.
+// One CTA a row, 2,048 rows came in two rounds of CTAs, each a trip to memory, two meetings of all warps and a write.
+inline int row_ctas(int rows, int threads) {
+  const int room = 148 * (1536 / threads < 1 ? 1 : 1536 / threads);
+  return rows <= room ? rows : room;
+}
+
 // 4 consecutive elements as floats, and back.
 __device__ __forceinline__ void load4(const float* p, float* v) {
   const float4 a = *reinterpret_cast<const float4*>(p);

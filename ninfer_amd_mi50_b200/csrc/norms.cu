@@ -98,6 +98,71 @@ __global__ void add_layernorm_kernel(float* __restrict__ h, const T* __restrict_
   }
 }
 
+// The same for rows of up to 8,192 numbers in runs of four, all rows in place (no list, no pending sum): the row in
+// registers, rows walked as `row_ctas` gives them out.  Same sums in the same order.
+template <typename T, int R>
+__global__ void __launch_bounds__(512)
+add_layernorm_regs_kernel(float* __restrict__ h, const T* __restrict__ delta, const float* __restrict__ w, float eps,
+                          T* __restrict__ out, int hidden, int rows) {
+  __shared__ float red[33];
+  chain_release_if_small();
+  float wk[R][4], v[R][4], hn[R][4], dn[R][4];
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 4;
+    if (i < hidden) load4(w + i, wk[c]);
+  }
+  chain_wait(h, delta);
+  auto ask = [&](int r) {
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+      const int i = (c * blockDim.x + threadIdx.x) * 4;
+      if (i < hidden) {
+        load4(h + (size_t)r * hidden + i, hn[c]);
+        if (delta) load4(delta + (size_t)r * hidden + i, dn[c]);
+      }
+    }
+  };
+  ask(blockIdx.x);
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    float s = 0.f;
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+      const int i = (c * blockDim.x + threadIdx.x) * 4;
+      if (i >= hidden) continue;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        v[c][e] = hn[c][e];
+        if (delta) v[c][e] += dn[c][e];
+        s += v[c][e];
+      }
+      if (delta) store4(h + (size_t)r * hidden + i, v[c]);
+    }
+    if (r + (int)gridDim.x < rows) ask(r + gridDim.x);
+    const float mean = block_sum(s, red) / (float)hidden;
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < R; ++c)
+      if ((c * (int)blockDim.x + (int)threadIdx.x) * 4 < hidden) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float d = v[c][e] - mean;
+          ss += d * d;
+        }
+      }
+    const float rstd = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+      const int i = (c * blockDim.x + threadIdx.x) * 4;
+      if (i >= hidden) continue;
+      float o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = (v[c][e] - mean) * rstd * wk[c][e];
+      store4(out + (size_t)r * hidden + i, o);
+    }
+  }
+}
+
 // RMS norm in `groups` equal consecutive parts, fused with the residual sum of up to two contributions (a
 // mixer's and a feed-forward's that ran side by side):
 //   h[t] += d1[t] (+ d2[t]);  out[t] = part / sqrt(mean(part^2) + eps) * w   for each part of h[t].
@@ -189,29 +254,38 @@ add_group_rmsnorm_kernel(float* __restrict__ h, const T* __restrict__ d1, const 
 template <typename TY, typename TZ, typename T, int R, int MODE>
 __global__ void __launch_bounds__(512)
 part_norm_vec_kernel(const TY* __restrict__ y, int ldy, int ycol0, const TZ* __restrict__ zsrc, int ldz, int zcol0,
-                     const float* __restrict__ w, float eps, T* __restrict__ out, int ldo, int n) {
+                     const float* __restrict__ w, float eps, T* __restrict__ out, int ldo, int n, int rows) {
   __shared__ float red[33];
-  const int t = blockIdx.x, c0 = blockIdx.y * n;
+  const int c0 = blockIdx.y * n;
   chain_release_if_small();
-  float wk[R][4], v[R][4], z[R][4];
+  float wk[R][4], v[R][4], z[R][4], vn[R][4], zn[R][4];
 #pragma unroll
   for (int c = 0; c < R; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 4;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) { wk[c][e] = 1.f; v[c][e] = z[c][e] = 0.f; }
+    for (int e = 0; e < 4; ++e) { wk[c][e] = 1.f; vn[c][e] = zn[c][e] = 0.f; }
     if (w && i < n) load4(w + c0 + i, wk[c]);
   }
   chain_wait(y, zsrc);
-  const TY* yr = y + (size_t)t * ldy + ycol0 + c0;
-  const TZ* zr = MODE ? zsrc + (size_t)t * ldz + zcol0 + c0 : nullptr;
+  auto ask = [&](int t) {
+    const TY* yr = y + (size_t)t * ldy + ycol0 + c0;
+    const TZ* zr = MODE ? zsrc + (size_t)t * ldz + zcol0 + c0 : nullptr;
 #pragma unroll
-  for (int c = 0; c < R; ++c) {
-    const int i = (c * blockDim.x + threadIdx.x) * 4;
-    if (i < n) {
-      load4(yr + i, v[c]);
-      if (MODE) load4(zr + i, z[c]);
+    for (int c = 0; c < R; ++c) {
+      const int i = (c * blockDim.x + threadIdx.x) * 4;
+      if (i < n) {
+        load4(yr + i, vn[c]);
+        if (MODE) load4(zr + i, zn[c]);
+      }
     }
-  }
+  };
+  ask(blockIdx.x);
+  for (int t = blockIdx.x; t < rows; t += gridDim.x) {
+#pragma unroll
+  for (int c = 0; c < R; ++c)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { v[c][e] = vn[c][e]; z[c][e] = zn[c][e]; }
+  if (t + (int)gridDim.x < rows) ask(t + gridDim.x);
   float ss = 0.f;
 #pragma unroll
   for (int c = 0; c < R; ++c)
@@ -234,6 +308,7 @@ part_norm_vec_kernel(const TY* __restrict__ y, int ldy, int ycol0, const TZ* __r
     for (int e = 0; e < 4; ++e) o[e] = v[c][e] * inv * wk[c][e] * (MODE >= 2 ? z[c][e] : 1.f);
     store4(out + (size_t)t * ldo + c0 + i, o);
   }
+  }
 }
 // Whether rows of `n` numbers at `p` (first column `col0`, `ld` apart, `el` bytes a number) can be moved four at a time.
 static inline bool runs_of_four(const void* p, size_t el, long ld, long col0) {
@@ -249,8 +324,8 @@ static int part_norm_vec(const void* y, int ldy, int ycol0, const void* z, int l
   const int units = n / 4, runs = units <= 512 ? 1 : (units <= 1024 ? 2 : 4);
   const int th = ((units + runs - 1) / runs + 31) / 32 * 32;
 #define NF_PN(RR)                                                                                                        \
-  launch_chained(part_norm_vec_kernel<TY, TZ, T, RR, MODE>, dim3(R, parts), dim3(th), 0, stream, (const TY*)y, ldy, ycol0, \
-                 (const TZ*)z, ldz, zcol0, w, eps, (T*)out, ldo, n)
+  launch_chained(part_norm_vec_kernel<TY, TZ, T, RR, MODE>, dim3(parts > 1 ? R : row_ctas(R, th), parts), dim3(th), 0, stream, (const TY*)y, \
+                 ldy, ycol0, (const TZ*)z, ldz, zcol0, w, eps, (T*)out, ldo, n, R)
   if (runs == 1) NF_PN(1); else if (runs == 2) NF_PN(2); else NF_PN(4);
 #undef NF_PN
   return 1;
@@ -388,6 +463,11 @@ extern "C" int nf_add_layernorm(float* h, const void* delta, const int* rows, co
   const size_t smem = (size_t)hidden * sizeof(float);
   NF_REQUIRE(smem <= 160 * 1024, "add_layernorm: a row of %d does not fit shared memory", hidden);
   const int threads = hidden >= 2048 ? 512 : 256;
+  const int runs = (hidden / 4 + threads - 1) / threads;
+#define NF_LN_R(T, RR)                                                                                                  \
+  launch_chained(add_layernorm_regs_kernel<T, RR>, dim3(row_ctas(R, threads)), dim3(threads), 0, stream, h, (const T*)delta, w, \
+                 eps, (T*)out, hidden, R)
+#define NF_LN_REGS(T) do { if (runs <= 1) NF_LN_R(T, 1); else if (runs <= 2) NF_LN_R(T, 2); else NF_LN_R(T, 4); } while (0)
 #define NF_LN(T, G, V)                                                                                      \
   do {                                                                                                      \
     if (smem > 48 * 1024)                                                                                   \
@@ -399,9 +479,16 @@ extern "C" int nf_add_layernorm(float* h, const void* delta, const int* rows, co
   const size_t tsize = dtype == kF32 ? 4 : 2;
   const bool vec = hidden % 4 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)w % 16 == 0 && (uintptr_t)out % (4 * tsize) == 0 &&
                    (!delta || (uintptr_t)delta % (4 * tsize) == 0) && (!y || (uintptr_t)y % (4 * tsize) == 0);
-  if (dtype == kF32) { if (rows) NF_LN_V(float, true); else NF_LN_V(float, false); }
-  else { if (rows) NF_LN_V(__nv_bfloat16, true); else NF_LN_V(__nv_bfloat16, false); }
+  if (vec && !rows && !y && runs <= 4) {
+    if (dtype == kF32) NF_LN_REGS(float); else NF_LN_REGS(__nv_bfloat16);
+  } else if (dtype == kF32) {
+    if (rows) NF_LN_V(float, true); else NF_LN_V(float, false);
+  } else {
+    if (rows) NF_LN_V(__nv_bfloat16, true); else NF_LN_V(__nv_bfloat16, false);
+  }
 #undef NF_LN_V
+#undef NF_LN_REGS
+#undef NF_LN_R
 #undef NF_LN
   return check_launch("add_layernorm");
 }
@@ -553,38 +640,48 @@ __global__ void scaled_norm_add_kernel(float* __restrict__ h, const TD* __restri
 template <typename TD, typename TO, int R>
 __global__ void __launch_bounds__(512)
 scaled_norm_add_regs_kernel(float* __restrict__ h, const TD* __restrict__ delta, const float* __restrict__ bias,
-                            const float* __restrict__ w, const float* __restrict__ ls, float eps, TO* __restrict__ out, int hidden) {
+                            const float* __restrict__ w, const float* __restrict__ ls, float eps, TO* __restrict__ out, int hidden,
+                            int rows) {
   __shared__ float red[33];
-  const int r = blockIdx.x;
   chain_release_if_small();
-  float wk[R], lk[R], d[R], hk[R];
+  float wk[R], lk[R], bk[R], d[R], hk[R], hn[R];
 #pragma unroll
   for (int c = 0; c < R; ++c) {
     const int i = c * blockDim.x + threadIdx.x;
     wk[c] = lk[c] = 1.f;
-    d[c] = hk[c] = 0.f;
+    bk[c] = d[c] = hk[c] = hn[c] = 0.f;
     if (i < hidden) {
       wk[c] = w[i];
       if (ls) lk[c] = ls[i];
-      if (bias) d[c] = bias[i];
+      if (bias) bk[c] = bias[i];
     }
   }
   chain_wait(h, delta);
-  float* hr = h + (size_t)r * hidden;
-  const TD* dr = delta + (size_t)r * hidden;
   TD raw[R];
+  auto ask = [&](int r) {
+    const float* hr = h + (size_t)r * hidden;
+    const TD* dr = delta + (size_t)r * hidden;
 #pragma unroll
-  for (int c = 0; c < R; ++c) {
-    const int i = c * blockDim.x + threadIdx.x;
-    if (i < hidden) { raw[c] = dr[i]; hk[c] = hr[i]; }
-  }
+    for (int c = 0; c < R; ++c) {
+      const int i = c * blockDim.x + threadIdx.x;
+      if (i < hidden) { raw[c] = dr[i]; hn[c] = hr[i]; }
+    }
+  };
+  constexpr bool AHEAD = R < 16;
+  if (AHEAD) ask(blockIdx.x);
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+  if (!AHEAD) ask(r);
+  float* hr = h + (size_t)r * hidden;
   float ss = 0.f;
 #pragma unroll
-  for (int c = 0; c < R; ++c)
+  for (int c = 0; c < R; ++c) {
+    hk[c] = hn[c];
     if (c * (int)blockDim.x + (int)threadIdx.x < hidden) {
-      d[c] = to_float(raw[c]) + d[c];
+      d[c] = to_float(raw[c]) + bk[c];
       ss = fmaf(d[c], d[c], ss);
     }
+  }
+  if (AHEAD && r + (int)gridDim.x < rows) ask(r + gridDim.x);
   const float inv = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
 #pragma unroll
   for (int c = 0; c < R; ++c) {
@@ -593,6 +690,7 @@ scaled_norm_add_regs_kernel(float* __restrict__ h, const TD* __restrict__ delta,
     const float v = scaled_norm_sum(d[c], inv, wk[c], ls, lk[c], hk[c]);
     hr[i] = v;
     if (out) out[(size_t)r * hidden + i] = from_float<TO>(v);
+  }
   }
 }
 
@@ -754,7 +852,7 @@ extern "C" int nf_scaled_norm_add(float* h, const void* delta, int delta_dtype, 
   const dim3 grid(R), block(norm_threads(hidden));
   const int each = (hidden + (int)block.x - 1) / (int)block.x;
 #define NF_SNV(TD, TO, RR) \
-  launch_chained(scaled_norm_add_regs_kernel<TD, TO, RR>, grid, block, 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden)
+  launch_chained(scaled_norm_add_regs_kernel<TD, TO, RR>, dim3(row_ctas(R, (int)block.x)), block, 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden, R)
 #define NF_SNA(TD, TO)                                                                                                     \
   do {                                                                                                                     \
     if (each <= 4) NF_SNV(TD, TO, 4); else if (each <= 8) NF_SNV(TD, TO, 8); else if (each <= 16) NF_SNV(TD, TO, 16);      \

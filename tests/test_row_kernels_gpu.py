@@ -83,3 +83,47 @@ def test_float32_products_of_few_rows(K, rows, n, k):
     assert torch.equal(out, torch.cat([K.linear(x[r:r + 1].contiguous(), w) for r in range(rows)]))
     # a chain of k float32 products and sums
     assert (out - x.double() @ w.double().T).abs().max() <= 2 ** -24 * k ** 0.5 * 5 * k ** 0.5
+
+
+@pytest.mark.parametrize("hidden", [64, 1024, 2048, 2052, 4096, 6144, 8192])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norms_whose_ctas_walk_rows(K, hidden, dtype):
+    """More rows than CTAs: every row's bits are those it has alone (one row a CTA), and the values are right."""
+    rows = 148 * 12 * 2 + 5 if hidden <= 2052 else 148 * 4 + 3
+    g = torch.Generator().manual_seed(3)
+    h = torch.randn((rows, hidden), generator=g).cuda()
+    a, b = (torch.randn((rows, hidden), generator=g).to(dtype).cuda() for _ in range(2))
+    w, w2 = torch.rand((hidden,), generator=g).cuda() + 0.5, torch.rand((hidden,), generator=g).cuda() + 0.5
+    some = [0, 1, rows // 2, rows - 2, rows - 1]
+    tol = dict(rtol=2 ** -8, atol=2 ** -8) if dtype == torch.bfloat16 else dict(rtol=2e-5, atol=2e-5)
+
+    def layernorm(h, a, b):
+        h, out = h.clone(), torch.empty_like(a)
+        K.add_layernorm(h, a, None, w, 1e-6, out)
+        return h, out
+
+    def scaled(h, a, b):
+        h = h.clone()
+        return h, K.scaled_norm_add(h, a, None, w, w2, 1e-6, dtype)
+
+    def residual(h, a, b):
+        h, out = h.clone(), torch.empty_like(a)
+        K.residual_norm(h, w2, 1e-6, out, a=a, scale_a=0.5, b=b, scale_b=2.0, inner_weight=w, inner_eps=1e-6)
+        return h, out
+
+    def gated(h, a, b):
+        return (K.group_rmsnorm_gate(h, a, 0, w, 1e-6, 1, 1, dtype),)
+
+    rms = lambda x: x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6)
+    x = h.double() + a.double()
+    mean = x - x.mean(-1, keepdim=True)
+    s = h.double() + rms(a.double()) * w.double() * w2.double()
+    r = h.double() + rms(0.5 * a.double() + 2.0 * b.double()) * w.double()
+    wants = {layernorm: (x, mean / torch.sqrt((mean * mean).mean(-1, keepdim=True) + 1e-6) * w.double()), scaled: (s, s),
+             residual: (r, rms(r) * w2.double()), gated: (rms(h.double()) * w.double() * torch.sigmoid(a.double()),)}
+    for fn, want in wants.items():
+        got = fn(h, a, b)
+        alone = [torch.cat(t) for t in zip(*(fn(h[i:i + 1].contiguous(), a[i:i + 1].contiguous(), b[i:i + 1].contiguous()) for i in some))]
+        for t, one, v in zip(got, alone, want):
+            assert torch.equal(t[some], one), fn.__name__
+            torch.testing.assert_close(t.double(), v, **(tol if t.dtype == torch.bfloat16 else dict(rtol=2e-5, atol=2e-5)))
