@@ -62,11 +62,29 @@ struct __align__(8) Barriers {
   int stop;
 };
 
-// Persistent: one CTA per SM walks the work items (group, pass of 256 rows, feature tile)
-// cta, cta + grid, ... with feature tiles varying fastest, so CTAs that run together share an
-// expert's token rows in L2, and the passes of a heavily loaded expert - which re-read its
-// weights - run next to each other and find them in L2.  Items cost about the same, so the
-// static assignment stays balanced however unevenly the router loads the experts.  448 threads: warp 0 producer, warp 1 MMA + tensor memory, warps 2..13 epilogue.  The
+// The item a CTA takes after `item`.  BACK_AND_FORTH: rounds of gridDim.x items are dealt out forwards
+// and backwards in turn, so that the CTA with the longest item of one round has the shortest of the next.
+template <bool BACK_AND_FORTH>
+__device__ __forceinline__ int next_item(int item) {
+  const int g = gridDim.x;
+  if (!BACK_AND_FORTH) return item + g;
+  const int round = item / g + 1;
+  return round * g + ((round & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
+}
+
+// Persistent: one CTA per SM walks the work items (group, pass of 256 rows, feature tile), one of
+// every round of as many items as there are CTAs, with feature tiles varying fastest, so CTAs that
+// run together share an expert's token rows in L2, and the passes of a heavily loaded expert - which
+// re-read its weights - run next to each other and find them in L2.
+// Groups are walked by falling number of rows.  An item's time is that of its weights' way from HBM
+// (1,440 cycles a k step of 32 KB with all SMs at it) until its rows' products take as long; routers
+// load experts unevenly (of 60 experts 3 to 1,291 of 8,192 rows), so items differ, 4 to 6 rounds do not
+// even that out, and the last round is thin.  By falling rows it is made of the shortest items, and
+// dealt back and forth the long and short ones meet (60 experts of 2 x 1408 x 2048, 8,192 rows: first
+// product 157 us in the experts' order, 153 by rows, 150 back and forth; second 90, 86, 86; 64 experts of
+// 16,384 rows: 529, 515, 508).  With a second accumulator, unpaired, dealing back and forth costs 4 %
+// (207 -> 216 us): there the order alone is kept.
+// 448 threads: warp 0 producer, warp 1 MMA + tensor memory, warps 2..13 epilogue.  The
 // producer is not held back by the epilogue: while the epilogue warps drain an item's
 // accumulator, the stages fill with the next item's first k tiles, so the memory pipe never
 // goes idle between items.  Wp: packed weights [groups][feature tiles][k tiles][A_ROWS][64].
@@ -100,8 +118,10 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
   // tensor memory are set up meanwhile, and everything that reads what that kernel (or the
   // routing before it) wrote comes after the wait.
   Barriers* bars = reinterpret_cast<Barriers*>(smem);
-  int* s_pass_start = reinterpret_cast<int*>(bars + 1);     // [groups + 1] first pass index of every group
-  const int head_bytes = ((int)sizeof(Barriers) + (groups + 1) * (int)sizeof(int) + 1023) & ~1023;
+  int* s_pass_start = reinterpret_cast<int*>(bars + 1);     // [groups + 1] first pass index of every place in that order
+  int* s_group = s_pass_start + groups + 1;                 // [groups] the groups by falling number of rows
+  int* s_rows = s_group + groups;                           // [groups] rows of every group
+  const int head_bytes = ((int)sizeof(Barriers) + (3 * groups + 1) * (int)sizeof(int) + 1023) & ~1023;
   unsigned char* stage0 = smem + head_bytes;
   volatile int* stop = &bars->stop;
   if (threadIdx.x == 0) {
@@ -125,9 +145,20 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
     for (int g = threadIdx.x; g < groups; g += blockDim.x) {
       const int n = offsets[g + 1] - offsets[g];
       mx = max(mx, n);
-      s_pass_start[g + 1] = (n + kBNMax - 1) / kBNMax;
+      s_rows[g] = n;
     }
     if (mx) atomicMax(&s_max_rows, mx);
+  }
+  __syncthreads();
+  for (int g = threadIdx.x; g < groups; g += blockDim.x) {
+    const int n = s_rows[g];
+    int before = g;
+    if (groups <= kTcThreads) {      // a thread a group; ranking more by comparisons would take longer than it gains
+      before = 0;
+      for (int o = 0; o < groups; ++o) before += s_rows[o] > n || (s_rows[o] == n && o < g);
+    }
+    s_group[before] = g;
+    s_pass_start[before + 1] = (n + kBNMax - 1) / kBNMax;
   }
   __syncthreads();
   if (warp == 0) {
@@ -160,11 +191,11 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
     if (lane == 0) {
       int it = 0, issued = 0;
       bool ok = true;
-      int group = 0;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+      int place = 0;
+      for (int item = blockIdx.x; item < n_items && ok; item = next_item<SWIGLU || PAIR>(item)) {
         const int gp = item / n_fitems, ft = (item - gp * n_fitems) * FT_STEP;      // global pass index, feature tile
-        while (s_pass_start[group + 1] <= gp) ++group;
-        const int pass = gp - s_pass_start[group];
+        while (s_pass_start[place + 1] <= gp) ++place;
+        const int group = s_group[place], pass = gp - s_pass_start[place];
         const int row_begin = offsets[group], n_rows = offsets[group + 1] - row_begin;
         constexpr int W_TILE_BYTES = SWIGLU ? 2 * TILE_BYTES : TILE_BYTES;    // one feature tile's weights of one k step
         const unsigned char* w_tile = reinterpret_cast<const unsigned char*>(Wp) +
@@ -212,11 +243,11 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
     if (lane == 0) {
       int it = 0, pass_ctr = 0;
       bool ok = true;
-      int group = 0;
-      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++pass_ctr) {
+      int place = 0;
+      for (int item = blockIdx.x; item < n_items && ok; item = next_item<SWIGLU || PAIR>(item), ++pass_ctr) {
         const int gp = item / n_fitems;
-        while (s_pass_start[group + 1] <= gp) ++group;
-        const int pass = gp - s_pass_start[group];
+        while (s_pass_start[place + 1] <= gp) ++place;
+        const int group = s_group[place], pass = gp - s_pass_start[place];
         const int n_rows = offsets[group + 1] - offsets[group];
         const bool second = SWIGLU || (PAIR && (item - gp * n_fitems) * FT_STEP + 1 < n_ftiles);
         {
@@ -254,11 +285,11 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
     const int quad = warp & 3, half = (warp - 2) >> 2;     // the warps of a quadrant's lanes take 32 columns in turn
     int pass_ctr = 0;
     bool ok = true;
-    int group = 0;
-    for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++pass_ctr) {
+    int place = 0;
+    for (int item = blockIdx.x; item < n_items && ok; item = next_item<SWIGLU || PAIR>(item), ++pass_ctr) {
       const int gp = item / n_fitems, ft0 = (item - gp * n_fitems) * FT_STEP;
-      while (s_pass_start[group + 1] <= gp) ++group;
-      const int pass = gp - s_pass_start[group];
+      while (s_pass_start[place + 1] <= gp) ++place;
+      const int group = s_group[place], pass = gp - s_pass_start[place];
       const int row_begin = offsets[group], n_rows = offsets[group + 1] - row_begin;
       const int tiles_here = (PAIR && ft0 + 1 < n_ftiles) ? 2 : 1;      // accumulators of this item to drain
       {

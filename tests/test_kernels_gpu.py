@@ -741,6 +741,35 @@ def test_grouped_gemm_on_tensor_cores(K, T, H, I, E, k):
     assert K.tensor_core_status() == 0
 
 
+@pytest.mark.parametrize("T,E,k", [(300, 1, 1), (517, 60, 4), (450, 448, 3), (450, 449, 3)])
+def test_grouped_gemm_walks_experts_by_falling_rows(K, T, E, k):
+    """Experts of very unequal numbers of rows, in an order that is neither rising nor falling; as
+    many as one thread a group can rank and one more, from where they are taken as they come;
+    more items than CTAs, so that later rounds are dealt backwards."""
+    dtype, H, I = torch.bfloat16, 192, 264
+    g = torch.Generator().manual_seed(T + E)
+    x = rnd((T, H), dtype, 61)
+    w13, w2 = rnd((E, 2 * I, H), dtype, 62, 0.1), rnd((E, H, I), dtype, 63, 0.1)
+    load = 1.0 / (1 + torch.arange(E, dtype=torch.float32)[torch.randperm(E, generator=g)])
+    idx = torch.multinomial(load.expand(T, E), k, generator=g).to(torch.int32).cuda()
+    plan = K.moe_plan(idx, E)
+    old = dict(K.TUNING)
+    lib = K.load()
+    try:
+        K.TUNING.update(bf16_moe="simt", skinny_moe_max_tokens=0)
+        ract = K.moe_gemm1(x, w13, plan, k)
+        ry = K.moe_gemm2(ract, w2, plan)
+        pw13, pw2 = K.pack_weights(w13, swiglu=True), K.pack_weights(w2, swiglu=False)
+        close(K.moe_gemm1(x, pw13, plan, k), ract, dtype)
+        for pair in (0, 1):
+            lib.nf_set_grouped_gemm_pair(pair, 1)
+            close(K.moe_gemm2(ract, pw2, plan), ry, dtype)
+    finally:
+        lib.nf_set_grouped_gemm_pair(1, 64)
+        K.TUNING.update(old)
+    assert K.tensor_core_status() == 0
+
+
 @pytest.mark.parametrize("T,H,I,E,k", [(1, 256, 128, 4, 2), (5, 200, 136, 6, 3), (8, 2048, 1408, 60, 4),
                                        (13, 512, 264, 7, 2), (3, 40, 24, 3, 1)])
 def test_streaming_experts_with_an_early_start(K, T, H, I, E, k):
