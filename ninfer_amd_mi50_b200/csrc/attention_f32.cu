@@ -5,7 +5,7 @@
 //
 // What bounds it: nothing but the way the keys reach the multiply-add units.  With one warp a row and head, every row
 // fetched all keys for itself, 32 lanes from 32 rows of memory: 308 us for 256 rows of 16 heads of 128 over 257 keys
-// (0.27 GFLOP, 4 us at the pipes' rate).  Here a CTA takes up to 16 queries that see the same keys (rows of a segment
+// (0.27 GFLOP, 4 us at the pipes' rate), now 60; four single rows over 257 keys 185, now 19.  Here a CTA takes up to 16 queries that see the same keys (rows of a segment
 // times the heads of a key head), and brings 64 or 128 keys and values to shared memory once for all of them, the
 // next keys while the softmax and the values are worked on, the next values while the scores are.
 //   scores   a lane a key, a warp a block of 32 keys and a share of the queries: a 16-byte piece of the key's row

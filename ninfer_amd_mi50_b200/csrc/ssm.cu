@@ -418,8 +418,8 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ldx, int x_col0, int b_col0, int 
 // nobody to meet.  A warp owns CP columns of one request's head, with all their states asked for before the wait (the
 // request's own, last written a step ago or, where a model runs a layer twice in a step, before the projection that feeds
 // this kernel), and B and C straight into the registers of the lanes that hold their states.  Same sums in the same order
-// as above.  (8 requests of 64 heads of 64 x 128, 33 MB: 21 us with the kernel above, whose 1,024 CTAs of 20 KB of shared
-// memory came in two rounds of load, barrier, sixteen tokens' worth of reductions and barrier.)
+// as above.  (8 requests of 64 heads of 64 x 128, 33 MB: 18.3 us with the kernel above, whose 1,024 CTAs of 20 KB of shared
+// memory came in two rounds of load, barrier, sixteen tokens' worth of reductions and barrier; now 8.5.  32 requests: 63, now 27.)
 template <typename T, int NPER, int CP>
 __global__ void __launch_bounds__(kScanThreads, NPER <= 4 ? 4 : 3)
 ssd_scan_row_kernel(const T* __restrict__ xbc, int ldx, int x_col0, int b_col0, int c_col0,

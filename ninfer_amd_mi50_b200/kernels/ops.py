@@ -646,7 +646,8 @@ def _plain_attention(q, Hq, Hkv, D, pages, block_table, page_size, ctx, window, 
     """The kernels that sum in float32 on CUDA cores: in float32 one whose CTAs share the keys among the rows of a
     segment, where rows are whole 16-byte pieces; else one warp a row and head.  Same sums in both."""
     T = q.shape[0]
-    if q.dtype == torch.float32 and D % 4 == 0 and D <= 256 and pages.data_ptr() % 16 == 0 and hasattr(ctx, "seg_row0"):
+    if (q.dtype == torch.float32 and D % 4 == 0 and D <= 256 and q.shape[1] % 4 == 0 and q.data_ptr() % 16 == 0
+            and pages.data_ptr() % 16 == 0 and hasattr(ctx, "seg_row0")):
         _lib.call("nf_paged_attention_f32", _p(q), c_int(q.shape[1]), _p(pages), _p(block_table), c_int(block_table.shape[1]),
                   _p(ctx.positions), _p(ctx.row_seg), _p(ctx.seg_row0), c_int(ctx.seg_row0.shape[0] - 1),
                   c_int(ctx.max_rows_per_seg), _p(out), c_int(T), c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size),
@@ -787,10 +788,12 @@ def biased_window_attention(q: torch.Tensor, Hq: int, Hkv: int, D: int, pages: t
                     _decode_attention(q, Hq, Hkv, D, pages, block_table, page_size, ctx, window, scale, out, rows, n_single,
                                       sigmoid_bias=sigmoid_bias)
                 singles = None
-            elif sigmoid_bias is None and D in DECODE_HEAD_DIMS:
+            elif (sigmoid_bias is None and D in DECODE_HEAD_DIMS and Hq <= 128 * Hkv
+                  and (n := int(_lib.load().nf_decode_attention_biased_splits(c_int(window), c_int(keep), c_int(int(ctx.max_context)))))
+                  <= DECODE_MAX_SPLITS):
+                # (more key blocks than a merge takes, or more heads a key head than its CTA holds: the shares below)
                 rows, n_single = (None, T) if ctx.all_single else ctx.single_rows()
                 if n_single:
-                    n = int(_lib.load().nf_decode_attention_biased_splits(c_int(window), c_int(keep), c_int(int(ctx.max_context))))
                     ws_acc = torch.empty((n_single, Hq, n, D), dtype=torch.float32, device=q.device)
                     ws_ml = torch.empty((n_single, Hq, n, 2), dtype=torch.float32, device=q.device)
                     _lib.call("nf_decode_attention_biased", _p(q), c_int(q.shape[1]), _p(pages), _p(block_table),

@@ -148,6 +148,22 @@ def test_biased_attention_of_single_rows(K, Hq, Hkv, D, page, window, keep, mixe
     K.check_status()
 
 
+@pytest.mark.parametrize("blocks,Hq,Hkv", [(1024, 4, 2), (1025, 4, 2), (16, 136, 1)])
+def test_biased_attention_of_single_rows_where_a_merge_ends(K, blocks, Hq, Hkv):
+    """A step whose context bound is as many key blocks as a merge takes, one more, and a key head of more
+    query heads than the split kernel is given: answered all the same."""
+    D, page = 64, 16
+    pages, bt, ctx, positions, row_seg, g = make_step(torch.bfloat16, [1, 1, 1], [0, 300, 1151], Hkv, D, page, 11)
+    ctx = replace(ctx, max_context=blocks * 128, _tiles={})
+    q = torch.randn((ctx.T, Hq * D), generator=g).bfloat16().cuda()
+    slopes = torch.tensor([0.05 / (i + 1) for i in range(Hq)]).cuda()
+    gate = torch.randn((ctx.T, Hq), generator=g).cuda()
+    out = K.biased_window_attention(q, Hq, Hkv, D, pages, bt, page, ctx, 0, 0, D ** -0.5, slopes, gate, 0)
+    want = exact_attention(q.view(ctx.T, Hq, D), pages, bt, positions, row_seg, Hq, page, 0, 0, D ** -0.5, slopes, gate)
+    assert (out.view(ctx.T, Hq, D) - want).abs().max() <= 2 ** -8 * 4.5      # (the bound of the test above)
+    K.check_status()
+
+
 @pytest.mark.parametrize("heads,P,N,groups", [(8, 64, 128, 2), (6, 20, 64, 3), (3, 7, 16, 1), (4, 33, 200, 4), (2, 64, 256, 1)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_scan_of_single_rows_has_the_walking_kernels_bits(K, heads, P, N, groups, dtype):
