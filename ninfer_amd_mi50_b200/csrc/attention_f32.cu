@@ -1,20 +1,31 @@
-// Causal grouped-query attention over the paged cache in float32: the all-32-bit path's, with the options, the
-// mathematics and the sums of paged_attention_generic_kernel (attention_generic.cu).  Scores are one chain of products
+// Causal grouped-query attention over the paged cache in float32: the all-32-bit path's, with the options and the
+// mathematics of paged_attention_generic_kernel (attention_generic.cu).  Scores are one chain of products
 // over the head size, keys are taken in blocks of 32 that begin at multiples of 32, in ascending order, and a block's
-// values are added one key after the other; so a row's bits depend on its own position alone, however the step was cut.
+// values are added one key after the other; so a row's bits depend on its own position alone, however the step was cut,
+// and are the same in every form below.  (The other kernel's blocks begin at a window's first key, and the kept first
+// keys are a run of their own there: the same bits in both where no window passes a key, roundings apart where one does.)
 //
 // What bounds it: nothing but the way the keys reach the multiply-add units.  With one warp a row and head, every row
 // fetched all keys for itself, 32 lanes from 32 rows of memory: 308 us for 256 rows of 16 heads of 128 over 257 keys
-// (0.27 GFLOP, 4 us at the pipes' rate), now 60; four single rows over 257 keys 185, now 19.  Here a CTA takes up to 16 queries that see the same keys (rows of a segment
-// times the heads of a key head), and brings 64 or 128 keys and values to shared memory once for all of them, the
-// next keys while the softmax and the values are worked on, the next values while the scores are.
+// (0.27 GFLOP, 4 us at the pipes' rate), now 49; four single rows over 257 keys 139, now 18.  Here a CTA takes up to 8
+// queries that see the same keys (rows of a segment times the heads of a key head; 16 with more than 8 heads a key head),
+// and brings 32, 64 or 128 keys and values to shared memory once for all of them, the next keys while the softmax and the
+// values are worked on, the next values while the scores are.
 //   scores   a lane a key, a warp a block of 32 keys and a share of the queries: a 16-byte piece of the key's row
 //            against the same piece of each query's (a broadcast); rows lie D + 4 floats apart, so that eight lanes'
 //            pieces meet no bank conflict
 //   softmax  a warp a query, its blocks one after the other
 //   values   a thread a dimension (two for heads beyond 128), every query's sum in a register
-// Steps of single rows take the smallest form that holds a key head's query heads, and four blocks at a time: there the
-// chain from key to key is what counts.
+// Steps of single rows take forms of 1, 2 or 4 queries.  With few CTAs the chain from key to key is what counts, and four
+// blocks at a time are the fastest; but that is one CTA a SM at heads of 128, and more CTAs come in rounds: the form is
+// the one of most blocks whose CTAs all find room (af_blocks).  A tile whose keys are one block has all warps fetch and
+// score it.  us, heads of 128, four blocks at a time always / now / one warp a row and head (attention_generic.cu):
+//   64 rows of 16 heads (16 key heads)    8 keys 52.4 / 10.4 / 9.7,  100 69 / 30 / 115,   1,024 330 / 245 / 1,197
+//   32 rows of 16 heads                   8 keys 29.9 / 5.7 / 9.4,   100 35 / 16 / 59,    1,024 188 / 105 / 1,205
+//   4 rows of 16 heads                    8 keys 8.1 / 5.1 / 9.0,    100 9.4 / 9.3 / 57,  1,024 46 / 47 / 582
+//   4 rows of 28 heads (4 key heads)      8 keys 13.2 / 5.7 / 9.2,   100 28 / 14 / 58,    1,024 192 / 97 / 537
+//   256 rows of 28 heads                  257 keys 142 / 67 / 246;   96 rows of 32 prompts of 2 and 4 tokens 19.8 / 8.8 / 8.6
+// Where it is still behind one warp a row: more than 888 CTAs (six a SM) of requests of fewer than ten tokens.
 #define NF_CHAIN_CLASS 8
 #include "common.cuh"
 
@@ -46,10 +57,16 @@ constexpr size_t af_floats(int D) {
   return (size_t)KB * 32 * (D + 4) + (size_t)KB * 32 * D + (size_t)Q * D + (size_t)Q * KB * 32 + (size_t)Q * KB;
 }
 
+// What a CTA works on: rows row0.. of one segment, `heads` query heads of a key head from head0 on.  Query x: row
+// row0 + x / heads, head head0 + x % heads.
+struct AfTile {
+  const int* bt;
+  int row0, rows, head0, heads, kvh, pos_most, pos_least;
+};
+
 // DP: the head size rounded up (32, 64, 128, 256)
 template <int Q, int KB, int DP>
-__global__ void __launch_bounds__(kAfThreads)
-paged_attention_f32_kernel(const AfArgs args) {
+__device__ __forceinline__ void af_tile(const AfArgs& a, const AfTile& t, float* af_smem, int* q_pos, int* q_lo, float* q_slope) {
   constexpr int NW = kAfThreads / 32;
   constexpr int KT = KB * 32;                               // keys at a time
   constexpr int SHARES = NW / KB;                           // warps that share a block of keys, each with its queries
@@ -60,10 +77,6 @@ paged_attention_f32_kernel(const AfArgs args) {
   constexpr int QW = (Q + NW - 1) / NW;                     // queries whose softmax a warp keeps
   constexpr int RW = KT / NW;                               // key rows a warp fetches
   constexpr int LR = DP / 4 < 32 ? DP / 4 : 32;             // lanes a row
-  extern __shared__ __align__(16) float af_smem[];
-  __shared__ int q_pos[Q], q_lo[Q];
-  __shared__ float q_slope[Q];
-  AfArgs a = args;
   const int D = a.D, DK = D + 4;
   float* const ks = af_smem;                                // [KT][D + 4]
   float* const vs = ks + (size_t)KT * DK;                   // [KT][D]
@@ -71,46 +84,10 @@ paged_attention_f32_kernel(const AfArgs args) {
   float* const ps = qs + (size_t)Q * D;                     // [Q][KT] scores, then weights; a weight below 0: not seen
   float* const as = ps + (size_t)Q * KT;                    // [KB][Q] what a block scales the sums before it by
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  chain_wait(a.qkv, a.pages, a.gate, a.block_table, a.positions, a.row_seg, a.seg_row0);
-
-  // which rows: the tile-th run of rows_tile rows of a segment
-  int seg, row0, rows;
-  if (a.rows_tile == 1) {
-    row0 = blockIdx.x, rows = 1;
-    seg = a.row_seg[row0];
-  } else {
-    int left = blockIdx.x;
-    seg = -1;
-    for (int s0 = 0; s0 < a.S; s0 += 32) {
-      const int s = s0 + lane;
-      const int own = s < a.S ? (a.seg_row0[s + 1] - a.seg_row0[s] + a.rows_tile - 1) / a.rows_tile : 0;
-      int upto = own;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += v;
-      }
-      const unsigned past = __ballot_sync(0xffffffffu, upto > left);
-      if (past) {
-        const int at = __ffs(past) - 1;
-        left -= __shfl_sync(0xffffffffu, upto - own, at);
-        seg = s0 + at;
-        break;
-      }
-      left -= __shfl_sync(0xffffffffu, upto, 31);
-    }
-    if (seg < 0) return;                                    // the grid is an upper bound
-    row0 = a.seg_row0[seg] + left * a.rows_tile;
-    rows = min(a.rows_tile, a.seg_row0[seg + 1] - row0);
-    seg = a.row_seg[row0];
-  }
-  const int kvh = blockIdx.y / a.head_tiles, group = a.Hq / a.Hkv;
-  const int head0 = kvh * group + (blockIdx.y % a.head_tiles) * a.heads_tile;
-  const int heads = min(a.heads_tile, (kvh + 1) * group - head0);
-  const int nq = rows * heads;                              // query x: row row0 + x / heads, head head0 + x % heads
-  const int* bt = a.block_table + (size_t)seg * a.bt_width;
+  const int row0 = t.row0, head0 = t.head0, heads = t.heads, nq = t.rows * t.heads, pos_most = t.pos_most, pos_least = t.pos_least;
+  const int* const bt = t.bt;
   const size_t head_stride = (size_t)a.page_size * D, page_stride = (size_t)2 * a.Hkv * head_stride;
-  const float* const kv_head = a.pages + (size_t)kvh * head_stride;
+  const float* const kv_head = a.pages + (size_t)t.kvh * head_stride;
 
   for (int x = warp; x < nq; x += NW) {
     const float* q = a.qkv + (size_t)(row0 + x / heads) * a.q_row_stride + (size_t)(head0 + x % heads) * D;
@@ -121,11 +98,6 @@ paged_attention_f32_kernel(const AfArgs args) {
     q_pos[tid] = p;
     q_lo[tid] = a.window > 0 ? max(0, p - a.window + 1) : 0;
     q_slope[tid] = a.slopes ? a.slopes[head0 + tid % heads] : 0.f;
-  }
-  int pos_most = -1, pos_least = 0x7fffffff;
-  for (int r = 0; r < rows; ++r) {
-    const int p = a.positions[row0 + r];
-    pos_most = max(pos_most, p), pos_least = min(pos_least, p);
   }
   const int lo_least = a.window > 0 ? max(0, pos_least - a.window + 1) : 0;
   const int lo_most = a.window > 0 ? max(0, pos_most - a.window + 1) : 0;
@@ -278,8 +250,9 @@ paged_attention_f32_kernel(const AfArgs args) {
 #pragma unroll 1
       for (int b = 0; b < KB; ++b) {
         if (j0 + b * 32 > pos_most) break;
-        // are all these keys seen by all queries?  Otherwise a weight below 0 leaves its value out.
-        const bool all = j0 + b * 32 + 31 <= pos_least && j0 + b * 32 >= lo_most && nq == Q;
+        // are all these keys seen by all queries of a whole tile?  Otherwise a weight below 0 leaves its value out.
+        const int live = min(32, pos_most + 1 - (j0 + b * 32));
+        const bool all = j0 + b * 32 + 31 <= pos_least && j0 + b * 32 >= lo_most && nq == a.rows_tile * a.heads_tile;
 #pragma unroll
         for (int x = 0; x < QV; ++x)
           if (vq0 + x < nq) {
@@ -288,7 +261,7 @@ paged_attention_f32_kernel(const AfArgs args) {
             for (int i = 0; i < DI; ++i) acc[i][x] *= alpha;
           }
 #pragma unroll(QV > 8 ? 1 : 2)
-        for (int r = 0; r < 32; r += 4) {
+        for (int r = 0; r < live; r += 4) {
           const float* v = vs + (size_t)(b * 32 + r) * D + vd;
           float vv[DI][4];
 #pragma unroll
@@ -352,6 +325,59 @@ paged_attention_f32_kernel(const AfArgs args) {
 }
 
 template <int Q, int KB, int DP>
+__global__ void __launch_bounds__(kAfThreads)
+paged_attention_f32_kernel(const AfArgs args) {
+  extern __shared__ __align__(16) float af_smem[];
+  __shared__ int q_pos[Q], q_lo[Q];
+  __shared__ float q_slope[Q];
+  AfArgs a = args;
+  const int lane = threadIdx.x & 31;
+  chain_wait(a.qkv, a.pages, a.gate, a.block_table, a.positions, a.row_seg, a.seg_row0);
+
+  // which rows: the tile-th run of rows_tile rows of a segment
+  AfTile t;
+  if (a.rows_tile == 1) {
+    t.row0 = blockIdx.x, t.rows = 1;
+  } else {
+    int left = blockIdx.x;
+    t.rows = 0;
+    for (int s0 = 0; s0 < a.S; s0 += 32) {
+      const int s = s0 + lane;
+      const int begin = s < a.S ? a.seg_row0[s] : 0, own_rows = s < a.S ? a.seg_row0[s + 1] - begin : 0;
+      const int own = (own_rows + a.rows_tile - 1) / a.rows_tile;
+      int upto = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const unsigned past = __ballot_sync(0xffffffffu, upto > left);
+      if (past) {
+        const int at = __ffs(past) - 1;
+        left = (left - __shfl_sync(0xffffffffu, upto - own, at)) * a.rows_tile;
+        t.row0 = __shfl_sync(0xffffffffu, begin, at) + left;
+        t.rows = min(a.rows_tile, __shfl_sync(0xffffffffu, own_rows, at) - left);
+        break;
+      }
+      left -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (t.rows == 0) return;                                // the grid is an upper bound
+  }
+  const int group = a.Hq / a.Hkv;
+  t.kvh = blockIdx.y / a.head_tiles;
+  t.head0 = t.kvh * group + (blockIdx.y % a.head_tiles) * a.heads_tile;
+  t.heads = min(a.heads_tile, (t.kvh + 1) * group - t.head0);
+  t.bt = a.block_table + (size_t)a.row_seg[t.row0] * a.bt_width;
+  static_assert(Q <= 32, "a lane a row");
+  const int p = a.positions[t.row0 + (lane < t.rows ? lane : 0)];
+  t.pos_most = __reduce_max_sync(0xffffffffu, p);
+  t.pos_least = __reduce_min_sync(0xffffffffu, p);
+  // a tile whose keys are one block has it fetched and scored by all warps
+  if (KB > 1 && t.pos_most < 32) af_tile<Q, 1, DP>(a, t, af_smem, q_pos, q_lo, q_slope);
+  else af_tile<Q, KB, DP>(a, t, af_smem, q_pos, q_lo, q_slope);
+}
+
+template <int Q, int KB, int DP>
 int af_launch(AfArgs a, int row_tiles, cudaStream_t stream) {
   const size_t smem = af_floats<Q, KB>(a.D) * sizeof(float);
   static const cudaError_t e = cudaFuncSetAttribute(paged_attention_f32_kernel<Q, KB, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -361,12 +387,30 @@ int af_launch(AfArgs a, int row_tiles, cudaStream_t stream) {
   return check_launch("paged_attention_f32");
 }
 
+// CTAs of this form that a SM holds beside one another: by their shared memory (228 KB, 1 KB of it taken by each CTA), and
+// by their registers six
+template <int Q, int KB>
+int af_resident(int D) {
+  const int fit = (int)(228 * 1024 / (af_floats<Q, KB>(D) * sizeof(float) + 1024));
+  return fit < 6 ? fit : 6;
+}
+
 template <int Q, int KB>
 int af_heads(const AfArgs& a, int row_tiles, cudaStream_t stream) {
   if (a.D <= 32) return af_launch<Q, KB, 32>(a, row_tiles, stream);
   if (a.D <= 64) return af_launch<Q, KB, 64>(a, row_tiles, stream);
   if (a.D <= 128) return af_launch<Q, KB, 128>(a, row_tiles, stream);
-  return af_launch<Q, 2, 256>(a, row_tiles, stream);       // four blocks of such rows do not fit
+  return af_launch<Q, (KB < 2 ? KB : 2), 256>(a, row_tiles, stream);       // four blocks of such rows do not fit
+}
+
+// The form of most blocks at a time (up to MOST) whose CTAs all lie beside one another; figures at the top.  (Four queries
+// of more than 64 dimensions gain nothing from four blocks: 4 rows of 28 heads over 1,024 keys 87 us with two, 88 with four.)
+template <int Q, int MOST>
+int af_blocks(const AfArgs& a, int row_tiles, cudaStream_t stream) {
+  const long long ctas = (long long)row_tiles * a.Hkv * a.head_tiles;
+  if (MOST >= 4 && ctas <= 148ll * af_resident<Q, 4>(a.D)) return af_heads<Q, (MOST >= 4 ? 4 : 1)>(a, row_tiles, stream);
+  if (ctas <= 148ll * af_resident<Q, 2>(a.D)) return af_heads<Q, 2>(a, row_tiles, stream);
+  return af_heads<Q, 1>(a, row_tiles, stream);
 }
 
 }  // namespace
@@ -387,14 +431,15 @@ extern "C" int nf_paged_attention_f32(const float* qkv, int q_row_stride, const 
   AfArgs a{qkv, pages, block_table, positions, row_seg, seg_row0, out, slopes, gate, sig_bias, q_row_stride, bt_width, T, S, Hq,
            Hkv, D, page_size, num_pages, window, window > 0 ? keep_first : 0, gate_ld, 0, 0, 0, scale, softcap};
   const int group = Hq / Hkv;
-  const int q = max_rows > 1 || group > 4 ? 16 : group > 2 ? 4 : group;
+  const int q = max_rows > 1 ? (group > 8 ? 16 : 8) : group > 2 ? 4 : group;
   a.heads_tile = group < q ? group : q;
   a.rows_tile = max_rows > 1 ? q / a.heads_tile : 1;
   a.head_tiles = (group + a.heads_tile - 1) / a.heads_tile;
   NF_REQUIRE((long long)Hkv * a.head_tiles <= 65535, "attention: too many heads (%d)", Hq);
   const long long tiles = a.rows_tile == 1 ? T : (long long)T / a.rows_tile + S < T ? T / a.rows_tile + S : T;
-  if (q == 16) return af_heads<16, 2>(a, (int)tiles, stream);
-  if (q == 4) return af_heads<4, 4>(a, (int)tiles, stream);
-  if (q == 2) return af_heads<2, 4>(a, (int)tiles, stream);
-  return af_heads<1, 4>(a, (int)tiles, stream);
+  if (q == 16) return af_blocks<16, 2>(a, (int)tiles, stream);
+  if (q == 8) return af_blocks<8, 2>(a, (int)tiles, stream);
+  if (q == 4) return D <= 64 ? af_blocks<4, 4>(a, (int)tiles, stream) : af_blocks<4, 2>(a, (int)tiles, stream);
+  if (q == 2) return af_blocks<2, 4>(a, (int)tiles, stream);
+  return af_blocks<1, 4>(a, (int)tiles, stream);
 }

@@ -644,9 +644,10 @@ def paged_attention(qkv: torch.Tensor, Hq: int, Hkv: int, D: int, pages: torch.T
 def _plain_attention(q, Hq, Hkv, D, pages, block_table, page_size, ctx, window, scale, out, slopes=None, keep=0, gate_p=None,
                      gate_ld=0, sigmoid_bias=None, softcap=0.0) -> None:
     """The kernels that sum in float32 on CUDA cores: in float32 one whose CTAs share the keys among the rows of a
-    segment, where rows are whole 16-byte pieces; else one warp a row and head.  Same sums in both."""
+    segment, where rows are whole 16-byte pieces and the step says which rows are a segment's; else one warp a row and head.
+    The same bits in both where no window passes a key (attention_f32.cu says why not where one does)."""
     T = q.shape[0]
-    if (q.dtype == torch.float32 and D % 4 == 0 and D <= 256 and q.shape[1] % 4 == 0 and q.data_ptr() % 16 == 0
+    if (q.dtype == torch.float32 and D % 4 == 0 and D <= 256 and Hq <= 65535 and q.shape[1] % 4 == 0 and q.data_ptr() % 16 == 0
             and pages.data_ptr() % 16 == 0 and hasattr(ctx, "seg_row0")):
         _lib.call("nf_paged_attention_f32", _p(q), c_int(q.shape[1]), _p(pages), _p(block_table), c_int(block_table.shape[1]),
                   _p(ctx.positions), _p(ctx.row_seg), _p(ctx.seg_row0), c_int(ctx.seg_row0.shape[0] - 1),

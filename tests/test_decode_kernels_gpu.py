@@ -116,6 +116,55 @@ def test_float32_attention_that_shares_keys(K, Hq, Hkv, D, page, lens, pos0s, fo
         at += n
 
 
+@pytest.mark.parametrize("Hq,Hkv,D", [(16, 16, 128), (28, 4, 128), (6, 2, 64), (16, 1, 32), (8, 8, 256), (4, 2, 64)])
+@pytest.mark.parametrize("lens", [[1] * 9, [1] * 33, [1] * 70, [1, 2, 3, 9] * 8 + [4], [8, 1, 9] * 23 + [1], [17, 16]])
+@pytest.mark.parametrize("window,keep", [(0, 0), (40, 3)])
+def test_float32_attention_of_many_segments(K, Hq, Hkv, D, lens, window, keep):
+    """More segments than a warp looks over at once, of a run of rows, one less and one more; steps whose CTAs fit the device
+    with four, two and one block of keys at a time, and tiles whose keys are one block beside others.  Against 64 bits and,
+    where no window passes a key, the bits of one warp a row."""
+    pos0s = [(0, 3, 31, 32, 33, 95, 96, 150)[(5 * s) % 8] for s in range(len(lens))]
+    pages, bt, ctx, positions, row_seg, g = make_step(torch.float32, lens, pos0s, Hkv, D, 16, 21)
+    q = torch.randn((ctx.T, Hq * D), generator=g).cuda()
+    slopes = torch.tensor([0.3 / (i + 1) for i in range(Hq)]).cuda()
+
+    def run(ctx):
+        return K.biased_window_attention(q, Hq, Hkv, D, pages, bt, 16, ctx, window, keep, D ** -0.5, slopes, None, 0, None)
+    out = run(ctx)
+    want = exact_attention(q.view(ctx.T, Hq, D), pages, bt, positions, row_seg, Hq, 16, window, keep, D ** -0.5, slopes)
+    assert (out.view(ctx.T, Hq, D) - want).abs().max() <= 6e-6 * max(1.0, want.abs().max().item())     # (the bound above)
+    if window == 0:
+        assert torch.equal(out, run(SimpleNamespace(positions=ctx.positions, row_seg=ctx.row_seg)))
+
+
+@pytest.mark.parametrize("rows,Hq,Hkv,D,keys", [(64, 16, 16, 128, 32), (32, 16, 16, 128, 8), (64, 16, 16, 64, 8), (16, 28, 4, 128, 8),
+                                                (64, 28, 4, 128, 8), (8, 32, 2, 128, 8), (64, 8, 8, 256, 16), (64, 16, 16, 128, 257)])
+def test_float32_attention_of_short_rows_is_no_slower_than_one_warp_a_row(K, rows, Hq, Hkv, D, keys):
+    """Single rows of requests with few keys, where CTAs that come in rounds took up to five times as long; 1.3 times is
+    more than any of these differs by from run to run."""
+    pages, bt, ctx, _, _, g = make_step(torch.float32, [1] * rows, [keys - 1] * rows, Hkv, D, 16, 22)
+    qkv = torch.randn((rows, (Hq + 2 * Hkv) * D), generator=g).cuda()
+
+    def timed(ctx):
+        run = lambda: K.paged_attention(qkv, Hq, Hkv, D, pages, bt, 16, ctx, 0, D ** -0.5)
+        run()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                run()
+        times = []
+        for _ in range(7):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+    assert timed(ctx) <= 1.3 * timed(SimpleNamespace(positions=ctx.positions, row_seg=ctx.row_seg))
+
+
 def test_float32_attention_keeps_a_number_that_is_not_finite_behind_its_row(K):
     """Later rows of a segment hold NaN: rows before them see nothing of it."""
     pages, bt, ctx, positions, row_seg, g = make_step(torch.float32, [40], [3], 2, 64, 16, 6)
