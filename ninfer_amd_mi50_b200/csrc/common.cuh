@@ -30,6 +30,7 @@ void note_launch_error(cudaError_t e);
 // For the first kernel after a wait on another stream's event: its dependency is then not the
 // kernel before it in its own stream, and a programmatic edge does not describe it.
 bool take_chain_break();
+void set_chain_break();
 // Whether a launch of class `cls` on `stream` gets the attribute: the class is switched on and no
 // break is pending.  (It used to be given only while the stream was being captured: driven from
 // the host, one decode step in some ten thousand came out different.  That was the stale read

@@ -415,10 +415,12 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ldx, int x_col0, int b_col0, int 
 }
 
 // Steps of single rows: one row's share of the scan is reading and writing the state, so there is nothing to stage and
-// nobody to meet.  A warp owns CP columns of one request's head, with all their states asked for before the wait (the
-// request's own, last written a step ago or, where a model runs a layer twice in a step, before the projection that feeds
-// this kernel), and B and C straight into the registers of the lanes that hold their states.  Same sums in the same order
-// as above.  (8 requests of 64 heads of 64 x 128, 33 MB: 18.3 us with the kernel above, whose 1,024 CTAs of 20 KB of shared
+// nobody to meet.  A warp owns CP columns of one request's head, with all their states asked for before the wait, and B and
+// C straight into the registers of the lanes that hold their states.  Same sums in the same order as above.
+// A state read before the wait must have been written before the kernel that precedes this one in the stream was launched,
+// and that kernel must wait itself and release nobody before its end (the short convolution does): only a caller that says
+// so (`settled`) gets a chained launch; any other gets an ordinary one, which begins when all before it is done.
+// (8 requests of 64 heads of 64 x 128, 33 MB: 18.3 us with the kernel above, whose 1,024 CTAs of 20 KB of shared
 // memory came in two rounds of load, barrier, sixteen tokens' worth of reductions and barrier; now 8.5.  32 requests: 63, now 27.)
 template <typename T, int NPER, int CP>
 __global__ void __launch_bounds__(kScanThreads, NPER <= 4 ? 4 : 3)
@@ -586,16 +588,20 @@ extern "C" int nf_causal_conv_silu(const void* src, int lds, int col0, int C, co
 }
 
 // skip_rows > 0: segments of that many rows or more are left alone.  single != 0: every segment brings one row.
+// settled != 0: the kernel before this one in the stream wrote no part of the states, waited for its own predecessor and
+// releases at its end only.
 extern "C" int nf_ssd_scan(const void* xbc, int ldx, int x_col0, int b_col0, int c_col0, const void* dt_src,
                            int ld_dt, int dt_col0, const float* dt_bias, const float* A_log, const float* Dskip,
                            float* state, long long slot_stride, const int* seg_row0, const int* seg_slot, float* y,
-                           int S, int heads, int P, int N, int groups, int dtype, int skip_rows, int single, cudaStream_t stream) {
+                           int S, int heads, int P, int N, int groups, int dtype, int skip_rows, int single, int settled,
+                           cudaStream_t stream) {
   if (S == 0) return 0;
   if (skip_rows <= 0) skip_rows = 0x7fffffff;
   NF_REQUIRE(heads > 0 && groups > 0 && heads % groups == 0, "ssd_scan: %d heads do not split into %d groups", heads, groups);
   NF_REQUIRE(N > 0 && N <= kScanLanes * kScanMaxPer, "ssd_scan: state size %d (1..%d)", N, kScanLanes * kScanMaxPer);
   NF_REQUIRE(P > 0, "ssd_scan: bad head width");
   if (single && (long long)heads * P <= 65535ll * kScanGroups) {
+    if (!settled) set_chain_break();
     if (dtype == kF32)
       launch_scan_rows<float>(xbc, ldx, x_col0, b_col0, c_col0, dt_src, ld_dt, dt_col0, dt_bias, A_log, Dskip, state, (long)slot_stride, seg_row0, seg_slot, y, S, heads, P, N, groups, stream);
     else

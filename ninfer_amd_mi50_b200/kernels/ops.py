@@ -1759,11 +1759,13 @@ def causal_conv_silu(src: torch.Tensor, col0: int, C: int, taps: torch.Tensor, b
 
 def ssd_scan(xbc: torch.Tensor, x_col0: int, b_col0: int, c_col0: int, dt_src: torch.Tensor, dt_col0: int,
              dt_bias: torch.Tensor, A_log: torch.Tensor, D: torch.Tensor, state: torch.Tensor, state_off: int,
-             ctx, heads: int, P: int, N: int, groups: int) -> torch.Tensor:
+             ctx, heads: int, P: int, N: int, groups: int, state_settled: bool = False) -> torch.Tensor:
     """The selective scan of a step's rows, request by request, from and into each request's
     state (float32 [slots, ...], the [heads, P, N] block starting at element `state_off`):
     S <- exp(-exp(A_log) dt) S + dt B x^T, y = S^T C + D x, dt = softplus(raw + dt_bias).
-    x, B, C are columns of `xbc`, raw dt a column of `dt_src`.  Returns y float32 [T, heads * P]."""
+    x, B, C are columns of `xbc`, raw dt a column of `dt_src`.  Returns y float32 [T, heads * P].
+    `state_settled`: the call before this one on the stream is `causal_conv_silu`, which leaves this block of the states
+    alone; steps of single rows may then read them while that kernel ends.  Without it they are read when all before is done."""
     _chk(xbc, "xbc"); _chk(dt_src, "dt_src", xbc.dtype); _chk(state, "state", torch.float32)
     for t, n in ((dt_bias, "dt_bias"), (A_log, "A_log"), (D, "D")):
         _chk(t, n, torch.float32)
@@ -1786,7 +1788,7 @@ def ssd_scan(xbc: torch.Tensor, x_col0: int, b_col0: int, c_col0: int, dt_src: t
               c_int(dt_src.shape[1]), c_int(dt_col0), _p(dt_bias), _p(A_log), _p(D),
               state_p, c_longlong(state.stride(0)), _p(ctx.seg_row0), _p(ctx.seg_slot), _p(y), c_int(ctx.S), c_int(heads),
               c_int(P), c_int(N), c_int(groups), c_int(_dt(xbc)), c_int(skip_rows),
-              c_int(1 if getattr(ctx, "all_single", False) else 0), _stream())
+              c_int(1 if getattr(ctx, "all_single", False) else 0), c_int(1 if state_settled else 0), _stream())
     return y
 
 

@@ -98,6 +98,7 @@ class StateSpaceDual(Mixer):
         proj = kernels.linear(x, self.w_in)                                     # [T, z | x | B | C | dt]
         xbc = kernels.causal_conv_silu(proj, inner, self.conv_channels, self.conv_w, self.conv_b, state, ctx)
         y = kernels.ssd_scan(xbc, 0, inner, inner + GN, proj, 2 * inner + 2 * GN, self.dt_bias, self.A_log, self.D,
-                             state, self.conv_state, ctx, self.heads, self.head_dim, self.state_size, self.groups)
+                             state, self.conv_state, ctx, self.heads, self.head_dim, self.state_size, self.groups,
+                             state_settled=True)      # (right behind the convolution, which writes its own block alone)
         g = kernels.gated_group_rmsnorm(y, proj, 0, self.norm_w, self.eps, self.norm_groups, x.dtype)
         return kernels.linear(g, self.w_out)

@@ -230,3 +230,28 @@ def test_scan_of_single_rows_has_the_walking_kernels_bits(K, heads, P, N, groups
                        replace(ctx, max_rows_per_seg=bound, _tiles={}), heads, P, N, groups)
         results.append((y, st))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("heads,P,N,groups,rows", [(8, 64, 128, 2, 1), (64, 64, 128, 8, 8), (3, 7, 16, 1, 3)])
+@pytest.mark.parametrize("behind_convolution", [False, True])
+def test_scan_of_single_rows_again_and_again_on_one_state(K, heads, P, N, groups, rows, behind_convolution):
+    """Sixty steps from and into one state with no copy between: by themselves, and behind the convolution of a layer with
+    what its call says.  The bits are those of the kernel that walks rows, which reads the state after its wait."""
+    dtype = torch.bfloat16
+    _, _, ctx, _, _, g = make_step(dtype, [1] * rows, [5] * rows, 1, 16, 16, 9)
+    C, taps = heads * P + 2 * groups * N, 4
+    src = [torch.randn((rows, C), generator=g).to(dtype).cuda() for _ in range(3)]
+    dt = torch.randn((rows, heads), generator=g).to(dtype).cuda()
+    w, b = torch.randn((taps, C), generator=g).cuda(), torch.randn((C,), generator=g).cuda()
+    bias, rate, D = (torch.randn((heads,), generator=g).cuda() for _ in range(3))
+    first = torch.randn((rows, (taps - 1) * C + heads * P * N), generator=g).cuda()
+    results = []
+    for bound in (1, 2):                                      # 2: rows are walked
+        c = replace(ctx, max_rows_per_seg=bound, _tiles={})
+        state, ys = first.clone(), []
+        for i in range(60):
+            xbc = K.causal_conv_silu(src[i % 3], 0, C, w, b, state, ctx) if behind_convolution else src[i % 3]
+            ys.append(K.ssd_scan(xbc, 0, heads * P, heads * P + groups * N, dt, 0, bias, rate, D, state, (taps - 1) * C, c, heads,
+                                 P, N, groups, **({"state_settled": True} if behind_convolution else {})))
+        results.append((torch.stack(ys), state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
