@@ -40,28 +40,65 @@ def context_bucket(n: int, limit: int) -> int:
     return min((n + 511) // 512 * 512, max(limit, 1))
 
 
-STAGES = 16                          # steps of one graph whose index data may be on its way
+STAGES = 16                          # steps whose index data may be on its way, at most ...
+STAGING_BYTES = 32 << 20             # ... and what the buffers of all of them may take, two kept in any case
+
+
+class Staging:
+    """Pinned buffers out of which a runner's graphs send their steps' index data, used in turn, each with the event of its
+    last copy: the host runs ahead of the device on purpose, so the copy out of a buffer may still be queued when the next
+    steps are being prepared; a buffer is rewritten only after its own last copy has finished.  They belong to no graph:
+    each is filled from end to end at every step, and there are no more of them for a service that has passed through many
+    row counts and context bounds.  As many as STAGES steps ahead is what a caller gets that knows its tokens beforehand:
+    the time that decode steps give the host is what it prepares the next prompt's eager step in (with two buffers it waited
+    a step's length at every step: 1.4 of 5.3 ms over four prompts of 2,048 tokens and 12 decode steps).  Generation, which
+    reads every step's tokens, is one step ahead."""
+
+    def __init__(self):
+        self.hosts: List[torch.Tensor] = []
+        self.nps: List[np.ndarray] = []
+        self.views: Dict[int, List[torch.Tensor]] = {}          # their first so many numbers, one entry a row count
+        self.copied: List[Optional[torch.cuda.Event]] = []      # made at the first use, recorded again at every other
+        self.turn = 0
+
+    def fit(self, total: int) -> None:
+        """Buffers of `total` int32 numbers at least, and their views of that many."""
+        if self.hosts and self.hosts[0].numel() >= total:
+            self.views.setdefault(total, [h[:total] for h in self.hosts])
+            return
+        for e in self.copied:
+            if e is not None:
+                e.synchronize()
+        stages = max(2, min(STAGES, STAGING_BYTES // (4 * total)))
+        self.hosts = list(torch.empty((stages, total), dtype=torch.int32).pin_memory().unbind(0))
+        self.nps = [h.numpy() for h in self.hosts]
+        self.views = {n: [h[:n] for h in self.hosts] for n in [*self.views, total]}
+        self.copied, self.turn = [None] * stages, 0
+
+    def take(self) -> int:
+        """The buffer to fill next; waits for the copy that last read it."""
+        i = self.turn % len(self.hosts)
+        self.turn += 1
+        if self.copied[i] is not None:
+            self.copied[i].synchronize()
+        return i
+
+    def send(self, i: int, dev: torch.Tensor) -> None:
+        dev.copy_(self.views[dev.numel()][i], non_blocking=True)
+        if self.copied[i] is None:
+            self.copied[i] = torch.cuda.Event()
+        self.copied[i].record(torch.cuda.current_stream(dev.device))
 
 
 class DecodeGraph:
-    def __init__(self, runner, rows: int, context_bound: int):
-        self.runner, self.S, self.context_bound = runner, rows, context_bound
+    def __init__(self, runner, staging: Staging, rows: int, context_bound: int):
+        self.runner, self.staging, self.S, self.context_bound = runner, staging, rows, context_bound
         cache, dev = runner.cache, runner.device
         S = rows
         self.width = cache.max_pages_per_request
         sizes = [S, S, S, S + 1, S, S, S] + [S * self.width for _ in cache.groups]
-        self.offsets = np.cumsum([0] + sizes)
-        total = int(self.offsets[-1])
-        # Pinned staging buffers used in turn, each with the event of its last copy: the host runs
-        # ahead of the device on purpose, so the copy out of a buffer may still be queued when the
-        # next steps are being prepared; a buffer is rewritten only after its own last copy has
-        # finished.  As many as STAGES steps ahead: the time that decode steps give the host is what
-        # it prepares the next prompt's eager step in (with two buffers it waited a step's length at
-        # every step: 1.4 of 5.3 ms over four prompts of 2,048 tokens and 12 decode steps).
-        self.hosts = list(torch.empty((STAGES, total), dtype=torch.int32).pin_memory().unbind(0))
-        self.nps = [h.numpy() for h in self.hosts]
-        self.copied: List[Optional[torch.cuda.Event]] = [None] * STAGES      # made at the first use, recorded again at every other
-        self.turn = 0
+        self.offsets = np.cumsum([0] + sizes).tolist()
+        total = self.offsets[-1]
         self.dev = torch.zeros((total,), dtype=torch.int32, device=dev)
         parts = [self.dev[self.offsets[i]:self.offsets[i + 1]] for i in range(len(sizes))]
         self.ctx = StepContext(
@@ -71,14 +108,12 @@ class DecodeGraph:
             max_context=context_bound, graph_mode=True)
         for gi, g in enumerate(cache.groups):
             self.ctx.block_tables[g.index] = parts[7 + gi].view(S, self.width)
-        # the parts of the buffer that never change
-        o = self.offsets
-        for a in self.nps:
-            a[o[2]:o[3]] = np.arange(S)
-            a[o[3]:o[4]] = np.arange(S + 1)
-            a[o[6]:o[7]] = np.arange(S)
-            self._fill(a, [], [])
-        self.dev.copy_(self.hosts[0])
+        # a row is its own segment, and its logits are wanted: row_seg, seg_row0 and logit_rows of every step
+        self.counting = np.concatenate([np.arange(S), np.arange(S + 1)]).astype(np.int32)
+        staging.fit(total)
+        i = staging.take()
+        self._fill(staging.nps[i], [], [])
+        staging.send(i, self.dev)
         # warm up on a side stream (library handles, lazily set kernel attributes), then capture
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
@@ -111,6 +146,8 @@ class DecodeGraph:
         a[o[0] + n:o[1]] = 0
         a[o[1]:o[1] + n] = lengths
         a[o[1] + n:o[2]] = 0
+        a[o[2]:o[4]] = self.counting
+        a[o[6]:o[7]] = self.counting[:S]
         a[o[4]:o[4] + n] = lengths
         a[o[4] + n:o[5]] = 0
         a[o[5]:o[5] + n] = [cache.slot(e.req) for e in entries]
@@ -130,15 +167,9 @@ class DecodeGraph:
         device) replace the entries' token ids: the tokens a step before has just drawn, which
         the host has not read yet."""
         lengths = [self.runner.cache.length(e.req) for e in entries]
-        i = self.turn % STAGES
-        self.turn += 1
-        if self.copied[i] is not None:
-            self.copied[i].synchronize()        # the copy that last read this buffer is done
-        self._fill(self.nps[i], entries, lengths)
-        self.dev.copy_(self.hosts[i], non_blocking=True)
-        if self.copied[i] is None:
-            self.copied[i] = torch.cuda.Event()
-        self.copied[i].record(torch.cuda.current_stream(self.dev.device))
+        i = self.staging.take()
+        self._fill(self.staging.nps[i], entries, lengths)
+        self.staging.send(i, self.dev)
         if device_tokens is not None:
             self.dev[self.offsets[0]:self.offsets[0] + len(entries)].copy_(device_tokens)
         self.graph.replay()
@@ -151,6 +182,7 @@ class DecodeGraphs:
 
     def __init__(self, runner, max_rows: int):
         self.runner, self.max_rows = runner, max_rows
+        self.staging = Staging()
         self.graphs: Dict[Tuple[int, int], DecodeGraph] = {}
 
     def eligible(self, entries: Sequence[StepEntry]) -> bool:
@@ -162,5 +194,5 @@ class DecodeGraphs:
         longest = max(cache.length(e.req) for e in entries) + 1
         key = (rows, context_bucket(longest, cache.max_context))
         if key not in self.graphs:
-            self.graphs[key] = DecodeGraph(self.runner, *key)
+            self.graphs[key] = DecodeGraph(self.runner, self.staging, *key)
         return self.graphs[key]

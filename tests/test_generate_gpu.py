@@ -347,3 +347,55 @@ def _replay_and_compare(d, cfg, rows):
     for _ in range(300 if rows < 8 else 100):
         graph.graph.replay()
         assert torch.equal(graph.logits, ref)
+
+
+def _staging_runner(folders, rows, **more):
+    from ninfer_amd_mi50_b200.config import EngineOptions
+    from ninfer_amd_mi50_b200.engine import StepEntry, load_runner
+    d, cfg, _, _ = folders["A"]
+    runner = load_runner(d, options=EngineOptions(dtype="bfloat16", page_size=16, num_sequences=rows, **more))
+    return runner, StepEntry, cfg["vocab_size"]
+
+
+def test_steps_prepared_far_ahead_of_the_device(folders):
+    """More decode steps than there are staging buffers, of two graphs in turn, queued behind a busy device: the logits of
+    steps taken one at a time."""
+    outs = []
+    for waits in (True, False):
+        runner, StepEntry, vocab = _staging_runner(folders, 4, max_context=256, cache_tokens=1024)
+        for r in range(3):
+            runner.open(r)
+            runner.step([StepEntry(r, random_tokens(20 + 7 * r, vocab, 40 + r), [])])
+        for n in (3, 1):                                      # both graphs exist before the device is kept busy
+            runner.step([StepEntry(r, [1], [0]) for r in range(n)])
+        a = torch.randn((8192, 8192), device="cuda")
+        torch.cuda.synchronize()
+        if not waits:
+            for _ in range(30):
+                a @ a
+        got = []
+        for s in range(50):
+            n = 1 if s % 3 == 2 else 3
+            got.append(runner.step([StepEntry(r, [(37 * s + 11 * r) % vocab], [0]) for r in range(n)]).clone())
+            if waits:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        outs.append(got)
+    assert all(torch.equal(x, y) for x, y in zip(*outs))
+
+
+def test_staging_memory_does_not_grow_with_the_graphs(folders):
+    """A service whose context passes one bound after another, with many rows and with few."""
+    pinned = lambda: torch.cuda.memory.host_memory_stats()["allocated_bytes.current"]
+    runner, StepEntry, vocab = _staging_runner(folders, 16, max_context=4096, cache_tokens=16 * 2048)
+    for r in range(16):
+        runner.open(r)
+    before = pinned()
+    sizes = []
+    for bound in range(3):
+        runner.step([StepEntry(0, random_tokens(500, vocab, bound), [])])
+        for n in (16, 5):
+            runner.step([StepEntry(r, [3], [0]) for r in range(n)])
+            sizes.append(pinned() - before)
+    assert len(runner.graphs.graphs) == 6
+    assert sizes[-1] == sizes[0] > 0
