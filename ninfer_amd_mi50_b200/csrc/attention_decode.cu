@@ -20,7 +20,7 @@
 // BIASED: slopes[h] * (pos - j) off a key's score, a window that keeps the request's first keys visible, and a gate a head
 // (in the merge).  A row's blocks are then those of the kept keys that lie before the window's first block, and the
 // window's; the workspace holds these alone, in ascending order, however long the context (a window of 1,024 keys and one
-// row of 16 heads: 20.3 us a layer, now 8.9, while such rows took shares of four blocks of 64 keys of attention_prefill.cu's kernel).
+// row of 16 heads: 8.9 us a layer; as shares of four blocks of 64 keys of attention_prefill.cu's kernel, before, 20.3).
 //
 // Further forms.  SIGMOID: a key weighs sigmoid(score + sig_bias[h]), not normalised over keys - blocks carry the
 // maximum 0 and simply add.  CAPPED: the softmax over cap * tanh(score / cap).  Turned values: the merge turns the first `turn_dims` numbers of a head's result by minus
@@ -618,18 +618,23 @@ static int decode_attention_impl(const void* qkv, int q_row_stride, const void* 
                                  T, Hq, Hkv, D, page_size, num_pages, window, scale, nsplit, row_list, sig_bias, softcap, stream);
   } else
 #define NF_DA_CALL(DD, SG) launch_split<DD, SG>(qkv, q_row_stride, pages, block_table, bt_width, positions, row_seg, ws_acc, ws_ml, T, Hq, Hkv, page_size, num_pages, window, scale, nsplit, counters, out, row_list, sig_bias, softcap, &merged, slopes, keep_first, stream)
-#define NF_DA(DD) case DD: rc = biased ? NF_DA_CALL(DD, kFormBiased) : sig_bias ? NF_DA_CALL(DD, kFormSigmoid) : (softcap > 0.f ? NF_DA_CALL(DD, kFormCapped) : NF_DA_CALL(DD, kFormSoftmax)); break;
+#define NF_DA_PLAIN(DD) (sig_bias ? NF_DA_CALL(DD, kFormSigmoid) : (softcap > 0.f ? NF_DA_CALL(DD, kFormCapped) : NF_DA_CALL(DD, kFormSoftmax)))
+#define NF_DA(DD) case DD: rc = biased ? NF_DA_CALL(DD, kFormBiased) : NF_DA_PLAIN(DD); break;
   switch (D) {
     NF_DA(16)
     NF_DA(32)
     NF_DA(64)
     NF_DA(128)
-    NF_DA(256)
+    case 256:      // (attention with slopes is given to the tensor cores for heads of up to 128 only)
+      NF_REQUIRE(!biased, "decode attention: no biased form for head_dim 256");
+      rc = NF_DA_PLAIN(256);
+      break;
     default:
       set_error("decode attention: head_dim %d is not one of 16, 32, 64, 128, 256", D);
       return 1;
   }
 #undef NF_DA
+#undef NF_DA_PLAIN
 #undef NF_DA_CALL
   if (rc || counters || merged) return rc;      // with counters the split kernel's last CTAs have merged
   dim3 grid(T, Hq);
@@ -701,7 +706,7 @@ extern "C" int nf_decode_attention_biased_splits(int window, int keep_first, int
   return own < all ? own : all;
 }
 
-// The biased form: slopes float32 [Hq] or null; keep_first >= 0 (it counts only with a window); gate float32 [rows, gate_ld]
+// The biased form, head_dim in {16, 32, 64, 128}: slopes float32 [Hq] or null; keep_first >= 0 (it counts only with a window); gate float32 [rows, gate_ld]
 // (column h: head h's gate logit) or null.  nsplit: at least nf_decode_attention_biased_splits() of the longest context.
 extern "C" int nf_decode_attention_biased(const void* qkv, int q_row_stride, const void* pages, const int* block_table,
                                           int bt_width, const int* positions, const int* row_seg, void* out, float* ws_acc,

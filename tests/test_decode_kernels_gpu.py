@@ -1,6 +1,7 @@
 """Kernels of decode steps and of the all-32-bit path at the sizes where they can go wrong: float32 attention that shares
 its keys among a segment's rows, the biased split-key attention of single rows, the scan of single rows."""
 
+import ctypes
 import math
 from dataclasses import replace
 from types import SimpleNamespace
@@ -211,6 +212,24 @@ def test_biased_attention_of_single_rows_where_a_merge_ends(K, blocks, Hq, Hkv):
     want = exact_attention(q.view(ctx.T, Hq, D), pages, bt, positions, row_seg, Hq, page, 0, 0, D ** -0.5, slopes, gate)
     assert (out.view(ctx.T, Hq, D) - want).abs().max() <= 2 ** -8 * 4.5      # (the bound of the test above)
     K.check_status()
+
+
+def test_biased_attention_of_heads_beyond_the_split_kernels_biased_form(K):
+    """Heads of 256 in bfloat16 are answered by one warp a row and head, and no split kernel is built for them."""
+    Hq, Hkv, D, page = 4, 2, 256, 16
+    pages, bt, ctx, positions, row_seg, g = make_step(torch.bfloat16, [1, 1, 1], [0, 130, 300], Hkv, D, page, 13)
+    q = torch.randn((3, Hq * D), generator=g).bfloat16().cuda()
+    slopes = torch.tensor([0.05 / (i + 1) for i in range(Hq)]).cuda()
+    out = K.biased_window_attention(q, Hq, Hkv, D, pages, bt, page, ctx, 100, 4, D ** -0.5, slopes)
+    want = exact_attention(q.view(3, Hq, D), pages, bt, positions, row_seg, Hq, page, 100, 4, D ** -0.5, slopes)
+    assert (out.view(3, Hq, D) - want).abs().max() <= 2 ** -8 * 4.5      # (the bound of the tests above)
+    n, none = ctypes.c_int, None
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    ws = torch.empty((3 * Hq * 3 * (D + 2),), device="cuda")
+    rc = K.load().nf_decode_attention_biased(p(q), n(Hq * D), p(pages), p(bt), n(bt.shape[1]), p(ctx.positions), p(ctx.row_seg), p(out),
+                                             p(ws), p(ws[3 * Hq * 3 * D:]), none, n(3), n(Hq), n(Hkv), n(D), n(page), n(pages.shape[0]),
+                                             n(100), ctypes.c_float(D ** -0.5), n(3), p(slopes), n(4), none, n(0), none)
+    assert rc != 0 and b"256" in K.load().nf_last_error()
 
 
 @pytest.mark.parametrize("heads,P,N,groups", [(8, 64, 128, 2), (6, 20, 64, 3), (3, 7, 16, 1), (4, 33, 200, 4), (2, 64, 256, 1)])
