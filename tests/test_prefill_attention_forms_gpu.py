@@ -80,3 +80,43 @@ def test_biased_form_leaves_out_what_a_page_held_before(D, page, window, monkeyp
             pages[bt[s, e // page], :, :, e % page:] = float("nan")
             pages[bt[s, e // page], :, :, e % page:, ::2] = float("inf")
     assert torch.equal(attend(), want) and want.isfinite().all()
+
+
+@pytest.mark.parametrize("D,page", [(64, 32), (128, 64)])
+@pytest.mark.parametrize("form", ["softmax", "biased"])
+@pytest.mark.parametrize("heights", ["rising", "uneven"])
+def test_reference_maximum_that_rises_block_after_block(D, page, form, heights, monkeypatch):
+    """Scores that outgrow the reference maximum by more than 2^8 in every block of 128 keys, or in two out of three: O is
+    scaled, by a millionth or less, while the product of the block before may still be adding to it."""
+    from ninfer_amd_mi50_b200 import kernels
+    dtype, Hq, Hkv, scale = torch.bfloat16, 4, 2, 1 / math.sqrt(D)
+    seg_lens, pos0s = [129, 300, 128, 257], [0, 723, 896, 40]
+    n_pages = sum((p + n + page - 1) // page for p, n in zip(pos0s, seg_lens)) + 2
+    pages, bt, c, qkv = make_cache_case(dtype, Hq, Hkv, D, page, seg_lens, pos0s, n_pages, 17)
+    slopes = None
+    if form == "biased":
+        slopes = torch.tensor([0.05, 0.12, 0.2, 0.3], device="cuda")      # 9 to 55 powers of two a block
+        if heights == "uneven":
+            slopes = torch.tensor([0.04, 0.044, 0.05, 0.06], device="cuda")      # around the 8 that a maximum is left at
+    else:
+        # the first number of every query undoes the scale: that of a key is what its score has more, 7 (10 powers of two) a block
+        qkv.view(len(qkv), -1, D)[:, :Hq, 0] = math.sqrt(D)
+        step = [0, 7, 14, 8, 22, 30, 29, 45, 60, 61, 70] if heights == "uneven" else [7 * b for b in range(11)]
+        for s, (n, p0) in enumerate(zip(seg_lens, pos0s)):
+            j = torch.arange(p0 + n, device="cuda")
+            pages[bt[s, j // page].long(), 0, :, j % page, 0] = torch.tensor(step, device="cuda").to(dtype)[j // 128][:, None]
+    q = qkv[:, :Hq * D].contiguous()
+
+    def attend(**how):
+        for k, v in how.items():
+            monkeypatch.setitem(kernels.TUNING, k, v)
+        ctx = _step_context(c, seg_lens, pos0s, dtype, 1024)
+        if form == "biased":
+            return kernels.biased_window_attention(q, Hq, Hkv, D, pages, bt, page, ctx, 0, 0, scale, slopes)
+        return kernels.paged_attention(qkv, Hq, Hkv, D, pages, bt, page, ctx, 0, scale)
+
+    out = attend(prefill_attention_tc_min_rows=1, bf16_attention="auto")
+    again = [attend() for _ in range(20)]
+    assert kernels.tensor_core_status() == 0
+    torch.testing.assert_close(out.float(), attend(bf16_attention="generic").float(), **tol(dtype))
+    assert all(torch.equal(o, out) for o in again)
