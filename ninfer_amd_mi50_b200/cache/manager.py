@@ -53,8 +53,8 @@ class RequestEntry:
     reserved: int = 0                      # tokens for which pages are held
     # per group: logical page index -> physical page (-1 once released or never held)
     tables: List[List[int]] = field(default_factory=list)
-    # the same numbers as int32 arrays (a table's length of them count): a decode step copies a request's row of the block
-    # table as it is, instead of turning a list of a hundred numbers into an array every step
+    # the same numbers as rows of int32 arrays that the manager keeps, -1 behind a table's end: a step copies its requests'
+    # rows as they are, instead of turning lists of a hundred numbers into arrays
     rows: List[np.ndarray] = field(default_factory=list)
 
 
@@ -98,6 +98,9 @@ class CacheManager:
                     self.state[layer] = torch.zeros((self.max_requests + 1, *sp.shape), dtype=sp.dtype,
                                                     device=self.device)
         self.requests: Dict[Hashable, RequestEntry] = {}
+        # every slot's rows, kept from request to request: an array made by every open cost a step of 60 prompts of two tokens 75 us
+        self._rows = np.full((len(self.groups), self.max_requests, self.max_pages_per_request), -1, np.int32)
+        self._slot_rows = [list(self._rows[:, s]) for s in range(self.max_requests)]
 
     @property
     def null_slot(self) -> int:
@@ -125,15 +128,15 @@ class CacheManager:
         slot = self._free_slots.pop()
         for slab in self.state.values():
             slab[slot].zero_()
-        self.requests[req] = RequestEntry(slot, tables=[[] for _ in self.groups],
-                                          rows=[np.full(self.max_pages_per_request, -1, np.int32) for _ in self.groups])
+        self.requests[req] = RequestEntry(slot, tables=[[] for _ in self.groups], rows=self._slot_rows[slot])
         return slot
 
     def close(self, req: Hashable) -> None:
         """Give back everything the request holds."""
         ent = self.requests.pop(req)
-        for g, table in zip(self.groups, ent.tables):
+        for g, table, row in zip(self.groups, ent.tables, ent.rows):
             g.pool.give_back([p for p in table if p >= 0])
+            row.fill(-1)
         self._free_slots.append(ent.slot)
 
     def is_open(self, req: Hashable) -> bool:
@@ -187,7 +190,10 @@ class CacheManager:
             first_new = len(table)
             taken, again = g.pool.take_marking_reuse(n)
             table.extend(taken)
-            row[first_new:first_new + n] = taken
+            if n == 1:
+                row[first_new] = taken[0]
+            else:
+                row[first_new:first_new + n] = taken
             if not (again and self.clear_reused_pages and g.pages is not None):
                 continue
             # A page that is handed out again still holds its earlier owner's entries.  Kernels
@@ -228,10 +234,11 @@ class CacheManager:
         """Drop a reservation that was never committed (a step that did not run)."""
         ent = self.requests[req]
         keep = self._pages_for(ent.length)
-        for g, table in zip(self.groups, ent.tables):
+        for g, table, row in zip(self.groups, ent.tables, ent.rows):
             extra = [p for p in table[keep:] if p >= 0]
             g.pool.give_back(extra)
             del table[keep:]
+            row[keep:] = -1
         ent.reserved = ent.length
 
     def block_table(self, group: int, req: Hashable) -> List[int]:
@@ -241,6 +248,10 @@ class CacheManager:
         """The same as an int32 array; a view that the next reservation or commit may change."""
         ent = self.requests[req]
         return ent.rows[group][:len(ent.tables[group])]
+
+    def block_rows(self, group: int, slots: Sequence[int], width: int) -> np.ndarray:
+        """The rows of requests by their slots, int32 [requests, width], -1 behind each table's end."""
+        return self._rows[group][slots, :width]
 
     # ---- what a mixer call sees ------------------------------------------------------
     def view(self, cache_slot: int, block_tables: Dict[int, torch.Tensor], append: bool

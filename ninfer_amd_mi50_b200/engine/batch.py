@@ -88,13 +88,13 @@ def pack_step(entries: Sequence[StepEntry], cache: CacheManager, dtype: torch.dt
     # block tables, one per cache group, padded to a common width with -1
     tables = []
     for g in cache.groups:
-        rows = [cache.block_row(g.index, e.req) for e in entries]
-        width = table_width or max(1, max(len(r) for r in rows))
-        tbl = np.full((S, width), -1, dtype=np.int32)
-        for i, r in enumerate(rows):
-            if len(r) > width:
-                raise BatchError("a block table is wider than the step's table width")
-            tbl[i, :len(r)] = r
+        longest = max(len(cache.block_table(g.index, e.req)) for e in entries)
+        width = table_width or max(1, longest)
+        if longest > width:
+            raise BatchError("a block table is wider than the step's table width")
+        tbl = cache.block_rows(g.index, seg_slot, width)
+        if tbl.shape[1] < width:
+            tbl = np.pad(tbl, ((0, 0), (0, width - tbl.shape[1])), constant_values=-1)
         tables.append((g.index, width, tbl.reshape(-1)))
     sizes = [T, T, T, S + 1, S, S, len(logit_rows)] + [S * w for _, w, _ in tables]
     small = lambda v: np.asarray(v, dtype=np.int32)

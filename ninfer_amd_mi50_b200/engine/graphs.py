@@ -150,14 +150,13 @@ class DecodeGraph:
         a[o[6]:o[7]] = self.counting[:S]
         a[o[4]:o[4] + n] = lengths
         a[o[4] + n:o[5]] = 0
-        a[o[5]:o[5] + n] = [cache.slot(e.req) for e in entries]
+        slots = [cache.slot(e.req) for e in entries]
+        a[o[5]:o[5] + n] = slots
         a[o[5] + n:o[6]] = cache.null_slot
         for gi, g in enumerate(cache.groups):
             tbl = a[o[7 + gi]:o[8 + gi]].reshape(S, self.width)
-            for s, e in enumerate(entries):
-                row = cache.block_row(g.index, e.req)
-                tbl[s, :len(row)] = row
-                tbl[s, len(row):] = -1
+            if n:
+                tbl[:n] = cache.block_rows(g.index, slots, self.width)
             tbl[n:, 0] = g.null_page
             tbl[n:, 1:] = -1
 

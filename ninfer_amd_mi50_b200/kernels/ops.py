@@ -789,21 +789,22 @@ def biased_window_attention(q: torch.Tensor, Hq: int, Hkv: int, D: int, pages: t
                     _decode_attention(q, Hq, Hkv, D, pages, block_table, page_size, ctx, window, scale, out, rows, n_single,
                                       sigmoid_bias=sigmoid_bias)
                 singles = None
-            elif (sigmoid_bias is None and D in DECODE_HEAD_DIMS and Hq <= 128 * Hkv
-                  and (n := int(_lib.load().nf_decode_attention_biased_splits(c_int(window), c_int(keep), c_int(int(ctx.max_context)))))
-                  <= DECODE_MAX_SPLITS):
-                # (more key blocks than a merge takes, or more heads a key head than its CTA holds: the shares below)
+            elif sigmoid_bias is None and D in DECODE_HEAD_DIMS and Hq <= 128 * Hkv:
                 rows, n_single = (None, T) if ctx.all_single else ctx.single_rows()
-                if n_single:
-                    ws_acc = torch.empty((n_single, Hq, n, D), dtype=torch.float32, device=q.device)
-                    ws_ml = torch.empty((n_single, Hq, n, 2), dtype=torch.float32, device=q.device)
-                    _lib.call("nf_decode_attention_biased", _p(q), c_int(q.shape[1]), _p(pages), _p(block_table),
-                              c_int(block_table.shape[1]), _p(ctx.positions), _p(ctx.row_seg), _p(out), _p(ws_acc), _p(ws_ml),
-                              _p(rows), c_int(n_single), c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size),
-                              c_int(pages.shape[0]), c_int(window), c_float(scale), c_int(n), _p(slopes), c_int(keep), gate_p,
-                              c_int(gate_ld), _stream())
                 singles = None
-            else:
+                if n_single:
+                    n = int(_lib.load().nf_decode_attention_biased_splits(c_int(window), c_int(keep), c_int(int(ctx.max_context))))
+                    if n <= DECODE_MAX_SPLITS:
+                        ws_acc = torch.empty((n_single, Hq, n, D), dtype=torch.float32, device=q.device)
+                        ws_ml = torch.empty((n_single, Hq, n, 2), dtype=torch.float32, device=q.device)
+                        _lib.call("nf_decode_attention_biased", _p(q), c_int(q.shape[1]), _p(pages), _p(block_table),
+                                  c_int(block_table.shape[1]), _p(ctx.positions), _p(ctx.row_seg), _p(out), _p(ws_acc), _p(ws_ml),
+                                  _p(rows), c_int(n_single), c_int(Hq), c_int(Hkv), c_int(D), c_int(page_size),
+                                  c_int(pages.shape[0]), c_int(window), c_float(scale), c_int(n), _p(slopes), c_int(keep), gate_p,
+                                  c_int(gate_ld), _stream())
+                    else:                             # more key blocks than a merge takes: the shares below
+                        singles, n_single = ctx.one_row_tiles()
+            else:                                     # (more heads a key head than the split kernel's CTA holds, sizes of no decode kernel)
                 singles, n_single = ctx.one_row_tiles()
             if singles is not None and n_single:
                 flash(singles, n_single, int(_lib.load().nf_prefill_attention_shares(c_int(window), c_int(int(ctx.max_context)))))
