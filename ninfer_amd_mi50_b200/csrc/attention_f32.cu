@@ -45,9 +45,6 @@ struct AfArgs {
   float scale, softcap;
 };
 
-__device__ __forceinline__ void af_cp16(float* dst, const float* src, bool ok) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
 __device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void af_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -124,7 +121,7 @@ __device__ __forceinline__ void af_tile(const AfArgs& a, const AfTile& t, float*
       const float* src = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), r));
 #pragma unroll
       for (int c = c0; c < DP; c += LR * 4)
-        if (c < D) af_cp16(dst + (size_t)(warp * RW + r) * ld + c, src ? src + off + c : a.pages, src != nullptr);
+        if (c < D) cp16_or_zeros(dst + (size_t)(warp * RW + r) * ld + c, src ? src + off + c : a.pages, src != nullptr);
     }
     af_commit();
   };

@@ -173,9 +173,16 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // CTAs of a row-wise kernel with `threads` threads each: one a row as long as they find room beside one another,
 // beyond that as many, which walk the rows with the next one's numbers on their way while one is summed up and written.
 // One CTA a row, 2,048 rows came in two rounds of CTAs, each a trip to memory, two meetings of all warps and a write.
+// The room is an estimate, 1,536 threads (42 registers each) on each of 148 SMs: a kernel that takes more registers has its
+// CTAs come in rounds, of which each walks the fewer rows.
 inline int row_ctas(int rows, int threads) {
   const int room = 148 * (1536 / threads < 1 ? 1 : 1536 / threads);
   return rows <= room ? rows : room;
+}
+
+// 16 bytes to shared memory on their way, zeros where not `ok` (`src` is then not read, but any valid address).
+__device__ __forceinline__ void cp16_or_zeros(float* dst, const float* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
 // 4 consecutive elements as floats, and back.

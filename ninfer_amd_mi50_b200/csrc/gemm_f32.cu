@@ -33,10 +33,6 @@ constexpr size_t kGfL2 = 126u << 20, kGfFar = 230u << 20;    // bytes of a matri
 constexpr int kGfK = 32;                  // k a stage
 constexpr int kGfRow = kGfK + 4;          // floats between two rows of a stage
 
-__device__ __forceinline__ void gf_cp16(float* dst, const float* src, bool ok) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
-
 // UNROLL: fours of k whose reads may be in flight together
 template <int BM, int BN, int TM, int TN, int STAGES, bool GATED, int UNROLL = (BM > 16 ? 2 : 8)>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), BM >= 64 ? 2 : 1)
@@ -79,7 +75,7 @@ gemm_f32_kernel(const float* __restrict__ A, int lda, const float* __restrict__ 
           if (PIECES % NT == 0 || x < PIECES) {
             const int r = x / (kGfK / 4), k = step * kGfK + (x % (kGfK / 4)) * 4;
             const bool ok = src[i] != nullptr && k < K;
-            gf_cp16(st + r * kGfRow + (x % (kGfK / 4)) * 4, ok ? src[i] + k : A, ok);
+            cp16_or_zeros(st + r * kGfRow + (x % (kGfK / 4)) * 4, ok ? src[i] + k : A, ok);
           }
         }
       }

@@ -282,32 +282,32 @@ part_norm_vec_kernel(const TY* __restrict__ y, int ldy, int ycol0, const TZ* __r
   ask(blockIdx.x);
   for (int t = blockIdx.x; t < rows; t += gridDim.x) {
 #pragma unroll
-  for (int c = 0; c < R; ++c)
+    for (int c = 0; c < R; ++c)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) { v[c][e] = vn[c][e]; z[c][e] = zn[c][e]; }
-  if (t + (int)gridDim.x < rows) ask(t + gridDim.x);
-  float ss = 0.f;
+      for (int e = 0; e < 4; ++e) { v[c][e] = vn[c][e]; z[c][e] = zn[c][e]; }
+    if (t + (int)gridDim.x < rows) ask(t + gridDim.x);
+    float ss = 0.f;
 #pragma unroll
-  for (int c = 0; c < R; ++c)
+    for (int c = 0; c < R; ++c)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (MODE) {
-        const float sg = 1.f / (1.f + expf(-z[c][e]));
-        if (MODE == 1) v[c][e] *= z[c][e] * sg;
-        else z[c][e] = MODE == 3 ? sg : z[c][e] * sg;
+      for (int e = 0; e < 4; ++e) {
+        if (MODE) {
+          const float sg = 1.f / (1.f + expf(-z[c][e]));
+          if (MODE == 1) v[c][e] *= z[c][e] * sg;
+          else z[c][e] = MODE == 3 ? sg : z[c][e] * sg;
+        }
+        ss += v[c][e] * v[c][e];
       }
-      ss += v[c][e] * v[c][e];
+    const float inv = rsqrtf(block_sum(ss, red) / (float)n + eps);
+#pragma unroll
+    for (int c = 0; c < R; ++c) {
+      const int i = (c * blockDim.x + threadIdx.x) * 4;
+      if (i >= n) continue;
+      float o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = v[c][e] * inv * wk[c][e] * (MODE >= 2 ? z[c][e] : 1.f);
+      store4(out + (size_t)t * ldo + c0 + i, o);
     }
-  const float inv = rsqrtf(block_sum(ss, red) / (float)n + eps);
-#pragma unroll
-  for (int c = 0; c < R; ++c) {
-    const int i = (c * blockDim.x + threadIdx.x) * 4;
-    if (i >= n) continue;
-    float o[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = v[c][e] * inv * wk[c][e] * (MODE >= 2 ? z[c][e] : 1.f);
-    store4(out + (size_t)t * ldo + c0 + i, o);
-  }
   }
 }
 // Whether rows of `n` numbers at `p` (first column `col0`, `ld` apart, `el` bytes a number) can be moved four at a time.
@@ -670,27 +670,27 @@ scaled_norm_add_regs_kernel(float* __restrict__ h, const TD* __restrict__ delta,
   constexpr bool AHEAD = R < 16;
   if (AHEAD) ask(blockIdx.x);
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-  if (!AHEAD) ask(r);
-  float* hr = h + (size_t)r * hidden;
-  float ss = 0.f;
+    if (!AHEAD) ask(r);
+    float* hr = h + (size_t)r * hidden;
+    float ss = 0.f;
 #pragma unroll
-  for (int c = 0; c < R; ++c) {
-    hk[c] = hn[c];
-    if (c * (int)blockDim.x + (int)threadIdx.x < hidden) {
-      d[c] = to_float(raw[c]) + bk[c];
-      ss = fmaf(d[c], d[c], ss);
+    for (int c = 0; c < R; ++c) {
+      hk[c] = hn[c];
+      if (c * (int)blockDim.x + (int)threadIdx.x < hidden) {
+        d[c] = to_float(raw[c]) + bk[c];
+        ss = fmaf(d[c], d[c], ss);
+      }
     }
-  }
-  if (AHEAD && r + (int)gridDim.x < rows) ask(r + gridDim.x);
-  const float inv = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
+    if (AHEAD && r + (int)gridDim.x < rows) ask(r + gridDim.x);
+    const float inv = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
 #pragma unroll
-  for (int c = 0; c < R; ++c) {
-    const int i = c * blockDim.x + threadIdx.x;
-    if (i >= hidden) continue;
-    const float v = scaled_norm_sum(d[c], inv, wk[c], ls, lk[c], hk[c]);
-    hr[i] = v;
-    if (out) out[(size_t)r * hidden + i] = from_float<TO>(v);
-  }
+    for (int c = 0; c < R; ++c) {
+      const int i = c * blockDim.x + threadIdx.x;
+      if (i >= hidden) continue;
+      const float v = scaled_norm_sum(d[c], inv, wk[c], ls, lk[c], hk[c]);
+      hr[i] = v;
+      if (out) out[(size_t)r * hidden + i] = from_float<TO>(v);
+    }
   }
 }
 

@@ -152,50 +152,51 @@ causal_conv_silu_rows_kernel(const T* __restrict__ src, int lds, int col0, int C
     if (t0 + i < t1) raw[i] = *reinterpret_cast<const uint4*>(src + (size_t)(t0 + i) * lds + col0 + c);
   float u[K][VE];                                  // the last K inputs, oldest first
   int seg = -1;
-  for (int ta = t0; ta < t1; ta += AHEAD)
+  for (int ta = t0; ta < t1; ta += AHEAD) {
 #pragma unroll
-  for (int i = 0; i < AHEAD; ++i) {
-    const int t = ta + i;
-    if (t >= t1) break;
-    const int sg = row_seg[t];
-    if (sg != seg) {                               // a tile's or a request's first row: what came before it
-      seg = sg;
-      const int r0 = seg_row0[sg];
-      const float* st = state + (size_t)seg_slot[sg] * slot_stride;
+    for (int i = 0; i < AHEAD; ++i) {
+      const int t = ta + i;
+      if (t >= t1) break;
+      const int sg = row_seg[t];
+      if (sg != seg) {                               // a tile's or a request's first row: what came before it
+        seg = sg;
+        const int r0 = seg_row0[sg];
+        const float* st = state + (size_t)seg_slot[sg] * slot_stride;
 #pragma unroll
-      for (int j = 1; j < K; ++j) {                // u[j] is the input K - j tokens back (it moves down below)
-        const int r = t - (K - j);
-        if (r >= r0) {
-          load_row(r, u[j]);
-        } else {
-          const int i = (K - 1) - (r0 - r);
+        for (int j = 1; j < K; ++j) {                // u[j] is the input K - j tokens back (it moves down below)
+          const int r = t - (K - j);
+          if (r >= r0) {
+            load_row(r, u[j]);
+          } else {
+            const int i = (K - 1) - (r0 - r);
 #pragma unroll
-          for (int e = 0; e < VE; ++e) u[j][e] = i >= 0 ? st[(size_t)i * C + c + e] : 0.f;
+            for (int e = 0; e < VE; ++e) u[j][e] = i >= 0 ? st[(size_t)i * C + c + e] : 0.f;
+          }
         }
       }
+#pragma unroll
+      for (int j = 0; j + 1 < K; ++j)
+#pragma unroll
+        for (int e = 0; e < VE; ++e) u[j][e] = u[j + 1][e];
+      if (VE == 8) {
+        unpack8(raw[i], u[K - 1]);
+      } else {
+        u[K - 1][0] = __uint_as_float(raw[i].x), u[K - 1][1] = __uint_as_float(raw[i].y);
+        u[K - 1][2] = __uint_as_float(raw[i].z), u[K - 1][3] = __uint_as_float(raw[i].w);
+      }
+      if (t + AHEAD < t1) raw[i] = *reinterpret_cast<const uint4*>(src + (size_t)(t + AHEAD) * lds + col0 + c);
+      float acc[VE];
+#pragma unroll
+      for (int e = 0; e < VE; ++e) {
+        acc[e] = bs[e];
+#pragma unroll
+        for (int j = 0; j < K; ++j) acc[e] = fmaf(w[j][e], u[j][e], acc[e]);
+        acc[e] = acc[e] / (1.f + expf(-acc[e]));
+      }
+      T* o = out + (size_t)t * C + c;
+#pragma unroll
+      for (int e = 0; e < VE; e += 4) store4(o + e, acc + e);
     }
-#pragma unroll
-    for (int j = 0; j + 1 < K; ++j)
-#pragma unroll
-      for (int e = 0; e < VE; ++e) u[j][e] = u[j + 1][e];
-    if (VE == 8) {
-      unpack8(raw[i], u[K - 1]);
-    } else {
-      u[K - 1][0] = __uint_as_float(raw[i].x), u[K - 1][1] = __uint_as_float(raw[i].y);
-      u[K - 1][2] = __uint_as_float(raw[i].z), u[K - 1][3] = __uint_as_float(raw[i].w);
-    }
-    if (t + AHEAD < t1) raw[i] = *reinterpret_cast<const uint4*>(src + (size_t)(t + AHEAD) * lds + col0 + c);
-    float acc[VE];
-#pragma unroll
-    for (int e = 0; e < VE; ++e) {
-      acc[e] = bs[e];
-#pragma unroll
-      for (int j = 0; j < K; ++j) acc[e] = fmaf(w[j][e], u[j][e], acc[e]);
-      acc[e] = acc[e] / (1.f + expf(-acc[e]));
-    }
-    T* o = out + (size_t)t * C + c;
-#pragma unroll
-    for (int e = 0; e < VE; e += 4) store4(o + e, acc + e);
   }
 }
 
