@@ -216,6 +216,12 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
     for (int m = 0; m < 2; ++m)
 #pragma unroll
       for (int i = 0; i < 4; ++i) c[m][i] = 0.f;
+    float slope[2] = {0.f, 0.f};        // of this lane's two heads, on their way during the products
+    if constexpr (BIASED) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (slopes && h0 + 2 * tq + i < G) slope[i] = slopes[kvh * G + h0 + 2 * tq + i];
+    }
     const bool head_ok = h0 + g < G;
     const __nv_bfloat16* qh = qrow + (size_t)(h0 + g) * D;
 #pragma unroll
@@ -244,7 +250,7 @@ decode_attention_split_kernel(const __nv_bfloat16* __restrict__ qkv, int q_row_s
           float v = CAPPED ? cap_score(c[m][i], softcap, in2) : c[m][i] * scale;
           if constexpr (BIASED) {
             const int j = k_base + r;
-            if (slopes) v = fmaf(-slopes[kvh * G + h], (float)(pos - j), v);
+            v = fmaf(-slope[i & 1], (float)(pos - j), v);
             if (j < lo && j >= kept) v = -INFINITY;      // between the kept keys and the window
           }
           sc[h * kSplit + r] = v;
@@ -400,7 +406,9 @@ constexpr int kMaxMergeSplits = 1024;
 constexpr int kMergeRun = 16;        // blocks one thread adds in a row
 // dthreads: threads that share the D dims (a power of two); blockDim.x is a multiple of it.
 // Dynamic shared memory: ceil(nsplit / kMergeRun) * D floats if nsplit > kMergeRun, else none.
-template <typename T>
+// BIASED: the workspace begins with the row's first block, and there may be a gate.  (A branch instead of the form, and the
+// gate's test for everybody: one row at 2,047 keys 8.4 us a layer, with the form 7.7.)
+template <typename T, bool BIASED>
 __global__ void decode_attention_merge_kernel(const float* __restrict__ ws_acc,
                                               const float* __restrict__ ws_ml,
                                               const int* __restrict__ positions, T* __restrict__ out,
@@ -419,14 +427,16 @@ __global__ void decode_attention_merge_kernel(const float* __restrict__ ws_acc,
   const int t = row_list ? row_list[wi] : wi;
   int pos = positions[t], lo;
   int s0 = 0, n;                       // the row's first block in the workspace, and how many it has
-  if (keep_first >= 0) {
+  if constexpr (BIASED) {
     n = min(nsplit, kept_key_range(pos, window, keep_first, kSplit).blocks);
   } else {
     decode_key_range(pos, lo, window, nsplit, kSplit);
     s0 = lo / kSplit;
     n = pos / kSplit - s0 + 1;
   }
-  chain_wait(ws_acc, ws_ml, gate);
+  chain_wait(ws_acc, ws_ml, gate);      // (the gate is null but in the biased form)
+  float gate_logit = 0.f;
+  if (BIASED && gate && threadIdx.x == 0) gate_logit = gate[(size_t)t * gate_ld + h];
   const float* ml = ws_ml + (((size_t)wi * Hq + h) * nsplit + s0) * 2;
   const float* acc = ws_acc + (((size_t)wi * Hq + h) * nsplit + s0) * D;
   // every block's (m, l) in one parallel read; the serial parts below then walk shared memory
@@ -449,7 +459,7 @@ __global__ void decode_attention_merge_kernel(const float* __restrict__ ws_acc,
     float l = 0.f;
     for (int s = 0; s < n; ++s) l += wl[s] * wgt[s];                              // ascending order
     float inv = !normalise ? 1.f : (l > 0.f ? 1.f / l : 0.f);
-    if (gate) inv *= 1.f / (1.f + expf(-gate[(size_t)t * gate_ld + h]));
+    if (BIASED && gate) inv *= 1.f / (1.f + expf(-gate_logit));
     s_inv = inv;
   }
   __syncthreads();
@@ -643,17 +653,20 @@ static int decode_attention_impl(const void* qkv, int q_row_stride, const void* 
   const int max_runs = (nsplit + kMergeRun - 1) / kMergeRun;
   int groups = 1024 / dthreads < max_runs ? 1024 / dthreads : max_runs;
   const size_t smem = max_runs > 1 ? (size_t)max_runs * D * sizeof(float) : 0;
-  static size_t allowed = 48 * 1024;
-  if (smem > allowed) {
-    cudaError_t e = cudaFuncSetAttribute(decode_attention_merge_kernel<__nv_bfloat16>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    NF_REQUIRE(e == cudaSuccess, "decode attention: the merge cannot have %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    allowed = smem;
-  }
-  launch_chained(decode_attention_merge_kernel<__nv_bfloat16>, grid, dim3(dthreads * groups), smem, stream,
-                 (const float*)ws_acc, (const float*)ws_ml, positions, (__nv_bfloat16*)out, Hq, D, window, nsplit,
-                 dthreads, row_list, sig_bias ? 0 : 1, turn_freq, turn_dims, interleaved, keep_first, gate, gate_ld);
-  return check_launch("decode_attention_merge");
+  auto merge = [&](auto kernel, size_t* allowed) -> int {
+    if (smem > *allowed) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      NF_REQUIRE(e == cudaSuccess, "decode attention: the merge cannot have %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+      *allowed = smem;
+    }
+    launch_chained(kernel, grid, dim3(dthreads * groups), smem, stream, (const float*)ws_acc, (const float*)ws_ml, positions,
+                   (__nv_bfloat16*)out, Hq, D, window, nsplit, dthreads, row_list, sig_bias ? 0 : 1, turn_freq, turn_dims,
+                   interleaved, keep_first, gate, gate_ld);
+    return check_launch("decode_attention_merge");
+  };
+  static size_t allowed_plain = 48 * 1024, allowed_biased = 48 * 1024;
+  return biased ? merge(decode_attention_merge_kernel<__nv_bfloat16, true>, &allowed_biased)
+                : merge(decode_attention_merge_kernel<__nv_bfloat16, false>, &allowed_plain);
 }
 
 extern "C" int nf_decode_attention(const void* qkv, int q_row_stride, const void* pages,
