@@ -100,7 +100,7 @@ __global__ void add_layernorm_kernel(float* __restrict__ h, const T* __restrict_
 
 // The same for rows of up to 8,192 numbers in runs of four, all rows in place (no list, no pending sum): the row in
 // registers, rows walked as `row_ctas` gives them out.  Same sums in the same order.
-template <typename T, int R>
+template <typename T, int R, bool WALK>
 __global__ void __launch_bounds__(512)
 add_layernorm_regs_kernel(float* __restrict__ h, const T* __restrict__ delta, const float* __restrict__ w, float eps,
                           T* __restrict__ out, int hidden, int rows) {
@@ -138,7 +138,7 @@ add_layernorm_regs_kernel(float* __restrict__ h, const T* __restrict__ delta, co
       }
       if (delta) store4(h + (size_t)r * hidden + i, v[c]);
     }
-    if (r + (int)gridDim.x < rows) ask(r + gridDim.x);
+    if (WALK && r + (int)gridDim.x < rows) ask(r + gridDim.x);
     const float mean = block_sum(s, red) / (float)hidden;
     float ss = 0.f;
 #pragma unroll
@@ -160,6 +160,7 @@ add_layernorm_regs_kernel(float* __restrict__ h, const T* __restrict__ delta, co
       for (int e = 0; e < 4; ++e) o[e] = (v[c][e] - mean) * rstd * wk[c][e];
       store4(out + (size_t)r * hidden + i, o);
     }
+    if (!WALK) return;
   }
 }
 
@@ -251,41 +252,35 @@ add_group_rmsnorm_kernel(float* __restrict__ h, const T* __restrict__ d1, const 
 // scans and delta rules 10.87 -> 10.55.
 // MODE 0: out = x / rms(x) * w.  1: x = y * silu(z), out = x / rms(x) * w.  2, 3: out = y / rms(y) * w * act(z), act the
 // silu or the sigmoid.  blockIdx.y: the part of the row.
-template <typename TY, typename TZ, typename T, int R, int MODE>
+template <typename TY, typename TZ, typename T, int R, int MODE, bool WALK>
 __global__ void __launch_bounds__(512)
 part_norm_vec_kernel(const TY* __restrict__ y, int ldy, int ycol0, const TZ* __restrict__ zsrc, int ldz, int zcol0,
                      const float* __restrict__ w, float eps, T* __restrict__ out, int ldo, int n, int rows) {
   __shared__ float red[33];
   const int c0 = blockIdx.y * n;
   chain_release_if_small();
-  float wk[R][4], v[R][4], z[R][4], vn[R][4], zn[R][4];
+  float wk[R][4], v[R][4], z[R][4], vn[R][4], zn[R][4];        // vn, zn: the next row's, where rows are walked
 #pragma unroll
   for (int c = 0; c < R; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 4;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) { wk[c][e] = 1.f; vn[c][e] = zn[c][e] = 0.f; }
+    for (int e = 0; e < 4; ++e) { wk[c][e] = 1.f; v[c][e] = z[c][e] = vn[c][e] = zn[c][e] = 0.f; }
     if (w && i < n) load4(w + c0 + i, wk[c]);
   }
   chain_wait(y, zsrc);
-  auto ask = [&](int t) {
+  auto ask = [&](int t, float (&yv)[R][4], float (&zv)[R][4]) {
     const TY* yr = y + (size_t)t * ldy + ycol0 + c0;
     const TZ* zr = MODE ? zsrc + (size_t)t * ldz + zcol0 + c0 : nullptr;
 #pragma unroll
     for (int c = 0; c < R; ++c) {
       const int i = (c * blockDim.x + threadIdx.x) * 4;
       if (i < n) {
-        load4(yr + i, vn[c]);
-        if (MODE) load4(zr + i, zn[c]);
+        load4(yr + i, yv[c]);
+        if (MODE) load4(zr + i, zv[c]);
       }
     }
   };
-  ask(blockIdx.x);
-  for (int t = blockIdx.x; t < rows; t += gridDim.x) {
-#pragma unroll
-    for (int c = 0; c < R; ++c)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { v[c][e] = vn[c][e]; z[c][e] = zn[c][e]; }
-    if (t + (int)gridDim.x < rows) ask(t + gridDim.x);
+  auto norm_row = [&](int t) {
     float ss = 0.f;
 #pragma unroll
     for (int c = 0; c < R; ++c)
@@ -308,6 +303,20 @@ part_norm_vec_kernel(const TY* __restrict__ y, int ldy, int ycol0, const TZ* __r
       for (int e = 0; e < 4; ++e) o[e] = v[c][e] * inv * wk[c][e] * (MODE >= 2 ? z[c][e] : 1.f);
       store4(out + (size_t)t * ldo + c0 + i, o);
     }
+  };
+  if constexpr (WALK) {
+    ask(blockIdx.x, vn, zn);
+    for (int t = blockIdx.x; t < rows; t += gridDim.x) {
+#pragma unroll
+      for (int c = 0; c < R; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { v[c][e] = vn[c][e]; z[c][e] = zn[c][e]; }
+      if (t + (int)gridDim.x < rows) ask(t + gridDim.x, vn, zn);
+      norm_row(t);
+    }
+  } else {
+    ask(blockIdx.x, v, z);
+    norm_row(blockIdx.x);
   }
 }
 // Whether rows of `n` numbers at `p` (first column `col0`, `ld` apart, `el` bytes a number) can be moved four at a time.
@@ -323,10 +332,19 @@ static int part_norm_vec(const void* y, int ldy, int ycol0, const void* z, int l
     return 0;
   const int units = n / 4, runs = units <= 512 ? 1 : (units <= 1024 ? 2 : 4);
   const int th = ((units + runs - 1) / runs + 31) / 32 * 32;
-#define NF_PN(RR)                                                                                                        \
-  launch_chained(part_norm_vec_kernel<TY, TZ, T, RR, MODE>, dim3(parts > 1 ? R : row_ctas(R, th), parts), dim3(th), 0, stream, (const TY*)y, \
-                 ldy, ycol0, (const TZ*)z, ldz, zcol0, w, eps, (T*)out, ldo, n, R)
-  if (runs == 1) NF_PN(1); else if (runs == 2) NF_PN(2); else NF_PN(4);
+#define NF_PN(RR, WALK, CTAS)                                                                                              \
+  launch_chained(part_norm_vec_kernel<TY, TZ, T, RR, MODE, WALK>, dim3(CTAS, parts), dim3(th), 0, stream, (const TY*)y, ldy, ycol0, \
+                 (const TZ*)z, ldz, zcol0, w, eps, (T*)out, ldo, n, R)
+  // Rows are walked where a row is a thread's one run of four and has no gate beside it: wider ones take so many registers
+  // for the next row that fewer CTAs fit (rows of 8,192 with a gate, 2,048 of them: 31 us, walked 62; of 3,584 17 and 22),
+  // with a gate nothing is gained (rows of 2,048, 4,096 of them: 17.6 and 17.1, 512 of them 3.3 and 3.5; without 10.7 and 9.1).
+  if (runs == 1) {
+    if (MODE == 0 && parts == 1 && 2 * row_ctas(R, th) <= R) NF_PN(1, MODE == 0, row_ctas(R, th)); else NF_PN(1, false, R);
+  } else if (runs == 2) {
+    NF_PN(2, false, R);
+  } else {
+    NF_PN(4, false, R);
+  }
 #undef NF_PN
   return 1;
 }
@@ -464,10 +482,16 @@ extern "C" int nf_add_layernorm(float* h, const void* delta, const int* rows, co
   NF_REQUIRE(smem <= 160 * 1024, "add_layernorm: a row of %d does not fit shared memory", hidden);
   const int threads = hidden >= 2048 ? 512 : 256;
   const int runs = (hidden / 4 + threads - 1) / threads;
-#define NF_LN_R(T, RR)                                                                                                  \
-  launch_chained(add_layernorm_regs_kernel<T, RR>, dim3(row_ctas(R, threads)), dim3(threads), 0, stream, h, (const T*)delta, w, \
-                 eps, (T*)out, hidden, R)
-#define NF_LN_REGS(T) do { if (runs <= 1) NF_LN_R(T, 1); else if (runs <= 2) NF_LN_R(T, 2); else NF_LN_R(T, 4); } while (0)
+#define NF_LN_R(T, RR, WALK)                                                                                            \
+  launch_chained(add_layernorm_regs_kernel<T, RR, WALK>, dim3(WALK ? row_ctas(R, threads) : R), dim3(threads), 0, stream, h, \
+                 (const T*)delta, w, eps, (T*)out, hidden, R)
+  // (rows of more than a run a thread take so many registers for the next one that fewer CTAs fit: they are not walked)
+#define NF_LN_REGS(T)                                                                                                   \
+  do {                                                                                                                  \
+    if (runs <= 1) { if (2 * row_ctas(R, threads) <= R) NF_LN_R(T, 1, true); else NF_LN_R(T, 1, false); }                    \
+    else if (runs <= 2) NF_LN_R(T, 2, false);                                                                           \
+    else NF_LN_R(T, 4, false);                                                                                          \
+  } while (0)
 #define NF_LN(T, G, V)                                                                                      \
   do {                                                                                                      \
     if (smem > 48 * 1024)                                                                                   \
@@ -637,14 +661,14 @@ __global__ void scaled_norm_add_kernel(float* __restrict__ h, const TD* __restri
 
 // Rows of up to R numbers a thread: the same sums in the same order, with the row in registers between the two passes, all
 // its numbers asked for at once and the weights, which no kernel writes, before the wait (see part_norm_vec_kernel).
-template <typename TD, typename TO, int R>
+template <typename TD, typename TO, int R, bool WALK>
 __global__ void __launch_bounds__(512)
 scaled_norm_add_regs_kernel(float* __restrict__ h, const TD* __restrict__ delta, const float* __restrict__ bias,
                             const float* __restrict__ w, const float* __restrict__ ls, float eps, TO* __restrict__ out, int hidden,
                             int rows) {
   __shared__ float red[33];
   chain_release_if_small();
-  float wk[R], lk[R], bk[R], d[R], hk[R], hn[R];
+  float wk[R], lk[R], bk[R], d[R], hk[R], hn[R];      // hn: the next row's, where rows are walked
 #pragma unroll
   for (int c = 0; c < R; ++c) {
     const int i = c * blockDim.x + threadIdx.x;
@@ -658,38 +682,52 @@ scaled_norm_add_regs_kernel(float* __restrict__ h, const TD* __restrict__ delta,
   }
   chain_wait(h, delta);
   TD raw[R];
-  auto ask = [&](int r) {
+  auto ask = [&](int r, float (&hv)[R]) {
     const float* hr = h + (size_t)r * hidden;
     const TD* dr = delta + (size_t)r * hidden;
 #pragma unroll
     for (int c = 0; c < R; ++c) {
       const int i = c * blockDim.x + threadIdx.x;
-      if (i < hidden) { raw[c] = dr[i]; hn[c] = hr[i]; }
+      if (i < hidden) { raw[c] = dr[i]; hv[c] = hr[i]; }
     }
   };
-  constexpr bool AHEAD = R < 16;
-  if (AHEAD) ask(blockIdx.x);
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-    if (!AHEAD) ask(r);
-    float* hr = h + (size_t)r * hidden;
+  auto sum_row = [&]() {
     float ss = 0.f;
 #pragma unroll
-    for (int c = 0; c < R; ++c) {
-      hk[c] = hn[c];
+    for (int c = 0; c < R; ++c)
       if (c * (int)blockDim.x + (int)threadIdx.x < hidden) {
         d[c] = to_float(raw[c]) + bk[c];
         ss = fmaf(d[c], d[c], ss);
       }
-    }
-    if (AHEAD && r + (int)gridDim.x < rows) ask(r + gridDim.x);
+    return ss;
+  };
+  auto add_row = [&](int r, float ss) {
     const float inv = rsqrtf(block_sum(ss, red) / (float)hidden + eps);
 #pragma unroll
     for (int c = 0; c < R; ++c) {
       const int i = c * blockDim.x + threadIdx.x;
       if (i >= hidden) continue;
       const float v = scaled_norm_sum(d[c], inv, wk[c], ls, lk[c], hk[c]);
-      hr[i] = v;
+      h[(size_t)r * hidden + i] = v;
       if (out) out[(size_t)r * hidden + i] = from_float<TO>(v);
+    }
+  };
+  if constexpr (!WALK) {
+    ask(blockIdx.x, hk);
+    add_row(blockIdx.x, sum_row());
+  } else if constexpr (R < 16) {
+    ask(blockIdx.x, hn);
+    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+      const float ss = sum_row();
+#pragma unroll
+      for (int c = 0; c < R; ++c) hk[c] = hn[c];
+      if (r + (int)gridDim.x < rows) ask(r + gridDim.x, hn);
+      add_row(r, ss);
+    }
+  } else {                             // (no registers for a next row)
+    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+      ask(r, hk);
+      add_row(r, sum_row());
     }
   }
 }
@@ -851,8 +889,16 @@ extern "C" int nf_scaled_norm_add(float* h, const void* delta, int delta_dtype, 
   NF_REQUIRE(R > 0 && hidden > 0 && h && delta && w, "scaled_norm_add: bad arguments R=%d hidden=%d", R, hidden);
   const dim3 grid(R), block(norm_threads(hidden));
   const int each = (hidden + (int)block.x - 1) / (int)block.x;
-#define NF_SNV(TD, TO, RR) \
-  launch_chained(scaled_norm_add_regs_kernel<TD, TO, RR>, dim3(row_ctas(R, (int)block.x)), block, 0, stream, h, (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden, R)
+  // Rows are walked from two a CTA on.  (257 rows of 3,584 4.9 us, as walks of one row 5.4; 512 of 4,096, walks of one or
+  // two, 9.0 and 9.6; 1,024 20.5 and 16.1; rows of 256 gain nothing: 2,048 of them 5.5 and 5.7.)
+  const bool walk = hidden >= 512 && 2 * row_ctas(R, (int)block.x) <= R;
+#define NF_SNV(TD, TO, RR)                                                                                                 \
+  do {                                                                                                                     \
+    if (walk) launch_chained(scaled_norm_add_regs_kernel<TD, TO, RR, true>, dim3(row_ctas(R, (int)block.x)), block, 0, stream, h, \
+                             (const TD*)delta, bias, w, ls, eps, (TO*)out, hidden, R);                                     \
+    else launch_chained(scaled_norm_add_regs_kernel<TD, TO, RR, false>, dim3(R), block, 0, stream, h, (const TD*)delta, bias, w,  \
+                        ls, eps, (TO*)out, hidden, R);                                                                     \
+  } while (0)
 #define NF_SNA(TD, TO)                                                                                                     \
   do {                                                                                                                     \
     if (each <= 4) NF_SNV(TD, TO, 4); else if (each <= 8) NF_SNV(TD, TO, 8); else if (each <= 16) NF_SNV(TD, TO, 16);      \

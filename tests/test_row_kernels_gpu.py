@@ -127,3 +127,33 @@ def test_norms_whose_ctas_walk_rows(K, hidden, dtype):
         for t, one, v in zip(got, alone, want):
             assert torch.equal(t[some], one), fn.__name__
             torch.testing.assert_close(t.double(), v, **(tol if t.dtype == torch.bfloat16 else dict(rtol=2e-5, atol=2e-5)))
+
+
+def median_time(fn):
+    """Of twenty calls in a graph, the fastest of seven replays."""
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(20):
+            fn()
+    times = []
+    for _ in range(7):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        graph.replay()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b))
+    return min(times)
+
+
+def test_norms_of_wide_rows_take_their_numbers_time(K):
+    """1,024 rows of 8,192 against 4,096 of 2,048, as many numbers: 1.4 times as long while wide rows were walked."""
+    times = {}
+    for rows, hidden in ((4096, 2048), (1024, 8192)):
+        h, a, w = torch.randn((rows, hidden), device="cuda"), torch.randn((rows, hidden), device="cuda").bfloat16(), torch.rand((hidden,), device="cuda")
+        out = torch.empty_like(a)
+        times[hidden] = (median_time(lambda: K.group_rmsnorm_gate(h, a, 0, w, 1e-6, 1, 1, torch.bfloat16)),
+                         median_time(lambda: K.add_layernorm(h, a, None, w, 1e-6, out)))
+    assert times[8192][0] <= 1.15 * times[2048][0] and times[8192][1] <= 1.15 * times[2048][1]
