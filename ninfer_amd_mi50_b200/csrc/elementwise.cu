@@ -496,53 +496,43 @@ __global__ void gated_bias_act_kernel(const TI* __restrict__ gu, const float* __
   act[(size_t)m * inner + i] = from_float<T>(gated_act(g, u, kind, limit, alpha));
 }
 
-// The same in runs of four columns, one access each, and ROWS rows a thread, all asked for at once: the biases are read
-// once for them (rows x columns 2,048 x 5,632 of float32 sums, 115 MB: element by element 46 us).
-template <typename TI, typename T, int ROWS>
+// The same in runs of four columns, one access each (2,048 rows of 5,632 columns of float32 sums, 115 MB: element by element
+// 41 us, now 19).
+template <typename TI, typename T>
 __global__ void __launch_bounds__(256)
-gated_bias_act_x4_kernel(const TI* __restrict__ gu, const float* __restrict__ bias, T* __restrict__ act, int M, int inner, int kind,
+gated_bias_act_x4_kernel(const TI* __restrict__ gu, const float* __restrict__ bias, T* __restrict__ act, int inner, int kind,
                          float limit, float alpha) {
-  const int m0 = blockIdx.y * ROWS, i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  float bg[4] = {0.f, 0.f, 0.f, 0.f}, bu[4] = {0.f, 0.f, 0.f, 0.f};
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  float bg[4] = {0.f, 0.f, 0.f, 0.f}, bu[4] = {0.f, 0.f, 0.f, 0.f}, g[4], u[4];
   if (bias && i < inner) {
     load4(bias + i, bg);
     load4(bias + inner + i, bu);
   }
   chain_wait(gu);
   if (i >= inner) return;
-  float g[ROWS][4], u[ROWS][4];
+  const TI* row = gu + (size_t)blockIdx.y * 2 * inner;
+  load4(row + i, g);
+  load4(row + inner + i, u);
 #pragma unroll
-  for (int r = 0; r < ROWS; ++r)
-    if (m0 + r < M) {
-      const TI* row = gu + (size_t)(m0 + r) * 2 * inner;
-      load4(row + i, g[r]);
-      load4(row + inner + i, u[r]);
-    }
-#pragma unroll
-  for (int r = 0; r < ROWS; ++r)
-    if (m0 + r < M) {
-      if (bias) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { g[r][e] += bg[e]; u[r][e] += bu[e]; }
-      }
-#pragma unroll
-      for (int e = 0; e < 4; ++e) g[r][e] = gated_act(g[r][e], u[r][e], kind, limit, alpha);
-      store4(act + (size_t)(m0 + r) * inner + i, g[r]);
-    }
+  for (int e = 0; e < 4; ++e) {
+    if (bias) { g[e] += bg[e]; u[e] += bu[e]; }
+    g[e] = gated_act(g[e], u[e], kind, limit, alpha);
+  }
+  store4(act + (size_t)blockIdx.y * inner + i, g);
 }
 
 template <typename TI, typename T>
 static void launch_gated_bias_act(const TI* gu, const float* bias, T* act, int M, int inner, int kind, float limit, float alpha,
                                   cudaStream_t stream) {
-  if (inner % 4 == 0 && (uintptr_t)gu % (4 * sizeof(TI)) == 0 && (uintptr_t)act % (4 * sizeof(T)) == 0 && (uintptr_t)bias % 16 == 0) {
-    const int tiles = (inner / 4 + 255) / 256;
-    if (M >= 64)      // (rows enough for every SM to have several CTAs all the same)
-      launch_chained(gated_bias_act_x4_kernel<TI, T, 4>, dim3(tiles, (M + 3) / 4), dim3(256), 0, stream, gu, bias, act, M, inner, kind, limit, alpha);
-    else
-      launch_chained(gated_bias_act_x4_kernel<TI, T, 1>, dim3(tiles, M), dim3(256), 0, stream, gu, bias, act, M, inner, kind, limit, alpha);
-  } else {
+  // Runs of four once a thread an element is more threads than the device holds at once, in rows that fill a CTA: below,
+  // one element a thread has the shorter chain (1,408 columns, 64 rows 1.4 and 1.5 us, 200 rows 1.8 both, 600 rows 3.3 and
+  // 2.7; of 256 columns 4,096 rows 3.6 and 4.1).  More rows a thread gave nothing (two: the same within 4 %; four, once the
+  // rule from 64 rows on: 64 rows 2.4, 600 rows 3.5).
+  if ((long long)M * inner > 148ll * 2048 && inner >= 512 && inner % 4 == 0 && (uintptr_t)gu % (4 * sizeof(TI)) == 0 &&
+      (uintptr_t)act % (4 * sizeof(T)) == 0 && (uintptr_t)bias % 16 == 0)
+    launch_chained(gated_bias_act_x4_kernel<TI, T>, dim3((inner / 4 + 255) / 256, M), dim3(256), 0, stream, gu, bias, act, inner, kind, limit, alpha);
+  else
     launch_chained(gated_bias_act_kernel<TI, T>, dim3((inner + 255) / 256, M), dim3(256), 0, stream, gu, bias, act, inner, kind, limit, alpha);
-  }
 }
 
 }  // namespace nf

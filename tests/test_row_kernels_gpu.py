@@ -148,6 +148,17 @@ def median_time(fn):
     return min(times)
 
 
+@pytest.mark.parametrize("inner", [704, 1408, 5632])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_activation_of_one_row_more_takes_no_jump(K, inner, dtype):
+    """64 rows took up to twice as long as 63 when a thread took four of them."""
+    times = []
+    for rows in (63, 64):
+        gu = torch.randn((rows, 2 * inner), device="cuda").to(dtype)
+        times.append(median_time(lambda: K.gated_bias_act(gu, None, None, torch.bfloat16)))
+    assert times[1] <= 1.3 * times[0]
+
+
 def test_norms_of_wide_rows_take_their_numbers_time(K):
     """1,024 rows of 8,192 against 4,096 of 2,048, as many numbers: 1.4 times as long while wide rows were walked."""
     times = {}
