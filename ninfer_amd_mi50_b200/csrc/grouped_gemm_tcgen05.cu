@@ -46,6 +46,7 @@ constexpr int kWarpCols = 48;      // accumulator columns a warp holds in regist
 constexpr int kRoundCols = kWarpCols * kEpilogueWarps / 4;
 constexpr int kXBox = 64;         // token rows per TMA box
 constexpr int kMaxStages = 8;
+constexpr int kUnevenRows = 192;     // groups are ordered by rows only from so many in the largest on
 constexpr int kMaxGroupsTc = 1024;   // groups one launch may have (their pass counts live in shared memory)
 constexpr int kSmemBudget = 225 * 1024;   // + 1 KB of alignment slack + a few static bytes <= the 227 KB a CTA may have
 
@@ -62,12 +63,11 @@ struct __align__(8) Barriers {
   int stop;
 };
 
-// The item a CTA takes after `item`.  BACK_AND_FORTH: rounds of gridDim.x items are dealt out forwards
+// The item a CTA takes after `item`.  `back_and_forth`: rounds of gridDim.x items are dealt out forwards
 // and backwards in turn, so that the CTA with the longest item of one round has the shortest of the next.
-template <bool BACK_AND_FORTH>
-__device__ __forceinline__ int next_item(int item) {
+__device__ __forceinline__ int next_item(int item, bool back_and_forth) {
   const int g = gridDim.x;
-  if (!BACK_AND_FORTH) return item + g;
+  if (!back_and_forth) return item + g;
   const int round = item / g + 1;
   return round * g + ((round & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
 }
@@ -76,14 +76,22 @@ __device__ __forceinline__ int next_item(int item) {
 // every round of as many items as there are CTAs, with feature tiles varying fastest, so CTAs that
 // run together share an expert's token rows in L2, and the passes of a heavily loaded expert - which
 // re-read its weights - run next to each other and find them in L2.
-// Groups are walked by falling number of rows.  An item's time is that of its weights' way from HBM
+// Unequal groups are walked by falling number of rows.  An item's time is that of its weights' way from HBM
 // (1,440 cycles a k step of 32 KB with all SMs at it) until its rows' products take as long; routers
 // load experts unevenly (of 60 experts 3 to 1,291 of 8,192 rows), so items differ, 4 to 6 rounds do not
 // even that out, and the last round is thin.  By falling rows it is made of the shortest items, and
-// dealt back and forth the long and short ones meet (60 experts of 2 x 1408 x 2048, 8,192 rows: first
-// product 157 us in the experts' order, 153 by rows, 150 back and forth; second 90, 86, 86; 64 experts of
-// 16,384 rows: 529, 515, 508).  With a second accumulator, unpaired, dealing back and forth costs 4 %
+// dealt back and forth the long and short ones meet (60 experts of 2 x 1408 x 2048, 4,096 rows, the largest group 12 times
+// the mean: first product 133 -> 127 us, second 80 -> 74; 8,192 rows 169 -> 160, 92 -> 88; 32 experts of 2 x 704 x 1024,
+// 2,048 rows 35 -> 29).  With a second accumulator, unpaired, dealing back and forth costs 4 %
 // (207 -> 216 us): there the order alone is kept.
+// Where groups are about equal, or all so small that their weights bound every item, the experts' own order is the
+// faster.  60 experts, us in their order and by rows (largest group, times the mean):
+//   first product   4,096 rows (92, 1.4) 124 and 127;  6,144 (287, 2.8) 144 and 141;  8,192 (171, 1.3) 138 and 143,
+//                   (321, 2.4) 144 and 147, (394, 2.9) 153 and 148, of a prompt (956, 7.0) 165 and 159
+//   second          4,096 (92, 1.4) 77 and 79, (188, 2.8) 82 and 80;  6,144 (182, 1.8) 90 and 88;  8,192 (171, 1.3) 94 and 96,
+//                   (251, 1.8) 101 and 97, of a prompt (956, 7.0) 116 and 102;  16,384 (312, 1.1) 165 and 144
+// Hence the rule: kUnevenRows rows in the largest group, and it 2.5 times the mean, 1.75 in the second product, or there a
+// group of more than one pass.
 // 448 threads: warp 0 producer, warp 1 MMA + tensor memory, warps 2..13 epilogue.  The
 // producer is not held back by the epilogue: while the epilogue warps drain an item's
 // accumulator, the stages fill with the next item's first k tiles, so the memory pipe never
@@ -98,7 +106,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_constant__ CUtensorMap map_x,
                        const __grid_constant__ CUtensorMap map_x_half,
                        const int* __restrict__ offsets, __nv_bfloat16* __restrict__ out, int ldo,
-                       int n_features, int K, int groups, GatedActParams act) {
+                       int n_features, int K, int groups, long long total_rows, GatedActParams act) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   static_assert(!(SWIGLU && PAIR), "the first product already has two weight tiles an item");
@@ -118,8 +126,8 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
   // tensor memory are set up meanwhile, and everything that reads what that kernel (or the
   // routing before it) wrote comes after the wait.
   Barriers* bars = reinterpret_cast<Barriers*>(smem);
-  int* s_pass_start = reinterpret_cast<int*>(bars + 1);     // [groups + 1] first pass index of every place in that order
-  int* s_group = s_pass_start + groups + 1;                 // [groups] the groups by falling number of rows
+  int* s_pass_start = reinterpret_cast<int*>(bars + 1);     // [groups + 1] first pass index of every place in the walk
+  int* s_group = s_pass_start + groups + 1;                 // [groups] the groups in the walk's order
   int* s_rows = s_group + groups;                           // [groups] rows of every group
   const int head_bytes = ((int)sizeof(Barriers) + (3 * groups + 1) * (int)sizeof(int) + 1023) & ~1023;
   unsigned char* stage0 = smem + head_bytes;
@@ -146,21 +154,25 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
       const int n = offsets[g + 1] - offsets[g];
       mx = max(mx, n);
       s_rows[g] = n;
+      s_group[g] = g;
+      s_pass_start[g + 1] = (n + kBNMax - 1) / kBNMax;
     }
     if (mx) atomicMax(&s_max_rows, mx);
   }
   __syncthreads();
-  for (int g = threadIdx.x; g < groups; g += blockDim.x) {
-    const int n = s_rows[g];
-    int before = g;
-    if (groups <= kTcThreads) {      // a thread a group; ranking more by comparisons would take longer than it gains
-      before = 0;
+  const long long most = (long long)s_max_rows * groups;          // against total_rows: the largest group to the mean
+  const bool by_rows = groups <= kTcThreads && ((s_max_rows >= kUnevenRows && 4 * most >= (SWIGLU ? 10 : 7) * total_rows) ||
+                                                (!SWIGLU && s_max_rows > kBNMax));
+  if (by_rows) {                     // a thread a group; ranking more by comparisons would take longer than it gains
+    for (int g = threadIdx.x; g < groups; g += blockDim.x) {
+      const int n = s_rows[g];
+      int before = 0;
       for (int o = 0; o < groups; ++o) before += s_rows[o] > n || (s_rows[o] == n && o < g);
+      s_group[before] = g;
+      s_pass_start[before + 1] = (n + kBNMax - 1) / kBNMax;
     }
-    s_group[before] = g;
-    s_pass_start[before + 1] = (n + kBNMax - 1) / kBNMax;
+    __syncthreads();
   }
-  __syncthreads();
   if (warp == 0) {
     int run = 0;
     if (lane == 0) s_pass_start[0] = 0;
@@ -176,6 +188,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
       run += __shfl_sync(0xffffffffu, v, 31);
     }
   }
+  const bool back_and_forth = (SWIGLU || PAIR) && by_rows;
   constexpr int kAccBuffers = (SWIGLU || PAIR) ? 1 : 2;      // accumulators of kBNMax columns that fit beside each other
   const int max_boxes = (min(max(s_max_rows, 1), kBNMax) + kXBox - 1) / kXBox;
   const int stage_bytes = A_BYTES + max_boxes * BOX_BYTES;
@@ -192,7 +205,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
       int it = 0, issued = 0;
       bool ok = true;
       int place = 0;
-      for (int item = blockIdx.x; item < n_items && ok; item = next_item<SWIGLU || PAIR>(item)) {
+      for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, back_and_forth)) {
         const int gp = item / n_fitems, ft = (item - gp * n_fitems) * FT_STEP;      // global pass index, feature tile
         while (s_pass_start[place + 1] <= gp) ++place;
         const int group = s_group[place], pass = gp - s_pass_start[place];
@@ -244,7 +257,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
       int it = 0, pass_ctr = 0;
       bool ok = true;
       int place = 0;
-      for (int item = blockIdx.x; item < n_items && ok; item = next_item<SWIGLU || PAIR>(item), ++pass_ctr) {
+      for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, back_and_forth), ++pass_ctr) {
         const int gp = item / n_fitems;
         while (s_pass_start[place + 1] <= gp) ++place;
         const int group = s_group[place], pass = gp - s_pass_start[place];
@@ -286,7 +299,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
     int pass_ctr = 0;
     bool ok = true;
     int place = 0;
-    for (int item = blockIdx.x; item < n_items && ok; item = next_item<SWIGLU || PAIR>(item), ++pass_ctr) {
+    for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, back_and_forth), ++pass_ctr) {
       const int gp = item / n_fitems, ft0 = (item - gp * n_fitems) * FT_STEP;
       while (s_pass_start[place + 1] <= gp) ++place;
       const int group = s_group[place], pass = gp - s_pass_start[place];
@@ -367,7 +380,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
 
 template <bool SWIGLU, bool PAIR>
 static int launch_tc(const void* Wp, const CUtensorMap& mx, const CUtensorMap& mx_half, const int* offsets, void* out, int ldo,
-                     int n_features, int K, int groups, GatedActParams act, cudaStream_t stream) {
+                     int n_features, int K, int groups, long long total_rows, GatedActParams act, cudaStream_t stream) {
   const size_t smem = (size_t)kSmemBudget + 1024;
   static bool set = false;
   if (!set) {
@@ -386,7 +399,7 @@ static int launch_tc(const void* Wp, const CUtensorMap& mx, const CUtensorMap& m
   // at least one pass per non-empty group; the kernel itself counts the exact number of items
   const int grid = n_sm;
   launch_chained(grouped_gemm_tc_kernel<SWIGLU, PAIR>, dim3(grid), dim3(kTcThreads), smem, stream,
-                 (const __nv_bfloat16*)Wp, mx, mx_half, offsets, (__nv_bfloat16*)out, ldo, n_features, K, groups, act);
+                 (const __nv_bfloat16*)Wp, mx, mx_half, offsets, (__nv_bfloat16*)out, ldo, n_features, K, groups, total_rows, act);
   return check_launch("grouped_gemm_tc");
 }
 
@@ -425,12 +438,12 @@ extern "C" int nf_grouped_gemm_tc(const void* X, long long total_rows, int ldx, 
   if (int rc = make_map(&mx_half, X, total_rows, K, kXBox / 2, ldx)) return rc;
   NF_REQUIRE(swiglu >= 0 && swiglu <= 3, "grouped_gemm_tc: epilogue %d (0 none, 1 silu-gated, 2 capped, 3 ungated GELU)", swiglu);
   const GatedActParams act{swiglu, act_limit, act_alpha};
-  if (swiglu == kActSilu || swiglu == kActCapped) return launch_tc<true, false>(Wp, mx, mx_half, offsets, out, ldo, n_features, K, groups, act, stream);
+  if (swiglu == kActSilu || swiglu == kActCapped) return launch_tc<true, false>(Wp, mx, mx_half, offsets, out, ldo, n_features, K, groups, total_rows, act, stream);
   // two feature tiles an item once an expert's rows weigh about as much as a tile's weights
   // (decided by the counts the host knows: all rows, all groups)
   if (g_tc_pair && total_rows >= (long long)g_tc_pair_min_rows * groups)
-    return launch_tc<false, true>(Wp, mx, mx_half, offsets, out, ldo, n_features, K, groups, act, stream);
-  return launch_tc<false, false>(Wp, mx, mx_half, offsets, out, ldo, n_features, K, groups, act, stream);
+    return launch_tc<false, true>(Wp, mx, mx_half, offsets, out, ldo, n_features, K, groups, total_rows, act, stream);
+  return launch_tc<false, false>(Wp, mx, mx_half, offsets, out, ldo, n_features, K, groups, total_rows, act, stream);
 }
 
 // A wait that nothing will ever satisfy, given `polls` polls: the bounded wait runs out, records

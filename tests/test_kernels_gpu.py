@@ -770,6 +770,29 @@ def test_grouped_gemm_walks_experts_by_falling_rows(K, T, E, k):
     assert K.tensor_core_status() == 0
 
 
+@pytest.mark.parametrize("loads", [[10, 191, 3, 40], [10, 192, 3, 40], [0, 192, 90, 96, 6, 0], [192, 96, 96, 1, 95], [20, 500, 0, 300, 7],
+                                   [240, 250, 257, 255]])
+def test_grouped_gemm_where_the_order_by_rows_begins(K, loads):
+    """Groups on either side of the rules for the walk by falling rows: 192 rows in the largest, which is 1.75 or 2.5 times the
+    mean, or more than a pass."""
+    dtype, H, I, E = torch.bfloat16, 128, 136, len(loads)
+    idx = torch.tensor([e for e, n in enumerate(loads) for _ in range(n)], dtype=torch.int32)
+    idx = idx[torch.randperm(len(idx), generator=torch.Generator().manual_seed(9))].view(-1, 1).cuda()
+    x = rnd((len(idx), H), dtype, 64)
+    w13, w2 = rnd((E, 2 * I, H), dtype, 65, 0.1), rnd((E, H, I), dtype, 66, 0.1)
+    plan = K.moe_plan(idx, E)
+    old = dict(K.TUNING)
+    try:
+        K.TUNING.update(bf16_moe="simt", skinny_moe_max_tokens=0)
+        ract = K.moe_gemm1(x, w13, plan, 1)
+        ry = K.moe_gemm2(ract, w2, plan)
+        close(K.moe_gemm1(x, K.pack_weights(w13, swiglu=True), plan, 1), ract, dtype)
+        close(K.moe_gemm2(ract, K.pack_weights(w2, swiglu=False), plan), ry, dtype)
+    finally:
+        K.TUNING.update(old)
+    assert K.tensor_core_status() == 0
+
+
 @pytest.mark.parametrize("T,H,I,E,k", [(1, 256, 128, 4, 2), (5, 200, 136, 6, 3), (8, 2048, 1408, 60, 4),
                                        (13, 512, 264, 7, 2), (3, 40, 24, 3, 1)])
 def test_streaming_experts_with_an_early_start(K, T, H, I, E, k):
