@@ -171,7 +171,8 @@ int gf_dispatch(const GfCall& c, cudaStream_t stream) {
   const bool alone = c.groups == 1;
   const size_t matrix = (size_t)c.N * (GATED ? 2 : 1) * c.K * sizeof(float);
   if constexpr (!GATED)
-    if (alone && rows > 4 && rows <= 32 && (c.N + 31) / 32 * ((c.max_rows + 7) / 8) <= 400 && matrix <= kGfL2)
+    if (alone && rows > 4 && rows <= 32 && (c.N + 31) / 32 * ((c.max_rows + 7) / 8) <= 400 && matrix <= kGfL2 &&
+        (rows > 24 || (c.N + 31) / 32 * ((c.max_rows + 3) / 4) > 148))      // up to one CTA a SM of the tile below: that one
       return gf_launch<8, 32, 4, 1, 8, false>(c, tiles(8), stream);
   if (rows <= (!alone ? 5 : matrix > kGfFar ? 4 : matrix > kGfL2 ? 10 : 24)) return gf_launch<4, GATED ? 64 : 32, 4, GATED ? 2 : 1, 6, GATED>(c, tiles(4), stream);
   if (rows <= 64) return gf_launch<16, 64, 8, 2, 4, GATED>(c, tiles(16), stream);
