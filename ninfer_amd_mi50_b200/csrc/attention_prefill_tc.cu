@@ -116,8 +116,12 @@ __device__ __forceinline__ float max3(float x, float y, float z) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(v) : "f"(x), "f"(y), "f"(z));
   return v;
 }
+// Buffers of P: two in tensor memory, or one in shared memory: where a weight is given as two numbers, and in the biased form
+// at heads of 64, which must fence its values in shared memory for every block all the same (16 heads on 4 key heads, 512 rows
+// behind 3,000 keys: 52.9 us, out of tensor memory 54.0; at heads of 128 29.9 and 29.4).
+constexpr int fa_p_buffers(int d, int rot, int form) { return rot || (form == kFormBiased && d == 64) ? 1 : 2; }
 // shared memory for P: none where it lives in tensor memory
-constexpr int fa_p_bytes(int parts) { return parts == 1 ? 0 : parts * 2 * kAtom; }
+constexpr int fa_p_bytes(int d, int rot, int form) { return fa_p_buffers(d, rot, form) == 2 ? 0 : (rot ? 2 : 1) * 2 * kAtom; }
 
 struct TileInfo {
   int seg, row0, n_rows, pos_first, pos_last, kb_first, n_kept, n_blocks;
@@ -158,14 +162,14 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   constexpr int KATOMS = (D + ROT) / 64;          // ... across a query or key
   constexpr int QB = KATOMS * kAtom, VB = ATOMS * kAtom;   // bytes of the Q tile and of a K block; of a V block
   constexpr int STAGES = ROT ? 1 : 2, PARTS = ROT ? 2 : 1; // K and V stages; bfloat16 numbers a weight is given as
-  constexpr int PBUF = PARTS == 1 ? 2 : 1;        // buffers of P: two in tensor memory, or one in shared memory
+  constexpr int PBUF = fa_p_buffers(D, ROT, FORM);
   static_assert(!ROT || (DENSE && FORM == kFormSoftmax), "the further dimensions go with the dense softmax form");
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* Qs = smem;
   unsigned char* KV = Qs + QB;                    // [stages][K block, V block]
   unsigned char* Ps = KV + STAGES * (QB + VB);    // [parts][2 atoms][128 rows][128 bytes]
-  FaBarriers* bars = reinterpret_cast<FaBarriers*>(Ps + fa_p_bytes(PARTS));
+  FaBarriers* bars = reinterpret_cast<FaBarriers*>(Ps + fa_p_bytes(D, ROT, FORM));
   float* s_rowsum = reinterpret_cast<float*>(bars + 1);      // [2 halves][128 rows]: the two threads of a row add up
   float* s_rowmax = s_rowsum + 2 * kQ;                       // [2 block parities][2 halves][128 rows]
   volatile int* stop = &bars->stop;
@@ -592,7 +596,7 @@ int launch_prefill_tc(const CUtensorMap& mq, const CUtensorMap& mkv, const CUten
                       const int* kv_base, const void* gate, int gate_ld, float softcap, const float* slopes, int keep_first,
                       cudaStream_t stream) {
   constexpr int QB = (D + ROT) / 64 * kAtom, VB = D / 64 * kAtom;
-  const size_t smem = 1024 + QB + (ROT ? 1 : 2) * (size_t)(QB + VB) + fa_p_bytes(ROT ? 2 : 1) + sizeof(FaBarriers) + 6 * kQ * sizeof(float);
+  const size_t smem = 1024 + QB + (ROT ? 1 : 2) * (size_t)(QB + VB) + fa_p_bytes(D, ROT, FORM) + sizeof(FaBarriers) + 6 * kQ * sizeof(float);
   static bool set = false;
   if (!set) {
     cudaError_t e = cudaFuncSetAttribute(prefill_attention_tc_kernel<D, ROT, FORM, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
