@@ -27,10 +27,10 @@
 //              one of two buffers in tensor memory, out of which the second product reads it; at the
 //              end of the tile O divided by the row sum is stored
 //
-// What bounds a tile is the chain of its softmax, block after block.  With one buffer of P in shared memory 550 of a
-// block's 2,780 cycles were waiting for the product of the block before; 2,048 rows of 16 heads 42.5 us, now 40.5, behind
-// 6,144 further keys 183.7, now 181.4.  (A quarter or half of the exponentials as polynomials on the multiply-add units
-// instead of the special-function unit: 41.9 and 45.7, it is issue slots that are short.)
+// What bounds a tile is the chain of its softmax, block after block.  With one buffer of P in shared memory it also waited for
+// the product of the block before: in a chain of such calls 2,048 rows of 16 heads 38.2 us, now 36.7, 512 rows behind 3,000
+// keys 49.5, now 48.4.  (A quarter or half of the exponentials as polynomials on the multiply-add units instead of the
+// special-function unit: 3 and 13 % slower.)
 //
 // The SIGMOID form has weights sigmoid(score + sig_bias[h]) that are not normalised over keys: no maximum, no rescaling,
 // no sum; P = 1 / (1 + 2^-(s + b)) and O is stored as it stands.

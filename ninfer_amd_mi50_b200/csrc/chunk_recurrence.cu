@@ -23,11 +23,10 @@
 // products whose weight is at least 2^-16 of the leading one are all taken (three where one operand is bfloat16, six
 // where both are float32) with float32 sums.
 //
-// One prompt of 2,048 tokens, before (row by row) and after: scan of 64 heads of 128 x 64 755 -> 177 us (the outputs take
-// 100 of it, the chunks' states 45, the chain over 16 chunks, which moves 67 MB, the rest), 32 heads of 64 x 64 394 -> 77;
-// linear attention of 16 heads of 128 x 128 with float32 q, k and v 499 -> 218 (six products each: bound by the tensor
-// pipe), 64 x 128 with bfloat16 values 347 -> 97; the delta rule of 16 heads of 128 x 128 431 -> 198, of 8 heads
-// 421 -> 138.  Chunks of 128 rows halve the states' traffic where the operands are bfloat16; with three parts of each
+// One prompt of 2,048 tokens, row by row and now: scan of 64 heads of 128 x 64 755 and 135 us (under a profiler, from a cold
+// cache, the outputs 95, the chunks' states 47, the chain over 16 chunks, which moves 67 MB, 15), 32 heads of 64 x 64 394 and 57;
+// linear attention of 16 heads of 128 x 128 with float32 q, k and v 499 and 150 (outputs 95, states 41, chain 22), 64 x 128 with
+// bfloat16 values 347 and 74; the delta rule of 16 heads of 128 x 128 431 and 172.  Chunks of 128 rows halve the states' traffic where the operands are bfloat16; with three parts of each
 // operand in shared memory 64 rows fit.
 #define NF_CHAIN_CLASS 2
 #include "common.cuh"
@@ -198,8 +197,7 @@ __device__ __forceinline__ void cr_row_gates(const CrArgs& a, int head, int row,
 // What a chunk's CTA reads goes through registers in two halves: `ask` issues every load, `put` brings the numbers to
 // shared memory (in parts, where they are float32).  Between the two lies other work - gates, decay tables, the products
 // with the rows or the state before - so that a CTA, of which only two fit a SM, does not stand still for each of its reads
-// (loads and stores in one loop: 42 % of the issue slots of the output kernel lost to waiting for loads, 47 % of the
-// states').
+// (with loads and stores in one loop the scan of 2,048 rows above took 164 us, linear attention 213, the delta rule 197).
 //
 // ROWS rows of the keys (or queries) for planes [PARTS][.][D + pad]; zeros from `live` rows on.
 template <int D, int PARTS, int ROWS>

@@ -16,7 +16,8 @@
 //                   Between, where 8 x 32 tiles of two warps are few (up to 400 CTAs), those: what counts there is the chain
 //                   over k, and more CTAs beside one another (one matrix, rows x features x k: 16 x 6144 x 2048 29 us, with
 //                   the tile before 33, with the next one 42; 32 x 2048 x 5632 50, 67, 108; 32 x 2048 x 2048 20, 28, 41; 768
-//                   CTAs, 32 x 6144 x 2048: 65, 63, 48; 8 x 6144 x 2048 21, 23, 42)
+//                   CTAs, 32 x 6144 x 2048: 65, 63, 48; 8 x 6144 x 2048 21, 23, 42); up to 24 rows not before the tile above is
+//                   more than one CTA a SM (24 x 512 x 256 3.35 us, in 8 x 32 3.48; 8 x 2048 x 5632 42.1 and 43.0)
 //   up to 64        16 x 64, two warps with 8 x 2 sums a thread (34 rows a group 472 us, with the next tile 518)
 //   up to 128       32 x 64 with 4 x 4 sums a thread: 100 rows 112 us, with the tile before 152, with the one behind 140
 //   more            64 x 64 with 8 x 4 sums a thread (gated 4 x 4), bound by the products themselves: 256 rows 184 us,

@@ -346,7 +346,7 @@ static thread_local GatedActParams t_gated_act{kActNone, 0.f, 0.f};   // the cur
 // Weights in flight to registers lie in the L1's part of the SM's memory until they are there; what it is not given is
 // shared memory, which these CTAs need little of but the kernels beside and around them more.  A half is the split at
 // which the chain of a decode step was fastest: with the driver's choice (the least shared memory that the CTAs of an SM
-// need) 14.0 ms for a prompt and 16 tokens over 12 layers, now 13.7; with all of it as shared memory 18.4.
+// need) 14.02 ms for a prompt and 16 tokens over 12 layers, now 13.81; with all of it as shared memory 18.4.
 constexpr int kSharedPercent = 50;
 template <typename... KArgs>
 static void prefer_half_shared(void (*kernel)(KArgs...)) {

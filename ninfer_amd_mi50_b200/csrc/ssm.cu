@@ -142,7 +142,7 @@ causal_conv_silu_rows_kernel(const T* __restrict__ src, int lds, int col0, int C
     if (VE == 8) load8(reinterpret_cast<const __nv_bfloat16*>(src) + (size_t)r * lds + col0 + c, u);
     else load4(reinterpret_cast<const float*>(src) + (size_t)r * lds + col0 + c, u);
   };
-  // AHEAD rows are in flight: one at a time, every row cost the thread a trip to memory (2,048 rows of 6,144 channels 34 us)
+  // AHEAD rows are in flight: one at a time, every row cost the thread a trip to memory (2,048 rows of 6,144 channels 32 us, now 28.5)
   constexpr int AHEAD = 4;
   static_assert(ROWS % AHEAD == 0, "whole rounds of rows");
   const int t1 = min(t0 + ROWS, T_rows);
@@ -421,8 +421,8 @@ ssd_scan_kernel(const T* __restrict__ xbc, int ldx, int x_col0, int b_col0, int 
 // A state read before the wait must have been written before the kernel that precedes this one in the stream was launched,
 // and that kernel must wait itself and release nobody before its end (the short convolution does): only a caller that says
 // so (`settled`) gets a chained launch; any other gets an ordinary one, which begins when all before it is done.
-// (8 requests of 64 heads of 64 x 128, 33 MB: 18.3 us with the kernel above, whose 1,024 CTAs of 20 KB of shared
-// memory came in two rounds of load, barrier, sixteen tokens' worth of reductions and barrier; now 8.5.  32 requests: 63, now 27.)
+// (8 requests of 64 heads of 64 x 128, 33 MB: 17.6 us with the kernel above, whose 1,024 CTAs of 20 KB of shared memory came in
+// two rounds of load, barrier, sixteen tokens' worth of reductions and barrier; now 6.8.  32 requests: 60, now 21.)
 template <typename T, int NPER, int CP>
 __global__ void __launch_bounds__(kScanThreads, NPER <= 4 ? 4 : 3)
 ssd_scan_row_kernel(const T* __restrict__ xbc, int ldx, int x_col0, int b_col0, int c_col0,
