@@ -63,13 +63,12 @@ struct __align__(8) Barriers {
   int stop;
 };
 
-// The item a CTA takes after `item`.  `back_and_forth`: rounds of gridDim.x items are dealt out forwards
-// and backwards in turn, so that the CTA with the longest item of one round has the shortest of the next.
-__device__ __forceinline__ int next_item(int item, bool back_and_forth) {
-  const int g = gridDim.x;
-  if (!back_and_forth) return item + g;
-  const int round = item / g + 1;
-  return round * g + ((round & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
+// The item a CTA takes after `item`: one of every round of gridDim.x items, rounds dealt out forwards, or forwards and
+// backwards in turn, so that the CTA with the longest item of one round has the shortest of the next.  `odd`: from the CTA's
+// item of an even round to that of the next (in the order above 1 .. 2 gridDim.x - 1, so the remainder tells the rounds apart).
+__device__ __forceinline__ int next_item(int item, int odd) {
+  const int two = 2 * (int)gridDim.x;
+  return item + ((item - (int)blockIdx.x) % two == 0 ? odd : two - odd);
 }
 
 // Persistent: one CTA per SM walks the work items (group, pass of 256 rows, feature tile), one of
@@ -90,8 +89,8 @@ __device__ __forceinline__ int next_item(int item, bool back_and_forth) {
 //                   (321, 2.4) 144 and 147, (394, 2.9) 153 and 148, of a prompt (956, 7.0) 165 and 159
 //   second          4,096 (92, 1.4) 77 and 79, (188, 2.8) 82 and 80;  6,144 (182, 1.8) 90 and 88;  8,192 (171, 1.3) 94 and 96,
 //                   (251, 1.8) 101 and 97, of a prompt (956, 7.0) 116 and 102;  16,384 (312, 1.1) 165 and 144
-// Hence the rule: kUnevenRows rows in the largest group, and it 2.5 times the mean, 1.75 in the second product, or there a
-// group of more than one pass.
+// Hence the rule: kUnevenRows rows in the largest group, and it 2.5 times the mean, 1.75 in the second product, or a group
+// of more than one pass.
 // 448 threads: warp 0 producer, warp 1 MMA + tensor memory, warps 2..13 epilogue.  The
 // producer is not held back by the epilogue: while the epilogue warps drain an item's
 // accumulator, the stages fill with the next item's first k tiles, so the memory pipe never
@@ -114,7 +113,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
   constexpr int A_BYTES = (SWIGLU || PAIR ? 2 : 1) * TILE_BYTES;     // gate (+ up) tile, or two feature tiles
   constexpr int FT_STEP = PAIR ? 2 : 1;                               // feature tiles an item covers
   constexpr int BOX_BYTES = kXBox * kBK * 2;
-  __shared__ int s_max_rows;
+  __shared__ int s_max_rows, s_odd;      // (the latter, see next_item, here and not in a register: the epilogue has none to spare)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k_steps = (K + kBK - 1) / kBK;
@@ -162,7 +161,8 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
   __syncthreads();
   const long long most = (long long)s_max_rows * groups;          // against total_rows: the largest group to the mean
   const bool by_rows = groups <= kTcThreads && ((s_max_rows >= kUnevenRows && 4 * most >= (SWIGLU ? 10 : 7) * total_rows) ||
-                                                (!SWIGLU && s_max_rows > kBNMax));
+                                                s_max_rows > kBNMax);
+  if (threadIdx.x == 0) s_odd = (int)gridDim.x + ((SWIGLU || PAIR) && by_rows ? (int)gridDim.x - 1 - 2 * (int)blockIdx.x : 0);
   if (by_rows) {                     // a thread a group; ranking more by comparisons would take longer than it gains
     for (int g = threadIdx.x; g < groups; g += blockDim.x) {
       const int n = s_rows[g];
@@ -188,7 +188,6 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
       run += __shfl_sync(0xffffffffu, v, 31);
     }
   }
-  const bool back_and_forth = (SWIGLU || PAIR) && by_rows;
   constexpr int kAccBuffers = (SWIGLU || PAIR) ? 1 : 2;      // accumulators of kBNMax columns that fit beside each other
   const int max_boxes = (min(max(s_max_rows, 1), kBNMax) + kXBox - 1) / kXBox;
   const int stage_bytes = A_BYTES + max_boxes * BOX_BYTES;
@@ -205,7 +204,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
       int it = 0, issued = 0;
       bool ok = true;
       int place = 0;
-      for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, back_and_forth)) {
+      for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, s_odd)) {
         const int gp = item / n_fitems, ft = (item - gp * n_fitems) * FT_STEP;      // global pass index, feature tile
         while (s_pass_start[place + 1] <= gp) ++place;
         const int group = s_group[place], pass = gp - s_pass_start[place];
@@ -257,7 +256,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
       int it = 0, pass_ctr = 0;
       bool ok = true;
       int place = 0;
-      for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, back_and_forth), ++pass_ctr) {
+      for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, s_odd), ++pass_ctr) {
         const int gp = item / n_fitems;
         while (s_pass_start[place + 1] <= gp) ++place;
         const int group = s_group[place], pass = gp - s_pass_start[place];
@@ -299,7 +298,7 @@ grouped_gemm_tc_kernel(const __nv_bfloat16* __restrict__ Wp, const __grid_consta
     int pass_ctr = 0;
     bool ok = true;
     int place = 0;
-    for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, back_and_forth), ++pass_ctr) {
+    for (int item = blockIdx.x; item < n_items && ok; item = next_item(item, s_odd), ++pass_ctr) {
       const int gp = item / n_fitems, ft0 = (item - gp * n_fitems) * FT_STEP;
       while (s_pass_start[place + 1] <= gp) ++place;
       const int group = s_group[place], pass = gp - s_pass_start[place];
